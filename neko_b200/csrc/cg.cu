@@ -595,7 +595,7 @@ int cg_poll(CgRun &R, bool wait, nb_solve_result *res, nb_status *status) {
   if (P->take_error())
     *status = ws_fail(NB_ERR_TIMEOUT, "a bounded device wait expired (bulk copy never completed)");
   else if (R.pc && R.pc->take_error())
-    *status = ws_fail(NB_ERR_TIMEOUT, "a bounded device wait expired (coarse-level grid barrier)");
+    *status = ws_fail(NB_ERR_TIMEOUT, "a bounded device wait expired (preconditioner level operator)");
   else if (hs->nan)
     *status = ws_fail(NB_ERR_NAN, "residual became NaN or Inf");
   return 1;

@@ -481,7 +481,7 @@ nb_status gmres_solve(nb_problem *P, double *x, const double *f, const nb_solve_
   if (P->take_error())
     return gfail(NB_ERR_TIMEOUT, "a bounded device wait expired (bulk copy never completed)");
   if (pc && pc->take_error())
-    return gfail(NB_ERR_TIMEOUT, "a bounded device wait expired (coarse-level grid barrier)");
+    return gfail(NB_ERR_TIMEOUT, "a bounded device wait expired (preconditioner level operator)");
   if (hs->nan) return gfail(NB_ERR_NAN, "residual became NaN or Inf");
   return NB_OK;
 }

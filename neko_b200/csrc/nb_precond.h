@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "nb_gs.h"
+#include "nb_nodes.h"
 #include "nb_problem.h"
 
 namespace nb {
@@ -123,30 +124,31 @@ nb_status pipecg_solve(nb_problem *P, double *x, const double *f, const nb_solve
 nb_status gmres_solve(nb_problem *P, double *x, const double *f, const nb_solve_opts &o,
                       Precond *pc, nb_solve_result *res, cudaStream_t s);
 
-// Operands of the persistent coarse-level launch of hsmg (hsmg_coarse.cu).
-// T is the precision of the middle level; the coarse level is FP64.
+// Operands of hsmg's coarse level (hsmg_coarse.cu).  T is the precision of
+// the middle level; the coarse level is FP64.
 template <typename T>
 struct CoarseArgs {
   long nelv = 0;
   const T *w_mid = nullptr, *mult_m = nullptr;  // middle-level residual and weights
   const T *J = nullptr;                         // lm x 2 interpolation, column-major
-  T *e_mid = nullptr;                           // += prolonged correction
-  double *f = nullptr, *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *w = nullptr;
-  const double *h1 = nullptr, *g11 = nullptr, *g22 = nullptr, *g33 = nullptr, *g12 = nullptr,
-               *g13 = nullptr, *g23 = nullptr, *D = nullptr, *Dt = nullptr;
-  const double *dinv = nullptr, *mult = nullptr;  // inverse Jacobi diagonal, weights
-  GsDevice gs;
-  CgState *st = nullptr;    // norm_fac, abs_tol, max_iter in; iter, rnorm out
-  double *part = nullptr;   // 2 x 2 x (grid) doubles
-  unsigned *bar = nullptr;  // grid-barrier word (reset with err after a timeout)
-  int *err = nullptr;       // set to 1 when a barrier wait expired
+  double *f = nullptr;                          // restricted residual, 8 values an element
+};
+struct CoarseCg {
+  NodeOp A;                   // the assembled vertex operator
+  const double *f = nullptr;  // element-local right-hand side
+  double *x = nullptr;        // solution, one value a node
+  double *p = nullptr, *r = nullptr, *w = nullptr;  // work, one value a node
+  double norm_fac = 0.0, tol = 0.0;
+  int niter = 0, stage_slices = 0;
   const int *skip = nullptr;
 };
-constexpr int kCoarseMaxBlocks = 1024;
 
-// Restrict, solve and prolong in one cooperative launch (lm = 3 or 4).
+// f = restriction of (w_mid mult_m), element by element (lm = 3 or 4).
 template <typename T>
-cudaError_t hsmg_coarse_solve(const CoarseArgs<T> &a, int lm, int max_blocks, cudaStream_t s);
+cudaError_t hsmg_coarse_restrict(const CoarseArgs<T> &a, int lm, const int *skip,
+                                 cudaStream_t s);
+// The coarse Jacobi-CG, one cluster launch.
+cudaError_t hsmg_coarse_cg(const CoarseCg &a, const int *skip, cudaStream_t s);
 
 // hsmg preconditioner of problem P, built on first use (pc_hsmg.cu).
 nb_status hsmg_get(nb_problem *P, const nb_solve_opts &o, Precond **out);

@@ -3,7 +3,7 @@
 // 574-625, CPU order) with levels lx -> 4 -> 2 (pc_hsmg.f90:208-219),
 // overlapping Schwarz + FDM smoothing on the fine and middle levels
 // (src/math/schwarz.f90:506-596) and a Jacobi-CG coarse solve of
-// `coarse_iter` iterations.
+// `coarse_iter` iterations over its distinct vertices (hsmg_coarse.cu).
 //
 // B200 form of the Schwarz step.  The reference builds extended
 // (lx+2)^3 elements, fills the ghost layer through a gather-scatter on a
@@ -399,33 +399,85 @@ struct PrologDots {
   double *part = nullptr;  // 2 per element
 };
 
+// The coarse level's correction, added to the middle level's as the
+// prolongation reads it: in(i,j,k) + sum J(k,c) J(j,b) J(i,a) x(a,b,c) with x
+// the node values of the element's vertices (0 on masked ones).
+template <typename T>
+struct CoarseAdd {
+  const double *x = nullptr;     // per node
+  const int *node_of = nullptr;  // 8 per element, -1 masked
+  const T *J = nullptr;          // NI x 2, column-major
+};
+
 template <typename TIN, typename TOUT, typename T, int NI, int NO, bool TR, bool ACC,
           bool DOT = false>
 __global__ void __launch_bounds__(kT3Threads)
     tensor3_kernel(const TIN *__restrict__ in, const TIN *__restrict__ scale,
                    const float *__restrict__ scale_f,
                    const T *__restrict__ M, TOUT *__restrict__ out, long nelv,
-                   const int *__restrict__ skip, PrologDots dots = PrologDots{}) {
+                   const int *__restrict__ skip, PrologDots dots = PrologDots{},
+                   CoarseAdd<T> crs = CoarseAdd<T>{}) {
   if (skip && *skip) return;
   constexpr int I3 = NI * NI * NI, O3 = NO * NO * NO, NT = kT3Threads;
   __shared__ T su[I3], s1[NO * NI * NI], s2[NO * NO * NI], sA[NO * NI];
   const long e = blockIdx.x;
   const int tid = threadIdx.x;
-  {
+  if constexpr (ACC) {  // the element's vertex values and the vertex interpolation
+    __shared__ T sx[8], sJc[2 * NI];
+    if (crs.x) {
+      if (tid < 8) {
+        const int nd = __ldg(crs.node_of + e * 8 + tid);
+        sx[tid] = nd >= 0 ? (T)__ldg(crs.x + nd) : T(0);
+      }
+      if (tid >= 32 && tid < 32 + 2 * NI) sJc[tid - 32] = __ldg(crs.J + tid - 32);
+    }
+    constexpr int R = (I3 + NT - 1) / NT;
+    TIN v[R];
+#pragma unroll
+    for (int g = 0; g < R; g++) {
+      const int q = tid + g * NT;
+      v[g] = q < I3 ? in[e * I3 + q] : TIN(0);
+    }
+    if (crs.x) __syncthreads();
+#pragma unroll
+    for (int g = 0; g < R; g++) {
+      const int q = tid + g * NT;
+      if (q < I3) {
+        T t = (T)v[g];
+        if (crs.x) {
+          const int o = q % NI, pp = (q / NI) % NI, rr = q / (NI * NI);
+          T acc_z = 0;
+#pragma unroll
+          for (int k = 0; k < 2; k++) {
+            T acc_y = 0;
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+              T acc_x = 0;
+#pragma unroll
+              for (int i = 0; i < 2; i++) acc_x += sJc[o + NI * i] * sx[i + 2 * j + 4 * k];
+              acc_y += sJc[pp + NI * j] * acc_x;
+            }
+            acc_z += sJc[rr + NI * k] * acc_y;
+          }
+          t = t + acc_z;
+        }
+        su[q] = t;
+      }
+    }
+  } else {
     constexpr int R = (I3 + NT - 1) / NT;
     TIN v[R], c[R];
 #pragma unroll
     for (int g = 0; g < R; g++) {
       const int q = tid + g * NT;
       v[g] = q < I3 ? in[e * I3 + q] : TIN(0);
-      c[g] = (!ACC && scale && q < I3)
-                 ? (scale_f ? (TIN)scale_f[e * I3 + q] : scale[e * I3 + q])
-                 : TIN(1);
+      c[g] = (scale && q < I3) ? (scale_f ? (TIN)scale_f[e * I3 + q] : scale[e * I3 + q])
+                               : TIN(1);
     }
 #pragma unroll
     for (int g = 0; g < R; g++) {
       const int q = tid + g * NT;
-      if (q < I3) su[q] = (!ACC && scale) ? (T)(v[g] * c[g]) : (T)v[g];
+      if (q < I3) su[q] = scale ? (T)(v[g] * c[g]) : (T)v[g];
     }
   }
   for (int q = tid; q < NO * NI; q += NT) {
@@ -685,8 +737,8 @@ static cudaError_t restrict_level(int ni, int no, const TIN *in, const TIN *scal
 // prolongation out += (J x J x J) in from ni to no points (J: no x ni)
 template <typename TIN, typename TOUT, typename T>
 static cudaError_t prolong_add(int ni, int no, const TIN *in, const T *J, TOUT *out, long nelv,
-                               const int *skip, cudaStream_t s, const TIN *oscale = nullptr,
-                               const float *oscale_f = nullptr,
+                               const int *skip, cudaStream_t s, const CoarseAdd<T> &crs,
+                               const TIN *oscale = nullptr, const float *oscale_f = nullptr,
                                const PrologDots *dots = nullptr) {
   const PrologDots d0 = dots ? *dots : PrologDots{};
 #define NB_P(A, B)                                                                          \
@@ -694,10 +746,10 @@ static cudaError_t prolong_add(int ni, int no, const TIN *in, const T *J, TOUT *
     const unsigned g = (unsigned)nelv;                                                      \
     if (dots)                                                                               \
       tensor3_kernel<TIN, TOUT, T, A, B, false, true, true>                                 \
-          <<<g, kT3Threads, 0, s>>>(in, oscale, oscale_f, J, out, nelv, skip, d0);          \
+          <<<g, kT3Threads, 0, s>>>(in, oscale, oscale_f, J, out, nelv, skip, d0, crs);          \
     else                                                                                    \
       tensor3_kernel<TIN, TOUT, T, A, B, false, true>                                       \
-          <<<g, kT3Threads, 0, s>>>(in, oscale, oscale_f, J, out, nelv, skip);              \
+          <<<g, kT3Threads, 0, s>>>(in, oscale, oscale_f, J, out, nelv, skip, d0, crs);     \
     return cudaGetLastError();                                                              \
   }
   NB_P(2, 4) NB_P(2, 3) NB_P(4, 5) NB_P(4, 6) NB_P(4, 7) NB_P(4, 8) NB_P(4, 9) NB_P(4, 10)
@@ -716,13 +768,17 @@ struct HsmgState : public Precond {
   int niter = 10;
   double tol = 1e-9;
   bool mixed = false;
-  // The two branches of the additive scheme share only the input r: the
-  // fine-level Schwarz runs on `side`, the middle level and the coarse solve
-  // on `hi`, a stream of the greatest priority, so that the small,
-  // latency-bound coarse-branch kernels get SM slots ahead of the pending
-  // blocks of the large fine-level FDM launch instead of queueing behind it.
-  cudaStream_t side = nullptr, hi = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join_hi = nullptr;
+  // The branches of the additive scheme share only the input r.  The middle
+  // level's residual and its restriction come first, on `crs`; then the
+  // coarse solve (a cluster of at most 16 blocks, on `crs`), the middle
+  // level's Schwarz (on `hi`) and the fine level's (on `side`) run side by
+  // side.  `crs` and `hi` have the greatest priority: the cluster needs its
+  // multiprocessors at once, so it is placed before the fine-level FDM fills
+  // the device, and the FDM then takes the others.
+  cudaStream_t side = nullptr, hi = nullptr, crs_s = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_mid = nullptr, ev_join = nullptr, ev_join_hi = nullptr,
+              ev_join_crs = nullptr;
+  NodeOp nodes;  // the coarse problem over its distinct vertices
   cudaError_t ensure_side() {
     if (side) return cudaSuccess;
     cudaError_t e;
@@ -730,7 +786,11 @@ struct HsmgState : public Precond {
     if ((e = cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithPriority(&hi, cudaStreamNonBlocking, hi_prio)) != cudaSuccess ||
+        (e = cudaStreamCreateWithPriority(&crs_s, cudaStreamNonBlocking, hi_prio)) !=
+            cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&ev_mid, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&ev_join_crs, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ev_join_hi, cudaEventDisableTiming)) != cudaSuccess)
       return e;
@@ -739,7 +799,11 @@ struct HsmgState : public Precond {
   ~HsmgState() override {
     if (side) cudaStreamDestroy(side);
     if (hi) cudaStreamDestroy(hi);
+    if (crs_s) cudaStreamDestroy(crs_s);
     if (ev_fork) cudaEventDestroy(ev_fork);
+    if (ev_mid) cudaEventDestroy(ev_mid);
+    if (ev_join_crs) cudaEventDestroy(ev_join_crs);
+    if (nodes.base) cudaFree(nodes.base);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_join_hi) cudaEventDestroy(ev_join_hi);
     if (arena) cudaFree(arena);
@@ -755,30 +819,17 @@ struct HsmgImpl : public HsmgState {
   T *mult_f = nullptr, *mult_m = nullptr;
   T *zf = nullptr;                   // smoother-precision fine output (float path)
   T *w_mid = nullptr, *e_mid = nullptr;
-  double *r_crs = nullptr, *e_crs = nullptr;
-  double *rc = nullptr, *zc = nullptr, *pc = nullptr, *wc = nullptr;
-  CgState *stc = nullptr;
   CoarseArgs<T> ca;
+  CoarseCg cg;
 
   // The fine level has no masked point: its Schwarz gather-scatter merges
   // into the final one.
   bool merged_assembly() const { return fine->nmask == 0; }
 
   int launches() const override {
-    // 2 Schwarz x (fdm, post, gs) + restrict + gs + coarse (one launch) +
-    // prolong + final gs (+ convert); one gs fewer when merged
-    return 6 + 1 + 1 + 1 + 1 + 1 + (sizeof(T) == 4 ? 1 : 0) - (merged_assembly() ? 1 : 0);
-  }
-
-  int take_error() override {
-    int v = 0;
-    if (cudaMemcpy(&v, ca.err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
-    if (v) {  // leave the barrier words at rest for the next launch
-      cudaMemset(ca.err, 0, sizeof(int));
-      cudaMemset(ca.bar, 0, 2 * sizeof(unsigned));
-      cudaDeviceSynchronize();
-    }
-    return v;
+    // 2 Schwarz x (fdm, post, gs) + restrict + gs + coarse restrict + coarse
+    // CG + prolong + final gs (+ convert); one gs fewer when merged
+    return 6 + 1 + 1 + 1 + 1 + 1 + 1 + (sizeof(T) == 4 ? 1 : 0) - (merged_assembly() ? 1 : 0);
   }
 
   // FP32 smoothing levels: the output can stay in FP32 (zf)
@@ -819,37 +870,43 @@ struct HsmgImpl : public HsmgState {
                        const PrologDots *dots = nullptr) {
     cudaError_t e;
     const long nelv = fine->nelv;
-    // fine Schwarz on the side stream: zs = S_f r
     if ((e = ensure_side()) != cudaSuccess || (e = cudaEventRecord(ev_fork, s)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(side, ev_fork, 0)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(hi, ev_fork, 0)) != cudaSuccess)
+        (e = cudaStreamWaitEvent(crs_s, ev_fork, 0)) != cudaSuccess)
       return e;
-    // middle and coarse levels first, on the high-priority stream:
-    // restrict (r * mult) to the middle level, assemble, mask
+    // restrict (r * mult) to the middle level, assemble, mask: w; restrict
+    // (w * mult_mid) to the vertices (FP64)
     if ((e = restrict_level<double, T, T>(fine->lx, mid->lx, r, fine->mult, Jfm, w_mid, nelv,
-                                          skip, hi, fine->multf)) != cudaSuccess)
+                                          skip, crs_s, fine->multf)) != cudaSuccess ||
+        (e = gs_add_fused<T>(mid->gsd, w_mid, true, crs_s, skip)) != cudaSuccess ||
+        (e = hsmg_coarse_restrict<T>(ca, mid->lx, skip, crs_s)) != cudaSuccess ||
+        (e = cudaEventRecord(ev_mid, crs_s)) != cudaSuccess ||
+        (e = cudaStreamWaitEvent(hi, ev_mid, 0)) != cudaSuccess ||
+        (e = cudaStreamWaitEvent(side, ev_mid, 0)) != cudaSuccess)
       return e;
-    if ((e = gs_add_fused<T>(mid->gsd, w_mid, true, hi, skip)) != cudaSuccess) return e;
+    // coarse: assemble, mask, niter Jacobi-CG iterations (or abs tol)
+    if ((e = hsmg_coarse_cg(cg, skip, crs_s)) != cudaSuccess ||
+        (e = cudaEventRecord(ev_join_crs, crs_s)) != cudaSuccess)
+      return e;
     // middle Schwarz: e_mid = S_m w
-    if ((e = schwarz_apply<T, T>(sm, w_mid, e_mid, skip, hi)) != cudaSuccess) return e;
-    // restrict (w * mult_mid) to the coarse level (FP64), assemble, mask,
-    // niter Jacobi-CG iterations (or abs tol), e_mid += J e_crs: one launch
-    ca.skip = skip;
-    if ((e = hsmg_coarse_solve<T>(ca, mid->lx, kCoarseMaxBlocks, hi)) != cudaSuccess) return e;
-    if ((e = cudaEventRecord(ev_join_hi, hi)) != cudaSuccess) return e;
-    // fine Schwarz on the side stream: zs = S_f r (left unassembled when the
-    // final gather-scatter takes it, see below)
+    if ((e = schwarz_apply<T, T>(sm, w_mid, e_mid, skip, hi)) != cudaSuccess ||
+        (e = cudaEventRecord(ev_join_hi, hi)) != cudaSuccess)
+      return e;
+    // fine Schwarz: zs = S_f r (left unassembled when the final
+    // gather-scatter takes it, see below)
     const bool merged = merged_assembly();
     if ((e = schwarz_apply<double, T>(sf, r, zs, skip, side, !merged)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(ev_join, side)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(s, ev_join, 0)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(s, ev_join_hi, 0)) != cudaSuccess)
+        (e = cudaStreamWaitEvent(s, ev_join_hi, 0)) != cudaSuccess ||
+        (e = cudaStreamWaitEvent(s, ev_join_crs, 0)) != cudaSuccess)
       return e;
-    // prolong: zs += J e_mid; z = mult * gs(zs).  Without a mask the fine
+    // prolong: zs += J (e_mid + J_c e_crs); z = mult * gs(zs).  Without a mask the fine
     // Schwarz output's own gather-scatter is folded into this one: wt and
     // mult are the same at every copy of a point, so
     // mult gs(gs(wt e) + J e_mid) = gs(wt e + mult J e_mid).
-    if ((e = prolong_add<T, T, T>(mid->lx, fine->lx, e_mid, Jfm, zs, nelv, skip, s,
+    CoarseAdd<T> crs_add;
+    if (nodes.nn > 0) crs_add = CoarseAdd<T>{cg.x, nodes.node_of, Jmc};
+    if ((e = prolong_add<T, T, T>(mid->lx, fine->lx, e_mid, Jfm, zs, nelv, skip, s, crs_add,
                                   merged ? mult_f : nullptr,
                                   merged && sizeof(T) == 8 ? fine->multf : nullptr,
                                   merged ? dots : nullptr)) !=
@@ -873,14 +930,16 @@ void hsmg_free(nb_problem *p) {
 // of the fine h1 and the coarse problem has no h2; its Jacobi diagonal
 // follows.  The mesh is marked all-deformed (pc_hsmg.f90:267), which turns on
 // the corner cross terms of that diagonal.
-static cudaError_t hsmg_set_h(nb_problem *P, nb_problem *C) {
+static cudaError_t hsmg_set_h(nb_problem *P, HsmgState *h) {
+  nb_problem *C = h->crs;
   cudaError_t e;
   if ((e = cudaMemcpy(C->h1, P->h1, C->n * 8, cudaMemcpyDeviceToDevice)) != cudaSuccess ||
       (e = cudaMemset(C->dfrmd, 1, C->nelv)) != cudaSuccess)
     return e;
   C->ifh2 = false;
   C->invalidate_solver_cache();
-  return C->update_jacobi(nullptr);
+  if ((e = C->update_jacobi(nullptr)) != cudaSuccess) return e;
+  return node_update(C, h->nodes, nullptr);
 }
 
 // Constant h1 on the coarse levels of p's preconditioners, on stream s
@@ -892,6 +951,7 @@ cudaError_t hsmg_set_h_const(nb_problem *p, double h1, cudaStream_t s) {
     cudaError_t e = fill_const(C->h1, h1, C->n, s);
     if (e != cudaSuccess) return e;
     if ((e = C->update_jacobi(s)) != cudaSuccess) return e;
+    if ((e = node_update(C, h->nodes, s)) != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
@@ -899,7 +959,7 @@ cudaError_t hsmg_set_h_const(nb_problem *p, double h1, cudaStream_t s) {
 cudaError_t hsmg_refresh_coefficients(nb_problem *p) {
   for (auto *h : p->hsmg) {
     if (!h) continue;
-    cudaError_t e = hsmg_set_h(p, h->crs);
+    cudaError_t e = hsmg_set_h(p, h);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -1026,10 +1086,9 @@ static nb_status upload_impl(HsmgImpl<T> *H, const SchwarzHost &hf, const Schwar
   const size_t o_mf = f32 ? c.take(n * sizeof(T)) : 0, o_mm = c.take(nm * sizeof(T));
   const size_t o_zf = f32 ? c.take(n * sizeof(T)) : 0;
   const size_t o_wm = c.take(nm * sizeof(T)), o_em = c.take(nm * sizeof(T));
-  const size_t o_rc = c.take(nc * 8), o_ec = c.take(nc * 8), o_r = c.take(nc * 8),
-               o_z = c.take(nc * 8), o_p = c.take(nc * 8), o_w = c.take(nc * 8);
-  const size_t o_st = c.take(sizeof(CgState)),
-               o_part = c.take(2 * 2 * kCoarseMaxBlocks * sizeof(double) + 64);
+  const size_t nn = (size_t)H->nodes.nn + 1;
+  const size_t o_rc = c.take(nc * 8), o_ec = c.take(nn * 8), o_r = c.take(nn * 8),
+               o_p = c.take(nn * 8), o_w = c.take(nn * 8);
   if (cudaMalloc(&H->arena, c.off) != cudaSuccess) return hfail(NB_ERR_OOM, "hsmg: device arena");
   char *A = (char *)H->arena;
   auto Tp = [&](size_t o) { return (T *)(A + o); };
@@ -1052,21 +1111,13 @@ static nb_status upload_impl(HsmgImpl<T> *H, const SchwarzHost &hf, const Schwar
   H->mult_m = Tp(o_mm);
   H->zf = f32 ? Tp(o_zf) : nullptr;
   H->w_mid = Tp(o_wm), H->e_mid = Tp(o_em);
-  H->r_crs = Dp(o_rc), H->e_crs = Dp(o_ec), H->rc = Dp(o_r), H->zc = Dp(o_z), H->pc = Dp(o_p),
-  H->wc = Dp(o_w);
-  H->stc = (CgState *)(A + o_st);
   CoarseArgs<T> &ca = H->ca;
   ca.nelv = nelv;
-  ca.w_mid = H->w_mid, ca.mult_m = H->mult_m, ca.J = H->Jmc, ca.e_mid = H->e_mid;
-  ca.f = H->r_crs, ca.x = H->e_crs, ca.r = H->rc, ca.z = H->zc, ca.p = H->pc, ca.w = H->wc;
-  ca.h1 = C->h1, ca.g11 = C->g11, ca.g22 = C->g22, ca.g33 = C->g33, ca.g12 = C->g12,
-  ca.g13 = C->g13, ca.g23 = C->g23, ca.D = C->D, ca.Dt = C->Dt;
-  ca.dinv = C->jdiag, ca.mult = C->mult;
-  ca.gs = C->gsd;
-  ca.st = H->stc;
-  ca.part = Dp(o_part);
-  ca.bar = (unsigned *)(A + o_part + 2 * 2 * kCoarseMaxBlocks * sizeof(double));
-  ca.err = (int *)(ca.bar + 2);
+  ca.w_mid = H->w_mid, ca.mult_m = H->mult_m, ca.J = H->Jmc, ca.f = Dp(o_rc);
+  CoarseCg &cg = H->cg;
+  cg.A = H->nodes;
+  cg.f = ca.f, cg.x = Dp(o_ec), cg.r = Dp(o_r), cg.p = Dp(o_p), cg.w = Dp(o_w);
+  cg.norm_fac = 1.0 / std::sqrt(C->volume), cg.tol = H->tol, cg.niter = H->niter;
   auto upv = [&](size_t o, const std::vector<double> &v) {
     std::vector<T> t = cast_vec<T>(v);
     return t.empty() ? cudaSuccess
@@ -1083,19 +1134,13 @@ static nb_status upload_impl(HsmgImpl<T> *H, const SchwarzHost &hf, const Schwar
     if (cudaMemcpy(hf_mult.data(), P->mult, n * 8, cudaMemcpyDeviceToHost) != cudaSuccess)
       return hfail(NB_ERR_CUDA, "hsmg: mult copy failed");
   }
-  CgState cs{};
-  cs.norm_fac = 1.0 / std::sqrt(C->volume);
-  cs.abs_tol = H->tol;
-  cs.max_iter = H->niter;
-  cs.done = 1;
   if (upv(o_Sf, hf.S) || upv(o_Lf, hf.lam) || upv(o_Ef, hf.eps) || upv(o_Wf, hf.wt) ||
       upi(o_Ff, hf.fn) || upv(o_Sm, hm.S) || upv(o_Lm, hm.lam) || upv(o_Em, hm.eps) ||
       upv(o_Wm, hm.wt) || upi(o_Fm, hm.fn) || upv(o_Jfm, Jfm) || upv(o_Jmc, Jmc) ||
       upv(o_mm, hm_mult) || (f32 && upv(o_mf, hf_mult)) ||
       (!ornt.empty() &&
        cudaMemcpy(A + o_or, ornt.data(), ornt.size(), cudaMemcpyHostToDevice) != cudaSuccess) ||
-      cudaMemcpy(A + o_st, &cs, sizeof(cs), cudaMemcpyHostToDevice) ||
-      cudaMemset(A + o_part, 0, 2 * 2 * kCoarseMaxBlocks * sizeof(double) + 64))
+      cudaMemset(A + o_ec, 0, nn * 8) != cudaSuccess)
     return hfail(NB_ERR_CUDA, "hsmg: upload failed");
   return NB_OK;
 }
@@ -1142,7 +1187,11 @@ nb_status hsmg_get(nb_problem *P, const nb_solve_opts &o, Precond **out) {
     delete H;
     return st;
   }
-  if (hsmg_set_h(P, H->crs) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+  if ((st = node_create(H->crs, H->nodes)) != NB_OK) {
+    delete H;
+    return st;
+  }
+  if (hsmg_set_h(P, H) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
     delete H;
     return hfail(NB_ERR_CUDA, "hsmg: coarse coefficients failed");
   }
@@ -1185,10 +1234,6 @@ nb_status hsmg_apply_once(nb_problem *P, double *z, const double *r, cudaStream_
   if (st != NB_OK) return st;
   NB_CUDA_TRY(pc->apply(z, r, nullptr, s));
   NB_CUDA_TRY(cudaStreamSynchronize(s));
-  if (pc->take_error()) {
-    set_error("a bounded device wait expired (coarse-level grid barrier)");
-    return NB_ERR_TIMEOUT;
-  }
   return NB_OK;
 }
 

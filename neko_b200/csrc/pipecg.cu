@@ -342,7 +342,7 @@ nb_status pipecg_solve(nb_problem *P, double *x, const double *f, const nb_solve
   if (P->take_error())
     return pfail(NB_ERR_TIMEOUT, "a bounded device wait expired (bulk copy never completed)");
   if (pc && pc->take_error())
-    return pfail(NB_ERR_TIMEOUT, "a bounded device wait expired (coarse-level grid barrier)");
+    return pfail(NB_ERR_TIMEOUT, "a bounded device wait expired (preconditioner level operator)");
   if (hs->nan) return pfail(NB_ERR_NAN, "residual became NaN or Inf");
   return NB_OK;
 }
