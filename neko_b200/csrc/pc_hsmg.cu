@@ -58,17 +58,27 @@ __device__ __forceinline__ void face_map(unsigned code, int lx, int s1, int s2, 
 // last (out(m,n,i) = sum_l M(i,l) in(l,m,n)), so after three passes the
 // order is back to (i,j,k).  A lane owns M lines of the pass and all NL
 // outputs of each: for every l it reads its M line values and the NL matrix
-// entries M(., l), which are the same for the whole warp (broadcast reads),
-// and updates M*NL independent sums, so a matrix read serves M lines.  Lines
-// sit at pos(t, l) = NLP t + C (t >> G) + l, the padding chosen per NL so
-// that the consecutive lines of a warp's reads and rotated writes fall in
-// distinct banks.  The D^-1 scaling of the third forward pass is applied to
-// each value as the first backward pass reads it (the same product, stored
-// one pass later).  The ghost-layer gather and the factor loads are
-// asynchronous copies straight into shared memory (zero-filled where a face
-// has no neighbour) when the input needs no conversion.  Every sum runs over
-// l in ascending order from zero; the eigenvalue scaling multiplies by
-// 1/diag, zero where the sum of the three spectra is <= eps
+// entries M(., l), which are the same for the whole element (broadcast
+// reads), and updates M*NL independent sums, so a matrix read serves M lines.
+//
+// The passes are bound by shared-memory wavefronts.  Line t starts at P t,
+// and for even NL a lane reads its lines two values at a time: with P / 2
+// odd, the eight lanes of a quarter-warp (sixteen of a half-warp in FP32)
+// then hit distinct banks, and where P = NL the rotated writes of
+// consecutive lines are consecutive addresses.  For nl = 10 in FP64 that is
+// 80 + 80 + 50 wavefronts a pass (line reads, writes, matrix rows) against
+// 140 + 84 + 50 with single-value reads of a padded layout.  Odd NL read
+// single values, conflict-free at their odd pitch.
+//
+// Every pass works in place: the lanes read their lines, the block meets at
+// a barrier and the rotated output overwrites the same buffer, so that more
+// elements fit a multiprocessor.  The D^-1 scaling of the third forward pass
+// is applied to each value as the first backward pass reads it (the same
+// product, stored one pass later).  The ghost-layer gather and the factor
+// loads are asynchronous copies straight into shared memory (zero-filled
+// where a face has no neighbour) when the input needs no conversion.  Every
+// sum runs over l in ascending order from zero; the eigenvalue scaling
+// multiplies by 1/diag, zero where the sum of the three spectra is <= eps
 // (fdm_setup_fast, src/math/fdm.f90:373-393).
 template <typename T, int NL>
 struct FdmCfg {
@@ -80,31 +90,21 @@ struct FdmCfg {
   static constexpr int LPE = TPE / EPW;                          // lanes per element
   static constexpr int M = (N2 + LPE - 1) / LPE;                 // lines per lane
   static constexpr int LA = (N2 + M - 1) / M;                    // lanes with lines
-  static constexpr int NLP = NL == 16 ? 17 : NL;
-  static constexpr int G = NL == 8 ? 2 : NL == 12 ? 3 : 4;
-  static constexpr int C = (NL % 2 == 0 && NL != 16) ? 1 : 0;
-  static constexpr int BUF = (NLP * (N2 - 1) + ((N2 - 1) >> G) * C + NL + 1) / 2 * 2;
-  // One element a block: the matrices are kept twice, each row l of the
-  // forward (S(l, .)) and backward (S(., l)) forms contiguous with a pitch of
-  // whole 16-byte vectors, so a lane reads a row with NL*sizeof(T)/16 vector
-  // loads instead of NL scalar ones.
-  static constexpr bool VEC = EPW == 1;
+  static constexpr bool PAIR = NL % 2 == 0;                      // two values a read
+  static constexpr int P = PAIR && (NL / 2) % 2 == 0 ? NL + 2 : NL;
   static constexpr int VW = 16 / (int)sizeof(T);            // values per vector
-  static constexpr int NLR = (NL + VW - 1) / VW * VW;        // row pitch
-  // FP32 one-element blocks pass in place: every lane reads its lines, the
-  // block meets at a barrier, then the rotated output overwrites the same
-  // buffer; the second buffer shrinks to the matrix staging area (3 N2), so
-  // more blocks fit an SM.  FP64 keeps two buffers (its registers, not its
-  // shared memory, bound its residency).
-  static constexpr bool INPLACE = VEC && sizeof(T) == 4;
-  static constexpr int BUF2 = INPLACE ? (3 * N2 + 1) / 2 * 2 : BUF;
-  static constexpr int OFFM = (BUF + BUF2 + VW - 1) / VW * VW;  // matrices, aligned
-  static_assert(!INPLACE || BUF2 >= 3 * N2, "the staging area holds the three raw matrices");
-  static constexpr int MAT = VEC ? 6 * NL * NLR : 3 * N2;
-  static constexpr int STR0 = VEC ? OFFM + MAT + 3 * NL + 1 : 2 * BUF + 3 * N2 + 3 * NL + 1;
-  // per-element stride; with several elements in a warp it is 9 mod 16
-  // values, which keeps the line reads of neighbouring elements in distinct banks
-  static constexpr int STR = EPW > 1 ? STR0 + ((9 - STR0 % 16) + 16) % 16 : STR0;
+  static constexpr int BUF = (P * N2 + VW - 1) / VW * VW;
+  // The matrices are kept twice, each row l of the forward (S(l, .)) and
+  // backward (S(., l)) forms contiguous with a pitch of whole 16-byte
+  // vectors, so a lane reads a row with NL*sizeof(T)/16 vector loads.
+  static constexpr int NLR = (NL + VW - 1) / VW * VW;       // row pitch
+  static constexpr int MS = NL * NLR;                       // one matrix
+  static constexpr int MAT = 6 * MS;
+  static constexpr int STR0 = BUF + MAT + 3 * NL + 1;
+  // per-element stride in whole vectors; with several elements in a warp an
+  // odd number of them, so that their broadcast rows fall in distinct banks
+  static constexpr int STRV = (STR0 + VW - 1) / VW;
+  static constexpr int STR = (EPW > 1 ? STRV + 1 - STRV % 2 : STRV) * VW;
   static constexpr size_t SMEM = ((size_t)EPW * STR * sizeof(T) + 15) / 16 * 16;
   // resident blocks per SM the register allocation is sized for: what the
   // shared memory allows (228 KB, 1 KB reserved per block), fewer if the
@@ -114,7 +114,7 @@ struct FdmCfg {
   static constexpr int RB = 65536 / (TPE * REGS);
   static constexpr int MINB0 = OCC < RB ? OCC : RB;
   static constexpr int MINB = MINB0 < 1 ? 1 : MINB0 > 32 / W ? 32 / W : MINB0;
-  __device__ static __forceinline__ int pos(int t, int l) { return NLP * t + (t >> G) * C + l; }
+  __device__ static __forceinline__ int pos(int t, int l) { return P * t + l; }
 };
 
 template <typename T>
@@ -139,24 +139,22 @@ __device__ __forceinline__ void gather_elem(T *dst, const TIN *src, bool valid) 
     *dst = valid ? (T)__ldg(src) : T(0);
 }
 
-// One pass over the element: FWD contracts with S(l,i) at Sd[l + NL*i],
-// otherwise with S(i,l) at Sd[i + NL*l].  SCALE multiplies each value read
-// by D^-1 (the first backward pass reads the third forward pass's output);
-// `out` != nullptr writes the natural (i,j,k) order to global memory (last
-// pass) instead of the rotated shared-memory layout.
-template <typename T, int NL, bool FWD, bool SCALE>
-__device__ __forceinline__ void fdm_pass(const T *__restrict__ src, T *__restrict__ dst,
-                                         const T *__restrict__ Sd, const T *__restrict__ sL,
-                                         T *__restrict__ out, int u) {
+// One pass over the element, in place: out(m,n,i) = sum_l R(l, i) in(l,m,n)
+// with row l of the pass's matrix at rows[NLR l].  SCALE multiplies each
+// value read by D^-1 (the first backward pass reads the third forward pass's
+// output); `out` != nullptr writes the natural (i,j,k) order to global memory
+// (last pass) instead of the rotated order over the buffer.
+template <typename T, int NL, bool SCALE>
+__device__ __forceinline__ void fdm_pass(T *__restrict__ buf, const T *__restrict__ rows,
+                                         const T *__restrict__ sL, T *__restrict__ out, int u) {
   using C = FdmCfg<T, NL>;
-  constexpr int N2 = C::N2, M = C::M, LA = C::LA;
-  // in place (src == dst), lanes without lines still meet the barrier
-  // between the reads and the writes
-  if (!C::INPLACE && u >= LA) return;
-  const bool lines = u < LA;
+  constexpr int N2 = C::N2, M = C::M, LA = C::LA, LS = C::PAIR ? 2 : 1;
+  using V = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
+  using V2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+  const bool lines = u < LA;  // lanes without lines only meet the barrier
   T o[M][NL];
   int base[M];
-  T ljk[M];  // SCALE: spectra sum of the line's second index, added to the first's
+  T ljk[M];  // SCALE: spectra of the line's second and third index
   T lz[M];
   const T ep = sL[3 * NL];
 #pragma unroll
@@ -170,42 +168,42 @@ __device__ __forceinline__ void fdm_pass(const T *__restrict__ src, T *__restric
 #pragma unroll
     for (int i = 0; i < NL; i++) o[j][i] = T(0);
   }
-#pragma unroll 2
-  for (int l = 0; l < (lines ? NL : 0); l++) {
-    T x[M];
+#pragma unroll(C::PAIR ? 1 : 2)
+  for (int l = 0; l < (lines ? NL : 0); l += LS) {
+    T x[M][LS];
 #pragma unroll
     for (int j = 0; j < M; j++) {
-      x[j] = src[base[j] + l];
+      if constexpr (C::PAIR) {
+        const V2 v = *reinterpret_cast<const V2 *>(buf + base[j] + l);
+        x[j][0] = v.x;
+        x[j][1] = v.y;
+      } else {
+        x[j][0] = buf[base[j] + l];
+      }
       if (SCALE) {  // (lx + ly) + lz, as the third forward pass forms it
-        const T d = (sL[l] + ljk[j]) + lz[j];
-        x[j] = x[j] * (d > ep ? T(1) / d : T(0));
+#pragma unroll
+        for (int h = 0; h < LS; h++) {
+          const T d = (sL[l + h] + ljk[j]) + lz[j];
+          x[j][h] = x[j][h] * (d > ep ? T(1) / d : T(0));
+        }
       }
     }
-    if constexpr (C::VEC) {
+#pragma unroll
+    for (int h = 0; h < LS; h++) {
       // row l of the pass's matrix in 16-byte vector loads (broadcast)
       T mr[C::NLR];
-      using V = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
-      const V *row = reinterpret_cast<const V *>(Sd + C::NLR * l);
+      const V *row = reinterpret_cast<const V *>(rows + C::NLR * (l + h));
 #pragma unroll
       for (int q = 0; q < C::NLR / C::VW; q++) reinterpret_cast<V *>(mr)[q] = row[q];
 #pragma unroll
       for (int i = 0; i < NL; i++) {
 #pragma unroll
-        for (int j = 0; j < M; j++) o[j][i] += mr[i] * x[j];
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < NL; i++) {
-        const T mv = Sd[FWD ? l + NL * i : i + NL * l];
-#pragma unroll
-        for (int j = 0; j < M; j++) o[j][i] += mv * x[j];
+        for (int j = 0; j < M; j++) o[j][i] += mr[i] * x[j][h];
       }
     }
   }
-  if constexpr (C::INPLACE) {
-    if (!out) __syncthreads();  // every read of src done before dst (= src) is written
-    if (!lines) return;
-  }
+  if (!out) __syncthreads();  // every read done before the buffer is overwritten
+  if (!lines) return;
 #pragma unroll
   for (int j = 0; j < M; j++) {
     const int t = u + LA * j;
@@ -216,7 +214,7 @@ __device__ __forceinline__ void fdm_pass(const T *__restrict__ src, T *__restric
     } else {
       const int m = t % NL, n = t / NL;
 #pragma unroll
-      for (int i = 0; i < NL; i++) dst[C::pos(n + NL * i, m)] = o[j][i];
+      for (int i = 0; i < NL; i++) buf[C::pos(n + NL * i, m)] = o[j][i];
     }
   }
 }
@@ -232,13 +230,11 @@ __global__ void __launch_bounds__(FdmCfg<T, NL>::TPE, FdmCfg<T, NL>::MINB)
   constexpr int LX = NL - 2, L2 = LX * LX, L3 = L2 * LX, N2 = C::N2, N3 = C::N3;
   extern __shared__ __align__(16) unsigned char fdm_smem[];
   const int es = threadIdx.x / C::LPE, ul = threadIdx.x - es * C::LPE;
-  T *b0 = reinterpret_cast<T *>(fdm_smem) + es * C::STR, *b1 = b0 + C::BUF;
-  // scalar form: S_x, S_y, S_z with S(l,i) at l + NL*i; vector form: the
-  // forward rows (S(l, i) at i + NLR*l) then the backward rows (S(i, l) at
-  // i + NLR*l), the factors staged in b1 first
-  T *sS = C::VEC ? b0 + C::OFFM : b1 + C::BUF;
-  T *sL = sS + C::MAT;  // spectra + eps
-  T *stage = C::VEC ? b1 : sS;
+  T *b0 = reinterpret_cast<T *>(fdm_smem) + es * C::STR;
+  // the forward rows (S(l, i) at i + NLR*l), then the backward rows (S(i, l)
+  // at i + NLR*l), direction by direction
+  T *fwd = b0 + C::BUF, *bwd = fwd + 3 * C::MS;
+  T *sL = fwd + C::MAT;  // spectra + eps
   const long e = (long)blockIdx.x * C::EPW + es;
   if ((long)blockIdx.x * C::EPW >= nelv) return;
   const bool active = e < nelv;
@@ -286,39 +282,28 @@ __global__ void __launch_bounds__(FdmCfg<T, NL>::TPE, FdmCfg<T, NL>::MINB)
       }
       b0[C::pos(b + NL * c, a)] = T(0);
     }
-    for (int q = u; q < 3 * N2; q += LPE) cp_async_elem<T>(stage + q, S + e * 3 * N2 + q, true);
+    for (int q = u; q < 3 * N2; q += LPE) {  // S_d(a, b), copied to its place in both forms
+      const int d = q / N2, w = q - d * N2, a = w % NL, b = w / NL;
+      const T *src = S + e * 3 * N2 + q;
+      cp_async_elem<T>(fwd + d * C::MS + b + C::NLR * a, src, true);
+      cp_async_elem<T>(bwd + d * C::MS + a + C::NLR * b, src, true);
+    }
     for (int q = u; q < 3 * NL; q += LPE) cp_async_elem<T>(sL + q, lam + e * 3 * NL + q, true);
     if (u == 0) cp_async_elem<T>(sL + 3 * NL, eps + e, true);
   }
   cp_async_wait_all();
   __syncthreads();
-  // matrix of direction d for the forward / backward passes
-  constexpr int MS = C::VEC ? NL * C::NLR : N2;
-  T *fwd = sS, *bwd = C::VEC ? sS + 3 * MS : sS;
-  if constexpr (C::VEC) {
-    if (active)
-      for (int q = u; q < 3 * N2; q += LPE) {
-        const int d = q / N2, r = q - d * N2, a = r % NL, b = r / NL;
-        const T v = stage[q];  // S_d(a, b)
-        fwd[d * MS + b + C::NLR * a] = v;
-        bwd[d * MS + a + C::NLR * b] = v;
-      }
-    __syncthreads();
-  }
-  // forward: b0 -> b1 -> b0 -> b1; backward (D^-1 on the first read): b1 -> b0 -> b1 -> out
-  // (in place: b0 -> b0 throughout)
-  if constexpr (C::INPLACE) b1 = b0;
-  fdm_pass<T, NL, true, false>(b0, b1, fwd, sL, nullptr, u);
+  fdm_pass<T, NL, false>(b0, fwd, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, true, false>(b1, b0, fwd + MS, sL, nullptr, u);
+  fdm_pass<T, NL, false>(b0, fwd + C::MS, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, true, false>(b0, b1, fwd + 2 * MS, sL, nullptr, u);
+  fdm_pass<T, NL, false>(b0, fwd + 2 * C::MS, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false, true>(b1, b0, bwd, sL, nullptr, u);
+  fdm_pass<T, NL, true>(b0, bwd, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false, false>(b0, b1, bwd + MS, sL, nullptr, u);
+  fdm_pass<T, NL, false>(b0, bwd + C::MS, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false, false>(b1, nullptr, bwd + 2 * MS, sL, out + e * N3, u);
+  fdm_pass<T, NL, false>(b0, bwd + 2 * C::MS, sL, out + e * N3, u);
 }
 
 // e(i,j,k) = ext interior + neighbours' ghost results on the first interior
@@ -642,49 +627,47 @@ __global__ void __launch_bounds__(FdmCfg<double, NL>::TPE, FdmCfg<double, NL>::M
                       const double *__restrict__ s, const double *__restrict__ d, int nelv) {
   using T = double;
   using C = FdmCfg<T, NL>;
-  static_assert(C::VEC && C::EPW == 1, "vector form only");
-  constexpr int N2 = C::N2, N3 = C::N3, LPE = C::LPE, MS = NL * C::NLR;
-  static_assert(6 * N2 <= C::BUF, "matrix staging fits the second buffer");
+  static_assert(C::EPW == 1, "one element a block");
+  constexpr int N2 = C::N2, N3 = C::N3, LPE = C::LPE, MS = C::MS;
   extern __shared__ __align__(16) unsigned char fdm_smem[];
   const int u = threadIdx.x;
-  T *b0 = reinterpret_cast<T *>(fdm_smem), *b1 = b0 + C::BUF;
-  T *sS = b0 + C::OFFM, *sL = sS + C::MAT, *stage = b1;
+  T *b0 = reinterpret_cast<T *>(fdm_smem);
+  T *fwd = b0 + C::BUF, *bwd = fwd + 3 * MS, *sL = fwd + C::MAT;
   const long e = blockIdx.x;
   if (e >= nelv) return;
   for (int q = u; q < N3; q += LPE) cp_async_elem<T>(b0 + C::pos(q / NL, q % NL), r + e * N3 + q, true);
-  for (int q = u; q < 6 * N2; q += LPE) cp_async_elem<T>(stage + q, s + e * 6 * N2 + q, true);
-  cp_async_wait_all();
-  __syncthreads();
   // Row l of a pass's matrix holds the weights of input l for outputs
   // i = 0..nl-1.  The reference's transforms are tnsr3d(s(2,x), s(1,y),
   // s(1,z)) forward and tnsr3d(s(1,x), s(2,y), s(2,z)) backward, whose
   // first matrix contracts as A(i, l) and the other two as Bt(l, j).
-  T *fwd = sS, *bwd = sS + 3 * MS;
-  for (int q = u; q < 3 * N2; q += LPE) {
-    const int dd = q / N2, rr = q - dd * N2, i = rr % NL, l = rr / NL;
-    const T *s1 = stage + (2 * dd) * N2, *s2 = stage + (2 * dd + 1) * N2;
-    fwd[dd * MS + i + C::NLR * l] = dd == 0 ? s2[i + NL * l] : s1[l + NL * i];
-    bwd[dd * MS + i + C::NLR * l] = dd == 0 ? s1[i + NL * l] : s2[l + NL * i];
+  for (int q = u; q < 6 * N2; q += LPE) {
+    const int dm = q / N2, w = q - dm * N2, dd = dm >> 1, a = w % NL, b = w / NL;
+    // s(., ., 1, .) serves the forward pass (the backward one of x), s(., .,
+    // 2, .) the backward pass (the forward one of x)
+    T *to = ((dm & 1) == 0) == (dd != 0) ? fwd : bwd;
+    cp_async_elem<T>(to + dd * MS + (dd == 0 ? a + C::NLR * b : b + C::NLR * a),
+                     s + e * 6 * N2 + q, true);
   }
+  cp_async_wait_all();
   __syncthreads();
-  fdm_pass<T, NL, true, false>(b0, b1, fwd, sL, nullptr, u);
+  fdm_pass<T, NL, false>(b0, fwd, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, true, false>(b1, b0, fwd + MS, sL, nullptr, u);
+  fdm_pass<T, NL, false>(b0, fwd + MS, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, true, false>(b0, b1, fwd + 2 * MS, sL, nullptr, u);
+  fdm_pass<T, NL, false>(b0, fwd + 2 * MS, sL, nullptr, u);
   __syncthreads();
   for (int q = u; q < N3; q += LPE) {  // r = d * (forward transform), kept for the backward one
     const int p = C::pos(q / NL, q % NL);
-    const T v = b1[p] * d[e * N3 + q];
-    b1[p] = v;
+    const T v = b0[p] * d[e * N3 + q];
+    b0[p] = v;
     r[e * N3 + q] = v;
   }
   __syncthreads();
-  fdm_pass<T, NL, false, false>(b1, b0, bwd, sL, nullptr, u);
+  fdm_pass<T, NL, false>(b0, bwd, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false, false>(b0, b1, bwd + MS, sL, nullptr, u);
+  fdm_pass<T, NL, false>(b0, bwd + MS, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false, false>(b1, nullptr, bwd + 2 * MS, sL, eo + e * N3, u);
+  fdm_pass<T, NL, false>(b0, bwd + 2 * MS, sL, eo + e * N3, u);
 }
 
 template <int NL>
