@@ -347,8 +347,7 @@ nb_status nb_problem_sync(nb_problem *p, void *stream);
 /* The direction update and operator of one CG iteration in one streaming
  * pass: pdir = z + beta pdir, w = A pdir (element-local, before the
  * gather-scatter), and *pap = sum over the local points of pdir * w (pap a
- * device double, may be NULL).  One launch when the problem has no mask and
- * no h2 term (lx 6, 8, 10); separate passes otherwise.  It fuses what
+ * device double, may be NULL), in one launch.  It fuses what
  * fusedcg_device_solve does with cuda_fusedcg_update_p followed by
  * ax_t%compute (src/krylov/bcknd/device/fusedcg_device.F90:382-384), and
  * adds the curvature sum.  Asynchronous on `stream`; calls on one problem

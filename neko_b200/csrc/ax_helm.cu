@@ -310,16 +310,21 @@ cudaError_t ax_helm_stream(T *w, const T *u, const T *D, const T *Dt, const T *h
   }
 }
 // ---------------------------------------------------------------------------
-// The streaming kernel fused with the two CG steps around it, for a problem
-// with no masked points and no h2 term: p = z + beta p (cg_update_p),
-// w = A p (element-local, before the gather-scatter), and pap = sum over the
-// local points of p * w with alpha = rtz / pap (cg_pap).  p is continuous
-// (z is), so the local sum equals (p, mult gs(w)), the form the reference
-// evaluates after the gather-scatter (cg_device.f90:211-214): each global
-// point's weights 1/k over its k copies add up to one.  The ring carries z
-// and the old p in place of u; each thread forms the new p for its own
-// points, stores it, and the element's operator then reads it from the
-// stage.  Returns at once when st->done is set.
+// The streaming kernel fused with the two CG steps around it: p = z + beta p
+// (cg_update_p), w = A p (element-local, before the gather-scatter, with the
+// h2 B p term when H2), and pap = sum over the local points of p * w with
+// alpha = rtz / pap (cg_pap).  p is continuous and zero on masked points (z
+// is), so the local sum equals (p, mult gs(w)) with the mask, the form the
+// reference evaluates after the gather-scatter (cg_device.f90:211-214): each
+// global point's weights 1/k over its k copies add up to one.  The ring
+// carries z and the old p in place of u; each thread forms the new p for its
+// own points, stores it, and the element's operator then reads it from the
+// stage.  h2 and B are read by each thread for its own points, issued before
+// the wait for the stage, so they cost no shared memory.  Returns at once
+// when st->done is set.
+//
+// Bound by HBM: 88 B a point, 104 with h2 (the separate passes: direction 24,
+// operator 72, h2 term 40, curvature 20).
 // ---------------------------------------------------------------------------
 // AL (lx = 10): the three work planes live in the stage itself, over the
 // G11, G22, G33 arrays of the element being computed (each thread reads the
@@ -336,7 +341,7 @@ struct AxCgCfg {
       S * NA * ABYTES + (AL ? 0 : 3 * ABYTES) + 2 * L2 * sizeof(double) + 16 * S;
 };
 
-template <int LX, int S, int KS, typename TZ, bool AL = false>
+template <int LX, int S, int KS, typename TZ, bool AL, bool H2>
 __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
     ax_cg_fused_kernel(double *__restrict__ w, double *__restrict__ p,
                        const TZ *__restrict__ z, const double *__restrict__ D,
@@ -344,6 +349,7 @@ __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
                        const double *__restrict__ g11, const double *__restrict__ g22,
                        const double *__restrict__ g33, const double *__restrict__ g12,
                        const double *__restrict__ g13, const double *__restrict__ g23,
+                       const double *__restrict__ h2, const double *__restrict__ Bm,
                        const int nelv, CgState *st, double beta_arg, double *pap_out,
                        double *partials, unsigned *counter, int *__restrict__ err) {
   using C = AxCgCfg<LX, S, KS, AL>;
@@ -400,12 +406,20 @@ __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
   bool failed = false;
   for (; t < nt; t++) {
     const int s = t % S;
+    const long e = b + (long)t * G;
+    double hb[H2 ? KP : 1];  // h2 B at this thread's points
+    if (H2 && act) {
+#pragma unroll
+      for (int kk = 0; kk < KP; kk++) {
+        const long g = e * L3 + col + L2 * (k0 + kk);
+        hb[kk] = __ldg(h2 + g) * __ldg(Bm + g);
+      }
+    }
     const bool ok = mbar_wait(&full[s], (uint32_t)((t / S) & 1));
     if (__syncthreads_or(!ok)) {
       failed = true;
       break;
     }
-    const long e = b + (long)t * G;
     const TZ *sz = reinterpret_cast<const TZ *>(stage + (size_t)s * NA * L3);
     double *su = stage + (size_t)s * NA * L3 + L3;  // old p, replaced by the new
     const double *sh = su + L3, *s11 = su + 2 * L3, *s22 = su + 3 * L3, *s33 = su + 4 * L3,
@@ -464,7 +478,8 @@ __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
           c += Dtj[l] * wsp[i + LX * l + L2 * k];
           d += sDt[k + LX * l] * rt[l];
         }
-        const double wq = a + c + d;
+        double wq = a + c + d;
+        if (H2) wq = wq + hb[kk] * pown[kk];
         w[e * L3 + col + L2 * k] = wq;
         pap += pown[kk] * wq;
       }
@@ -491,15 +506,23 @@ __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
   }
 }
 
-template <int LX, int S, int KS, typename TZ, bool AL = false>
-static cudaError_t launch_ax_cg(double *w, double *p, const TZ *z, const double *D,
-                                const double *Dt, const double *h1, const double *g11,
-                                const double *g22, const double *g33, const double *g12,
-                                const double *g13, const double *g23, int nelv, CgState *st,
-                                double beta, double *pap_out, double *partials,
-                                unsigned *counter, int max_grid, cudaStream_t s, int *err) {
+// Operands of one fused step (see ax_cg_fused).
+template <typename TZ>
+struct AxCgArgs {
+  double *w, *p;
+  const TZ *z;
+  const double *D, *Dt, *h1, *g[6], *h2, *B;
+  int nelv;
+  CgState *st;
+  double beta, *pap_out, *partials;
+  unsigned *counter;
+  int max_grid, *err;
+};
+
+template <int LX, int S, int KS, typename TZ, bool AL, bool H2>
+static cudaError_t launch_ax_cg(const AxCgArgs<TZ> &a, cudaStream_t s) {
   using C = AxCgCfg<LX, S, KS, AL>;
-  auto kern = ax_cg_fused_kernel<LX, S, KS, TZ, AL>;
+  auto kern = ax_cg_fused_kernel<LX, S, KS, TZ, AL, H2>;
   static int grid_per_dev[64] = {0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -515,43 +538,176 @@ static cudaError_t launch_ax_cg(double *w, double *p, const TZ *z, const double 
     if (e != cudaSuccess) return e;
     g = (per_sm > 0 ? per_sm : 1) * sms;
   }
-  if (nelv <= 0) return cudaErrorNotSupported;
-  int grid = nelv < g ? nelv : g;
-  if (grid > max_grid) grid = max_grid;
-  kern<<<grid, C::THREADS, C::SMEM, s>>>(w, p, z, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv,
-                                          st, beta, pap_out, partials, counter, err);
+  int grid = a.nelv < g ? a.nelv : g;
+  if (grid > a.max_grid) grid = a.max_grid;
+  kern<<<grid, C::THREADS, C::SMEM, s>>>(a.w, a.p, a.z, a.D, a.Dt, a.h1, a.g[0], a.g[1], a.g[2],
+                                         a.g[3], a.g[4], a.g[5], a.h2, a.B, a.nelv, a.st, a.beta,
+                                         a.pap_out, a.partials, a.counter, a.err);
+  return cudaGetLastError();
+}
+
+// The fused step for the other orders and for operands that are not 16-byte
+// aligned (a bulk copy moves whole 16-byte units, and lx^3 values are not one
+// for odd lx): NE elements a block with plain coalesced loads, the element
+// loop of ax_helm_kernel.
+template <int LX, int NE>
+struct AxCgGen {
+  static constexpr int L2 = LX * LX, L3 = L2 * LX;
+  static constexpr int THREADS = ((L2 * NE + 31) / 32) * 32;
+  static constexpr size_t SMEM = sizeof(double) * (2 * L2 + (size_t)NE * 3 * L3);
+};
+
+template <int LX, int NE, typename TZ>
+__global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS)
+    ax_cg_gen_kernel(const AxCgArgs<TZ> a) {
+  using C = AxCgGen<LX, NE>;
+  constexpr int L2 = C::L2, L3 = C::L3;
+  if (a.st && a.st->done) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *sD = reinterpret_cast<double *>(smem_raw), *sDt = sD + L2;
+  const int tid = threadIdx.x, tz = tid / L2, col = tid - tz * L2;
+  const int i = col % LX, j = col / LX;
+  double *su = sDt + L2 + (tz < NE ? tz : 0) * 3 * L3, *sur = su + L3, *sus = sur + L3;
+  for (int q = tid; q < L2; q += C::THREADS) {
+    sD[q] = a.D[q];
+    sDt[q] = a.Dt[q];
+  }
+  const double beta = a.st ? a.st->beta : a.beta;
+  double pap = 0.0;
+  for (long eb = (long)blockIdx.x * NE; eb < a.nelv; eb += (long)gridDim.x * NE) {
+    const long e = eb + tz;
+    const bool active = tz < NE && e < a.nelv;
+    const long base = e * L3 + col;
+    double rp[LX], rut[LX];
+    __syncthreads();  // matrices loaded; planes of the previous elements read
+    if (active) {
+#pragma unroll
+      for (int k = 0; k < LX; k++) {
+        const long g = base + k * L2;
+        rp[k] = (double)a.z[g] + beta * a.p[g];
+      }
+#pragma unroll
+      for (int k = 0; k < LX; k++) {
+        a.p[base + k * L2] = rp[k];
+        su[col + L2 * k] = rp[k];
+      }
+    }
+    __syncthreads();
+    if (active) {
+#pragma unroll
+      for (int k = 0; k < LX; k++) {
+        double ur = 0, us = 0, ut = 0;
+#pragma unroll
+        for (int l = 0; l < LX; l++) {
+          ur += sD[i + LX * l] * su[l + LX * j + L2 * k];
+          us += sD[j + LX * l] * su[i + LX * l + L2 * k];
+          ut += sD[k + LX * l] * rp[l];
+        }
+        const long g = base + k * L2;
+        const double G11 = __ldg(a.g[0] + g), G22 = __ldg(a.g[1] + g), G33 = __ldg(a.g[2] + g),
+                     G12 = __ldg(a.g[3] + g), G13 = __ldg(a.g[4] + g), G23 = __ldg(a.g[5] + g),
+                     H = __ldg(a.h1 + g);
+        sur[col + L2 * k] = H * (G11 * ur + G12 * us + G13 * ut);
+        sus[col + L2 * k] = H * (G12 * ur + G22 * us + G23 * ut);
+        rut[k] = H * (G13 * ur + G23 * us + G33 * ut);
+      }
+    }
+    __syncthreads();
+    if (active) {
+#pragma unroll
+      for (int k = 0; k < LX; k++) {
+        double c0 = 0, c1 = 0, c2 = 0;
+#pragma unroll
+        for (int l = 0; l < LX; l++) {
+          c0 += sDt[i + LX * l] * sur[l + LX * j + L2 * k];
+          c1 += sDt[j + LX * l] * sus[i + LX * l + L2 * k];
+          c2 += sDt[k + LX * l] * rut[l];
+        }
+        const long g = base + k * L2;
+        double wv = c0 + c1 + c2;
+        if (a.h2) wv = wv + __ldg(a.h2 + g) * __ldg(a.B + g) * rp[k];
+        a.w[g] = wv;
+        pap += rp[k] * wv;
+      }
+    }
+  }
+  double tot;
+  if (grid_sum<C::THREADS>(pap, a.partials, a.counter, &tot)) {
+    if (a.st) {
+      a.st->pap = tot;
+      a.st->alpha = a.st->rtz1 / tot;
+    } else if (a.pap_out) {
+      *a.pap_out = tot;
+    }
+  }
+}
+
+template <int LX, typename TZ>
+static cudaError_t launch_ax_cg_gen(const AxCgArgs<TZ> &a, cudaStream_t s) {
+  using C = AxCgGen<LX, AxCfg<LX>::NE>;
+  auto kern = ax_cg_gen_kernel<LX, AxCfg<LX>::NE, TZ>;
+  if (C::SMEM > 48 * 1024) {
+    cudaError_t e =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    if (e != cudaSuccess) return e;
+  }
+  // every partial sum has a slot: blocks loop over the elements beyond that
+  const int ne = AxCfg<LX>::NE, need = (a.nelv + ne - 1) / ne;
+  kern<<<need < a.max_grid ? need : a.max_grid, C::THREADS, C::SMEM, s>>>(a);
   return cudaGetLastError();
 }
 
 template <typename TZ>
 cudaError_t ax_cg_fused(double *w, double *p, const TZ *z, const double *D, const double *Dt,
                         const double *h1, const double *g11, const double *g22, const double *g33,
-                        const double *g12, const double *g13, const double *g23, int nelv, int lx,
-                        CgState *st, double beta, double *pap_out, double *partials,
-                        unsigned *counter, int max_grid, cudaStream_t s, int *err) {
+                        const double *g12, const double *g13, const double *g23,
+                        const double *h2, const double *B, int nelv, int lx, CgState *st,
+                        double beta, double *pap_out, double *partials, unsigned *counter,
+                        int max_grid, cudaStream_t s, int *err) {
+  if (nelv <= 0) return cudaErrorNotSupported;
+  const AxCgArgs<TZ> a{w,    p,  z,    D,       Dt,       h1,      {g11, g22, g33, g12, g13, g23},
+                       h2,   B,  nelv, st,      beta,     pap_out, partials,
+                       counter, max_grid, err};
+  bool aligned = ((size_t)lx * lx * lx * sizeof(TZ)) % 16 == 0;
   const void *ptrs[] = {z, p, h1, g11, g22, g33, g12, g13, g23};
   for (const void *q : ptrs)
-    if (reinterpret_cast<uintptr_t>(q) & 15) return cudaErrorNotSupported;
-  if (((size_t)lx * lx * lx * sizeof(TZ)) % 16) return cudaErrorNotSupported;
+    if (reinterpret_cast<uintptr_t>(q) & 15) aligned = false;
+  if (aligned) {
+#define NB_CG_CASE(LX, S, KS, AL)                                              \
+  case LX:                                                                     \
+    return h2 ? launch_ax_cg<LX, S, KS, TZ, AL, true>(a, s)                    \
+              : launch_ax_cg<LX, S, KS, TZ, AL, false>(a, s);
+    switch (lx) {
+      NB_CG_CASE(4, 4, 4, false)
+      NB_CG_CASE(6, 3, 2, false)
+      NB_CG_CASE(8, 2, 2, false)
+      NB_CG_CASE(10, 3, 5, true)
+      default: break;
+    }
+#undef NB_CG_CASE
+  }
   switch (lx) {
-    case 6: return launch_ax_cg<6, 3, 2, TZ>(w, p, z, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, st, beta, pap_out, partials, counter, max_grid, s, err);
-    case 8: return launch_ax_cg<8, 2, 2, TZ>(w, p, z, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, st, beta, pap_out, partials, counter, max_grid, s, err);
-    case 10: return launch_ax_cg<10, 3, 5, TZ, true>(w, p, z, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, st, beta, pap_out, partials, counter, max_grid, s, err);
+#define NB_CG_GEN(N) \
+  case N: return launch_ax_cg_gen<N, TZ>(a, s);
+    NB_CG_GEN(2) NB_CG_GEN(3) NB_CG_GEN(4) NB_CG_GEN(5) NB_CG_GEN(6) NB_CG_GEN(7) NB_CG_GEN(8)
+    NB_CG_GEN(9) NB_CG_GEN(10) NB_CG_GEN(11) NB_CG_GEN(12) NB_CG_GEN(13) NB_CG_GEN(14)
+    NB_CG_GEN(15) NB_CG_GEN(16)
+#undef NB_CG_GEN
     default: return cudaErrorNotSupported;
   }
 }
 template cudaError_t ax_cg_fused<double>(double *, double *, const double *, const double *,
                                          const double *, const double *, const double *,
                                          const double *, const double *, const double *,
-                                         const double *, const double *, int, int, CgState *,
-                                         double, double *, double *, unsigned *, int,
-                                         cudaStream_t, int *);
+                                         const double *, const double *, const double *,
+                                         const double *, int, int, CgState *, double, double *,
+                                         double *, unsigned *, int, cudaStream_t, int *);
 template cudaError_t ax_cg_fused<float>(double *, double *, const float *, const double *,
                                         const double *, const double *, const double *,
                                         const double *, const double *, const double *,
-                                        const double *, const double *, int, int, CgState *,
-                                        double, double *, double *, unsigned *, int,
-                                        cudaStream_t, int *);
+                                        const double *, const double *, const double *,
+                                        const double *, int, int, CgState *, double, double *,
+                                        double *, unsigned *, int, cudaStream_t, int *);
 
 int *dropin_error_word() {
   static int *cache[64] = {nullptr};

@@ -10,12 +10,17 @@
 // alpha, rnorm) live in device memory and are produced by the last block of
 // each reduction, so no iteration waits for the host (the reference copies
 // three dot products to the host and synchronises per iteration,
-// math.cu:765-797); the vector updates and the mult-weighted inner products
-// are fused (x/r update + (r,mult r) in one pass, z = d r + (r, mult z) in
-// one pass); the gather-scatter and the mask are one launch; and a chunk of
-// iterations is captured in a CUDA graph and replayed, each kernel
-// returning at once after the convergence flag is set, so the iteration
-// count is exact.
+// math.cu:765-797); p = z + beta p, w = A p and (w, mult p) are one launch
+// (ax_cg_fused); the gather-scatter and the mask are one launch; with the
+// Jacobi preconditioner (or none) the x and r update, z = d r and the next
+// iteration's (r, mult z) are one pass, so an iteration is three launches;
+// and a chunk of iterations is captured in a CUDA graph and replayed, each
+// kernel returning at once after the convergence flag is set, so the
+// iteration count is exact.
+//
+// What the fusions are worth: a Jacobi-CG iteration on 262,144 points (8^3
+// elements, lx 8) took 30 us as six launches, a Helmholtz one on 7.1 M points
+// 301 us as seven.
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -54,32 +59,35 @@ __global__ void addcol4_kernel(double *w, const double *h2, const double *B, con
 // CG kernels.  Every kernel returns immediately once st->done is set.
 // ---------------------------------------------------------------------------
 
-// x = 0, p = 0, r = f, rtr = (r, mult r) -> res_start.
+// x = 0, p = 0, r = f, rtr = (r, mult r) -> res_start; with z given (the
+// folded preconditioner) z = d r (d null: z = r) and rtz = (r, mult z).
 __global__ void __launch_bounds__(kRedThreads)
     cg_init_kernel(double *__restrict__ x, double *__restrict__ p, double *__restrict__ r,
+                   double *__restrict__ z, const double *__restrict__ d,
                    const double *__restrict__ f, const double *__restrict__ mult, const float *__restrict__ multf, long n,
-                   CgState *st, double *partials, unsigned *counter,
-                   const int *__restrict__ outer_skip) {
-  if (outer_skip && *outer_skip) {  // enclosing solve finished: stay idle
-    if (blockIdx.x == 0 && threadIdx.x == 0) st->done = 1;
-    return;
-  }
-  double s = 0.0;
+                   CgState *st, double *partials, unsigned *counter) {
+  double s = 0.0, sz = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
        i += (long)gridDim.x * kRedThreads) {
-    const double ri = f[i];
+    const double ri = f[i], m = MW(i);
     x[i] = 0.0;
     p[i] = 0.0;
     r[i] = ri;
-    s += ri * MW(i) * ri;
+    s += ri * m * ri;
+    if (z) {
+      const double zi = d ? ri * d[i] : ri;
+      z[i] = zi;
+      sz += ri * m * zi;
+    }
   }
-  double tot;
-  if (grid_sum<kRedThreads>(s, partials, counter, &tot)) {
-    const double rn = sqrt(tot) * st->norm_fac;
-    st->rtr = tot;
+  double tot[2];
+  if (grid_sum2<kRedThreads>(s, sz, partials, counter, tot)) {
+    const double rn = sqrt(tot[0]) * st->norm_fac;
+    st->rtr = tot[0];
     st->rnorm = rn;
     st->res_start = rn;
-    st->rtz1 = 1.0;
+    st->rtz1 = z ? tot[1] : 1.0;
+    st->beta = 0.0;
     st->iter = 0;
     st->nan = 0;
     st->skip_rc = 1;
@@ -267,6 +275,68 @@ __global__ void __launch_bounds__(kRedThreads)
   }
 }
 
+// The update with the preconditioner folded in: x += alpha p; r -= alpha w;
+// z = d r (d null: z = r); (r, mult r), (r, mult z) and the convergence
+// test; beta of the next iteration.  68 B a point (60 with mult in FP32):
+// bound by HBM on large problems, by launch and reduction latency on small
+// ones.
+__global__ void __launch_bounds__(kRedThreads)
+    cg_update_xrz_kernel(double *__restrict__ r, double *__restrict__ z,
+                         const double *__restrict__ p, const double *__restrict__ w,
+                         const double *__restrict__ d, const double *__restrict__ mult,
+                         const float *__restrict__ multf, long n, CgState *st, double *partials,
+                         unsigned *counter) {
+  if (st->done) return;
+  double *__restrict__ x = st->x;
+  const double alpha = st->alpha, malpha = -alpha;
+  double s = 0.0, sz = 0.0;
+  // every operand of a pair of points is loaded before anything is stored
+  // (x comes from the state: the compiler cannot tell it from r)
+  const long stride = (long)gridDim.x * kRedThreads;
+  for (long i0 = blockIdx.x * (long)kRedThreads + threadIdx.x; i0 < n; i0 += 2 * stride) {
+    const long i1 = i0 + stride;
+    const bool two = i1 < n;
+    const double x0 = x[i0], p0 = p[i0], r0 = r[i0], w0 = w[i0], m0 = MW(i0),
+                 d0 = d ? d[i0] : 1.0;
+    double x1 = 0, p1 = 0, r1 = 0, w1 = 0, m1 = 0, d1 = 0;
+    if (two) {
+      x1 = x[i1], p1 = p[i1], r1 = r[i1], w1 = w[i1], m1 = MW(i1), d1 = d ? d[i1] : 1.0;
+    }
+    const double ri0 = r0 + malpha * w0, zi0 = ri0 * d0;
+    x[i0] = x0 + alpha * p0;
+    r[i0] = ri0;
+    z[i0] = zi0;
+    s += ri0 * m0 * ri0;
+    sz += ri0 * m0 * zi0;
+    if (two) {
+      const double ri1 = r1 + malpha * w1, zi1 = ri1 * d1;
+      x[i1] = x1 + alpha * p1;
+      r[i1] = ri1;
+      z[i1] = zi1;
+      s += ri1 * m1 * ri1;
+      sz += ri1 * m1 * zi1;
+    }
+  }
+  double tot[2];
+  if (grid_sum2<kRedThreads>(s, sz, partials, counter, tot)) {
+    const double rn = sqrt(tot[0]) * st->norm_fac;
+    st->rtr = tot[0];
+    st->rnorm = rn;
+    st->iter += 1;
+    int done = 0;
+    if (!(rn == rn) || isinf(rn)) {
+      st->nan = 1;
+      done = 1;
+    }
+    if (rn < st->abs_tol) done = 1;
+    if (st->iter >= st->max_iter) done = 1;
+    st->done = done;
+    st->rtz2 = st->rtz1;
+    st->rtz1 = tot[1];
+    st->beta = tot[1] / st->rtz2;
+  }
+}
+
 // True residual: r = f - w (w = A x just computed), rtr, rnorm and the
 // convergence test redone on it; the next direction restarts (beta = 0).
 __global__ void __launch_bounds__(kRedThreads)
@@ -394,20 +464,22 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, cuda
         cg_dot_rz_kernel<double><<<rb, kRedThreads, 0, s>>>(W.z, W.r, P->mult, P->multf, n,
                                                             W.st, W.partials, W.counter);
     }
-  } else {
+  } else if (!W.fold) {
     cg_precond_dot_kernel<<<rb, kRedThreads, 0, s>>>(W.z, W.r, W.use_jacobi ? P->jdiag : nullptr,
                                                      P->mult, P->multf, n, W.st, W.partials, W.counter);
   }
-  // p = z + beta p; w = A p; pap: one launch when the problem has no mask and
-  // no h2 term (the local form of pap needs p zero wherever w is masked)
+  // p = z + beta p; w = A p; pap: one launch (the local form of pap needs p
+  // continuous and zero wherever w is masked: f is assembled and masked, so r
+  // and every preconditioner's output are)
   cudaError_t e = cudaErrorNotSupported;
-  if (P->nmask == 0 && !P->ifh2 && P->use_stream_ax)
+  const double *h2 = P->ifh2 ? P->h2 : nullptr;
+  if (P->use_stream_ax)
     e = zf ? ax_cg_fused(W.w, W.p, zf, P->D, P->Dt, P->h1, P->g11, P->g22, P->g33, P->g12,
-                         P->g13, P->g23, (int)P->nelv, P->lx, W.st, 0.0, nullptr, W.partials,
-                         W.counter, kCgMaxPartials, s, P->err)
+                         P->g13, P->g23, h2, P->B, (int)P->nelv, P->lx, W.st, 0.0, nullptr,
+                         W.partials, W.counter, kCgMaxPartials, s, P->err)
            : ax_cg_fused(W.w, W.p, (const double *)W.z, P->D, P->Dt, P->h1, P->g11, P->g22,
-                         P->g33, P->g12, P->g13, P->g23, (int)P->nelv, P->lx, W.st, 0.0, nullptr,
-                         W.partials, W.counter, kCgMaxPartials, s, P->err);
+                         P->g33, P->g12, P->g13, P->g23, h2, P->B, (int)P->nelv, P->lx, W.st,
+                         0.0, nullptr, W.partials, W.counter, kCgMaxPartials, s, P->err);
   W.fused = e == cudaSuccess;
   if (e != cudaSuccess && e != cudaErrorNotSupported) return e;
   if (!W.fused) {
@@ -423,6 +495,12 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, cuda
   if (e != cudaSuccess) return e;
   if (!W.fused)
     cg_pap_kernel<<<rb, kRedThreads, 0, s>>>(W.w, W.p, P->mult, P->multf, n, W.st, W.partials, W.counter);
+  if (W.fold) {
+    cg_update_xrz_kernel<<<rb, kRedThreads, 0, s>>>(W.r, W.z, W.p, W.w,
+                                                    W.use_jacobi ? P->jdiag : nullptr, P->mult,
+                                                    P->multf, n, W.st, W.partials, W.counter);
+    return cudaGetLastError();
+  }
   cg_update_xr_kernel<<<rb, kRedThreads, 0, s>>>(W.r, W.p, W.w, P->mult, P->multf, n, W.st,
                                                  W.partials, W.counter);
   if (W.recompute_every > 0) {  // w = A x, gs, mask; r = f - w (scheduled iterations only)
@@ -480,6 +558,8 @@ nb_status cg_start(CgRun &R) {
   W.flexible = (o.flexible != 0 || o.mixed != 0) && pc != nullptr;
   W.recompute_every = o.mixed ? 50 : 0;
   W.use_dots = W.flexible && pc->dots_in_apply();
+  // z = d r moves into the update, except where r may change after it
+  W.fold = !pc && W.recompute_every == 0;
   if (W.use_dots && (!W.dots || W.dots_n != P->nelv)) {
     if (W.dots) cudaFree(W.dots);
     W.dots = nullptr;
@@ -501,15 +581,16 @@ nb_status cg_start(CgRun &R) {
   init.skip_rc = 1;
   NB_CUDA_TRY(cudaMemcpyAsync(W.st, &init, sizeof(CgState), cudaMemcpyHostToDevice, s));
   const long n = P->n;
-  cg_init_kernel<<<red_blocks(n), kRedThreads, 0, s>>>(R.x, W.p, W.r, R.f, P->mult, P->multf, n,
-                                                        W.st, W.partials, W.counter, nullptr);
+  cg_init_kernel<<<red_blocks(n), kRedThreads, 0, s>>>(
+      R.x, W.p, W.r, W.fold ? W.z : nullptr, W.use_jacobi ? P->jdiag : nullptr, R.f, P->mult,
+      P->multf, n, W.st, W.partials, W.counter);
   NB_CUDA_TRY(cudaGetLastError());
   // (Re)capture the iteration graph when the operands changed.
   // x and f are read from the state: the graph depends on neither
   const void *key[5] = {nullptr, nullptr, pc,
                         (const void *)(intptr_t)(W.use_jacobi | (W.flexible << 1) |
                                                  ((W.recompute_every > 0) << 2) |
-                                                 (W.use_dots << 3)),
+                                                 (W.use_dots << 3) | (W.fold << 4)),
                         (const void *)(intptr_t)P->ifh2};
   bool same = W.graph_exec && !memcmp(key, W.graph_key, sizeof(key));
   R.chunk = n > (1 << 22) ? 4 : 16;
@@ -529,7 +610,7 @@ nb_status cg_start(CgRun &R) {
     // inner products formed by the preconditioner a one-block finishing
     // launch replaces the dot pass
     const int pc_launches = pc ? pc->launches() - (pc->output_f32() ? 1 : 0) : 0;
-    W.launches_per_iter = (W.fused ? 4 : 6 + (P->ifh2 ? 1 : 0)) + pc_launches +
+    W.launches_per_iter = (W.fused ? 4 : 6 + (P->ifh2 ? 1 : 0)) - (W.fold ? 1 : 0) + pc_launches +
                           (W.recompute_every > 0 ? 4 + (P->ifh2 ? 1 : 0) : 0);
     cudaError_t ee = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);

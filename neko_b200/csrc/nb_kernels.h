@@ -63,19 +63,21 @@ cudaError_t ax_stress_part2(double *au, double *av, double *aw, const double *u,
                             const double *B, long n, cudaStream_t s, const int *skip);
 
 struct CgState;
-// p = z + beta p, w = A p (no gather-scatter) and pap = sum p * w in one
-// streaming launch (ax_helm.cu).  With a CG state, beta is read from it,
-// the launch returns at once when st->done is set, and pap and alpha =
-// rtz / pap are written to it; without one, beta is the argument and pap
-// goes to *pap_out (device, may be null).  cudaErrorNotSupported when lx or
-// alignment is not covered.
+// p = z + beta p, w = A p (+ h2 B p when h2 is given; no gather-scatter) and
+// pap = sum p * w in one launch (ax_helm.cu).  With a CG state, beta is read
+// from it, the launch returns at once when st->done is set, and pap and
+// alpha = rtz / pap are written to it; without one, beta is the argument and
+// pap goes to *pap_out (device, may be null).  The streaming kernel for lx 4,
+// 6, 8, 10 with 16-byte aligned operands, a general one otherwise;
+// cudaErrorNotSupported for lx outside 2..16.
 // z may be FP32 (a mixed-precision preconditioner's output), widened as read.
 template <typename TZ>
 cudaError_t ax_cg_fused(double *w, double *p, const TZ *z, const double *D, const double *Dt,
                         const double *h1, const double *g11, const double *g22, const double *g33,
-                        const double *g12, const double *g13, const double *g23, int nelv, int lx,
-                        CgState *st, double beta, double *pap_out, double *partials,
-                        unsigned *counter, int max_grid, cudaStream_t s, int *err);
+                        const double *g12, const double *g13, const double *g23,
+                        const double *h2, const double *B, int nelv, int lx, CgState *st,
+                        double beta, double *pap_out, double *partials, unsigned *counter,
+                        int max_grid, cudaStream_t s, int *err);
 
 // cuda_fdm_do_fast for nl 8..16 with the native FDM passes (pc_hsmg.cu);
 // cudaErrorNotSupported for other nl.

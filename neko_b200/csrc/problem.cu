@@ -630,10 +630,10 @@ extern "C" nb_status nb_ax_update_p(nb_problem *p, double *w, double *pdir, cons
   if (!p || !w || !pdir || !z) return fail(NB_ERR_ARG, "null argument");
   const cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = cudaErrorNotSupported;
-  if (p->nmask == 0 && !p->ifh2 && p->use_stream_ax)
+  if (p->use_stream_ax)
     e = ax_cg_fused(w, pdir, z, p->D, p->Dt, p->h1, p->g11, p->g22, p->g33, p->g12, p->g13,
-                    p->g23, p->nelv, p->lx, nullptr, beta, pap, p->red_partials, p->red_counter,
-                    kMaxRedBlocks, s, p->err);
+                    p->g23, p->ifh2 ? p->h2 : nullptr, p->B, p->nelv, p->lx, nullptr, beta, pap,
+                    p->red_partials, p->red_counter, kMaxRedBlocks, s, p->err);
   if (e != cudaErrorNotSupported) {
     NB_TRY(e);
     return NB_OK;
