@@ -12,13 +12,13 @@
 //
 // and the h2 B term (cuda_ax_helm_stress_vector_part2).
 //
-// B200 form: a persistent streaming kernel (lx 4, 6, 8) -- the three
+// B200 form: a persistent streaming kernel (lx 4, 6, 8, 10) -- the three
 // components, h1, 1/jac and the nine cofactors of an element (14 arrays)
 // arrive in one bulk-copy stage, the strain is formed once for the three
-// components, the nine flux planes are written to shared memory and the
-// transposed contractions read them back; the stage is refilled as soon as
-// the fluxes are formed.  112 B of coefficients and 48 B of fields per
-// point: 136 B per point moved (17 arrays of 8 B).  Other orders use a
+// components, the nine flux planes are written over the cofactors in the
+// stage and the transposed contractions read them back.  112 B of
+// coefficients and 48 B of fields per point: 136 B per point moved (17 arrays
+// of 8 B).  Other orders use a
 // general kernel (one element per block, fluxes kept in registers).
 #include <cstdint>
 #include <cstdio>
@@ -84,35 +84,50 @@ __device__ __forceinline__ void stress_point(const double g[3][3], const double 
 }
 
 // ---------------------------------------------------------------------------
-// Streaming kernel
+// Streaming kernel (lx 4, 6, 8, 10).  Bound by HBM (136 B a point, 152 with
+// h2; 184 / 200 in the CG form) with shared-memory wavefronts close behind.
+//
+// The nine flux planes lie over the nine cofactor arrays of the element's own
+// stage: a thread reads the nine cofactors of a point and writes that point's
+// nine fluxes over them, and no thread reads another point's cofactors.  So
+// a stage is all the memory an element needs (14 arrays), two blocks of two
+// stages share a multiprocessor at lx 8, and two stages of lx 10 (224 KB) fit
+// one.  With separate planes only one block of 256 threads was resident at
+// lx 8 (104 us a coupled-CG step on 2.1 M points, 62% of the copy rate) and
+// lx 10 had no streaming form (272 us on 2.2 M points, plus 29 us for the h2
+// term).  The CG form reads z straight into registers, issued before the wait
+// for the stage, instead of staging three more arrays.
+// Registers (two blocks of 256 threads, or one of 512: 128 a thread) hold two
+// rows of D at a time, reloaded for the second pass, and the components are
+// differentiated one after the other.
 // ---------------------------------------------------------------------------
-template <int LX, int S, int KS, bool CG = false>
+template <int LX, int S, int KS>
 struct StressCfg {
-  static constexpr int L2 = LX * LX, L3 = L2 * LX, NA = CG ? 17 : 14, NP = 9;
+  static constexpr int L2 = LX * LX, L3 = L2 * LX, NA = 14;
   static constexpr int THREADS = ((L2 * KS + 31) / 32) * 32;
   static constexpr size_t ABYTES = (size_t)L3 * sizeof(double);
-  static constexpr size_t SMEM =
-      S * NA * ABYTES + NP * ABYTES + ABYTES + 3 * L2 * sizeof(double) + 16 * S;
+  static constexpr size_t SMEM = S * NA * ABYTES + L2 * sizeof(double) + 16 * S;
+  static constexpr int BLOCKS0 = (int)(233472 / (SMEM + 1024 + 128));
+  static constexpr int BLOCKS1 = BLOCKS0 * THREADS > 512 ? 512 / THREADS : BLOCKS0;
+  static constexpr int BLOCKS = BLOCKS1 < 1 ? 1 : BLOCKS1;
 };
 
-template <int LX, int S, int KS, bool CG = false>
-__global__ void __launch_bounds__(StressCfg<LX, S, KS, CG>::THREADS)
+template <int LX, int S, int KS, bool CG>
+__global__ void __launch_bounds__(StressCfg<LX, S, KS>::THREADS, StressCfg<LX, S, KS>::BLOCKS)
     ax_stress_tma_kernel(StressIo io, StressGeo geo, const double *__restrict__ dx,
                          const double *__restrict__ dy, const double *__restrict__ dz,
                          const double *__restrict__ w3, const double *__restrict__ h2,
                          const double *__restrict__ Bm, const int nelv, int *__restrict__ err,
                          const int *__restrict__ skip, StressCg cg) {
-  using C = StressCfg<LX, S, KS, CG>;
+  using C = StressCfg<LX, S, KS>;
   constexpr int L2 = C::L2, L3 = C::L3, NA = C::NA, KP = LX / KS;
-  static_assert(LX % KS == 0, "k split must divide lx");
+  static_assert(LX % KS == 0 && LX % 2 == 0, "k split must divide an even lx");
   if (skip && *skip) return;
   if (CG && cg.st->done) return;
   const double beta = CG ? cg.st->beta : 0.0;
   extern __shared__ __align__(128) unsigned char smem_stress[];
   double *stage = reinterpret_cast<double *>(smem_stress);
-  double *planes = stage + S * NA * L3;  // 9 flux planes: component-major, (r, s, t)
-  double *sW3 = planes + 9 * L3;
-  double *sDx = sW3 + L3, *sDy = sDx + L2, *sDz = sDy + L2;
+  double *sDz = stage + S * NA * L3;
   uint64_t *full = reinterpret_cast<uint64_t *>(sDz + L2);
 
   const int tid = threadIdx.x;
@@ -122,23 +137,17 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS, CG>::THREADS)
     for (int s = 0; s < S; s++) mbar_init(&full[s], 1);
     fence_barrier_init();
   }
-  for (int q = tid; q < L2; q += C::THREADS) {
-    sDx[q] = dx[q];
-    sDy[q] = dy[q];
-    sDz[q] = dz[q];
-  }
-  for (int q = tid; q < L3; q += C::THREADS) sW3[q] = w3[q];
+  for (int q = tid; q < L2; q += C::THREADS) sDz[q] = dz[q];
   __syncthreads();
-  // stage slot: u, v, w, h1, 1/jac, the nine cofactors (+ z_1..z_3 in the
-  // CG form, where u, v, w are the old directions)
+  // stage slot: u, v, w (the old directions in the CG form), h1, 1/jac, the
+  // nine cofactors
   auto issue = [&](int t, int s) {
     const long e = b + (long)t * G;
     mbar_arrive_expect_tx(&full[s], (uint32_t)(NA * C::ABYTES));
 #pragma unroll
     for (int a = 0; a < NA; a++) {
       const double *src =
-          a < 3 ? io.in[a]
-                : (a == 3 ? geo.h1 : (a == 4 ? geo.jacinv : (a < 14 ? geo.c[a - 5] : cg.z[a - 14])));
+          a < 3 ? io.in[a] : (a == 3 ? geo.h1 : (a == 4 ? geo.jacinv : geo.c[a - 5]));
       bulk_g2s(stage + (size_t)(s * NA + a) * L3, src + e * L3, (uint32_t)C::ABYTES, &full[s]);
     }
   };
@@ -148,94 +157,103 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS, CG>::THREADS)
   const bool act = tid < L2 * KS;
   const int col = tid % L2, kh = tid / L2;
   const int i = col % LX, j = col / LX, k0 = kh * KP;
-  // rows of the derivative matrices: dx(i, l), dy(j, l), and transposed dx(l, i), dy(l, j)
-  double Dxi[LX], Dyj[LX], Dxti[LX], Dytj[LX];
-#pragma unroll
-  for (int l = 0; l < LX; l++) {
-    Dxi[l] = sDx[i + LX * l];
-    Dyj[l] = sDy[j + LX * l];
-    Dxti[l] = sDx[l + LX * i];
-    Dytj[l] = sDy[l + LX * j];
-  }
 
   int t = 0;
   bool failed = false;
   double pap = 0.0;
   for (; t < nt; t++) {
     const int s = t % S;
+    const long e = b + (long)t * G;
+    double *slot = stage + (size_t)s * NA * L3;
+    double *planes = slot + 5 * L3;  // fluxes: component-major, (r, s, t)
+    // global operands of this thread's points, in flight during the wait
+    double hb[KP], zc[CG ? 3 : 1][KP];
+    if (act) {
+#pragma unroll
+      for (int kk = 0; kk < KP; kk++) {
+        const long g = e * L3 + col + L2 * (k0 + kk);
+        hb[kk] = h2 ? __ldg(h2 + g) * __ldg(Bm + g) : 0.0;
+        if constexpr (CG) {
+#pragma unroll
+          for (int c = 0; c < 3; c++) zc[c][kk] = __ldg(cg.z[c] + g);
+        }
+      }
+    }
     const bool ok = mbar_wait(&full[s], (uint32_t)((t / S) & 1));
     if (__syncthreads_or(!ok)) {
       failed = true;
       break;
     }
-    const long e = b + (long)t * G;
-    const double *slot = stage + (size_t)s * NA * L3;
     if constexpr (CG) {  // p = z + beta p for this thread's points, in the stage and stored
-      double *sp = stage + (size_t)s * NA * L3;
       if (act) {
 #pragma unroll
         for (int c = 0; c < 3; c++)
 #pragma unroll
           for (int kk = 0; kk < KP; kk++) {
             const int q = col + L2 * (k0 + kk);
-            const double pn = sp[(14 + c) * L3 + q] + beta * sp[c * L3 + q];
-            sp[c * L3 + q] = pn;
+            const double pn = zc[c][kk] + beta * slot[c * L3 + q];
+            slot[c * L3 + q] = pn;
             cg.pout[c][e * L3 + q] = pn;
           }
       }
       __syncthreads();  // the element's new directions complete in the stage
     }
-    double uown[3][KP];  // u, v, w at this thread's points (for the h2 term)
     if (act) {
-      double cu[3][LX];  // this thread's (i, j) column of u, v, w
+      double Dxi[LX], Dyj[LX];  // dx(i, l), dy(j, l)
 #pragma unroll
-      for (int c = 0; c < 3; c++)
+      for (int l = 0; l < LX; l++) {
+        Dxi[l] = __ldg(dx + i + LX * l);
+        Dyj[l] = __ldg(dy + j + LX * l);
+      }
+      double g[KP][3][3];
 #pragma unroll
-        for (int l = 0; l < LX; l++) cu[c][l] = slot[c * L3 + col + L2 * l];
+      for (int c = 0; c < 3; c++) {
+        const double *su = slot + c * L3;
+        double cu[LX];  // this thread's (i, j) column
 #pragma unroll
-      for (int c = 0; c < 3; c++)
+        for (int l = 0; l < LX; l++) cu[l] = su[col + L2 * l];
 #pragma unroll
-        for (int kk = 0; kk < KP; kk++) uown[c][kk] = slot[c * L3 + col + L2 * (k0 + kk)];
-#pragma unroll
-      for (int kk = 0; kk < KP; kk++) {
-        const int k = k0 + kk;
-        const int p = col + L2 * k;
-        double g[3][3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const double *su = slot + c * L3;
+        for (int kk = 0; kk < KP; kk++) {
+          const int k = k0 + kk;
+          const double2 *row = reinterpret_cast<const double2 *>(su + LX * j + L2 * k);
           double ur = 0, us = 0, ut = 0;
 #pragma unroll
-          for (int l = 0; l < LX; l++) {
-            ur += Dxi[l] * su[l + LX * j + L2 * k];
+          for (int l = 0; l < LX; l += 2) {
+            const double2 v = row[l / 2];
+            ur += Dxi[l] * v.x;
             us += Dyj[l] * su[i + LX * l + L2 * k];
-            ut += sDz[k + LX * l] * cu[c][l];
+            ut += sDz[k + LX * l] * cu[l];
+            ur += Dxi[l + 1] * v.y;
+            us += Dyj[l + 1] * su[i + LX * (l + 1) + L2 * k];
+            ut += sDz[k + LX * (l + 1)] * cu[l + 1];
           }
-          g[c][0] = ur;
-          g[c][1] = us;
-          g[c][2] = ut;
+          g[kk][c][0] = ur;
+          g[kk][c][1] = us;
+          g[kk][c][2] = ut;
         }
+      }
+#pragma unroll
+      for (int kk = 0; kk < KP; kk++) {
+        const int p = col + L2 * (k0 + kk);
         double cf[9];
 #pragma unroll
-        for (int a = 0; a < 9; a++) cf[a] = slot[(5 + a) * L3 + p];
-        const double dj = slot[3 * L3 + p] * sW3[p] * slot[4 * L3 + p];
+        for (int a = 0; a < 9; a++) cf[a] = planes[a * L3 + p];
+        const double dj = slot[3 * L3 + p] * __ldg(w3 + p) * slot[4 * L3 + p];
         double f[3][3];
-        stress_point(g, cf, dj, f);
+        stress_point(g[kk], cf, dj, f);
 #pragma unroll
         for (int c = 0; c < 3; c++)
 #pragma unroll
           for (int d = 0; d < 3; d++) planes[(3 * c + d) * L3 + p] = f[c][d];
       }
     }
-    __syncthreads();  // flux planes complete, stage s consumed
-    if (tid == 0 && t + S < nt) issue(t + S, s);
+    __syncthreads();  // flux planes complete
     if (act) {
-      // h2 B at this thread's points (the part2 term, folded in)
-      double hb[KP];
+      double Dxti[LX], Dytj[LX];  // dx(l, i), dy(l, j)
 #pragma unroll
-      for (int kk = 0; kk < KP; kk++) {
-        const long g = e * L3 + col + L2 * (k0 + kk);
-        hb[kk] = h2 ? __ldg(h2 + g) * __ldg(Bm + g) : 0.0;
+      for (int l = 0; l < LX; l++) {
+        Dxti[l] = __ldg(dx + l + LX * i);
+        Dytj[l] = __ldg(dy + l + LX * j);
       }
 #pragma unroll
       for (int c = 0; c < 3; c++) {
@@ -247,21 +265,32 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS, CG>::THREADS)
 #pragma unroll
         for (int kk = 0; kk < KP; kk++) {
           const int k = k0 + kk;
+          const double2 *row = reinterpret_cast<const double2 *>(fr + LX * j + L2 * k);
+          const double2 *dk = reinterpret_cast<const double2 *>(sDz + LX * k);
           double a = 0, cc = 0, d = 0;
 #pragma unroll
-          for (int l = 0; l < LX; l++) {
-            a += Dxti[l] * fr[l + LX * j + L2 * k];
+          for (int l = 0; l < LX; l += 2) {
+            const double2 v = row[l / 2], z = dk[l / 2];
+            a += Dxti[l] * v.x;
             cc += Dytj[l] * fs[i + LX * l + L2 * k];
-            d += sDz[l + LX * k] * rt[l];
+            d += z.x * rt[l];
+            a += Dxti[l + 1] * v.y;
+            cc += Dytj[l + 1] * fs[i + LX * (l + 1) + L2 * k];
+            d += z.y * rt[l + 1];
           }
+          const int q = col + L2 * k;
+          const double u = slot[c * L3 + q];
           double v = a + cc + d;
-          if (h2) v = v + hb[kk] * uown[c][kk];  // au + h2 B u, the part2 order
-          wo[e * L3 + col + L2 * k] = v;
-          if (CG) pap += uown[c][kk] * v;
+          if (h2) v = v + hb[kk] * u;  // au + h2 B u, the part2 order
+          wo[e * L3 + q] = v;
+          if (CG) pap += u * v;
         }
       }
     }
-    __syncthreads();  // flux planes free for the next element
+    // this thread's writes to the stage come before the next copy into it
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();  // stage s consumed
+    if (tid == 0 && t + S < nt) issue(t + S, s);
   }
   if (failed) {
     if (tid == 0) {
@@ -286,7 +315,7 @@ static cudaError_t launch_stress_tma(const StressIo &io, const StressGeo &geo, c
                                      const double *h2, const double *Bm, int nelv,
                                      cudaStream_t st, int *err, const int *skip,
                                      const StressCg &cg = StressCg{}) {
-  using C = StressCfg<LX, S, KS, CG>;
+  using C = StressCfg<LX, S, KS>;
   auto kern = ax_stress_tma_kernel<LX, S, KS, CG>;
   static int grid_per_dev[64] = {0};
   int dev = 0;
@@ -453,7 +482,7 @@ static cudaError_t launch_stress_gen(const StressIo &io, const StressGeo &geo, c
 }
 
 // (au, av, aw) = A_stress (u, v, w), h1 part.  The streaming kernel for lx
-// 4, 6, 8 with 16-byte aligned operands, the general kernel otherwise.
+// 4, 6, 8, 10 with 16-byte aligned operands, the general kernel otherwise.
 cudaError_t ax_stress(double *au, double *av, double *aw, const double *u, const double *v,
                       const double *w, const double *dx, const double *dy, const double *dz,
                       const double *h1, const double *jacinv, const double *const cof[9],
@@ -469,9 +498,10 @@ cudaError_t ax_stress(double *au, double *av, double *aw, const double *u, const
     if (reinterpret_cast<uintptr_t>(q) & 15) aligned = false;
   if (aligned) {
     switch (lx) {
-      case 4: return launch_stress_tma<4, 4, 4>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
-      case 6: return launch_stress_tma<6, 3, 3>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
-      case 8: return launch_stress_tma<8, 3, 4>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
+      case 4: return launch_stress_tma<4, 3, 4>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
+      case 6: return launch_stress_tma<6, 2, 3>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
+      case 8: return launch_stress_tma<8, 2, 4>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
+      case 10: return launch_stress_tma<10, 2, 5>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
       default: break;
     }
   }
@@ -679,9 +709,10 @@ cudaError_t problem_ax_stress_cg(nb_problem *P, double *const w[3], double *cons
     if (reinterpret_cast<uintptr_t>(q) & 15) return cudaErrorNotSupported;
   const double *h2 = P->ifh2 ? P->h2 : nullptr, *Bm = P->ifh2 ? P->B : nullptr;
   switch (P->lx) {
-    case 4: return launch_stress_tma<4, 4, 4, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
-    case 6: return launch_stress_tma<6, 3, 3, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
+    case 4: return launch_stress_tma<4, 3, 4, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
+    case 6: return launch_stress_tma<6, 2, 3, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
     case 8: return launch_stress_tma<8, 2, 4, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
+    case 10: return launch_stress_tma<10, 2, 5, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
     default: return cudaErrorNotSupported;
   }
 }

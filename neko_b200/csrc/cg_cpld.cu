@@ -13,11 +13,12 @@
 //
 // Differences in form: the scalars live on the device; z_c = M r_c and the
 // next iteration's rtz are formed in the pass that updates x and r; with the
-// full-stress operator on its streaming kernel (lx 4, 6, 8) the direction
+// full-stress operator on its streaming kernel (lx 4, 6, 8, 10) the direction
 // update p = z + beta p and the curvature (p, w) (summed over local points
 // before the gather-scatter: p is continuous and zero on masked points) are
-// part of the operator's pass, so an iteration is the operator, three
-// gather-scatters and the update; a chunk of iterations is one CUDA graph.
+// part of the operator's pass, so an iteration is the operator, one
+// gather-scatter of the three components and the update; a chunk of
+// iterations is one CUDA graph.
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -125,17 +126,27 @@ __global__ void __launch_bounds__(kRedThreads)
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
        i += (long)gridDim.x * kRedThreads) {
     double rr = 0.0, rz = 0.0;
+    // every operand before the first store (the compiler cannot tell the
+    // arrays apart): all of a point's loads are in flight together
+    const double m = MW(i), di = d ? d[i] : 1.0;
+    double xi[3], pi[3], ri[3], wi[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      x.c[c][i] = x.c[c][i] + alpha * p.c[c][i];
-      const double ri = r.c[c][i] + alphm * w.c[c][i];
-      r.c[c][i] = ri;
-      const double zi = d ? d[i] * ri : ri;
-      z.c[c][i] = zi;
-      rr = rr + ri * ri;
-      rz = rz + zi * ri;
+      xi[c] = x.c[c][i];
+      pi[c] = p.c[c][i];
+      ri[c] = r.c[c][i];
+      wi[c] = w.c[c][i];
     }
-    const double m = MW(i);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      x.c[c][i] = xi[c] + alpha * pi[c];
+      const double rn = ri[c] + alphm * wi[c];
+      r.c[c][i] = rn;
+      const double zi = d ? di * rn : rn;
+      z.c[c][i] = zi;
+      rr = rr + rn * rn;
+      rz = rz + zi * rn;
+    }
     s0 += rr * m;
     s1 += rz * m;
   }
@@ -219,8 +230,7 @@ static cudaError_t cpld_op(nb_problem *P, int op, const V3 &w, const V3 &p, cons
       e = ax_stress_part2(w.c[0], w.c[1], w.c[2], p.c[0], p.c[1], p.c[2], P->h2, P->B, P->n, s,
                           skip);
   }
-  for (int c = 0; c < 3 && e == cudaSuccess; c++)
-    e = gs_add_fused<double>(P->gsd, w.c[c], true, s, skip);
+  if (e == cudaSuccess) e = gs_add_fused3(P->gsd, w.c[0], w.c[1], w.c[2], true, s, skip);
   return e;
 }
 
@@ -284,8 +294,7 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
               : cudaErrorNotSupported;
       if (fe == cudaSuccess) {
         fused = true;
-        for (int c = 0; c < 3 && ce == cudaSuccess; c++)
-          ce = gs_add_fused<double>(P->gsd, w.c[c], true, cs, &W.st->done);
+        ce = gs_add_fused3(P->gsd, w.c[0], w.c[1], w.c[2], true, cs, &W.st->done);
       } else if (fe != cudaErrorNotSupported) {
         ce = fe;
         break;
@@ -305,9 +314,10 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
     }
     // the operator: one launch, plus a separate h2 launch except on the
     // full-stress streaming kernel, which folds the h2 term in
-    const bool h2_folded = op == NB_AX_STRESS && (P->lx == 4 || P->lx == 6 || P->lx == 8);
+    const bool h2_folded =
+        op == NB_AX_STRESS && (P->lx == 4 || P->lx == 6 || P->lx == 8 || P->lx == 10);
     const int op_launches = 1 + (P->ifh2 && !h2_folded ? 1 : 0);
-    W.launches_per_iter = fused ? 1 + 3 + 1 : 1 + op_launches + 3 + 2;
+    W.launches_per_iter = fused ? 1 + 1 + 1 : 1 + op_launches + 1 + 2;
     cudaError_t ee = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
     if (ce != cudaSuccess) {

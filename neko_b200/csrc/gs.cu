@@ -92,9 +92,15 @@ __global__ void scatter_ref_kernel(const double *__restrict__ v, int m,
 // step: after step k the lane at position k holds ((u0 + u1) + ...) + uk,
 // the sequential sum of the reference's gather, so the segment's last lane
 // holds the total, which every lane of the segment then reads.
-template <typename T, int CPW>
-__global__ void __launch_bounds__(256) gs_add_warp_kernel(T *__restrict__ u, const GsDevice g,
-                                                          bool with_mask,
+// NC vectors share one pass over the index lists (the three components of a
+// velocity): one launch and one read of the indices instead of three.
+template <typename T, int NC>
+struct GsVec {
+  T *c[NC];
+};
+template <typename T, int CPW, int NC>
+__global__ void __launch_bounds__(256) gs_add_warp_kernel(const GsVec<T, NC> vec,
+                                                          const GsDevice g, bool with_mask,
                                                           const int *__restrict__ skip,
                                                           const T *__restrict__ scale) {
   if (skip && *skip) return;
@@ -105,7 +111,7 @@ __global__ void __launch_bounds__(256) gs_add_warp_kernel(T *__restrict__ u, con
     const long c0 = (t >> 5) * CPW;
     int idx[CPW];
     unsigned head[CPW];
-    T v[CPW];
+    T v[CPW][NC];
 #pragma unroll
     for (int j = 0; j < CPW; j++) {
       const bool ok = c0 + j < g.nchunk;  // uniform over the warp
@@ -113,7 +119,9 @@ __global__ void __launch_bounds__(256) gs_add_warp_kernel(T *__restrict__ u, con
       head[j] = ok ? __ldg(g.lane_head + c0 + j) : 0xffffffffu;
     }
 #pragma unroll
-    for (int j = 0; j < CPW; j++) v[j] = idx[j] >= 0 ? u[idx[j]] : T(0);
+    for (int j = 0; j < CPW; j++)
+#pragma unroll
+      for (int c = 0; c < NC; c++) v[j][c] = idx[j] >= 0 ? vec.c[c][idx[j]] : T(0);
     const unsigned upto = 0xffffffffu >> (31 - lane);  // bits 0..lane
 #pragma unroll
     for (int j = 0; j < CPW; j++) {
@@ -122,19 +130,28 @@ __global__ void __launch_bounds__(256) gs_add_warp_kernel(T *__restrict__ u, con
       const unsigned above = head[j] & ~upto;         // heads after this lane
       const int last = above ? __ffs(above) - 2 : 31; // last lane of the segment
       const int steps = (int)__reduce_max_sync(0xffffffffu, (unsigned)pos);
-      T acc = v[j];
+      T acc[NC];
+#pragma unroll
+      for (int c = 0; c < NC; c++) acc[c] = v[j][c];
       for (int k = 1; k <= steps; k++) {
-        const T up = __shfl_up_sync(0xffffffffu, acc, 1);
-        if (pos == k) acc = up + v[j];
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+          const T up = __shfl_up_sync(0xffffffffu, acc[c], 1);
+          if (pos == k) acc[c] = up + v[j][c];
+        }
       }
-      v[j] = __shfl_sync(0xffffffffu, acc, last);
+#pragma unroll
+      for (int c = 0; c < NC; c++) v[j][c] = __shfl_sync(0xffffffffu, acc[c], last);
     }
 #pragma unroll
     for (int j = 0; j < CPW; j++) {
       if (idx[j] < 0) continue;
-      T s = v[j];
-      if (with_mask && ((__ldg(g.lane_zero + c0 + j) >> lane) & 1u)) s = T(0);
-      u[idx[j]] = scale ? s * scale[idx[j]] : s;
+      const bool zero = with_mask && ((__ldg(g.lane_zero + c0 + j) >> lane) & 1u);
+#pragma unroll
+      for (int c = 0; c < NC; c++) {
+        const T s = zero ? T(0) : v[j][c];
+        vec.c[c][idx[j]] = scale ? s * scale[idx[j]] : s;
+      }
     }
     return;
   }
@@ -142,26 +159,32 @@ __global__ void __launch_bounds__(256) gs_add_warp_kernel(T *__restrict__ u, con
   if (q < g.nlong) {
     const int sg = __ldg(g.seg_long + q);
     const int a = __ldg(g.seg_ptr + sg), b = __ldg(g.seg_ptr + sg + 1);
-    T s = u[__ldg(g.seg_idx + a)];
-    for (int k = a + 1; k < b; k++) s = s + u[__ldg(g.seg_idx + k)];
-    if (with_mask && g.seg_masked && g.seg_masked[sg]) s = T(0);
-    for (int k = a; k < b; k++) {
-      const int i = __ldg(g.seg_idx + k);
-      u[i] = scale ? s * scale[i] : s;
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      T *u = vec.c[c];
+      T s = u[__ldg(g.seg_idx + a)];
+      for (int k = a + 1; k < b; k++) s = s + u[__ldg(g.seg_idx + k)];
+      if (with_mask && g.seg_masked && g.seg_masked[sg]) s = T(0);
+      for (int k = a; k < b; k++) {
+        const int i = __ldg(g.seg_idx + k);
+        u[i] = scale ? s * scale[i] : s;
+      }
     }
     return;
   }
   q -= g.nlong;
-  if (with_mask && q < g.nextra) u[__ldg(g.extra_mask + q)] = T(0);
+  if (with_mask && q < g.nextra)
+#pragma unroll
+    for (int c = 0; c < NC; c++) vec.c[c][__ldg(g.extra_mask + q)] = T(0);
 }
 
-template <typename T, int CPW>
-static void launch_warp_form(const GsDevice &g, T *u, bool with_mask, cudaStream_t s,
+template <typename T, int CPW, int NC>
+static void launch_warp_form(const GsDevice &g, const GsVec<T, NC> &u, bool with_mask, cudaStream_t s,
                              const int *skip, const T *scale) {
   const long total = 32L * ((g.nchunk + CPW - 1) / CPW) + g.nlong + (with_mask ? g.nextra : 0);
   const int threads = 256;
   const int blocks = (int)((total + threads - 1) / threads);
-  gs_add_warp_kernel<T, CPW><<<blocks, threads, 0, s>>>(u, g, with_mask, skip, scale);
+  gs_add_warp_kernel<T, CPW, NC><<<blocks, threads, 0, s>>>(u, g, with_mask, skip, scale);
 }
 
 template <typename T>
@@ -170,7 +193,15 @@ cudaError_t gs_add_fused(const GsDevice &g, T *u, bool with_mask, cudaStream_t s
   if (g.nchunk == 0 && g.nlong == 0 && (!with_mask || g.nextra == 0)) return cudaSuccess;
   // four chunks a warp: 70 us against 80 (two) and 77 (eight) for the
   // 9.7 M entries of a 32^3-element box at lx = 8
-  launch_warp_form<T, 4>(g, u, with_mask, s, skip, scale);
+  launch_warp_form<T, 4, 1>(g, GsVec<T, 1>{{u}}, with_mask, s, skip, scale);
+  return cudaGetLastError();
+}
+
+// Two chunks a warp: six scattered loads in flight a thread.
+cudaError_t gs_add_fused3(const GsDevice &g, double *u0, double *u1, double *u2, bool with_mask,
+                          cudaStream_t s, const int *skip) {
+  if (g.nchunk == 0 && g.nlong == 0 && (!with_mask || g.nextra == 0)) return cudaSuccess;
+  launch_warp_form<double, 2, 3>(g, GsVec<double, 3>{{u0, u1, u2}}, with_mask, s, skip, nullptr);
   return cudaGetLastError();
 }
 template cudaError_t gs_add_fused<double>(const GsDevice &, double *, bool, cudaStream_t,

@@ -50,5 +50,8 @@ bool gs_pairs_regular(const GsMaps &m);
 template <typename T>
 cudaError_t gs_add_fused(const GsDevice &g, T *u, bool with_mask, cudaStream_t s,
                          const int *skip = nullptr, const T *scale = nullptr);
+// The same on three vectors in one launch (no scale): each sum as above.
+cudaError_t gs_add_fused3(const GsDevice &g, double *u0, double *u1, double *u2, bool with_mask,
+                          cudaStream_t s, const int *skip = nullptr);
 
 }  // namespace nb
