@@ -15,15 +15,22 @@
 //   p = z + beta p | w = A p, (p, w) | x += alpha p, r -= alpha w, z = d r,
 //                                      (r, r), (r, z) |
 //
-// with three barriers (|).  The whole solve is one thread-block cluster (up
-// to 16 blocks on one GPC): its barriers are hardware barriers, and its
-// sums travel through distributed shared memory.  The vectors of a row stay
-// in the registers of the thread that owns it, the matrix in the shared
-// memory of its block when it fits.  A solve on 4096 vertices took 124 us as
-// a cooperative grid with barriers in global memory and element-local
-// vectors (33 barriers of about 3.7 us with their sums).  A cluster leaves the
-// other multiprocessors to the fine-level smoother, which runs beside it;
-// the grid form held one block on every one.
+// between barriers (|).  The whole solve is one thread-block cluster (up to
+// 16 blocks on one GPC): its barriers are hardware barriers, and its sums
+// travel through distributed shared memory, every warp's partial straight to
+// every block.  The vectors of a row stay in the registers of the thread that
+// owns it, the matrix in the shared memory of its block when it fits.  Up to
+// 8192 vertices each block also holds all of z and p in shared memory: a
+// thread sends its z to every block before the barrier of the sums, and each
+// block forms p for itself, which leaves two cluster barriers an iteration
+// and gathers that never leave the block.  Beyond, p is exchanged through
+// global memory at the price of a third barrier.
+//
+// A solve on 343 vertices (8^3 elements) took 124 us as a cooperative grid
+// with barriers in global memory and element-local vectors (33 barriers of
+// about 3.7 us with their sums), 67 us with p in global memory.
+// A cluster leaves the other multiprocessors to the fine-level smoother,
+// which runs beside it; the grid form held one block on every one.
 //
 // The arithmetic is that of cg_init / cg_precond_dot / cg_update_p /
 // ax_helm / gs / cg_update_xr with sums over distinct points: a mult-weighted
@@ -32,6 +39,7 @@
 #include <cmath>
 #include <string>
 
+#include "nb_cluster.cuh"
 #include "nb_nodes.h"
 #include "nb_precond.h"
 #include "nb_reduce.cuh"
@@ -39,77 +47,17 @@
 
 namespace nb {
 
-constexpr int kCoarseThreads = 512;
-constexpr int kCoarseWarps = kCoarseThreads / 32;
-constexpr int kMaxCluster = 16;
 // rows a block aims at when the cluster grows: below, the block's own work is
 // shorter than a larger cluster's barrier
-constexpr int kCoarseRowsPerBlock = 256;
-// shared memory a block may spend on its part of the matrix
-constexpr size_t kCoarseStageBytes = 160 * 1024;
-
-__device__ __forceinline__ unsigned cluster_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// All threads of the cluster; orders their global and shared writes.
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
-                   : "memory");
-}
-// *p = v in the shared memory of block `rank` of the cluster (p: this
-// block's address of the variable).
-__device__ __forceinline__ void cluster_store(double *p, unsigned rank, double v) {
-  unsigned a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-
-// Two sums over the cluster, identical in every thread: block sums, sent to
-// every block's slot of this block, a barrier, then each warp adds the slots
-// in one fixed tree.  Consecutive calls alternate `slots`.
-struct ClusterSums {
-  double slot[2][kMaxCluster][2];
-  double warp[kCoarseWarps][2];
-};
-__device__ __forceinline__ void cluster_allsum2(double v0, double v1, ClusterSums &sm, int buf,
-                                                unsigned rank, unsigned nblk, double &t0,
-                                                double &t1) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  v0 = warp_sum(v0);
-  v1 = warp_sum(v1);
-  if (lane == 0) {
-    sm.warp[wid][0] = v0;
-    sm.warp[wid][1] = v1;
-  }
-  __syncthreads();
-  if (wid == 0) {
-    v0 = lane < kCoarseWarps ? sm.warp[lane][0] : 0.0;
-    v1 = lane < kCoarseWarps ? sm.warp[lane][1] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-      v1 += __shfl_xor_sync(0xffffffffu, v1, o);
-    }
-    if (lane < (int)nblk) {
-      cluster_store(&sm.slot[buf][rank][0], lane, v0);
-      cluster_store(&sm.slot[buf][rank][1], lane, v1);
-    }
-  }
-  cluster_barrier();
-  t0 = lane < (int)nblk ? sm.slot[buf][lane][0] : 0.0;
-  t1 = lane < (int)nblk ? sm.slot[buf][lane][1] : 0.0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    t0 += __shfl_xor_sync(0xffffffffu, t0, o);
-    t1 += __shfl_xor_sync(0xffffffffu, t1, o);
-  }
-}
+constexpr int kCoarseRowsPerBlock = 128;
+// shared memory a block may spend on its part of the matrix and the vectors
+constexpr size_t kCoarseStageBytes = 200 * 1024;
+static_assert(kMaxCluster * kCoarseThreads * 2 * sizeof(double) <= kCoarseStageBytes,
+              "z and p of the resident form fit");
 
 // f(o,p,r) = sum_k J(k,r) sum_j J(j,p) sum_i J(i,o) (w mult)(i,j,k) per
 // element, in T and in the order of tensor3_kernel (x, then y, then z); one
-// thread a vertex of an element.
+// thread a vertex of an element, 32 elements a block.
 template <typename T, int LM>
 __global__ void __launch_bounds__(256)
     coarse_restrict_kernel(const T *__restrict__ w_mid, const T *__restrict__ mult_m,
@@ -117,14 +65,34 @@ __global__ void __launch_bounds__(256)
                            const int *__restrict__ skip) {
   if (skip && *skip) return;
   constexpr int M3 = LM * LM * LM;
+  constexpr int NE = 32;  // elements a block: its products read once, coalesced
   __shared__ T sJ[LM * 2];  // J(m, c) at m + LM c
-  if (threadIdx.x < LM * 2) sJ[threadIdx.x] = J[threadIdx.x];
+  __shared__ T sw[NE * M3 + NE];  // pitch M3 + 1
+  const int tid = threadIdx.x;
+  if (tid < LM * 2) sJ[tid] = J[tid];
+  const long e0 = (long)blockIdx.x * NE;
+  {
+    const long base = e0 * M3, left = (nc >> 3) * M3 - base;
+    constexpr int R = NE * M3 / 256 + (NE * M3 % 256 != 0);
+    T a[R], b[R];
+#pragma unroll
+    for (int g = 0; g < R; g++) {
+      const int q = tid + 256 * g;
+      const bool ok = q < NE * M3 && q < left;
+      a[g] = ok ? __ldg(w_mid + base + q) : T(0);
+      b[g] = ok ? __ldg(mult_m + base + q) : T(0);
+    }
+#pragma unroll
+    for (int g = 0; g < R; g++) {
+      const int q = tid + 256 * g;
+      if (q < NE * M3) sw[q + q / M3] = a[g] * b[g];
+    }
+  }
   __syncthreads();
-  const long q = blockIdx.x * 256L + threadIdx.x;
+  const long q = blockIdx.x * 256L + tid;
   if (q >= nc) return;
-  const long e = q >> 3;
   const int o = q & 1, pp = (q >> 1) & 1, rr = (q >> 2) & 1;
-  const T *in = w_mid + e * M3, *sc = mult_m + e * M3;
+  const T *in = sw + (tid >> 3) * (M3 + 1);
   T acc_z = 0;
 #pragma unroll
   for (int k = 0; k < LM; k++) {
@@ -133,10 +101,7 @@ __global__ void __launch_bounds__(256)
     for (int j = 0; j < LM; j++) {
       T acc_x = 0;
 #pragma unroll
-      for (int i = 0; i < LM; i++) {
-        const int m = i + LM * (j + LM * k);
-        acc_x += sJ[i + LM * o] * (T)(__ldg(in + m) * __ldg(sc + m));
-      }
+      for (int i = 0; i < LM; i++) acc_x += sJ[i + LM * o] * in[i + LM * (j + LM * k)];
       acc_y += sJ[j + LM * pp] * acc_x;
     }
     acc_z += sJ[k + LM * rr] * acc_y;
@@ -144,9 +109,112 @@ __global__ void __launch_bounds__(256)
   f[q] = (double)acc_z;
 }
 
-// niter Jacobi-CG iterations (or to the absolute tolerance) of A x = f from
-// zero, f the sum of the element-local `a.f` over a node's copies.  Warp t
-// of the cluster takes matrix slices t, t + warps, ...; with RPT > 0 a thread
+// sum of the element-local right-hand side over a node's copies, in order
+__device__ __forceinline__ double node_rhs(const NodeOp &A, const double *__restrict__ f,
+                                           int row) {
+  const int k0 = __ldg(A.eptr + row), k1 = __ldg(A.eptr + row + 1);
+  double acc = 0.0;
+  for (int k = k0; k < k1; k += 8) {  // eight copies at a time, loads in flight together
+    int q[8];
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) q[u] = k + u < k1 ? __ldg(A.ent + k + u) : -1;
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = q[u] >= 0 ? f[q[u]] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) acc += v[u];
+  }
+  return acc;
+}
+
+// one slice of the matrix to shared memory
+__device__ __forceinline__ void stage_slice(const NodeOp &A, int s, double *val, int *col,
+                                            int lane) {
+  const int o = __ldg(A.soff + s), w = __ldg(A.soff + s + 1) - o;
+  const double *gv = A.val + 32 * (size_t)o + lane;
+  const int *gc = A.col + 32 * (size_t)o + lane;
+#pragma unroll 9
+  for (int k = 0; k < w; k++) {
+    val[32 * k + lane] = __ldg(gv + 32 * k);
+    col[32 * k + lane] = __ldg(gc + 32 * k);
+  }
+}
+
+// The solve with at most one row a thread (8192 vertices): all of z and p in
+// every block's shared memory.
+__global__ void __launch_bounds__(kCoarseThreads) coarse_cg_resident_kernel(const CoarseCg a) {
+  if (a.skip && *a.skip) return;
+  extern __shared__ __align__(16) unsigned char coarse_smem[];
+  __shared__ ClusterSums sums;
+  const NodeOp &A = a.A;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const unsigned rank = cluster_rank(), nblk = gridDim.x;
+  const int s = wid * (int)nblk + (int)rank, row = 32 * s + lane;
+  const bool own = s < A.ns && row < A.nn;
+  double *zf = reinterpret_cast<double *>(coarse_smem), *pf = zf + A.nn;
+  double *sval = pf + A.nn;
+  int *scol = reinterpret_cast<int *>(sval + (size_t)a.stage_slices * A.maxw * 32);
+  const double *val = nullptr;
+  const int *col = nullptr;
+  int width = 0;
+  if (s < A.ns) {
+    const int o = __ldg(A.soff + s);
+    width = __ldg(A.soff + s + 1) - o;
+    val = A.val + 32 * (size_t)o + lane;
+    col = A.col + 32 * (size_t)o + lane;
+    if (a.stage_slices > 0) {
+      const size_t to = (size_t)wid * A.maxw * 32;
+      stage_slice(A, s, sval + to, scol + to, lane);
+      val = sval + to + lane;
+      col = scol + to + lane;
+    }
+  }
+  for (int i = tid; i < A.nn; i += kCoarseThreads) pf[i] = 0.0;
+  double x = 0.0, r = own ? node_rhs(A, a.f, row) : 0.0;
+  const double d = own ? __ldg(A.dinv + row) : 0.0;
+  double z = d * r;
+  cluster_barrier();  // every block runs before its shared memory is written to
+  auto send_z = [&] {
+    if (own)
+      for (unsigned b = 0; b < nblk; b++) cluster_store(zf + row, b, z);
+  };
+  send_z();
+  double rtr, rtz;
+  cluster_allsum2(r * r, r * z, sums, 0, rank, nblk, rtr, rtz);
+  double rn = sqrt(rtr) * a.norm_fac;
+  bool done = fabs(rn) < 2.220446049250313e-16;
+  int iter = 0;
+  double rtz_old = 1.0;
+  while (!done) {
+    const double beta = iter == 0 ? 0.0 : rtz / rtz_old;
+    for (int i = tid; i < A.nn; i += kCoarseThreads) pf[i] = zf[i] + beta * pf[i];
+    __syncthreads();
+    double w = 0.0, p = 0.0;
+    if (own) {
+      w = row_dot(val, col, width, [&](int c) { return pf[c]; });
+      p = pf[row];
+    }
+    double pap, unused;
+    cluster_allsum2(p * w, 0.0, sums, 1, rank, nblk, pap, unused);
+    const double alpha = rtz / pap, malpha = -alpha;
+    x = x + alpha * p;
+    r = r + malpha * w;
+    z = d * r;
+    if (!own) r = z = 0.0;  // a NaN alpha stays with the rows
+    send_z();
+    double rtz_new;
+    cluster_allsum2(r * r, r * z, sums, 0, rank, nblk, rtr, rtz_new);
+    rtz_old = rtz;
+    rtz = rtz_new;
+    rn = sqrt(rtr) * a.norm_fac;
+    iter += 1;
+    done = !(rn == rn) || isinf(rn) || rn < a.tol || iter >= a.niter;
+  }
+  if (own) a.x[row] = x;
+}
+
+// The solve on more vertices: p exchanged through global memory.  Warp t of
+// the cluster takes matrix slices t, t + warps, ...; with RPT > 0 a thread
 // owns at most RPT rows and keeps their vectors in registers, with RPT = 0
 // (more rows than that) they are kept in global memory.
 template <int RPT>
@@ -190,33 +258,18 @@ __global__ void __launch_bounds__(kCoarseThreads)
   if (a.stage_slices > 0) {
     int j = 0;
     for (int s = first; s < A.ns; s += warps, j++) {
-      const int o = __ldg(A.soff + s), w = __ldg(A.soff + s + 1) - o;
-      const size_t to = (size_t)(j * kCoarseWarps + wid) * A.maxw * 32 + lane;
-      for (int k = 0; k < w; k++) {
-        sval[to + 32 * k] = __ldg(A.val + 32 * ((size_t)o + k) + lane);
-        scol[to + 32 * k] = __ldg(A.col + 32 * ((size_t)o + k) + lane);
-      }
+      const size_t to = (size_t)(j * kCoarseWarps + wid) * A.maxw * 32;
+      stage_slice(A, s, sval + to, scol + to, lane);
     }
     __syncwarp();
   }
-  // (A p)(row) of slice s, the j-th of this warp: nine entries at a time (a
-  // third of a box row), their vector values in flight together
+  // (A p)(row) of slice s, the j-th of this warp
   auto matvec = [&](int j, int s) {
     const int o = __ldg(A.soff + s), w = __ldg(A.soff + s + 1) - o;
     const size_t st = (size_t)(j * kCoarseWarps + wid) * A.maxw * 32 + lane;
     const double *val = a.stage_slices > 0 ? sval + st : A.val + 32 * (size_t)o + lane;
     const int *col = a.stage_slices > 0 ? scol + st : A.col + 32 * (size_t)o + lane;
-    double acc = 0.0;
-    int k = 0;
-    for (; k + 9 <= w; k += 9) {
-      double v[9];
-#pragma unroll
-      for (int u = 0; u < 9; u++) v[u] = __ldcg(a.p + col[32 * (k + u)]);
-#pragma unroll
-      for (int u = 0; u < 9; u++) acc += val[32 * (k + u)] * v[u];
-    }
-    for (; k < w; k++) acc += val[32 * k] * __ldcg(a.p + col[32 * k]);
-    return acc;
+    return row_dot(val, col, w, [&](int c) { return __ldcg(a.p + c); });
   };
 
   // x = 0, r = f, z = d r, p = 0; (r, r), (r, z)
@@ -232,11 +285,8 @@ __global__ void __launch_bounds__(kCoarseThreads)
     }
   }
   rows([&](int, int, int row, double &xv, double &rv, double &zv, double &pv, double &dv) {
-    double f = 0.0;
-    for (int k = __ldg(A.eptr + row); k < __ldg(A.eptr + row + 1); k++)
-      f += a.f[__ldg(A.ent + k)];
     xv = 0.0;
-    rv = f;
+    rv = node_rhs(A, a.f, row);
     pv = 0.0;
     if (RPT > 0) dv = __ldg(A.dinv + row);
     zv = dv * rv;
@@ -297,61 +347,6 @@ __global__ void __launch_bounds__(kCoarseThreads)
     });
 }
 
-// Blocks of the largest cluster the device takes for this kernel: 16 (one
-// GPC, an opt-in size) where it is accepted, else the portable 8.
-template <int RPT>
-static cudaError_t cluster_limit(int &limit) {
-  static int known[64] = {0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  int &k = known[dev & 63];
-  if (k == 0) {
-    auto kern = coarse_cg_kernel<RPT>;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kCoarseStageBytes)) != cudaSuccess)
-      return e;
-    k = 8;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-        cudaSuccess) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(kMaxCluster);
-      cfg.blockDim = dim3(kCoarseThreads);
-      cfg.dynamicSmemBytes = kCoarseStageBytes;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = kMaxCluster;
-      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1) k = kMaxCluster;
-    }
-    cudaGetLastError();  // a refused cluster size is not an error of the caller
-  }
-  limit = k;
-  return cudaSuccess;
-}
-
-template <int RPT>
-static cudaError_t launch_cg(CoarseCg a, int nblk, cudaStream_t s) {
-  const int warps = kCoarseWarps * nblk, per_warp = (a.A.ns + warps - 1) / warps;
-  const size_t bytes = (size_t)per_warp * kCoarseWarps * a.A.maxw * 32 * (sizeof(double) + sizeof(int));
-  a.stage_slices = bytes <= kCoarseStageBytes ? per_warp * kCoarseWarps : 0;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)nblk);
-  cfg.blockDim = dim3(kCoarseThreads);
-  cfg.dynamicSmemBytes = a.stage_slices ? bytes : 0;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)nblk;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, coarse_cg_kernel<RPT>, a);
-}
-
 template <typename T>
 cudaError_t hsmg_coarse_restrict(const CoarseArgs<T> &a, int lm, const int *skip,
                                  cudaStream_t s) {
@@ -375,24 +370,35 @@ template cudaError_t hsmg_coarse_restrict<float>(const CoarseArgs<float> &, int,
 
 cudaError_t hsmg_coarse_cg(const CoarseCg &a, const int *skip, cudaStream_t s) {
   if (a.A.nn == 0) return cudaSuccess;  // every vertex masked: no correction
-  CoarseCg b = a;
-  b.skip = skip;
-  int limit = 0;
-  cudaError_t e = cluster_limit<1>(limit);
-  if (e != cudaSuccess) return e;
-  int nblk = 1;
-  while (nblk < limit && nblk * kCoarseRowsPerBlock < a.A.nn) nblk *= 2;
-  const int per_thread = (a.A.ns + kCoarseWarps * nblk - 1) / (kCoarseWarps * nblk);
-  if (per_thread <= 1) return launch_cg<1>(b, nblk, s);
-  if (per_thread <= 2) {
-    if ((e = cluster_limit<2>(limit)) != cudaSuccess) return e;
-    if (nblk <= limit) return launch_cg<2>(b, nblk, s);
-  } else if (per_thread <= 4) {
-    if ((e = cluster_limit<4>(limit)) != cudaSuccess) return e;
-    if (nblk <= limit) return launch_cg<4>(b, nblk, s);
+  // resident form (one row a thread), two, four rows a thread, any number
+  constexpr int kForms = 4;
+  using CoarseKernel = void (*)(CoarseCg);
+  static const CoarseKernel kernels[kForms] = {coarse_cg_resident_kernel, coarse_cg_kernel<2>,
+                                               coarse_cg_kernel<4>, coarse_cg_kernel<0>};
+  static const int rows[kForms] = {1, 2, 4, 0};
+  static int known[kForms][64];
+  const NodeOp &A = a.A;
+  const size_t slice = (size_t)A.maxw * 32 * (sizeof(double) + sizeof(int));
+  for (int v = 0; v < kForms; v++) {
+    int limit = 0, nblk = 1;
+    cudaError_t e = cluster_limit(kernels[v], kCoarseStageBytes, known[v], limit);
+    if (e != cudaSuccess) return e;
+    while (nblk < limit && nblk * kCoarseRowsPerBlock < A.nn) nblk *= 2;
+    const int per_block = (A.ns + nblk - 1) / nblk;
+    const int per_warp = (per_block + kCoarseWarps - 1) / kCoarseWarps;
+    if (rows[v] > 0 && per_warp > rows[v]) continue;
+    const size_t vectors = v == 0 ? 2 * (size_t)A.nn * sizeof(double) : 0;
+    CoarseCg b = a;
+    b.skip = skip;
+    // slices at a common pitch, warp by warp
+    const int staged = per_warp > 1 ? per_warp * kCoarseWarps : per_block;
+    b.stage_slices = vectors + staged * slice <= kCoarseStageBytes ? staged : 0;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    cluster_config(cfg, at, nblk, vectors + b.stage_slices * slice, s);
+    return cudaLaunchKernelEx(&cfg, kernels[v], b);
   }
-  if ((e = cluster_limit<0>(limit)) != cudaSuccess) return e;
-  return launch_cg<0>(b, nblk < limit ? nblk : limit, s);
+  return cudaErrorNotSupported;
 }
 
 }  // namespace nb

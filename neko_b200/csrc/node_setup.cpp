@@ -45,37 +45,38 @@ void node_setup(const GsMaps &maps, long n, const std::vector<int> &masked, Node
   H.slot.assign(8 * H.ent.size(), -1);
   H.soff.assign(1, 0);
   H.col.clear();
+  H.col.reserve(27 * (size_t)nn + 27 * 32);
   H.maxw = 0;
-  std::vector<std::vector<int>> rows(32);
+  // columns of a row in order of first appearance over its copies' corners;
+  // at[v] is the position of node v in the row that stamped it last
+  std::vector<int> at(nn), stamp(nn, -1), rows[32];
   for (int r0 = 0; r0 < nn; r0 += 32) {
     int width = 0;
     for (int l = 0; l < 32; l++) {
       std::vector<int> &c = rows[l];
       c.clear();
-      if (r0 + l >= nn) continue;
-      for (int k = H.eptr[r0 + l]; k < H.eptr[r0 + l + 1]; k++)
+      const int r = r0 + l;
+      if (r >= nn) continue;
+      for (int k = H.eptr[r]; k < H.eptr[r + 1]; k++)
         for (int b = 0; b < 8; b++) {
           const int v = H.node_of[(H.ent[k] & ~7) + b];
-          if (v >= 0) c.push_back(v);
+          if (v < 0) continue;
+          if (stamp[v] != r) {
+            stamp[v] = r;
+            at[v] = (int)c.size();
+            c.push_back(v);
+          }
+          H.slot[8 * (size_t)k + b] = at[v];
         }
-      std::sort(c.begin(), c.end());
-      c.erase(std::unique(c.begin(), c.end()), c.end());
       width = std::max(width, (int)c.size());
-      for (int k = H.eptr[r0 + l]; k < H.eptr[r0 + l + 1]; k++)
-        for (int b = 0; b < 8; b++) {
-          const int v = H.node_of[(H.ent[k] & ~7) + b];
-          if (v >= 0)
-            H.slot[8 * (size_t)k + b] =
-                (int)(std::lower_bound(c.begin(), c.end(), v) - c.begin());
-        }
     }
     const size_t base = H.col.size();
     H.col.resize(base + 32 * (size_t)width);
-    for (int l = 0; l < 32; l++)
+    for (int l = 0; l < 32; l++) {
+      const int own = std::min(r0 + l, nn - 1);
       for (int k = 0; k < width; k++)
-        H.col[base + 32 * (size_t)k + l] = k < (int)rows[l].size()
-                                               ? rows[l][k]
-                                               : std::min(r0 + l, nn - 1);
+        H.col[base + 32 * (size_t)k + l] = k < (int)rows[l].size() ? rows[l][k] : own;
+    }
     H.soff.push_back(H.soff.back() + width);
     H.maxw = std::max(H.maxw, width);
   }

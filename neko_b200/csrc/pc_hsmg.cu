@@ -853,7 +853,7 @@ struct HsmgImpl : public HsmgState {
                        const PrologDots *dots = nullptr) {
     cudaError_t e;
     const long nelv = fine->nelv;
-    if ((e = ensure_side()) != cudaSuccess || (e = cudaEventRecord(ev_fork, s)) != cudaSuccess ||
+    if ((e = cudaEventRecord(ev_fork, s)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(crs_s, ev_fork, 0)) != cudaSuccess)
       return e;
     // restrict (r * mult) to the middle level, assemble, mask: w; restrict
@@ -1194,7 +1194,7 @@ nb_status hsmg_get(nb_problem *P, const nb_solve_opts &o, Precond **out) {
              : upload_impl((HsmgImpl<double> *)H, hf, hm, Jfm, Jmc, ornt);
   // The uploads ran on the legacy stream (a pageable cudaMemcpy may return
   // before its DMA lands); finish them before any caller stream reads them.
-  if (st == NB_OK && cudaDeviceSynchronize() != cudaSuccess)
+  if (st == NB_OK && (cudaDeviceSynchronize() != cudaSuccess || H->ensure_side() != cudaSuccess))
     st = hfail(NB_ERR_CUDA, "hsmg: upload failed");
   if (st != NB_OK) {
     delete H;

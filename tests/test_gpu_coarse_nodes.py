@@ -1,7 +1,8 @@
 """The hsmg coarse solve over distinct vertices, at the sizes where its
-launch changes form: no unmasked vertex at all, one block, a cluster, two
-and four rows a thread, the matrix no longer in shared memory, and more rows
-than the registers hold.  One application against the CPU oracle with the
+launch changes form: no unmasked vertex at all, one block, clusters with the
+vectors resident in every block, two and four rows a thread with the vectors
+in global memory, the matrix no longer in shared memory, and more rows than
+the registers hold.  One application against the CPU oracle with the
 bounds of test_gpu_hsmg.py (lx 4 keeps the other levels small)."""
 import numpy as np
 import pytest
@@ -14,8 +15,8 @@ pytestmark = pytest.mark.gpu
 #        elements       periodic              vertices
 NODES = [((1, 1, 1), (False,) * 3),         # 0
          ((2, 2, 2), (False,) * 3),         # 1
-         ((9, 7, 8), (False,) * 3),         # 336: two blocks
-         ((17, 16, 18), (False,) * 3),      # 4080: sixteen blocks, staged
+         ((9, 7, 8), (False,) * 3),         # 336: four blocks
+         ((17, 16, 18), (False,) * 3),      # 4080: sixteen blocks
          ((21, 20, 22), (True, False, True)),   # 8778: two rows a thread
          ((26, 25, 27), (False,) * 3),      # 15600
          ((28, 28, 27), (True, False, False)),  # 19656: four rows a thread
