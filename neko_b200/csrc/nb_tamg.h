@@ -1,0 +1,32 @@
+// nb_tamg.h -- operands of the tree-AMG cycle launch (tamg_cluster.cu).
+#pragma once
+
+#include "nb_nodes.h"
+
+namespace nb {
+
+// Level 0: the distinct vertices.  Level l >= 1: one entry an aggregate.
+struct TamgClusterLevel {
+  int n = 0;
+  const int *agg = nullptr;                   // l >= 2: element -> aggregate (l = 1: itself)
+  const int *sptr = nullptr, *sidx = nullptr; // l >= 1: aggregate -> vertices of its points (-1 masked)
+  const int *rptr = nullptr, *ridx = nullptr; // l >= 2: aggregate -> entries of level l - 1
+  const int *spread = nullptr;                // l >= 2: entry of level l - 1 -> aggregate
+  double *x = nullptr, *b = nullptr, *r = nullptr, *d[2] = {nullptr, nullptr};
+  double tha = 0.0, dlt = 0.0;
+};
+struct TamgCluster {
+  NodeOp A;
+  const double *mean = nullptr;       // 1 / copies of each vertex
+  const TamgClusterLevel *lv = nullptr;  // device array of nlvls
+  int nlvls = 0, degree = 0, cycles = 0;
+  double *wn = nullptr, *yn = nullptr;   // work on the vertices
+  const double *rhs = nullptr;           // element-local, assembled and masked
+  double *z = nullptr;                   // element-local result
+  long npts = 0;
+  const int *skip = nullptr;
+};
+// z = `cycles` V-cycles from zero for the right-hand side rhs.
+cudaError_t tamg_cycle(const TamgCluster &a, const int *skip, cudaStream_t s);
+
+}  // namespace nb

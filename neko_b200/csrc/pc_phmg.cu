@@ -28,6 +28,7 @@
 #include "nb_phmg.h"
 #include "nb_precond.h"
 #include "nb_reduce.cuh"
+#include "nb_tamg.h"
 
 namespace nb {
 
@@ -249,6 +250,9 @@ struct TamgDev {
   std::vector<double *> x, b, r, cr, d, w;    // cycle vectors and smoother scratch
   double *wi = nullptr, *wo = nullptr;        // level-0 work of the flat matvec
   std::vector<double> tha, dlt, lam;
+  // the cycle as one launch, where C is a vertex level (lx = 2)
+  NodeOp nodes;
+  TamgCluster cl;
 };
 
 #define PH_LAUNCH(...)                                 \
@@ -281,6 +285,7 @@ struct PhmgImpl : public Precond {
 
   ~PhmgImpl() override {
     for (void *p : allocs) cudaFree(p);
+    if (A.nodes.base) cudaFree(A.nodes.base);
     for (auto &l : L)
       if (l.owned) nb_problem_destroy(l.P);
   }
@@ -432,14 +437,18 @@ struct PhmgImpl : public Precond {
     }
     // the tree AMG from zero on the last level, its rhs that level's r
     PhmgLevel &T = L[nl - 1];
-    A.x[0] = T.z;
-    A.b[0] = T.r;
-    if (!dry && (e = cudaMemsetAsync(T.z, 0, T.P->n * sizeof(double), s)) != cudaSuccess)
-      return e;
-    bool zero = true;
-    for (int c = 0; c < A.cycles; c++) {
-      if ((e = amg_cycle(zero, skip, s)) != cudaSuccess) return e;
-      zero = false;
+    if (A.cl.lv) {
+      PH_CALL(tamg_cycle(A.cl, skip, s));
+    } else {
+      A.x[0] = T.z;
+      A.b[0] = T.r;
+      if (!dry && (e = cudaMemsetAsync(T.z, 0, T.P->n * sizeof(double), s)) != cudaSuccess)
+        return e;
+      bool zero = true;
+      for (int c = 0; c < A.cycles; c++) {
+        if ((e = amg_cycle(zero, skip, s)) != cudaSuccess) return e;
+        zero = false;
+      }
     }
     for (int l = nl - 2; l >= 0; l--) {
       PhmgLevel &M = L[l], &C = L[l + 1];
@@ -569,6 +578,66 @@ nb_status amg_power(PhmgImpl &H, int l) {
   return NB_OK;
 }
 
+// Operands of the one-launch cycle: level 0 on the distinct vertices of C.
+// Left out (the separate launches stay) when C is not a vertex level or has
+// no unmasked vertex.
+nb_status tamg_cluster_build(PhmgImpl &H, const TamgHost &T) {
+  TamgDev &A = H.A;
+  nb_problem *C = A.C;
+  if (C->lx != 2) return NB_OK;
+  nb_status st = node_create(C, A.nodes);
+  if (st != NB_OK) return st;
+  const int nn = A.nodes.nn;
+  if (nn == 0) return NB_OK;
+  PH_TRY(node_update(C, A.nodes, nullptr));
+  std::vector<int> node_of(C->n), eptr(nn + 1);
+  PH_TRY(cudaMemcpy(node_of.data(), A.nodes.node_of, C->n * sizeof(int), cudaMemcpyDeviceToHost));
+  PH_TRY(cudaMemcpy(eptr.data(), A.nodes.eptr, (nn + 1) * sizeof(int), cudaMemcpyDeviceToHost));
+  std::vector<double> mean(nn);
+  for (int i = 0; i < nn; i++) mean[i] = 1.0 / (double)(eptr[i + 1] - eptr[i]);
+  const double *dmean = nullptr;
+  PH_TRY(upload(H, &dmean, mean));
+  std::vector<TamgClusterLevel> lv(A.nlvls);
+  for (int l = 0; l < A.nlvls; l++) {
+    TamgClusterLevel &L = lv[l];
+    L.n = l == 0 ? nn : (int)A.n[l];
+    L.tha = A.tha[l];
+    L.dlt = A.dlt[l];
+    PH_TRY(H.alloc(&L.x, L.n));
+    PH_TRY(H.alloc(&L.b, L.n));
+    L.r = A.cr[l];
+    L.d[0] = A.d[l];
+    L.d[1] = A.w[l];
+    if (l == 0) continue;
+    std::vector<int> sidx(T.lvl[l].fidx.size());
+    for (size_t k = 0; k < sidx.size(); k++) sidx[k] = node_of[T.lvl[l].fidx[k]];
+    PH_TRY(upload(H, &L.sidx, sidx));
+    L.sptr = A.fptr[l];
+    if (l == 1) continue;
+    std::vector<int> agg(C->nelv);
+    for (int e = 0; e < C->nelv; e++) agg[e] = T.lvl[l].finest[8 * (size_t)e];
+    PH_TRY(upload(H, &L.agg, agg));
+    L.rptr = A.rptr[l];
+    L.ridx = A.ridx[l];
+    L.spread = A.spread[l];
+  }
+  const TamgClusterLevel *dlv = nullptr;
+  PH_TRY(upload(H, &dlv, lv));
+  TamgCluster &c = A.cl;
+  c.A = A.nodes;
+  c.mean = dmean;
+  c.nlvls = A.nlvls;
+  c.degree = A.degree;
+  c.cycles = A.cycles;
+  c.wn = A.wi;
+  c.yn = A.wo;
+  c.rhs = H.L.back().r;
+  c.z = H.L.back().z;
+  c.npts = C->n;
+  c.lv = dlv;
+  return NB_OK;
+}
+
 nb_status phmg_build(nb_problem *P, const PhmgSettings &o, PhmgImpl *H) {
   H->itrs = o.smoother_iterations;
   H->nelv = P->nelv;
@@ -689,6 +758,7 @@ nb_status phmg_build(nb_problem *P, const PhmgSettings &o, PhmgImpl *H) {
     if ((st = level_power(*H, l)) != NB_OK) return st;
   for (int l = 0; l < A.nlvls; l++)
     if ((st = amg_power(*H, l)) != NB_OK) return st;
+  if ((st = tamg_cluster_build(*H, T)) != NB_OK) return st;
   PH_TRY(cudaDeviceSynchronize());
   // launches of one application, counted without launching
   H->dry = true;
