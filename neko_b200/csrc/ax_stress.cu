@@ -95,8 +95,9 @@ __device__ __forceinline__ void stress_point(const double g[3][3], const double 
 // one.  With separate planes only one block of 256 threads was resident at
 // lx 8 (104 us a coupled-CG step on 2.1 M points, 62% of the copy rate) and
 // lx 10 had no streaming form (272 us on 2.2 M points, plus 29 us for the h2
-// term).  The CG form reads z straight into registers, issued before the wait
-// for the stage, instead of staging three more arrays.
+// term).  h2, B and (CG form) z go straight to registers instead of
+// staging up to five more arrays; they are brought to L2 when the stage is
+// filled.
 // Registers (two blocks of 256 threads, or one of 512: 128 a thread) hold two
 // rows of D at a time, reloaded for the second pass, and the components are
 // differentiated one after the other.
@@ -149,6 +150,15 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS>::THREADS, StressCfg<LX, S
       const double *src =
           a < 3 ? io.in[a] : (a == 3 ? geo.h1 : (a == 4 ? geo.jacinv : geo.c[a - 5]));
       bulk_g2s(stage + (size_t)(s * NA + a) * L3, src + e * L3, (uint32_t)C::ABYTES, &full[s]);
+    }
+    // operands that go to registers, to L2 meanwhile
+    if (h2) {
+      bulk_prefetch_l2(h2 + e * L3, (uint32_t)C::ABYTES);
+      bulk_prefetch_l2(Bm + e * L3, (uint32_t)C::ABYTES);
+    }
+    if constexpr (CG) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) bulk_prefetch_l2(cg.z[c] + e * L3, (uint32_t)C::ABYTES);
     }
   };
   if (tid == 0)

@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kRedThreads)
 }
 
 // x += alpha p; r -= alpha w; rtr = (r, mult r); convergence test.
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, 4)
     cg_update_xr_kernel(double *__restrict__ r,
                         const double *__restrict__ p, const double *__restrict__ w,
                         const double *__restrict__ mult, const float *__restrict__ multf, long n, CgState *st,
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kRedThreads)
 // test; beta of the next iteration.  68 B a point (60 with mult in FP32):
 // bound by HBM on large problems, by launch and reduction latency on small
 // ones.
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, 4)
     cg_update_xrz_kernel(double *__restrict__ r, double *__restrict__ z,
                          const double *__restrict__ p, const double *__restrict__ w,
                          const double *__restrict__ d, const double *__restrict__ mult,
@@ -496,12 +496,12 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, cuda
   if (!W.fused)
     cg_pap_kernel<<<rb, kRedThreads, 0, s>>>(W.w, W.p, P->mult, P->multf, n, W.st, W.partials, W.counter);
   if (W.fold) {
-    cg_update_xrz_kernel<<<rb, kRedThreads, 0, s>>>(W.r, W.z, W.p, W.w,
+    cg_update_xrz_kernel<<<wave_blocks(n), kRedThreads, 0, s>>>(W.r, W.z, W.p, W.w,
                                                     W.use_jacobi ? P->jdiag : nullptr, P->mult,
                                                     P->multf, n, W.st, W.partials, W.counter);
     return cudaGetLastError();
   }
-  cg_update_xr_kernel<<<rb, kRedThreads, 0, s>>>(W.r, W.p, W.w, P->mult, P->multf, n, W.st,
+  cg_update_xr_kernel<<<wave_blocks(n), kRedThreads, 0, s>>>(W.r, W.p, W.w, P->mult, P->multf, n, W.st,
                                                  W.partials, W.counter);
   if (W.recompute_every > 0) {  // w = A x, gs, mask; r = f - w (scheduled iterations only)
     // x through z (free until the next preconditioner apply overwrites it)

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kRedThreads)
 
 // x_c += alpha p_c, r_c -= alpha w_c; rnorm, the convergence test; then the
 // next iteration's z_c = d r_c, rtz and beta.
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, 4)
     cpld_update_kernel(const V3 *__restrict__ xp, V3 r, V3 z, C3 p, C3 w,
                        const double *__restrict__ d, const double *__restrict__ mult,
                        const float *__restrict__ multf, long n, CgState *st, double *partials,
@@ -307,7 +307,7 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
                                                       W.partials, W.counter);
       }
       if (ce == cudaSuccess) {
-        cpld_update_kernel<<<rb, kRedThreads, 0, cs>>>(W.xdev, r, z, pc, wc, d, P->mult,
+        cpld_update_kernel<<<wave_blocks(n), kRedThreads, 0, cs>>>(W.xdev, r, z, pc, wc, d, P->mult,
                                                        P->multf, n, W.st, W.partials, W.counter);
         ce = cudaGetLastError();
       }

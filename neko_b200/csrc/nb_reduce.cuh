@@ -113,4 +113,13 @@ inline int red_blocks(long n) {
   return (int)b;
 }
 
+// Blocks of an update kernel built for four resident blocks a multiprocessor
+// (__launch_bounds__(kRedThreads, 4)) whose threads take two points a step:
+// one wave.  With eight blocks' worth of grid and three resident, the last
+// two thirds of a wave ran nearly alone: 98 us for 425 MB.
+inline int wave_blocks(long n) {
+  const long b = (n + 2 * kRedThreads - 1) / (2 * kRedThreads), cap = 4L * device_sms();
+  return (int)(b < 1 ? 1 : b < cap ? b : cap);
+}
+
 }  // namespace nb
