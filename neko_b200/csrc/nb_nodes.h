@@ -32,8 +32,10 @@ struct NodeHost {
   int maxw = 0;               // longest row
 };
 // maps: the level's gather-scatter maps (lx = 2, n local points); masked:
-// its zero-Dirichlet points (0-based).
-void node_setup(const GsMaps &maps, long n, const std::vector<int> &masked, NodeHost &H);
+// its zero-Dirichlet points (0-based).  Beyond most_nodes only nn and node_of
+// are filled.
+void node_setup(const GsMaps &maps, long n, const std::vector<int> &masked, int most_nodes,
+                NodeHost &H);
 
 // The same on the device (one allocation, `base`).
 struct NodeOp {
@@ -43,7 +45,8 @@ struct NodeOp {
   double *val = nullptr, *dinv = nullptr;  // matrix values; inverse Jacobi diagonal
   void *base = nullptr;
 };
-nb_status node_create(nb_problem *C, NodeOp &A);
+// Beyond most_nodes only A.nn is set (A.val stays null).
+nb_status node_create(nb_problem *C, NodeOp &A, int most_nodes = 0x7fffffff);
 // Matrix values and dinv from the level's current coefficients, on stream s.
 cudaError_t node_update(const nb_problem *C, const NodeOp &A, cudaStream_t s);
 

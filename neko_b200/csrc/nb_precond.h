@@ -120,14 +120,34 @@ struct CoarseArgs {
   const T *J = nullptr;                         // lm x 2 interpolation, column-major
   double *f = nullptr;                          // restricted residual, 8 values an element
 };
+// blocks of the element-local coarse solve at most (its partial sums)
+constexpr int kCoarseMaxBlocks = 1024;
+
+// Vertices up to which the coarse solve works on the assembled matrix: one row
+// a thread of the largest cluster (8192; 4096 where the device takes clusters
+// of the portable size only).
+cudaError_t hsmg_coarse_nodes(int &most);
+// The same without any mask.  That problem is singular, and a flexible CG
+// carries a change of rounding of its coarse solve into the solution, the more
+// the larger the mesh: 1e-14 of it on 12^3 elements, 6e-11 on 16^3, 1e-9 on
+// 20^3 and 5e-9 on 32^3 periodic ones, 2e-16 on any with a mask.
+constexpr int kCoarseFreeNodes = 4096;
 struct CoarseCg {
-  NodeOp A;                   // the assembled vertex operator
-  const double *f = nullptr;  // element-local right-hand side
-  double *x = nullptr;        // solution, one value a node
-  double *p = nullptr, *r = nullptr, *w = nullptr;  // work, one value a node
+  NodeOp A;                   // the assembled vertex operator (val null: not built)
+  double *f = nullptr;        // element-local right-hand side
+  double *x = nullptr;        // solution: a value a node, or 8 an element (val null)
   double norm_fac = 0.0, tol = 0.0;
-  int niter = 0, stage_slices = 0;
+  int niter = 0, lm = 0, stage_slices = 0;
   const int *skip = nullptr;
+  // element-local form
+  long nelv = 0;
+  double *r = nullptr, *z = nullptr, *p = nullptr, *w = nullptr;
+  const double *h1 = nullptr, *g[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr},
+               *D = nullptr, *Dt = nullptr, *dinv = nullptr, *mult = nullptr;
+  double *part = nullptr;   // 2 x 2 x (grid) doubles
+  unsigned *bar = nullptr;  // grid-barrier word (reset with err after a timeout)
+  int *err = nullptr;       // set to 1 when a barrier wait expired
+  GsDevice gs;
 };
 
 // f = restriction of (w_mid mult_m), element by element (lm = 3 or 4).
@@ -136,7 +156,6 @@ cudaError_t hsmg_coarse_restrict(const CoarseArgs<T> &a, int lm, const int *skip
                                  cudaStream_t s);
 // The coarse Jacobi-CG, one cluster launch.
 cudaError_t hsmg_coarse_cg(const CoarseCg &a, const int *skip, cudaStream_t s);
-
 // hsmg preconditioner of problem P, built on first use (pc_hsmg.cu).
 nb_status hsmg_get(nb_problem *P, const nb_solve_opts &o, Precond **out);
 

@@ -36,6 +36,25 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
   return r;
 }
 
+// Two sums at once: the same trees as two calls of block_sum, their stages
+// interleaved (one pair of barriers instead of two).
+template <int THREADS>
+__device__ __forceinline__ void block_sum2(double &v0, double &v1, double (&sh)[2][THREADS / 32]) {
+  v0 = warp_sum(v0);
+  v1 = warp_sum(v1);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) {
+    sh[0][wid] = v0;
+    sh[1][wid] = v1;
+  }
+  __syncthreads();
+  if (wid == 0) {
+    v0 = warp_sum(lane < THREADS / 32 ? sh[0][lane] : 0.0);
+    v1 = warp_sum(lane < THREADS / 32 ? sh[1][lane] : 0.0);
+  }
+  __syncthreads();
+}
+
 // Called by every thread of every block after computing `v` (its share).
 // partials: gridDim.x doubles; counter: one zero-initialised unsigned.
 // Returns true in thread 0 of the last block, with *out set to the total.
@@ -71,13 +90,12 @@ __device__ __forceinline__ bool grid_sum(double v, double *partials, unsigned *c
 template <int THREADS>
 __device__ __forceinline__ bool grid_sum2(double v0, double v1, double *partials,
                                           unsigned *counter, double *out) {
-  __shared__ double sh[THREADS / 32];
+  __shared__ double sh[2][THREADS / 32];
   __shared__ bool last;
-  const double b0 = block_sum<THREADS>(v0, sh);
-  const double b1 = block_sum<THREADS>(v1, sh);
+  block_sum2<THREADS>(v0, v1, sh);
   if (threadIdx.x == 0) {
-    partials[2 * blockIdx.x] = b0;
-    partials[2 * blockIdx.x + 1] = b1;
+    partials[2 * blockIdx.x] = v0;
+    partials[2 * blockIdx.x + 1] = v1;
     __threadfence();
     const unsigned done = atomicAdd(counter, 1u);
     last = done == gridDim.x - 1;
@@ -90,8 +108,7 @@ __device__ __forceinline__ bool grid_sum2(double v0, double v1, double *partials
     t0 += *((volatile double *)partials + 2 * b);
     t1 += *((volatile double *)partials + 2 * b + 1);
   }
-  t0 = block_sum<THREADS>(t0, sh);
-  t1 = block_sum<THREADS>(t1, sh);
+  block_sum2<THREADS>(t0, t1, sh);
   if (threadIdx.x == 0) {
     *counter = 0;
     out[0] = t0;

@@ -77,22 +77,23 @@ __global__ void __launch_bounds__(128) node_values_kernel(NodeOp A, NodeCoef c) 
 }
 
 cudaError_t node_update(const nb_problem *C, const NodeOp &A, cudaStream_t s) {
-  if (A.nn == 0) return cudaSuccess;
+  if (A.nn == 0 || !A.val) return cudaSuccess;
   const NodeCoef c{C->h1, {C->g11, C->g22, C->g33, C->g12, C->g13, C->g23}, C->D,
                    C->ifh2 ? C->h2 : nullptr, C->B, C->jdiag};
   node_values_kernel<<<(32 * A.ns + 127) / 128, 128, 0, s>>>(A, c);
   return cudaGetLastError();
 }
 
-nb_status node_create(nb_problem *C, NodeOp &A) {
+nb_status node_create(nb_problem *C, NodeOp &A, int most_nodes) {
   std::vector<int> masked(C->nmask);
   if (C->nmask > 0)
     NB_CUDA_TRY(cudaMemcpy(masked.data(), C->msk, C->nmask * sizeof(int),
                            cudaMemcpyDeviceToHost));
   for (int &m : masked) m -= 1;
   NodeHost H;
-  node_setup(C->maps, C->n, masked, H);
+  node_setup(C->maps, C->n, masked, most_nodes, H);
   A.nn = H.nn;
+  if (A.nn > most_nodes) return NB_OK;
   A.ns = (int)H.soff.size() - 1;
   A.maxw = H.maxw;
   const std::vector<int> *src[6] = {&H.node_of, &H.eptr, &H.ent, &H.soff, &H.col, &H.slot};

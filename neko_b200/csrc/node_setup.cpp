@@ -6,7 +6,8 @@
 
 namespace nb {
 
-void node_setup(const GsMaps &maps, long n, const std::vector<int> &masked, NodeHost &H) {
+void node_setup(const GsMaps &maps, long n, const std::vector<int> &masked, int most_nodes,
+                NodeHost &H) {
   // points with one gather-scatter id are one node; points outside the maps
   // are nodes of their own
   std::vector<int> id(n, -1);
@@ -33,6 +34,7 @@ void node_setup(const GsMaps &maps, long n, const std::vector<int> &masked, Node
     }
   }
   const int nn = H.nn;
+  if (nn > most_nodes) return;
   H.eptr.assign(nn + 1, 0);
   for (int v : H.node_of)
     if (v >= 0) H.eptr[v + 1]++;

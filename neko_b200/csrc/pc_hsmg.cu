@@ -386,10 +386,11 @@ struct PrologDots {
 
 // The coarse level's correction, added to the middle level's as the
 // prolongation reads it: in(i,j,k) + sum J(k,c) J(j,b) J(i,a) x(a,b,c) with x
-// the node values of the element's vertices (0 on masked ones).
+// the values of the element's vertices, by node (0 on masked ones) or, without
+// node_of, element by element.
 template <typename T>
 struct CoarseAdd {
-  const double *x = nullptr;     // per node
+  const double *x = nullptr;
   const int *node_of = nullptr;  // 8 per element, -1 masked
   const T *J = nullptr;          // NI x 2, column-major
 };
@@ -411,7 +412,7 @@ __global__ void __launch_bounds__(kT3Threads)
     __shared__ T sx[8], sJc[2 * NI];
     if (crs.x) {
       if (tid < 8) {
-        const int nd = __ldg(crs.node_of + e * 8 + tid);
+        const long nd = crs.node_of ? __ldg(crs.node_of + e * 8 + tid) : e * 8 + tid;
         sx[tid] = nd >= 0 ? (T)__ldg(crs.x + nd) : T(0);
       }
       if (tid >= 32 && tid < 32 + 2 * NI) sJc[tid - 32] = __ldg(crs.J + tid - 32);
@@ -758,6 +759,10 @@ struct HsmgState : public Precond {
   // side.  `crs` and `hi` have the greatest priority: the cluster needs its
   // multiprocessors at once, so it is placed before the fine-level FDM fills
   // the device, and the FDM then takes the others.
+  // As a grid on every multiprocessor (larger meshes) the coarse solve gains
+  // nothing from its place: there the fine level starts at once, and the coarse
+  // solve follows the middle level's Schwarz (27.0 against 27.4 ms a solve of
+  // 20 applications on 32^3 elements).
   cudaStream_t side = nullptr, hi = nullptr, crs_s = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_mid = nullptr, ev_join = nullptr, ev_join_hi = nullptr,
               ev_join_crs = nullptr;
@@ -815,6 +820,18 @@ struct HsmgImpl : public HsmgState {
     return 6 + 1 + 1 + 1 + 1 + 1 + 1 + (sizeof(T) == 4 ? 1 : 0) - (merged_assembly() ? 1 : 0);
   }
 
+  int take_error() override {
+    int v = 0;
+    if (!cg.err) return 0;
+    if (cudaMemcpy(&v, cg.err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
+    if (v) {  // leave the barrier words at rest for the next launch
+      cudaMemset(cg.err, 0, sizeof(int));
+      cudaMemset(cg.bar, 0, 2 * sizeof(unsigned));
+      cudaDeviceSynchronize();
+    }
+    return v;
+  }
+
   // FP32 smoothing levels: the output can stay in FP32 (zf)
   const float *output_f32() override {
     return sizeof(T) == 4 ? reinterpret_cast<const float *>(zf) : nullptr;
@@ -853,6 +870,7 @@ struct HsmgImpl : public HsmgState {
                        const PrologDots *dots = nullptr) {
     cudaError_t e;
     const long nelv = fine->nelv;
+    const bool grid = cg.err != nullptr;  // the coarse solve takes every multiprocessor
     if ((e = cudaEventRecord(ev_fork, s)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(crs_s, ev_fork, 0)) != cudaSuccess)
       return e;
@@ -864,16 +882,19 @@ struct HsmgImpl : public HsmgState {
         (e = hsmg_coarse_restrict<T>(ca, mid->lx, skip, crs_s)) != cudaSuccess ||
         (e = cudaEventRecord(ev_mid, crs_s)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(hi, ev_mid, 0)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(side, ev_mid, 0)) != cudaSuccess)
+        (e = cudaStreamWaitEvent(side, grid ? ev_fork : ev_mid, 0)) != cudaSuccess)
       return e;
     // coarse: assemble, mask, niter Jacobi-CG iterations (or abs tol)
-    if ((e = hsmg_coarse_cg(cg, skip, crs_s)) != cudaSuccess ||
-        (e = cudaEventRecord(ev_join_crs, crs_s)) != cudaSuccess)
-      return e;
+    auto coarse = [&](cudaStream_t cs) {
+      const cudaError_t r = hsmg_coarse_cg(cg, skip, cs);
+      return r != cudaSuccess ? r : cudaEventRecord(ev_join_crs, cs);
+    };
+    if (!grid && (e = coarse(crs_s)) != cudaSuccess) return e;
     // middle Schwarz: e_mid = S_m w
     if ((e = schwarz_apply<T, T>(sm, w_mid, e_mid, skip, hi)) != cudaSuccess ||
         (e = cudaEventRecord(ev_join_hi, hi)) != cudaSuccess)
       return e;
+    if (grid && (e = coarse(hi)) != cudaSuccess) return e;
     // fine Schwarz: zs = S_f r (left unassembled when the final
     // gather-scatter takes it, see below)
     const bool merged = merged_assembly();
@@ -1069,9 +1090,12 @@ static nb_status upload_impl(HsmgImpl<T> *H, const SchwarzHost &hf, const Schwar
   const size_t o_mf = f32 ? c.take(n * sizeof(T)) : 0, o_mm = c.take(nm * sizeof(T));
   const size_t o_zf = f32 ? c.take(n * sizeof(T)) : 0;
   const size_t o_wm = c.take(nm * sizeof(T)), o_em = c.take(nm * sizeof(T));
-  const size_t nn = (size_t)H->nodes.nn + 1;
-  const size_t o_rc = c.take(nc * 8), o_ec = c.take(nn * 8), o_r = c.take(nn * 8),
-               o_p = c.take(nn * 8), o_w = c.take(nn * 8);
+  // coarse solve: the solution by node, or element-local with its vectors
+  const bool local = H->nodes.nn > 0 && !H->nodes.val;
+  const size_t nx = local ? (size_t)nc : (size_t)H->nodes.nn + 1, nv = local ? (size_t)nc : 0;
+  const size_t o_rc = c.take(nc * 8), o_ec = c.take(nx * 8), o_r = c.take(nv * 8),
+               o_z = c.take(nv * 8), o_p = c.take(nv * 8), o_w = c.take(nv * 8),
+               o_part = c.take(local ? (2 * 2 * kCoarseMaxBlocks + 2) * sizeof(double) : 0);
   if (cudaMalloc(&H->arena, c.off) != cudaSuccess) return hfail(NB_ERR_OOM, "hsmg: device arena");
   char *A = (char *)H->arena;
   auto Tp = [&](size_t o) { return (T *)(A + o); };
@@ -1099,7 +1123,17 @@ static nb_status upload_impl(HsmgImpl<T> *H, const SchwarzHost &hf, const Schwar
   ca.w_mid = H->w_mid, ca.mult_m = H->mult_m, ca.J = H->Jmc, ca.f = Dp(o_rc);
   CoarseCg &cg = H->cg;
   cg.A = H->nodes;
-  cg.f = ca.f, cg.x = Dp(o_ec), cg.r = Dp(o_r), cg.p = Dp(o_p), cg.w = Dp(o_w);
+  cg.f = ca.f, cg.x = Dp(o_ec), cg.nelv = nelv, cg.lm = M->lx;
+  if (local) {
+    cg.r = Dp(o_r), cg.z = Dp(o_z), cg.p = Dp(o_p), cg.w = Dp(o_w);
+    cg.h1 = C->h1, cg.D = C->D, cg.Dt = C->Dt, cg.dinv = C->jdiag, cg.mult = C->mult;
+    cg.g[0] = C->g11, cg.g[1] = C->g22, cg.g[2] = C->g33, cg.g[3] = C->g12, cg.g[4] = C->g13,
+    cg.g[5] = C->g23;
+    cg.gs = C->gsd;
+    cg.part = Dp(o_part);  // followed by the barrier and error words
+    cg.bar = reinterpret_cast<unsigned *>(cg.part + 2 * 2 * kCoarseMaxBlocks);
+    cg.err = reinterpret_cast<int *>(cg.bar + 2);
+  }
   cg.norm_fac = 1.0 / std::sqrt(C->volume), cg.tol = H->tol, cg.niter = H->niter;
   auto upv = [&](size_t o, const std::vector<double> &v) {
     std::vector<T> t = cast_vec<T>(v);
@@ -1123,7 +1157,8 @@ static nb_status upload_impl(HsmgImpl<T> *H, const SchwarzHost &hf, const Schwar
       upv(o_mm, hm_mult) || (f32 && upv(o_mf, hf_mult)) ||
       (!ornt.empty() &&
        cudaMemcpy(A + o_or, ornt.data(), ornt.size(), cudaMemcpyHostToDevice) != cudaSuccess) ||
-      cudaMemset(A + o_ec, 0, nn * 8) != cudaSuccess)
+      cudaMemset(A + o_ec, 0, nx * 8) != cudaSuccess ||
+      (local && cudaMemset(cg.bar, 0, 2 * sizeof(double)) != cudaSuccess))
     return hfail(NB_ERR_CUDA, "hsmg: upload failed");
   return NB_OK;
 }
@@ -1170,7 +1205,11 @@ nb_status hsmg_get(nb_problem *P, const nb_solve_opts &o, Precond **out) {
     delete H;
     return st;
   }
-  if ((st = node_create(H->crs, H->nodes)) != NB_OK) {
+  int most_nodes = 0;
+  if (hsmg_coarse_nodes(most_nodes) != cudaSuccess)
+    st = hfail(NB_ERR_CUDA, "hsmg: coarse solve not available");
+  if (!dirichlet) most_nodes = std::min(most_nodes, kCoarseFreeNodes);
+  if (st != NB_OK || (st = node_create(H->crs, H->nodes, most_nodes)) != NB_OK) {
     delete H;
     return st;
   }

@@ -1,9 +1,9 @@
-"""The hsmg coarse solve over distinct vertices, at the sizes where its
-launch changes form: no unmasked vertex at all, one block, clusters with the
-vectors resident in every block, two and four rows a thread with the vectors
-in global memory, the matrix no longer in shared memory, and more rows than
-the registers hold.  One application against the CPU oracle with the
-bounds of test_gpu_hsmg.py (lx 4 keeps the other levels small)."""
+"""The hsmg coarse solve at the sizes where its launch changes form: no
+unmasked vertex at all, one block, clusters with the vectors and the matrix
+resident in every block, the matrix in global memory, and the element-local
+grid of larger meshes, with its vectors in registers and in memory.  One
+application against the CPU oracle with the bounds of test_gpu_hsmg.py (lx 4
+keeps the other levels small)."""
 import numpy as np
 import pytest
 import torch
@@ -17,10 +17,12 @@ NODES = [((1, 1, 1), (False,) * 3),         # 0
          ((2, 2, 2), (False,) * 3),         # 1
          ((9, 7, 8), (False,) * 3),         # 336: four blocks
          ((17, 16, 18), (False,) * 3),      # 4080: sixteen blocks
-         ((21, 20, 22), (True, False, True)),   # 8778: two rows a thread
+         ((21, 20, 21), (False,) * 3),      # 7600: matrix in global memory
+         ((21, 20, 22), (True, False, True)),   # 8400: element-local
          ((26, 25, 27), (False,) * 3),      # 15600
-         ((28, 28, 27), (True, False, False)),  # 19656: four rows a thread
-         ((33, 33, 34), (True, False, False))]  # 34848: vectors in memory
+         ((28, 28, 27), (True, False, False)),  # 19656
+         ((33, 33, 34), (True, False, False)),  # 34848
+         ((34, 34, 33), (True, False, False))]  # vectors in memory
 
 
 @pytest.mark.parametrize("nel,per", NODES)
