@@ -1256,6 +1256,10 @@ nb_status hsmg_apply_once(nb_problem *P, double *z, const double *r, cudaStream_
   if (st != NB_OK) return st;
   NB_CUDA_TRY(pc->apply(z, r, nullptr, s));
   NB_CUDA_TRY(cudaStreamSynchronize(s));
+  if (pc->take_error()) {
+    set_error("a bounded device wait expired (coarse-level grid barrier)");
+    return NB_ERR_TIMEOUT;
+  }
   return NB_OK;
 }
 
