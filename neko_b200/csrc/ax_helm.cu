@@ -20,6 +20,7 @@
 
 #include <cstdint>
 
+#include "nb_chain.cuh"
 #include "nb_kernels.h"
 #include "nb_precond.h"
 #include "nb_reduce.cuh"
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(LX *LX *NE)
                    const T *__restrict__ g12, const T *__restrict__ g13,
                    const T *__restrict__ g23, const int nelv,
                    const int *__restrict__ skip) {
+  chain();
   if (skip && *skip) return;  // solver finished: uniform early exit
   constexpr int L2 = LX * LX, L3 = L2 * LX;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -152,7 +154,6 @@ __global__ void __launch_bounds__(AxTmaCfg<T, LX, S, KS>::THREADS)
   using C = AxTmaCfg<T, LX, S, KS>;
   constexpr int L2 = C::L2, L3 = C::L3, NA = C::NA, KP = LX / KS;
   static_assert(LX % KS == 0, "k split must divide lx");
-  if (skip && *skip) return;
   extern __shared__ __align__(128) unsigned char smem_ring[];
   T *stage = reinterpret_cast<T *>(smem_ring);
   T *sur = stage + S * NA * L3, *sus = sur + L3, *sut = sus + L3;
@@ -166,6 +167,8 @@ __global__ void __launch_bounds__(AxTmaCfg<T, LX, S, KS>::THREADS)
     for (int s = 0; s < S; s++) mbar_init(&full[s], 1);
     fence_barrier_init();
   }
+  chain();
+  if (skip && *skip) return;
   for (int q = tid; q < L2; q += C::THREADS) {
     sD[q] = D[q];
     sDt[q] = Dt[q];
@@ -285,7 +288,8 @@ static cudaError_t launch_ax_tma(T *w, const T *u, const T *D, const T *Dt, cons
   }
   if (nelv <= 0) return cudaSuccess;
   const int grid = nelv < g ? nelv : g;
-  kern<<<grid, C::THREADS, C::SMEM, st>>>(w, u, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv,
+  launch_chained((long)nelv * C::L3, kern, grid, C::THREADS, C::SMEM, st, w, u, D, Dt, h1, g11,
+                 g22, g33, g12, g13, g23, nelv,
                                           skip, err);
   return cudaGetLastError();
 }
@@ -357,7 +361,6 @@ __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
   using C = AxCgCfg<LX, S, KS, AL>;
   constexpr int L2 = C::L2, L3 = C::L3, NA = C::NA, KP = LX / KS, THREADS = C::THREADS;
   static_assert(LX % KS == 0, "k split must divide lx");
-  if (st && st->done) return;
   extern __shared__ __align__(128) unsigned char smem_ring[];
   double *stage = reinterpret_cast<double *>(smem_ring);
   double *sur = stage + S * NA * L3, *sus = sur + L3, *sut = sus + L3;
@@ -367,7 +370,6 @@ __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
   const int tid = threadIdx.x;
   const int G = gridDim.x, b = blockIdx.x;
   const int nt = b < nelv ? (nelv - b + G - 1) / G : 0;
-  const double beta = st ? st->beta : beta_arg;
   if (tid == 0) {
     for (int s = 0; s < S; s++) mbar_init(&full[s], 1);
     fence_barrier_init();
@@ -377,6 +379,9 @@ __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
     sDt[q] = Dt[q];
   }
   __syncthreads();
+  chain();
+  if (st && st->done) return;
+  const double beta = st ? st->beta : beta_arg;
   // z (slot 0) arrives in its own precision: L3 values of TZ
   constexpr uint32_t ZBYTES = (uint32_t)(L3 * sizeof(TZ));
   const double *src[NA] = {nullptr, p, h1, g11, g22, g33, g12, g13, g23};
@@ -546,7 +551,8 @@ static cudaError_t launch_ax_cg(const AxCgArgs<TZ> &a, cudaStream_t s) {
   }
   int grid = a.nelv < g ? a.nelv : g;
   if (grid > a.max_grid) grid = a.max_grid;
-  kern<<<grid, C::THREADS, C::SMEM, s>>>(a.w, a.p, a.z, a.D, a.Dt, a.h1, a.g[0], a.g[1], a.g[2],
+  launch_chained((long)a.nelv * C::L3, kern, grid, C::THREADS, C::SMEM, s, a.w, a.p, a.z, a.D,
+                 a.Dt, a.h1, a.g[0], a.g[1], a.g[2],
                                          a.g[3], a.g[4], a.g[5], a.h2, a.B, a.nelv, a.st, a.beta,
                                          a.pap_out, a.partials, a.counter, a.err);
   return cudaGetLastError();
@@ -568,7 +574,6 @@ __global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS)
     ax_cg_gen_kernel(const AxCgArgs<TZ> a) {
   using C = AxCgGen<LX, NE>;
   constexpr int L2 = C::L2, L3 = C::L3;
-  if (a.st && a.st->done) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double *sD = reinterpret_cast<double *>(smem_raw), *sDt = sD + L2;
   const int tid = threadIdx.x, tz = tid / L2, col = tid - tz * L2;
@@ -578,6 +583,8 @@ __global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS)
     sD[q] = a.D[q];
     sDt[q] = a.Dt[q];
   }
+  chain();
+  if (a.st && a.st->done) return;
   const double beta = a.st ? a.st->beta : a.beta;
   double pap = 0.0;
   for (long eb = (long)blockIdx.x * NE; eb < a.nelv; eb += (long)gridDim.x * NE) {
@@ -659,7 +666,8 @@ static cudaError_t launch_ax_cg_gen(const AxCgArgs<TZ> &a, cudaStream_t s) {
   }
   // every partial sum has a slot: blocks loop over the elements beyond that
   const int ne = AxCfg<LX>::NE, need = (a.nelv + ne - 1) / ne;
-  kern<<<need < a.max_grid ? need : a.max_grid, C::THREADS, C::SMEM, s>>>(a);
+  launch_chained((long)a.nelv * C::L3, kern,
+                 need < a.max_grid ? need : a.max_grid, C::THREADS, C::SMEM, s, a);
   return cudaGetLastError();
 }
 
@@ -756,7 +764,8 @@ static cudaError_t launch_ax(T *w, const T *u, const T *dx, const T *dy, const T
   }
   dim3 block(LX, LX, NE), grid((nelv + NE - 1) / NE);
   if (nelv <= 0) return cudaSuccess;
-  kern<<<grid, block, smem, s>>>(w, u, dx, dy, dz, dxt, dyt, dzt, h1, g11, g22, g33, g12,
+  launch_chained((long)nelv * LX * LX * LX, kern, grid, block, smem, s, w, u, dx, dy, dz, dxt,
+                 dyt, dzt, h1, g11, g22, g33, g12,
                                  g13, g23, nelv, skip);
   return cudaGetLastError();
 }

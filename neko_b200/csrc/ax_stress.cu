@@ -24,6 +24,7 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include "nb_chain.cuh"
 #include "nb_kernels.h"
 #include "nb_precond.h"
 #include "nb_problem.h"
@@ -123,9 +124,6 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS>::THREADS, StressCfg<LX, S
   using C = StressCfg<LX, S, KS>;
   constexpr int L2 = C::L2, L3 = C::L3, NA = C::NA, KP = LX / KS;
   static_assert(LX % KS == 0 && LX % 2 == 0, "k split must divide an even lx");
-  if (skip && *skip) return;
-  if (CG && cg.st->done) return;
-  const double beta = CG ? cg.st->beta : 0.0;
   extern __shared__ __align__(128) unsigned char smem_stress[];
   double *stage = reinterpret_cast<double *>(smem_stress);
   double *sDz = stage + S * NA * L3;
@@ -138,6 +136,10 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS>::THREADS, StressCfg<LX, S
     for (int s = 0; s < S; s++) mbar_init(&full[s], 1);
     fence_barrier_init();
   }
+  chain();
+  if (skip && *skip) return;
+  if (CG && cg.st->done) return;
+  const double beta = CG ? cg.st->beta : 0.0;
   for (int q = tid; q < L2; q += C::THREADS) sDz[q] = dz[q];
   __syncthreads();
   // stage slot: u, v, w (the old directions in the CG form), h1, 1/jac, the
@@ -344,7 +346,8 @@ static cudaError_t launch_stress_tma(const StressIo &io, const StressGeo &geo, c
   if (!err) err = dropin_error_word();
   if (!err) return cudaErrorInvalidSymbol;
   const int grid = nelv < g ? nelv : g;
-  kern<<<grid, C::THREADS, C::SMEM, st>>>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, err, skip, cg);
+  launch_chained(3L * nelv * C::L3, kern, grid, C::THREADS, C::SMEM, st, io, geo, dx, dy, dz, w3,
+                 h2, Bm, nelv, err, skip, cg);
   return cudaGetLastError();
 }
 
@@ -538,6 +541,7 @@ __global__ void ax_stress_part2_kernel(double *__restrict__ au, double *__restri
                                        const double *__restrict__ h2,
                                        const double *__restrict__ B, long n,
                                        const int *__restrict__ skip) {
+  chain();
   if (skip && *skip) return;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n;
        q += (long)gridDim.x * blockDim.x) {
@@ -551,7 +555,8 @@ cudaError_t ax_stress_part2(double *au, double *av, double *aw, const double *u,
                             const double *v, const double *w, const double *h2,
                             const double *B, long n, cudaStream_t s, const int *skip) {
   if (n <= 0) return cudaSuccess;
-  ax_stress_part2_kernel<<<stream_grid(n, 256), 256, 0, s>>>(au, av, aw, u, v, w, h2, B, n,
+  launch_chained(3 * n, ax_stress_part2_kernel, stream_grid(n, 256), 256, 0, s, au, av, aw, u, v,
+                 w, h2, B, n,
                                                              skip);
   return cudaGetLastError();
 }

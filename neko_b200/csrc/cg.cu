@@ -26,6 +26,7 @@
 #include <cstring>
 #include <string>
 
+#include "nb_chain.cuh"
 #include "nb_kernels.h"
 #include "nb_precond.h"
 #include "nb_problem.h"
@@ -49,6 +50,7 @@ __global__ void jacobi_scale_kernel(double *d, const double *h1, const double *h
 
 __global__ void addcol4_kernel(double *w, const double *h2, const double *B, const double *u,
                                long n, const int *skip) {
+  chain();
   if (skip && *skip) return;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
        i += (long)gridDim.x * blockDim.x)
@@ -66,6 +68,7 @@ __global__ void __launch_bounds__(kRedThreads)
                    double *__restrict__ z, const double *__restrict__ d,
                    const double *__restrict__ f, const double *__restrict__ mult, const float *__restrict__ multf, long n,
                    CgState *st, double *partials, unsigned *counter) {
+  chain();
   double s = 0.0, sz = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
        i += (long)gridDim.x * kRedThreads) {
@@ -102,6 +105,7 @@ __global__ void __launch_bounds__(kRedThreads)
     cg_precond_dot_kernel(double *__restrict__ z, const double *__restrict__ r,
                           const double *__restrict__ d, const double *__restrict__ mult, const float *__restrict__ multf,
                           long n, CgState *st, double *partials, unsigned *counter) {
+  chain();
   if (st->done) return;
   double s = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
@@ -126,6 +130,7 @@ __global__ void __launch_bounds__(kRedThreads)
     cg_dot_rz_kernel(const TZ *__restrict__ z, const double *__restrict__ r,
                      const double *__restrict__ mult, const float *__restrict__ multf, long n, CgState *st, double *partials,
                      unsigned *counter) {
+  chain();
   if (st->done) return;
   double s = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
@@ -148,6 +153,7 @@ __global__ void __launch_bounds__(kRedThreads)
     cg_dot_rz_flex_kernel(const TZ *__restrict__ z, const double *__restrict__ r,
                           const double *__restrict__ w_prev, const double *__restrict__ mult, const float *__restrict__ multf,
                           long n, CgState *st, double *partials, unsigned *counter) {
+  chain();
   if (st->done) return;
   double s0 = 0.0, s1 = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
@@ -170,6 +176,7 @@ __global__ void __launch_bounds__(kRedThreads)
 // fixed order.
 __global__ void __launch_bounds__(1024)
     cg_finish_flex_kernel(const double *__restrict__ part, long nelv, CgState *st) {
+  chain();
   if (st->done) return;
   // four independent chains a thread (loads in flight together), summed in
   // a fixed order
@@ -201,6 +208,7 @@ __global__ void __launch_bounds__(1024)
 template <typename TZ>
 __global__ void cg_update_p_kernel(double *__restrict__ p, const TZ *__restrict__ z,
                                    long n, const CgState *st) {
+  chain();
   if (st->done) return;
   const double beta = st->beta;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
@@ -213,6 +221,7 @@ __global__ void __launch_bounds__(kRedThreads)
     cg_pap_kernel(const double *__restrict__ w, const double *__restrict__ p,
                   const double *__restrict__ mult, const float *__restrict__ multf, long n, CgState *st, double *partials,
                   unsigned *counter) {
+  chain();
   if (st->done) return;
   double s = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
@@ -231,6 +240,7 @@ __global__ void __launch_bounds__(kRedThreads, 4)
                         const double *__restrict__ p, const double *__restrict__ w,
                         const double *__restrict__ mult, const float *__restrict__ multf, long n, CgState *st,
                         double *partials, unsigned *counter) {
+  chain();
   if (st->done) return;
   double *__restrict__ x = st->x;
   const double alpha = st->alpha, malpha = -alpha;
@@ -286,6 +296,7 @@ __global__ void __launch_bounds__(kRedThreads, 4)
                          const double *__restrict__ d, const double *__restrict__ mult,
                          const float *__restrict__ multf, long n, CgState *st, double *partials,
                          unsigned *counter) {
+  chain();
   if (st->done) return;
   double *__restrict__ x = st->x;
   const double alpha = st->alpha, malpha = -alpha;
@@ -343,6 +354,7 @@ __global__ void __launch_bounds__(kRedThreads)
     cg_true_residual_kernel(double *__restrict__ r,
                             const double *__restrict__ w, const double *__restrict__ mult, const float *__restrict__ multf, long n,
                             CgState *st, double *partials, unsigned *counter) {
+  chain();
   if (st->skip_rc) return;
   const double *__restrict__ f = st->f;
   double s = 0.0;
@@ -369,6 +381,7 @@ __global__ void __launch_bounds__(kRedThreads)
 
 // y = st->x (the recompute's operator input), on scheduled iterations only
 __global__ void cg_copy_x_kernel(double *__restrict__ y, long n, const CgState *st) {
+  chain();
   if (st->skip_rc) return;
   const double *__restrict__ x = st->x;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
@@ -444,28 +457,33 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, cuda
     // unassembled output equal the mult-weighted ones of the assembled z)
     cudaError_t e = pc->apply_dots(W.z, W.r, W.w, W.dots, &W.st->done, s);
     if (e != cudaSuccess) return e;
-    cg_finish_flex_kernel<<<1, 1024, 0, s>>>(W.dots, W.dots_n, W.st);
+    launch_chained(n, cg_finish_flex_kernel, 1, 1024, 0, s, W.dots, W.dots_n, W.st);
   } else if (pc) {
     cudaError_t e = zf ? pc->apply_f32(W.r, &W.st->done, s) : pc->apply(W.z, W.r, &W.st->done, s);
     if (e != cudaSuccess) return e;
     if (W.flexible) {
       if (zf)
-        cg_dot_rz_flex_kernel<float><<<rb, kRedThreads, 0, s>>>(zf, W.r, W.w, P->mult, P->multf,
+        launch_chained(n, cg_dot_rz_flex_kernel<float>, rb, kRedThreads, 0, s, zf, W.r, W.w,
+                       P->mult, P->multf,
                                                                 n, W.st, W.partials, W.counter);
       else
-        cg_dot_rz_flex_kernel<double><<<rb, kRedThreads, 0, s>>>(W.z, W.r, W.w, P->mult,
+        launch_chained(n, cg_dot_rz_flex_kernel<double>, rb, kRedThreads, 0, s, W.z, W.r, W.w,
+                       P->mult,
                                                                  P->multf, n, W.st, W.partials,
                                                                  W.counter);
     } else {
       if (zf)
-        cg_dot_rz_kernel<float><<<rb, kRedThreads, 0, s>>>(zf, W.r, P->mult, P->multf, n, W.st,
+        launch_chained(n, cg_dot_rz_kernel<float>, rb, kRedThreads, 0, s, zf, W.r, P->mult,
+                       P->multf, n, W.st,
                                                            W.partials, W.counter);
       else
-        cg_dot_rz_kernel<double><<<rb, kRedThreads, 0, s>>>(W.z, W.r, P->mult, P->multf, n,
+        launch_chained(n, cg_dot_rz_kernel<double>, rb, kRedThreads, 0, s, W.z, W.r, P->mult,
+                       P->multf, n,
                                                             W.st, W.partials, W.counter);
     }
   } else if (!W.fold) {
-    cg_precond_dot_kernel<<<rb, kRedThreads, 0, s>>>(W.z, W.r, W.use_jacobi ? P->jdiag : nullptr,
+    launch_chained(n, cg_precond_dot_kernel, rb, kRedThreads, 0, s, W.z, W.r,
+                   W.use_jacobi ? P->jdiag : nullptr,
                                                      P->mult, P->multf, n, W.st, W.partials, W.counter);
   }
   // p = z + beta p; w = A p; pap: one launch (the local form of pap needs p
@@ -484,34 +502,39 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, cuda
   if (e != cudaSuccess && e != cudaErrorNotSupported) return e;
   if (!W.fused) {
     if (zf)
-      cg_update_p_kernel<float><<<eg, 256, 0, s>>>(W.p, zf, n, W.st);
+      launch_chained(n, cg_update_p_kernel<float>, eg, 256, 0, s, W.p, zf, n, W.st);
     else
-      cg_update_p_kernel<double><<<eg, 256, 0, s>>>(W.p, W.z, n, W.st);
+      launch_chained(n, cg_update_p_kernel<double>, eg, 256, 0, s, W.p, W.z, n, W.st);
     e = P->ax_raw(W.w, W.p, s, &W.st->done);
     if (e != cudaSuccess) return e;
-    if (P->ifh2) addcol4_kernel<<<eg, 256, 0, s>>>(W.w, P->h2, P->B, W.p, n, &W.st->done);
+    if (P->ifh2) launch_chained(n, addcol4_kernel, eg, 256, 0, s, W.w, P->h2, P->B, W.p, n,
+                                &W.st->done);
   }
   e = gs_add_fused<double>(P->gsd, W.w, true, s, &W.st->done);
   if (e != cudaSuccess) return e;
   if (!W.fused)
-    cg_pap_kernel<<<rb, kRedThreads, 0, s>>>(W.w, W.p, P->mult, P->multf, n, W.st, W.partials, W.counter);
+    launch_chained(n, cg_pap_kernel, rb, kRedThreads, 0, s, W.w, W.p, P->mult, P->multf, n, W.st,
+                   W.partials, W.counter);
   if (W.fold) {
-    cg_update_xrz_kernel<<<wave_blocks(n), kRedThreads, 0, s>>>(W.r, W.z, W.p, W.w,
+    launch_chained(n, cg_update_xrz_kernel, wave_blocks(n), kRedThreads, 0, s, W.r, W.z, W.p, W.w,
                                                     W.use_jacobi ? P->jdiag : nullptr, P->mult,
                                                     P->multf, n, W.st, W.partials, W.counter);
     return cudaGetLastError();
   }
-  cg_update_xr_kernel<<<wave_blocks(n), kRedThreads, 0, s>>>(W.r, W.p, W.w, P->mult, P->multf, n, W.st,
+  launch_chained(n, cg_update_xr_kernel, wave_blocks(n), kRedThreads, 0, s, W.r, W.p, W.w,
+                 P->mult, P->multf, n, W.st,
                                                  W.partials, W.counter);
   if (W.recompute_every > 0) {  // w = A x, gs, mask; r = f - w (scheduled iterations only)
     // x through z (free until the next preconditioner apply overwrites it)
-    cg_copy_x_kernel<<<eg, 256, 0, s>>>(W.z, n, W.st);
+    launch_chained(n, cg_copy_x_kernel, eg, 256, 0, s, W.z, n, W.st);
     e = P->ax_raw(W.w, W.z, s, &W.st->skip_rc);
     if (e != cudaSuccess) return e;
-    if (P->ifh2) addcol4_kernel<<<eg, 256, 0, s>>>(W.w, P->h2, P->B, W.z, n, &W.st->skip_rc);
+    if (P->ifh2) launch_chained(n, addcol4_kernel, eg, 256, 0, s, W.w, P->h2, P->B, W.z, n,
+                                &W.st->skip_rc);
     e = gs_add_fused<double>(P->gsd, W.w, true, s, &W.st->skip_rc);
     if (e != cudaSuccess) return e;
-    cg_true_residual_kernel<<<rb, kRedThreads, 0, s>>>(W.r, W.w, P->mult, P->multf, n, W.st,
+    launch_chained(n, cg_true_residual_kernel, rb, kRedThreads, 0, s, W.r, W.w, P->mult,
+                   P->multf, n, W.st,
                                                        W.partials, W.counter);
   }
   return cudaGetLastError();
@@ -581,7 +604,7 @@ nb_status cg_start(CgRun &R) {
   init.skip_rc = 1;
   NB_CUDA_TRY(cudaMemcpyAsync(W.st, &init, sizeof(CgState), cudaMemcpyHostToDevice, s));
   const long n = P->n;
-  cg_init_kernel<<<red_blocks(n), kRedThreads, 0, s>>>(
+  launch_chained(n, cg_init_kernel, red_blocks(n), kRedThreads, 0, s, 
       R.x, W.p, W.r, W.fold ? W.z : nullptr, W.use_jacobi ? P->jdiag : nullptr, R.f, P->mult,
       P->multf, n, W.st, W.partials, W.counter);
   NB_CUDA_TRY(cudaGetLastError());

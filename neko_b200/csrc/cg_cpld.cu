@@ -23,6 +23,7 @@
 #include <cstring>
 #include <string>
 
+#include "nb_chain.cuh"
 #include "nb_kernels.h"
 #include "nb_precond.h"
 #include "nb_problem.h"
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(kRedThreads)
     cpld_init_kernel(V3 x, V3 p, V3 r, V3 z, C3 f, const double *__restrict__ d,
                      const double *__restrict__ mult, const float *__restrict__ multf, long n,
                      CgState *st, double *partials, unsigned *counter) {
+  chain();
   double s0 = 0.0, s1 = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
        i += (long)gridDim.x * kRedThreads) {
@@ -87,6 +89,7 @@ __global__ void __launch_bounds__(kRedThreads)
 
 // p_c = z_c + beta p_c
 __global__ void cpld_update_p_kernel(V3 p, C3 z, long n, const CgState *st) {
+  chain();
   if (st->done) return;
   const double beta = st->beta;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
@@ -100,6 +103,7 @@ __global__ void __launch_bounds__(kRedThreads)
     cpld_pap_kernel(C3 w, C3 p, const double *__restrict__ mult,
                     const float *__restrict__ multf, long n, CgState *st, double *partials,
                     unsigned *counter) {
+  chain();
   if (st->done) return;
   double s = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
@@ -119,6 +123,7 @@ __global__ void __launch_bounds__(kRedThreads, 4)
                        const double *__restrict__ d, const double *__restrict__ mult,
                        const float *__restrict__ multf, long n, CgState *st, double *partials,
                        unsigned *counter) {
+  chain();
   if (st->done) return;
   const V3 x = *xp;  // the solve's x, y, z (device copy: one graph for every solve)
   const double alpha = st->alpha, alphm = -alpha;
@@ -266,7 +271,8 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
   init.max_iter = o.max_iter;
   NB_CUDA_TRY(cudaMemcpyAsync(W.st, &init, sizeof(init), cudaMemcpyHostToDevice, s));
   NB_CUDA_TRY(cudaMemcpyAsync(W.xdev, &x, sizeof(V3), cudaMemcpyHostToDevice, s));
-  cpld_init_kernel<<<rb, kRedThreads, 0, s>>>(x, p, r, z, f, d, P->mult, P->multf, n, W.st,
+  launch_chained(3 * n, cpld_init_kernel, rb, kRedThreads, 0, s, x, p, r, z, f, d, P->mult,
+                 P->multf, n, W.st,
                                               W.partials, W.counter);
   NB_CUDA_TRY(cudaGetLastError());
   // x, y, z are read from the device copy: the graph depends on neither
@@ -299,15 +305,17 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
         ce = fe;
         break;
       } else {
-        cpld_update_p_kernel<<<eg, 256, 0, cs>>>(p, zc, n, W.st);
+        launch_chained(3 * n, cpld_update_p_kernel, eg, 256, 0, cs, p, zc, n, W.st);
         ce = cudaGetLastError();
         if (ce == cudaSuccess) ce = cpld_op(P, op, w, p, &W.st->done, cs);
         if (ce == cudaSuccess)
-          cpld_pap_kernel<<<rb, kRedThreads, 0, cs>>>(wc, pc, P->mult, P->multf, n, W.st,
+          launch_chained(3 * n, cpld_pap_kernel, rb, kRedThreads, 0, cs, wc, pc, P->mult,
+                         P->multf, n, W.st,
                                                       W.partials, W.counter);
       }
       if (ce == cudaSuccess) {
-        cpld_update_kernel<<<wave_blocks(n), kRedThreads, 0, cs>>>(W.xdev, r, z, pc, wc, d, P->mult,
+        launch_chained(3 * n, cpld_update_kernel, wave_blocks(n), kRedThreads, 0, cs, W.xdev, r,
+                       z, pc, wc, d, P->mult,
                                                        P->multf, n, W.st, W.partials, W.counter);
         ce = cudaGetLastError();
       }

@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstdlib>
 
+#include "nb_chain.cuh"
 #include "nb_kernels.h"
 #include "nb_gs.h"
 #include "nb_gs_dev.cuh"
@@ -103,21 +104,22 @@ __global__ void __launch_bounds__(256) gs_add_warp_kernel(const GsVec<T, NC> vec
                                                           const GsDevice g, bool with_mask,
                                                           const int *__restrict__ skip,
                                                           const T *__restrict__ scale) {
-  if (skip && *skip) return;
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const long nwarps = (g.nchunk + CPW - 1) / CPW;
-  if (t < 32 * nwarps) {  // whole warps
-    const int lane = threadIdx.x & 31;
-    const long c0 = (t >> 5) * CPW;
-    int idx[CPW];
-    unsigned head[CPW];
-    T v[CPW][NC];
+  const int lane = threadIdx.x & 31;
+  const long c0 = (t >> 5) * CPW;
+  int idx[CPW];
+  unsigned head[CPW];
 #pragma unroll
-    for (int j = 0; j < CPW; j++) {
-      const bool ok = c0 + j < g.nchunk;  // uniform over the warp
-      idx[j] = ok ? __ldg(g.lane_idx + 32 * (c0 + j) + lane) : -1;
-      head[j] = ok ? __ldg(g.lane_head + c0 + j) : 0xffffffffu;
-    }
+  for (int j = 0; j < CPW; j++) {  // the maps are read while the predecessor ends
+    const bool ok = c0 + j < g.nchunk;  // uniform over the warp
+    idx[j] = ok ? __ldg(g.lane_idx + 32 * (c0 + j) + lane) : -1;
+    head[j] = ok ? __ldg(g.lane_head + c0 + j) : 0xffffffffu;
+  }
+  chain();
+  if (skip && *skip) return;
+  if (t < 32 * nwarps) {  // whole warps
+    T v[CPW][NC];
 #pragma unroll
     for (int j = 0; j < CPW; j++)
 #pragma unroll
@@ -184,7 +186,8 @@ static void launch_warp_form(const GsDevice &g, const GsVec<T, NC> &u, bool with
   const long total = 32L * ((g.nchunk + CPW - 1) / CPW) + g.nlong + (with_mask ? g.nextra : 0);
   const int threads = 256;
   const int blocks = (int)((total + threads - 1) / threads);
-  gs_add_warp_kernel<T, CPW, NC><<<blocks, threads, 0, s>>>(u, g, with_mask, skip, scale);
+  launch_chained(32L * NC * g.nchunk, gs_add_warp_kernel<T, CPW, NC>, blocks, threads, 0, s, u,
+                 g, with_mask, skip, scale);
 }
 
 template <typename T>

@@ -41,6 +41,7 @@
 #include <cmath>
 #include <string>
 
+#include "nb_chain.cuh"
 #include "nb_cluster.cuh"
 #include "nb_gs_dev.cuh"
 #include "nb_nodes.h"
@@ -66,6 +67,7 @@ __global__ void __launch_bounds__(256)
     coarse_restrict_kernel(const T *__restrict__ w_mid, const T *__restrict__ mult_m,
                            const T *__restrict__ J, double *__restrict__ f, long nc,
                            const int *__restrict__ skip) {
+  chain();
   if (skip && *skip) return;
   constexpr int M3 = LM * LM * LM;
   constexpr int NE = 32;  // elements a block: its products read once, coalesced
@@ -146,6 +148,7 @@ __device__ __forceinline__ double node_rhs(const NodeOp &A, const double *__rest
 // The solve with at most one row a thread: all of z and p in every block's
 // shared memory.
 __global__ void __launch_bounds__(kCoarseThreads) coarse_cg_resident_kernel(const CoarseCg a) {
+  chain();
   if (a.skip && *a.skip) return;
   extern __shared__ __align__(16) unsigned char coarse_smem[];
   __shared__ ClusterSums sums;
@@ -615,10 +618,12 @@ cudaError_t hsmg_coarse_restrict(const CoarseArgs<T> &a, int lm, const int *skip
   const unsigned grid = (unsigned)((nc + 255) / 256);
   switch (lm) {
     case 3:
-      coarse_restrict_kernel<T, 3><<<grid, 256, 0, s>>>(a.w_mid, a.mult_m, a.J, a.f, nc, skip);
+      launch_chained(nc, coarse_restrict_kernel<T, 3>, grid, 256, 0, s, a.w_mid, a.mult_m, a.J,
+                     a.f, nc, skip);
       break;
     case 4:
-      coarse_restrict_kernel<T, 4><<<grid, 256, 0, s>>>(a.w_mid, a.mult_m, a.J, a.f, nc, skip);
+      launch_chained(nc, coarse_restrict_kernel<T, 4>, grid, 256, 0, s, a.w_mid, a.mult_m, a.J,
+                     a.f, nc, skip);
       break;
     default: return cudaErrorNotSupported;
   }
@@ -650,7 +655,7 @@ cudaError_t hsmg_coarse_cg(const CoarseCg &a, const int *skip, cudaStream_t s) {
   int limit = 0, nblk = 1;
   cudaError_t e;
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at;
+  cudaLaunchAttribute at[2];
   if (A.val) {  // assembled: z, p and, where it fits, the matrix resident
     if ((e = resident_limit(limit)) != cudaSuccess) return e;
     while (nblk < limit && nblk * kCoarseRowsPerBlock < A.nn) nblk *= 2;
@@ -658,7 +663,7 @@ cudaError_t hsmg_coarse_cg(const CoarseCg &a, const int *skip, cudaStream_t s) {
     const size_t slice = (size_t)A.maxw * 32 * (sizeof(double) + sizeof(int)),
                  vectors = 2 * (size_t)A.nn * sizeof(double);
     b.stage_slices = vectors + slices * slice <= kCoarseStageBytes ? slices : 0;
-    cluster_config(cfg, at, nblk, vectors + b.stage_slices * slice, s);
+    cluster_config(cfg, at, nblk, vectors + b.stage_slices * slice, s, 8L * a.nelv);
     return cudaLaunchKernelEx(&cfg, coarse_cg_resident_kernel, b);
   }
   // element-local: a block for every 512 points of the middle level, at most one

@@ -8,6 +8,7 @@
 
 #include <cuda_runtime.h>
 
+#include "nb_chain.cuh"
 #include "nb_tma.cuh"
 
 namespace nb {
@@ -80,18 +81,22 @@ __device__ __forceinline__ double row_dot(const double *val, const int *col, int
   return (acc[0] + acc[1]) + acc[2];
 }
 
-inline void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at, int nblk,
-                           size_t bytes, cudaStream_t s) {
+// The cluster launch, chained to its predecessor in the stream when the level
+// has few points (nb_chain.cuh).
+inline void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[2], int nblk,
+                           size_t bytes, cudaStream_t s, long points) {
   cfg = {};
   cfg.gridDim = dim3((unsigned)nblk);
   cfg.blockDim = dim3(kCoarseThreads);
   cfg.dynamicSmemBytes = bytes;
   cfg.stream = s;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = (unsigned)nblk;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)nblk;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = points <= kChainPoints ? 2 : 1;
 }
 
 // Blocks of the largest cluster the device takes for a kernel: 16 (one GPC,
@@ -111,8 +116,8 @@ cudaError_t cluster_limit(K kern, size_t bytes, int *known, int &limit) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
         cudaSuccess) {
       cudaLaunchConfig_t cfg;
-      cudaLaunchAttribute at;
-      cluster_config(cfg, at, kMaxCluster, bytes, nullptr);
+      cudaLaunchAttribute at[2];
+      cluster_config(cfg, at, kMaxCluster, bytes, nullptr, 0);
       int n = 0;
       if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1)
         best = kMaxCluster;

@@ -24,6 +24,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "nb_chain.cuh"
 #include "nb_hsmg.h"
 #include "nb_kernels.h"
 #include "nb_precond.h"
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(FdmCfg<T, NL>::TPE, FdmCfg<T, NL>::MINB)
                const unsigned char *__restrict__ ornt, const T *__restrict__ S,
                const T *__restrict__ lam, const T *__restrict__ eps, T *__restrict__ out,
                int nelv, const int *__restrict__ skip) {
+  chain();
   if (skip && *skip) return;
   using C = FdmCfg<T, NL>;
   constexpr int LX = NL - 2, L2 = LX * LX, L3 = L2 * LX, N2 = C::N2, N3 = C::N3;
@@ -358,6 +360,7 @@ __global__ void __launch_bounds__(256)
     schwarz_post_kernel(const T *__restrict__ ext, const int *__restrict__ fn,
                         const unsigned char *__restrict__ ornt, const T *__restrict__ wt,
                         T *__restrict__ out, long nelv, const int *__restrict__ skip) {
+  chain();
   if (skip && *skip) return;
   constexpr int L3 = LX * LX * LX;
   const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -403,6 +406,7 @@ __global__ void __launch_bounds__(kT3Threads)
                    const T *__restrict__ M, TOUT *__restrict__ out, long nelv,
                    const int *__restrict__ skip, PrologDots dots = PrologDots{},
                    CoarseAdd<T> crs = CoarseAdd<T>{}) {
+  chain();
   if (skip && *skip) return;
   constexpr int I3 = NI * NI * NI, O3 = NO * NO * NO, NT = kT3Threads;
   __shared__ T su[I3], s1[NO * NI * NI], s2[NO * NO * NI], sA[NO * NI];
@@ -550,6 +554,7 @@ __global__ void __launch_bounds__(kT3Threads)
 template <typename TA, typename TB>
 __global__ void convert_kernel(TB *__restrict__ b, const TA *__restrict__ a, long n,
                                const int *__restrict__ skip) {
+  chain();
   if (skip && *skip) return;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
        i += (long)gridDim.x * blockDim.x)
@@ -590,10 +595,10 @@ static cudaError_t launch_fdm_post(const SchwarzLevel<T> &L, const TIN *r, T *e,
     if (err != cudaSuccess) return err;
     attr_set = true;
   }
-  kern<<<(unsigned)((L.nelv + C::EPW - 1) / C::EPW), C::TPE, C::SMEM, s>>>(
-      r, L.fn, L.ornt, L.S, L.lam, L.eps, L.ext, (int)L.nelv, skip);
+  launch_chained(4 * L.nelv * C::N3, kern, (unsigned)((L.nelv + C::EPW - 1) / C::EPW), C::TPE,
+                 C::SMEM, s, r, L.fn, L.ornt, L.S, L.lam, L.eps, L.ext, (int)L.nelv, skip);
   const long n = L.nelv * LX * LX * LX;
-  schwarz_post_kernel<T, LX><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
+  launch_chained(4 * n, schwarz_post_kernel<T, LX>, (unsigned)((n + 255) / 256), 256, 0, s, 
       L.ext, L.fn, L.ornt, L.wt, e, L.nelv, skip);
   return cudaGetLastError();
 }
@@ -708,8 +713,9 @@ static cudaError_t restrict_level(int ni, int no, const TIN *in, const TIN *scal
                                   const float *scale_f = nullptr) {
 #define NB_R(A, B)                                                                          \
   if (ni == A && no == B) {                                                                 \
-    tensor3_kernel<TIN, TOUT, T, A, B, true, false><<<(unsigned)nelv, kT3Threads, 0, s>>>(         \
-        in, scale, scale_f, J, out, nelv, skip);                                            \
+    launch_chained(4 * nelv * A * A * A, tensor3_kernel<TIN, TOUT, T, A, B, true, false>,   \
+                   (unsigned)nelv, kT3Threads, 0, s,          \
+        in, scale, scale_f, J, out, nelv, skip, PrologDots{}, CoarseAdd<T>{});              \
     return cudaGetLastError();                                                              \
   }
   NB_R(4, 2) NB_R(3, 2) NB_R(5, 4) NB_R(6, 4) NB_R(7, 4) NB_R(8, 4) NB_R(9, 4) NB_R(10, 4)
@@ -729,11 +735,12 @@ static cudaError_t prolong_add(int ni, int no, const TIN *in, const T *J, TOUT *
   if (ni == A && no == B) {                                                                 \
     const unsigned g = (unsigned)nelv;                                                      \
     if (dots)                                                                               \
-      tensor3_kernel<TIN, TOUT, T, A, B, false, true, true>                                 \
-          <<<g, kT3Threads, 0, s>>>(in, oscale, oscale_f, J, out, nelv, skip, d0, crs);          \
+      launch_chained(4 * nelv * B * B * B, tensor3_kernel<TIN, TOUT, T, A, B, false, true, true>,\
+                     g, kT3Threads, 0, s, in, oscale, oscale_f, J, out, nelv, skip, d0,     \
+                     crs);          \
     else                                                                                    \
-      tensor3_kernel<TIN, TOUT, T, A, B, false, true>                                       \
-          <<<g, kT3Threads, 0, s>>>(in, oscale, oscale_f, J, out, nelv, skip, d0, crs);     \
+      launch_chained(4 * nelv * B * B * B, tensor3_kernel<TIN, TOUT, T, A, B, false, true>, g,\
+                     kT3Threads, 0, s, in, oscale, oscale_f, J, out, nelv, skip, d0, crs);     \
     return cudaGetLastError();                                                              \
   }
   NB_P(2, 4) NB_P(2, 3) NB_P(4, 5) NB_P(4, 6) NB_P(4, 7) NB_P(4, 8) NB_P(4, 9) NB_P(4, 10)
@@ -861,7 +868,8 @@ struct HsmgImpl : public HsmgState {
     cudaError_t e = apply_to(zs, r, skip, s);
     if (e != cudaSuccess) return e;
     if (sizeof(T) == 4)
-      convert_kernel<T, double><<<stream_grid(fine->n, 256), 256, 0, s>>>(z, zs, fine->n, skip);
+      launch_chained(fine->n, convert_kernel<T, double>, stream_grid(fine->n, 256), 256, 0, s, z,
+                     zs, fine->n, skip);
     return cudaGetLastError();
   }
 

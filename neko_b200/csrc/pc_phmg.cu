@@ -23,6 +23,7 @@
 #include <string>
 #include <vector>
 
+#include "nb_chain.cuh"
 #include "nb_hsmg.h"
 #include "nb_kernels.h"
 #include "nb_phmg.h"
@@ -44,6 +45,7 @@ constexpr int kPhThreads = 256;
 
 __global__ void ph_mask_kernel(double *__restrict__ x, const int *__restrict__ msk, int m,
                                const int *skip) {
+  chain();
   PH_SKIP
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < m) x[msk[i] - 1] = 0.0;
@@ -57,6 +59,7 @@ __global__ void ph_cheby_first_kernel(double *__restrict__ x, double *__restrict
                                       const double *__restrict__ w,
                                       const double *__restrict__ dinv, double inv_tha, long n,
                                       int zero, const int *skip) {
+  chain();
   PH_SKIP
   PH_LOOP(i, n) {
     const double r = zero ? f[i] : f[i] - w[i];
@@ -73,6 +76,7 @@ __global__ void ph_cheby_step_kernel(double *__restrict__ x, double *__restrict_
                                      const double *__restrict__ w,
                                      const double *__restrict__ dinv, double tmp1, double tmp2,
                                      long n, const int *skip) {
+  chain();
   PH_SKIP
   PH_LOOP(i, n) {
     const double z = (f[i] - w[i]) * dinv[i];
@@ -86,6 +90,7 @@ __global__ void ph_cheby_step_kernel(double *__restrict__ x, double *__restrict_
 __global__ void ph_resid_weight_kernel(double *__restrict__ w, const double *__restrict__ r,
                                        const double *__restrict__ mult, long n,
                                        const int *skip) {
+  chain();
   PH_SKIP
   PH_LOOP(i, n) w[i] = (-1.0 * w[i] + r[i]) * mult[i];
 }
@@ -93,6 +98,7 @@ __global__ void ph_resid_weight_kernel(double *__restrict__ w, const double *__r
 // Correction after prolongation: z = z + w * mult (col2, add2).
 __global__ void ph_correct_kernel(double *__restrict__ z, const double *__restrict__ w,
                                   const double *__restrict__ mult, long n, const int *skip) {
+  chain();
   PH_SKIP
   PH_LOOP(i, n) z[i] = z[i] + w[i] * mult[i];
 }
@@ -105,6 +111,7 @@ __global__ void ph_tensor_kernel(double *__restrict__ v, int nv, const double *_
                                  int nu, const double *__restrict__ A,
                                  const double *__restrict__ Bt, const double *__restrict__ Ct,
                                  const int *skip) {
+  chain();
   PH_SKIP
   extern __shared__ double sm[];
   const int nu3 = nu * nu * nu, nvu2 = nv * nu * nu, nv2u = nv * nv * nu;
@@ -140,6 +147,7 @@ __global__ void ph_tensor_kernel(double *__restrict__ v, int nv, const double *_
 // AMG prolongation and the flat matvec's map to level 0).
 __global__ void amg_spread_kernel(double *__restrict__ out, const double *__restrict__ in,
                                   const int *__restrict__ node, long n, const int *skip) {
+  chain();
   PH_SKIP
   PH_LOOP(i, n) out[i] = in[node[i]];
 }
@@ -150,6 +158,7 @@ __global__ void amg_spread_kernel(double *__restrict__ out, const double *__rest
 __global__ void amg_sum_kernel(double *__restrict__ out, const double *__restrict__ in,
                                const int *__restrict__ ptr, const int *__restrict__ idx,
                                const double *__restrict__ scale, int nn, const int *skip) {
+  chain();
   PH_SKIP
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nn; c += gridDim.x * blockDim.x) {
     double acc = 0.0;
@@ -168,6 +177,7 @@ __global__ void amg_cheby_first_kernel(double *__restrict__ r, const double *__r
                                        const double *__restrict__ w, double *__restrict__ x,
                                        double *__restrict__ d, double inv_thet, long n,
                                        int zero, const int *skip) {
+  chain();
   PH_SKIP
   PH_LOOP(i, n) {
     const double rt = f[i] - (zero ? 0.0 : w[i]);
@@ -180,6 +190,7 @@ __global__ void amg_cheby_first_kernel(double *__restrict__ r, const double *__r
 __global__ void amg_cheby_step_kernel(double *__restrict__ r, const double *__restrict__ w,
                                       double *__restrict__ d, double *__restrict__ x,
                                       double tmp1, double tmp2, long n, const int *skip) {
+  chain();
   PH_SKIP
   PH_LOOP(i, n) {
     const double rt = r[i] - w[i];
@@ -193,11 +204,13 @@ __global__ void amg_cheby_step_kernel(double *__restrict__ r, const double *__re
 // r = b - r (calc_resid after the matvec); x = x + r (the correction).
 __global__ void amg_resid_kernel(double *__restrict__ r, const double *__restrict__ b, long n,
                                  const int *skip) {
+  chain();
   PH_SKIP
   PH_LOOP(i, n) r[i] = -1.0 * r[i] + b[i];
 }
 __global__ void ph_add2_kernel(double *__restrict__ x, const double *__restrict__ r, long n,
                                const int *skip) {
+  chain();
   PH_SKIP
   PH_LOOP(i, n) x[i] = x[i] + r[i];
 }
@@ -309,7 +322,8 @@ struct PhmgImpl : public Precond {
   cudaError_t op(nb_problem *P, double *w, const double *u, const int *skip, cudaStream_t s) {
     PH_CALL(P->ax_raw(w, u, s, skip));
     if (P->ifh2)
-      PH_LAUNCH(addcol4_kernel<<<grid(P->n), kPhThreads, 0, s>>>(w, P->h2, P->B, u, P->n, skip));
+      PH_LAUNCH(launch_chained(P->n, addcol4_kernel, grid(P->n), kPhThreads, 0, s, w, P->h2,
+                               P->B, u, P->n, skip));
     PH_CALL(gs_add_fused<double>(P->gsd, w, P->nmask > 0, s, skip));
     return cudaSuccess;
   }
@@ -321,7 +335,7 @@ struct PhmgImpl : public Precond {
     const long n = M.P->n;
     cudaError_t e;
     if (!zero && (e = op(M.P, M.w, x, skip, s)) != cudaSuccess) return e;
-    PH_LAUNCH(ph_cheby_first_kernel<<<grid(n), kPhThreads, 0, s>>>(
+    PH_LAUNCH(launch_chained(n, ph_cheby_first_kernel, grid(n), kPhThreads, 0, s, 
         x, M.d, f, M.w, M.dinv, 1.0 / M.tha, n, zero ? 1 : 0, skip));
     const double sig1 = M.tha / M.dlt;
     double rhok = 1.0 / sig1;
@@ -330,7 +344,8 @@ struct PhmgImpl : public Precond {
       const double tmp1 = rhokp1 * rhok, tmp2 = 2.0 * rhokp1 / M.dlt;
       rhok = rhokp1;
       if ((e = op(M.P, M.w, x, skip, s)) != cudaSuccess) return e;
-      PH_LAUNCH(ph_cheby_step_kernel<<<grid(n), kPhThreads, 0, s>>>(x, M.d, f, M.w, M.dinv,
+      PH_LAUNCH(launch_chained(n, ph_cheby_step_kernel, grid(n), kPhThreads, 0, s, x, M.d, f,
+                               M.w, M.dinv,
                                                                      tmp1, tmp2, n, skip));
     }
     return cudaSuccess;
@@ -340,7 +355,8 @@ struct PhmgImpl : public Precond {
                      const double *Bt, const double *Ct, const int *skip, cudaStream_t s) {
     const size_t smem = sizeof(double) * ((size_t)nu * nu * nu + (size_t)nv * nu * nu +
                                           (size_t)nv * nv * nu);
-    PH_LAUNCH(ph_tensor_kernel<<<nelv, 128, smem, s>>>(v, nv, u, nu, Am, Bt, Ct, skip));
+    PH_LAUNCH(launch_chained((long)nelv * std::max(nu, nv) * nu * nv, ph_tensor_kernel, nelv,
+                             128, smem, s, v, nv, u, nu, Am, Bt, Ct, skip));
     return cudaSuccess;
   }
 
@@ -349,16 +365,19 @@ struct PhmgImpl : public Precond {
     nb_problem *C = A.C;
     if (l == 0) return op(C, out, in, skip, s);
     const bool m = C->nmask > 0;
-    PH_LAUNCH(amg_spread_kernel<<<grid(C->n), kPhThreads, 0, s>>>(A.wi, in, A.fnode[l], C->n,
+    PH_LAUNCH(launch_chained(C->n, amg_spread_kernel, grid(C->n), kPhThreads, 0, s, A.wi, in,
+                             A.fnode[l], C->n,
                                                                    skip));
     PH_CALL(gs_add_fused<double>(C->gsd, A.wi, m, s, skip, (const double *)C->mult));
     PH_CALL(C->ax_raw(A.wo, A.wi, s, skip));
     if (C->ifh2)
-      PH_LAUNCH(addcol4_kernel<<<grid(C->n), kPhThreads, 0, s>>>(A.wo, C->h2, C->B, A.wi, C->n,
+      PH_LAUNCH(launch_chained(C->n, addcol4_kernel, grid(C->n), kPhThreads, 0, s, A.wo, C->h2,
+                               C->B, A.wi, C->n,
                                                                   skip));
     PH_CALL(gs_add_fused<double>(C->gsd, A.wo, m, s, skip, (const double *)C->mult));
     const int nn = (int)A.n[l];
-    PH_LAUNCH(amg_sum_kernel<<<(nn + 127) / 128, 128, 0, s>>>(out, A.wo, A.fptr[l], A.fidx[l],
+    PH_LAUNCH(launch_chained(nn, amg_sum_kernel, (nn + 127) / 128, 128, 0, s, out, A.wo,
+                             A.fptr[l], A.fidx[l],
                                                                nullptr, nn, skip));
     return cudaSuccess;
   }
@@ -369,7 +388,7 @@ struct PhmgImpl : public Precond {
     const long n = A.n[l];
     cudaError_t e;
     if (!zero && (e = matvec(l, A.w[l], x, skip, s)) != cudaSuccess) return e;
-    PH_LAUNCH(amg_cheby_first_kernel<<<grid(n), kPhThreads, 0, s>>>(
+    PH_LAUNCH(launch_chained(n, amg_cheby_first_kernel, grid(n), kPhThreads, 0, s, 
         A.cr[l], f, A.w[l], x, A.d[l], 1.0 / A.tha[l], n, zero ? 1 : 0, skip));
     const double s1 = A.tha[l] / A.dlt[l];
     double rhok = 1.0 / s1;
@@ -378,7 +397,8 @@ struct PhmgImpl : public Precond {
       const double rhokp1 = 1.0 / (2.0 * s1 - rhok);
       const double tmp1 = rhokp1 * rhok, tmp2 = 2.0 * rhokp1 / A.dlt[l];
       rhok = rhokp1;
-      PH_LAUNCH(amg_cheby_step_kernel<<<grid(n), kPhThreads, 0, s>>>(A.cr[l], A.w[l], A.d[l], x,
+      PH_LAUNCH(launch_chained(n, amg_cheby_step_kernel, grid(n), kPhThreads, 0, s, A.cr[l],
+                               A.w[l], A.d[l], x,
                                                                       tmp1, tmp2, n, skip));
     }
     return cudaSuccess;
@@ -392,10 +412,11 @@ struct PhmgImpl : public Precond {
     for (int l = 0; l < top; l++) {
       if ((e = amg_cheby(l, A.x[l], A.b[l], zero, skip, s)) != cudaSuccess) return e;
       if ((e = matvec(l, A.r[l], A.x[l], skip, s)) != cudaSuccess) return e;
-      PH_LAUNCH(amg_resid_kernel<<<grid(A.n[l]), kPhThreads, 0, s>>>(A.r[l], A.b[l], A.n[l],
+      PH_LAUNCH(launch_chained(A.n[l], amg_resid_kernel, grid(A.n[l]), kPhThreads, 0, s, A.r[l],
+                               A.b[l], A.n[l],
                                                                       skip));
       const int nn = (int)A.n[l + 1];
-      PH_LAUNCH(amg_sum_kernel<<<(nn + 127) / 128, 128, 0, s>>>(
+      PH_LAUNCH(launch_chained(nn, amg_sum_kernel, (nn + 127) / 128, 128, 0, s, 
           A.b[l + 1], A.r[l], A.rptr[l + 1], A.ridx[l + 1], l == 0 ? C->mult : nullptr, nn,
           skip));
       if (!dry && (e = cudaMemsetAsync(A.x[l + 1], 0, nn * sizeof(double), s)) != cudaSuccess)
@@ -405,13 +426,15 @@ struct PhmgImpl : public Precond {
     if ((e = amg_cheby(top, A.x[top], A.b[top], zero, skip, s)) != cudaSuccess) return e;
     zero = false;
     for (int l = top - 1; l >= 0; l--) {
-      PH_LAUNCH(amg_spread_kernel<<<grid(A.n[l]), kPhThreads, 0, s>>>(A.r[l], A.x[l + 1],
+      PH_LAUNCH(launch_chained(A.n[l], amg_spread_kernel, grid(A.n[l]), kPhThreads, 0, s, A.r[l],
+                               A.x[l + 1],
                                                                        A.spread[l + 1], A.n[l],
                                                                        skip));
       if (l == 0)
         PH_CALL(gs_add_fused<double>(C->gsd, A.r[0], C->nmask > 0, s, skip,
                                      (const double *)C->mult));
-      PH_LAUNCH(ph_add2_kernel<<<grid(A.n[l]), kPhThreads, 0, s>>>(A.x[l], A.r[l], A.n[l], skip));
+      PH_LAUNCH(launch_chained(A.n[l], ph_add2_kernel, grid(A.n[l]), kPhThreads, 0, s, A.x[l],
+                               A.r[l], A.n[l], skip));
       if ((e = amg_cheby(l, A.x[l], A.b[l], false, skip, s)) != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -428,7 +451,8 @@ struct PhmgImpl : public Precond {
       double *x = l == 0 ? z : M.z;
       if ((e = cheby(l, x, f, true, skip, s)) != cudaSuccess) return e;
       if ((e = op(M.P, M.w, x, skip, s)) != cudaSuccess) return e;
-      PH_LAUNCH(ph_resid_weight_kernel<<<grid(M.P->n), kPhThreads, 0, s>>>(M.w, f, M.P->mult,
+      PH_LAUNCH(launch_chained(M.P->n, ph_resid_weight_kernel, grid(M.P->n), kPhThreads, 0, s,
+                               M.w, f, M.P->mult,
                                                                             M.P->n, skip));
       if ((e = tensor(C.r, C.P->lx, M.w, M.P->lx, JT[l + 1], J[l + 1], J[l + 1], skip, s)) !=
           cudaSuccess)
@@ -458,7 +482,8 @@ struct PhmgImpl : public Precond {
           cudaSuccess)
         return e;
       PH_CALL(gs_add_fused<double>(M.P->gsd, M.w, false, s, skip));
-      PH_LAUNCH(ph_correct_kernel<<<grid(M.P->n), kPhThreads, 0, s>>>(x, M.w, M.P->mult, M.P->n,
+      PH_LAUNCH(launch_chained(M.P->n, ph_correct_kernel, grid(M.P->n), kPhThreads, 0, s, x, M.w,
+                               M.P->mult, M.P->n,
                                                                        skip));
       if ((e = cheby(l, x, f, false, skip, s)) != cudaSuccess) return e;
     }

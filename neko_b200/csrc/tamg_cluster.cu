@@ -22,12 +22,14 @@
 // direction d alternates between two buffers for the same reason, and the
 // update x += d of a step is made in the next one (the same additions in the
 // same order), when no other thread reads x any more.
+#include "nb_chain.cuh"
 #include "nb_cluster.cuh"
 #include "nb_tamg.h"
 
 namespace nb {
 
 __global__ void __launch_bounds__(kCoarseThreads) tamg_cycle_kernel(const TamgCluster a) {
+  chain();
   if (a.skip && *a.skip) return;
   const NodeOp &A = a.A;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -213,8 +215,8 @@ cudaError_t tamg_cycle(const TamgCluster &a, const int *skip, cudaStream_t s) {
   TamgCluster b = a;
   b.skip = skip;
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at;
-  cluster_config(cfg, at, nblk, 0, s);
+  cudaLaunchAttribute at[2];
+  cluster_config(cfg, at, nblk, 0, s, a.npts);
   return cudaLaunchKernelEx(&cfg, tamg_cycle_kernel, b);
 }
 
