@@ -32,7 +32,7 @@ sys.path.insert(0, ROOT)
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0}
 
 
-# DRAM bytes per point of ax_cg_fused_kernel measured by ncu on a 24^3-element
+# DRAM bytes per point of the fused CG step (ax_cg_fused) measured by ncu on a 24^3-element
 # case (dram__bytes_read.sum + dram__bytes_write.sum per launch over the
 # points; the part of p and w still dirty in L2 when the launch ends is not
 # counted).
@@ -1020,7 +1020,7 @@ def main():
                         "step k's solve on a second stream",
                 "serial_value": e2e_serial},
         "roofline": {"bound": "hbm",
-                     "kernel": f"ax_cg_fused_kernel<{cfg['lx']}> (p = z + beta p, w = A p, "
+                     "kernel": f"ax_stream_kernel<{cfg['lx']}> (p = z + beta p, w = A p, "
                                f"sum p w; the solve's largest kernel)",
                      "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"],
@@ -1030,7 +1030,7 @@ def main():
                                        "times the points",
                      "peak_source": peak_src, "bytes_per_launch": fused_bytes,
                      "launch_ms": t_fused * 1e3, "gdof_s": P.n / t_fused / 1e9},
-        "ax_helm": {"kernel": f"ax_helm_tma_kernel<double,{cfg['lx']}>",
+        "ax_helm": {"kernel": f"ax_stream_kernel<{cfg['lx']}>",
                     "achieved": ax_bytes / t_ax / 1e9, "unit": "GB/s",
                     "frac": ax_bytes / t_ax / 1e9 / peaks["hbm_gbs"],
                     "bytes_per_launch": ax_bytes, "launch_ms": t_ax * 1e3,

@@ -11,6 +11,7 @@
 // 180-290): ur = Dx u, us = Dy u, ut = Dz u; (ur,us,ut) <- h1 G (ur,us,ut);
 // w = Dxt ur + Dyt us + Dzt ut, with D matrices column-major as passed.
 #include <array>
+#include <initializer_list>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -49,8 +50,8 @@ __global__ void __launch_bounds__(LX *LX *NE)
                    const T *__restrict__ h1, const T *__restrict__ g11,
                    const T *__restrict__ g22, const T *__restrict__ g33,
                    const T *__restrict__ g12, const T *__restrict__ g13,
-                   const T *__restrict__ g23, const int nelv,
-                   const int *__restrict__ skip) {
+                   const T *__restrict__ g23, const T *__restrict__ h2,
+                   const T *__restrict__ Bm, const int nelv, const int *__restrict__ skip) {
   chain();
   if (skip && *skip) return;  // solver finished: uniform early exit
   constexpr int L2 = LX * LX, L3 = L2 * LX;
@@ -121,287 +122,149 @@ __global__ void __launch_bounds__(LX *LX *NE)
     T acc3 = 0;
 #pragma unroll
     for (int l = 0; l < LX; l++) acc3 += sDzt[k + LX * l] * rut[l];
-    if (active) w[base + k * L2] = acc + acc2 + acc3;
+    if (active) {
+      const long g = base + k * L2;
+      T v = acc + acc2 + acc3;
+      if (h2) v = v + __ldg(h2 + g) * __ldg(Bm + g) * ru[k];
+      w[g] = v;
+    }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Streaming variant for the native solver: a persistent kernel in which each
-// CTA walks its share of the elements (e = blockIdx.x + t * gridDim.x) and
-// keeps S elements in flight in a shared-memory ring.  One thread issues, per
-// element, eight 1-D bulk copies (u, h1, G11, G22, G33, G12, G13, G23; each
-// lx^3 contiguous values) completing on the stage's mbarrier, so the bytes
-// in flight per SM are S * 8 * lx^3 * sizeof(T) per CTA regardless of
-// register pressure.  KS thread groups split the k-planes of an element:
-// thread (i, j, kh) computes planes [kh*LX/KS, (kh+1)*LX/KS).
-// ---------------------------------------------------------------------------
-template <typename T, int LX, int S, int KS>
-struct AxTmaCfg {
-  static constexpr int L2 = LX * LX, L3 = L2 * LX, NA = 8;
-  static constexpr int THREADS = ((L2 * KS + 31) / 32) * 32;
-  static constexpr size_t ABYTES = (size_t)L3 * sizeof(T);
-  static constexpr size_t SMEM = S * NA * ABYTES + 3 * ABYTES + 2 * L2 * sizeof(T) + 16 * S;
-};
-
-template <typename T, int LX, int S, int KS>
-__global__ void __launch_bounds__(AxTmaCfg<T, LX, S, KS>::THREADS)
-    ax_helm_tma_kernel(T *__restrict__ w, const T *__restrict__ u, const T *__restrict__ D,
-                       const T *__restrict__ Dt, const T *__restrict__ h1,
-                       const T *__restrict__ g11, const T *__restrict__ g22,
-                       const T *__restrict__ g33, const T *__restrict__ g12,
-                       const T *__restrict__ g13, const T *__restrict__ g23, const int nelv,
-                       const int *__restrict__ skip, int *__restrict__ err) {
-  using C = AxTmaCfg<T, LX, S, KS>;
-  constexpr int L2 = C::L2, L3 = C::L3, NA = C::NA, KP = LX / KS;
-  static_assert(LX % KS == 0, "k split must divide lx");
-  extern __shared__ __align__(128) unsigned char smem_ring[];
-  T *stage = reinterpret_cast<T *>(smem_ring);
-  T *sur = stage + S * NA * L3, *sus = sur + L3, *sut = sus + L3;
-  T *sD = sut + L3, *sDt = sD + L2;
-  uint64_t *full = reinterpret_cast<uint64_t *>(sDt + L2);
-
-  const int tid = threadIdx.x;
-  const int G = gridDim.x, b = blockIdx.x;
-  const int nt = b < nelv ? (nelv - b + G - 1) / G : 0;
-  if (tid == 0) {
-    for (int s = 0; s < S; s++) mbar_init(&full[s], 1);
-    fence_barrier_init();
-  }
-  chain();
-  if (skip && *skip) return;
-  for (int q = tid; q < L2; q += C::THREADS) {
-    sD[q] = D[q];
-    sDt[q] = Dt[q];
-  }
-  __syncthreads();
-  const T *src[NA] = {u, h1, g11, g22, g33, g12, g13, g23};
-  auto issue = [&](int t, int s) {
-    const long e = b + (long)t * G;
-    mbar_arrive_expect_tx(&full[s], (uint32_t)(NA * C::ABYTES));
-#pragma unroll
-    for (int a = 0; a < NA; a++)
-      bulk_g2s(stage + (size_t)(s * NA + a) * L3, src[a] + e * L3, (uint32_t)C::ABYTES, &full[s]);
-  };
-  if (tid == 0)
-    for (int t = 0; t < S && t < nt; t++) issue(t, t);
-
-  const bool act = tid < L2 * KS;
-  const int col = tid % L2, kh = tid / L2;
-  const int i = col % LX, j = col / LX, k0 = kh * KP;
-  T Di[LX], Dj[LX], Dti[LX], Dtj[LX];
-#pragma unroll
-  for (int l = 0; l < LX; l++) {
-    Di[l] = sD[i + LX * l];
-    Dj[l] = sD[j + LX * l];
-    Dti[l] = sDt[i + LX * l];
-    Dtj[l] = sDt[j + LX * l];
-  }
-
-  int t = 0;
-  bool failed = false;
-  for (; t < nt; t++) {
-    const int s = t % S;
-    const bool ok = mbar_wait(&full[s], (uint32_t)((t / S) & 1));
-    if (__syncthreads_or(!ok)) {
-      failed = true;
-      break;
-    }
-    const T *su = stage + (size_t)s * NA * L3;
-    const T *sh = su + L3, *s11 = su + 2 * L3, *s22 = su + 3 * L3, *s33 = su + 4 * L3,
-            *s12 = su + 5 * L3, *s13 = su + 6 * L3, *s23 = su + 7 * L3;
-    if (act) {
-      T ru[LX];
-#pragma unroll
-      for (int l = 0; l < LX; l++) ru[l] = su[col + L2 * l];
-#pragma unroll
-      for (int kk = 0; kk < KP; kk++) {
-        const int k = k0 + kk;
-        T ur = 0, us = 0, ut = 0;
-#pragma unroll
-        for (int l = 0; l < LX; l++) {
-          ur += Di[l] * su[l + LX * j + L2 * k];
-          us += Dj[l] * su[i + LX * l + L2 * k];
-          ut += sD[k + LX * l] * ru[l];
-        }
-        const int p = col + L2 * k;
-        const T H = sh[p];
-        const T a11 = s11[p], a22 = s22[p], a33 = s33[p], a12 = s12[p], a13 = s13[p],
-                a23 = s23[p];
-        sur[p] = H * (a11 * ur + a12 * us + a13 * ut);
-        sus[p] = H * (a12 * ur + a22 * us + a23 * ut);
-        sut[p] = H * (a13 * ur + a23 * us + a33 * ut);
-      }
-    }
-    __syncthreads();  // stage s consumed, work planes complete
-    if (tid == 0 && t + S < nt) issue(t + S, s);
-    if (act) {
-      T rt[LX];
-#pragma unroll
-      for (int l = 0; l < LX; l++) rt[l] = sut[col + L2 * l];
-      const long e = b + (long)t * G;
-#pragma unroll
-      for (int kk = 0; kk < KP; kk++) {
-        const int k = k0 + kk;
-        T a = 0, c = 0, d = 0;
-#pragma unroll
-        for (int l = 0; l < LX; l++) {
-          a += Dti[l] * sur[l + LX * j + L2 * k];
-          c += Dtj[l] * sus[i + LX * l + L2 * k];
-          d += sDt[k + LX * l] * rt[l];
-        }
-        w[e * L3 + col + L2 * k] = a + c + d;
-      }
-    }
-    __syncthreads();  // work planes free for the next element
-  }
-  if (failed) {
-    if (tid == 0) {
-      atomicExch(err ? err : &nb_dropin_error, 1);
-      // bounded wait for this CTA's copies still in flight
-      for (int q = t; q < nt && q < t + S; q++) mbar_wait(&full[q % S], (uint32_t)((q / S) & 1));
-    }
-    __syncthreads();
-  }
-}
-
-template <typename T, int LX, int S, int KS>
-static cudaError_t launch_ax_tma(T *w, const T *u, const T *D, const T *Dt, const T *h1,
-                                 const T *g11, const T *g22, const T *g33, const T *g12,
-                                 const T *g13, const T *g23, int nelv, cudaStream_t st,
-                                 const int *skip, int *err) {
-  using C = AxTmaCfg<T, LX, S, KS>;
-  auto kern = ax_helm_tma_kernel<T, LX, S, KS>;
-  static int grid_per_dev[64] = {0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  int &g = grid_per_dev[dev & 63];
-  if (g == 0) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0, sms = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::THREADS, C::SMEM);
-    if (e != cudaSuccess) return e;
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    g = (per_sm > 0 ? per_sm : 1) * sms;
-  }
-  if (nelv <= 0) return cudaSuccess;
-  const int grid = nelv < g ? nelv : g;
-  launch_chained((long)nelv * C::L3, kern, grid, C::THREADS, C::SMEM, st, w, u, D, Dt, h1, g11,
-                 g22, g33, g12, g13, g23, nelv,
-                                          skip, err);
-  return cudaGetLastError();
-}
-
-// Dispatch of the streaming variant; returns cudaErrorNotSupported when no
-// instantiation covers (T, lx) or a pointer is not 16-byte aligned.
-template <typename T>
-cudaError_t ax_helm_stream(T *w, const T *u, const T *D, const T *Dt, const T *h1,
-                           const T *g11, const T *g22, const T *g33, const T *g12,
-                           const T *g13, const T *g23, int nelv, int lx, cudaStream_t s,
-                           const int *skip, int *err) {
-  const void *ptrs[] = {u, h1, g11, g22, g33, g12, g13, g23};
-  for (const void *p : ptrs)
-    if (reinterpret_cast<uintptr_t>(p) & 15) return cudaErrorNotSupported;
-  if (((size_t)lx * lx * lx * sizeof(T)) % 16) return cudaErrorNotSupported;
-  switch (lx) {
-    case 4: return launch_ax_tma<T, 4, 4, 1>(w, u, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, s, skip, err);
-    case 6: return launch_ax_tma<T, 6, 3, 2>(w, u, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, s, skip, err);
-    case 8: return launch_ax_tma<T, 8, 3, 2>(w, u, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, s, skip, err);
-    case 10: return launch_ax_tma<T, 10, 2, 5>(w, u, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, s, skip, err);
-    default: return cudaErrorNotSupported;
-  }
-}
-// ---------------------------------------------------------------------------
-// The streaming kernel fused with the two CG steps around it: p = z + beta p
-// (cg_update_p), w = A p (element-local, before the gather-scatter, with the
-// h2 B p term when H2), and pap = sum over the local points of p * w with
-// alpha = rtz / pap (cg_pap).  p is continuous and zero on masked points (z
-// is), so the local sum equals (p, mult gs(w)) with the mask, the form the
-// reference evaluates after the gather-scatter (cg_device.f90:211-214): each
-// global point's weights 1/k over its k copies add up to one.  The ring
-// carries z and the old p in place of u; each thread forms the new p for its
-// own points, stores it, and the element's operator then reads it from the
-// stage.  h2 and B are read by each thread for its own points, so they cost
-// no shared memory; they are brought to L2 when the element's stage is filled,
-// as their latency is not hidden behind the wait otherwise (139 us against the
-// 112 us of its 736 MB at 7.1 M points).  Returns at once when st->done is
-// set.
+// Streaming form: a persistent kernel in which each CTA walks its share of the
+// elements and keeps S of them in flight in a shared-memory ring.  One thread
+// issues, per element, 1-D bulk copies of the arrays it needs (u, h1, G11,
+// G22, G33, G12, G13, G23; each lx^3 contiguous values) completing on the
+// stage's mbarrier, so the bytes in flight per SM do not depend on register
+// pressure.  KS thread groups split the k-planes of an element: thread
+// (i, j, kh) computes planes [kh KP, (kh + 1) KP).
 //
-// Bound by HBM: 88 B a point, 104 with h2 (the separate passes: direction 24,
-// operator 72, h2 term 40, curvature 20).
+// A bulk copy moves whole 16-byte units, and lx^3 doubles are none for odd lx:
+// those orders stream two elements a stage (NE = 2), which start on a 16-byte
+// boundary whenever the array does.  The last element of an odd count arrives
+// as lx^3 - 1 copied values and one stored by the issuing thread.  At lx 7 and
+// 6.8 M points the general kernel took 181 us (260 with h2), this form takes
+// 101 (127): the blocks of the general kernel each wait for their own loads,
+// several times an element.
+//
+// With CG the kernel is fused with the two CG steps around the operator:
+// p = z + beta p (cg_update_p), w = A p (element-local, before the
+// gather-scatter), and pap = sum over the local points of p * w with alpha =
+// rtz / pap (cg_pap).  p is continuous and zero on masked points (z is), so
+// the local sum equals (p, mult gs(w)) with the mask, the form the reference
+// evaluates after the gather-scatter (cg_device.f90:211-214): each global
+// point's weights 1/k over its k copies add up to one.  The ring carries z
+// and the old p in place of u; each thread forms the new p for its own
+// points, stores it, and the element's operator then reads it from the stage.
+//
+// The h2 B u term, when h2 is given, is added in the same pass: each thread
+// reads h2 and B for its own points, so they cost no shared memory; they are
+// brought to L2 when the stage is filled, as their latency is not hidden
+// behind the wait otherwise (139 us against the 112 us of 736 MB for a fused
+// step on 7.1 M points, now 118).
+//
+// Bound by HBM: 72 B a point, 88 with the step, 16 more with h2; the next
+// limiter is the shared-memory pipe (81 % at lx 8).  At 7.1 M points and lx 8 the
+// step takes 105 us, 91 % of the measured copy rate (140 in three launches).
 // ---------------------------------------------------------------------------
-// AL (lx = 10): the three work planes live in the stage itself, over the
-// G11, G22, G33 arrays of the element being computed (each thread reads the
-// six factors of a point before it writes that point's three fluxes, and no
-// thread reads another point's factors), which frees the room for a third
-// stage; the stage is then refilled after the second pass instead of the
-// first, so two elements are in flight while one is computed.
-template <int LX, int S, int KS, bool AL = false>
-struct AxCgCfg {
-  static constexpr int L2 = LX * LX, L3 = L2 * LX, NA = 9;
-  static constexpr int THREADS = ((L2 * KS + 31) / 32) * 32;
-  static constexpr size_t ABYTES = (size_t)L3 * sizeof(double);
+// AL: the three work planes live in the stage itself, over the G11, G22, G33
+// arrays of the element being computed (each thread reads the six factors of a
+// point before it writes that point's three fluxes, and no thread reads
+// another point's factors), which frees room for a further stage or block; the
+// stage is then refilled after the second pass instead of the first.  At lx 8
+// the plain operator takes 88.2 us so at 7.1 M points, 90.2 otherwise; at lx 9
+// with h2 150 against 166.
+template <int LX, int S, int KS, int NE, bool CG, bool AL>
+struct AxCfgS {
+  static constexpr int L2 = LX * LX, L3 = L2 * LX, NA = CG ? 9 : 8;
+  static constexpr int KP = (LX + KS - 1) / KS;
+  static constexpr int THREADS = ((L2 * KS * NE + 31) / 32) * 32;
+  static constexpr size_t ABYTES = (size_t)L3 * sizeof(double);  // one array of one element
   static constexpr size_t SMEM =
-      S * NA * ABYTES + (AL ? 0 : 3 * ABYTES) + 2 * L2 * sizeof(double) + 16 * S;
+      (S * NA + (AL ? 0 : 3)) * NE * ABYTES + 2 * L2 * sizeof(double) + 16 * S;
+  static_assert((NE * L3 * sizeof(double)) % 16 == 0, "stage arrays are whole 16-byte units");
 };
 
-template <int LX, int S, int KS, typename TZ, bool AL, bool H2>
-__global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
-    ax_cg_fused_kernel(double *__restrict__ w, double *__restrict__ p,
-                       const TZ *__restrict__ z, const double *__restrict__ D,
-                       const double *__restrict__ Dt, const double *__restrict__ h1,
-                       const double *__restrict__ g11, const double *__restrict__ g22,
-                       const double *__restrict__ g33, const double *__restrict__ g12,
-                       const double *__restrict__ g13, const double *__restrict__ g23,
-                       const double *__restrict__ h2, const double *__restrict__ Bm,
-                       const int nelv, CgState *st, double beta_arg, double *pap_out,
-                       double *partials, unsigned *counter, int *__restrict__ err) {
-  using C = AxCgCfg<LX, S, KS, AL>;
-  constexpr int L2 = C::L2, L3 = C::L3, NA = C::NA, KP = LX / KS, THREADS = C::THREADS;
-  static_assert(LX % KS == 0, "k split must divide lx");
+// Operands; u of the plain operator, or z and p of the fused step.
+template <typename TZ>
+struct AxArgs {
+  double *w;
+  const double *u;
+  double *p;
+  const TZ *z;
+  const double *D, *Dt, *h1, *g[6], *h2, *B;
+  int nelv;
+  const int *skip;
+  int *err;
+  // fused step
+  CgState *st;
+  double beta, *pap_out, *partials;
+  unsigned *counter;
+  int max_grid;
+};
+
+template <int LX, int S, int KS, int NE, bool CG, bool AL, bool H2, typename TZ>
+__global__ void __launch_bounds__(AxCfgS<LX, S, KS, NE, CG, AL>::THREADS)
+    ax_stream_kernel(const AxArgs<TZ> a) {
+  using C = AxCfgS<LX, S, KS, NE, CG, AL>;
+  constexpr int L2 = C::L2, L3 = C::L3, NA = C::NA, KP = C::KP, THREADS = C::THREADS;
+  constexpr int AS = NE * L3;  // one array of a stage
+  constexpr int U0 = CG ? 1 : 0;
+  static_assert(NE == 1 || !CG || sizeof(TZ) == 8, "FP32 z of odd lx is not a whole unit");
   extern __shared__ __align__(128) unsigned char smem_ring[];
   double *stage = reinterpret_cast<double *>(smem_ring);
-  double *sur = stage + S * NA * L3, *sus = sur + L3, *sut = sus + L3;
-  double *sD = AL ? stage + S * NA * L3 : sut + L3, *sDt = sD + L2;
+  double *sD = stage + (S * NA + (AL ? 0 : 3)) * AS, *sDt = sD + L2;
   uint64_t *full = reinterpret_cast<uint64_t *>(sDt + L2);
 
   const int tid = threadIdx.x;
   const int G = gridDim.x, b = blockIdx.x;
-  const int nt = b < nelv ? (nelv - b + G - 1) / G : 0;
+  const int ngroup = (a.nelv + NE - 1) / NE;
+  const int nt = b < ngroup ? (ngroup - b + G - 1) / G : 0;
   if (tid == 0) {
     for (int s = 0; s < S; s++) mbar_init(&full[s], 1);
     fence_barrier_init();
   }
+  chain();
+  if (a.skip && *a.skip) return;
+  if (CG && a.st && a.st->done) return;
+  const double beta = CG ? (a.st ? a.st->beta : a.beta) : 0.0;
   for (int q = tid; q < L2; q += THREADS) {
-    sD[q] = D[q];
-    sDt[q] = Dt[q];
+    sD[q] = a.D[q];
+    sDt[q] = a.Dt[q];
   }
   __syncthreads();
-  chain();
-  if (st && st->done) return;
-  const double beta = st ? st->beta : beta_arg;
-  // z (slot 0) arrives in its own precision: L3 values of TZ
-  constexpr uint32_t ZBYTES = (uint32_t)(L3 * sizeof(TZ));
-  const double *src[NA] = {nullptr, p, h1, g11, g22, g33, g12, g13, g23};
+  // stage arrays: (z, p) or u, h1, G11, G22, G33, G12, G13, G23
   auto issue = [&](int t, int s) {
-    const long e = b + (long)t * G;
-    mbar_arrive_expect_tx(&full[s], (uint32_t)((NA - 1) * C::ABYTES) + ZBYTES);
-    bulk_g2s(stage + (size_t)(s * NA) * L3, z + e * L3, ZBYTES, &full[s]);
+    const long e0 = ((long)b + (long)t * G) * NE;
+    const bool odd = NE == 2 && e0 + 1 == a.nelv;  // the last element alone
+    const uint32_t count = (uint32_t)(odd ? L3 - 1 : AS);  // values an array copies
+    double *base = stage + (size_t)s * NA * AS;
+    auto source = [&](int q) {
+      return q < U0 ? nullptr
+                    : q == U0 ? (CG ? (const double *)a.p : a.u) : q == U0 + 1 ? a.h1 : a.g[q - U0 - 2];
+    };
+    if (odd) {  // its last value of each array, before the arrival below
+      if (CG) reinterpret_cast<TZ *>(base)[L3 - 1] = a.z[e0 * L3 + L3 - 1];
 #pragma unroll
-    for (int a = 1; a < NA; a++)
-      bulk_g2s(stage + (size_t)(s * NA + a) * L3, src[a] + e * L3, (uint32_t)C::ABYTES, &full[s]);
+      for (int q = U0; q < NA; q++) base[(size_t)q * AS + L3 - 1] = source(q)[e0 * L3 + L3 - 1];
+    }
+    const uint32_t zbytes = CG ? count * (uint32_t)sizeof(TZ) : 0u;
+    mbar_arrive_expect_tx(&full[s], (uint32_t)(NA - U0) * count * 8u + zbytes);
+    if (CG) bulk_g2s(base, a.z + e0 * L3, zbytes, &full[s]);
+#pragma unroll
+    for (int q = U0; q < NA; q++)
+      bulk_g2s(base + (size_t)q * AS, source(q) + e0 * L3, count * 8u, &full[s]);
     if (H2) {
-      bulk_prefetch_l2(h2 + e * L3, (uint32_t)C::ABYTES);
-      bulk_prefetch_l2(Bm + e * L3, (uint32_t)C::ABYTES);
+      bulk_prefetch_l2(a.h2 + e0 * L3, count * 8u);
+      bulk_prefetch_l2(a.B + e0 * L3, count * 8u);
     }
   };
   if (tid == 0)
     for (int t = 0; t < S && t < nt; t++) issue(t, t);
 
-  const bool act = tid < L2 * KS;
-  const int col = tid % L2, kh = tid / L2;
+  const int col = tid % L2, part = tid / L2;
+  const int kh = NE == 1 ? part : part % KS, el = NE == 1 ? 0 : part / KS;
   const int i = col % LX, j = col / LX, k0 = kh * KP;
   double Di[LX], Dj[LX], Dti[LX], Dtj[LX];
 #pragma unroll
@@ -417,45 +280,48 @@ __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
   bool failed = false;
   for (; t < nt; t++) {
     const int s = t % S;
-    const long e = b + (long)t * G;
-    double hb[H2 ? KP : 1];  // h2 B at this thread's points
-    if (H2 && act) {
-#pragma unroll
-      for (int kk = 0; kk < KP; kk++) {
-        const long g = e * L3 + col + L2 * (k0 + kk);
-        hb[kk] = __ldg(h2 + g) * __ldg(Bm + g);
-      }
-    }
+    const long e = ((long)b + (long)t * G) * NE + el;
+    const bool act = (L2 * KS * NE == THREADS || tid < L2 * KS * NE) && (NE == 1 || e < a.nelv);
+    auto plane = [&](int kk) { return LX % KS == 0 || k0 + kk < LX; };
     const bool ok = mbar_wait(&full[s], (uint32_t)((t / S) & 1));
     if (__syncthreads_or(!ok)) {
       failed = true;
       break;
     }
-    const TZ *sz = reinterpret_cast<const TZ *>(stage + (size_t)s * NA * L3);
-    double *su = stage + (size_t)s * NA * L3 + L3;  // old p, replaced by the new
-    const double *sh = su + L3, *s11 = su + 2 * L3, *s22 = su + 3 * L3, *s33 = su + 4 * L3,
-                 *s12 = su + 5 * L3, *s13 = su + 6 * L3, *s23 = su + 7 * L3;
+    double *base = stage + (size_t)s * NA * AS;
+    double *su = base + U0 * AS + el * L3;  // u, or the old p replaced by the new
+    const double *sh = su + AS, *s11 = su + 2 * AS, *s22 = su + 3 * AS, *s33 = su + 4 * AS,
+                 *s12 = su + 5 * AS, *s13 = su + 6 * AS, *s23 = su + 7 * AS;
     // work planes: separate, or over this stage's G11, G22, G33 (AL)
-    double *wr = AL ? su + 2 * L3 : sur, *wsp = AL ? su + 3 * L3 : sus,
-           *wtp = AL ? su + 4 * L3 : sut;
-    if (act) {
+    double *wr = AL ? su + 2 * AS : stage + (size_t)S * NA * AS + el * L3, *ws = wr + AS,
+           *wt = ws + AS;
+    if constexpr (CG) {
+      const TZ *sz = reinterpret_cast<const TZ *>(base) + el * L3;
+      if (act) {
 #pragma unroll
-      for (int kk = 0; kk < KP; kk++) {
-        const int q = col + L2 * (k0 + kk);
-        const double pn = (double)sz[q] + beta * su[q];
-        su[q] = pn;
-        p[e * L3 + q] = pn;
+        for (int kk = 0; kk < KP; kk++)
+          if (plane(kk)) {
+            const int q = col + L2 * (k0 + kk);
+            const double pn = (double)sz[q] + beta * su[q];
+            su[q] = pn;
+            a.p[e * L3 + q] = pn;
+          }
       }
+      __syncthreads();  // the new p complete in the stage
     }
-    __syncthreads();  // the element's new p complete in the stage
-    double ru[LX], pown[KP];  // p column; p at this thread's points
+    double own[H2 || CG ? KP : 1];  // u (p) at this thread's points
     if (act) {
+      double ru[LX];  // its column
 #pragma unroll
       for (int l = 0; l < LX; l++) ru[l] = su[col + L2 * l];
+      if constexpr (H2 || CG) {
 #pragma unroll
-      for (int kk = 0; kk < KP; kk++) pown[kk] = su[col + L2 * (k0 + kk)];
+        for (int kk = 0; kk < KP; kk++)
+          if (plane(kk)) own[kk] = su[col + L2 * (k0 + kk)];
+      }
 #pragma unroll
       for (int kk = 0; kk < KP; kk++) {
+        if (!plane(kk)) continue;
         const int k = k0 + kk;
         double ur = 0, us = 0, ut = 0;
 #pragma unroll
@@ -469,30 +335,43 @@ __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
         const double a11 = s11[q], a22 = s22[q], a33 = s33[q], a12 = s12[q], a13 = s13[q],
                      a23 = s23[q];
         wr[q] = H * (a11 * ur + a12 * us + a13 * ut);
-        wsp[q] = H * (a12 * ur + a22 * us + a23 * ut);
-        wtp[q] = H * (a13 * ur + a23 * us + a33 * ut);
+        ws[q] = H * (a12 * ur + a22 * us + a23 * ut);
+        wt[q] = H * (a13 * ur + a23 * us + a33 * ut);
       }
     }
+    // AL: this thread's writes over the factors come before the next copy
+    if (AL || CG) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();  // stage s consumed (but for AL's planes), work planes complete
     if (!AL && tid == 0 && t + S < nt) issue(t + S, s);
     if (act) {
+      double h2v[H2 ? KP : 1], bv[H2 ? KP : 1];  // in flight during the contractions
+      if constexpr (H2) {
+#pragma unroll
+        for (int kk = 0; kk < KP; kk++)
+          if (plane(kk)) {
+            const long g = e * L3 + col + L2 * (k0 + kk);
+            h2v[kk] = __ldg(a.h2 + g);
+            bv[kk] = __ldg(a.B + g);
+          }
+      }
       double rt[LX];
 #pragma unroll
-      for (int l = 0; l < LX; l++) rt[l] = wtp[col + L2 * l];
+      for (int l = 0; l < LX; l++) rt[l] = wt[col + L2 * l];
 #pragma unroll
       for (int kk = 0; kk < KP; kk++) {
+        if (!plane(kk)) continue;
         const int k = k0 + kk;
-        double a = 0, c = 0, d = 0;
+        double x = 0, y = 0, z = 0;
 #pragma unroll
         for (int l = 0; l < LX; l++) {
-          a += Dti[l] * wr[l + LX * j + L2 * k];
-          c += Dtj[l] * wsp[i + LX * l + L2 * k];
-          d += sDt[k + LX * l] * rt[l];
+          x += Dti[l] * wr[l + LX * j + L2 * k];
+          y += Dtj[l] * ws[i + LX * l + L2 * k];
+          z += sDt[k + LX * l] * rt[l];
         }
-        double wq = a + c + d;
-        if (H2) wq = wq + hb[kk] * pown[kk];
-        w[e * L3 + col + L2 * k] = wq;
-        pap += pown[kk] * wq;
+        double wq = x + y + z;
+        if constexpr (H2) wq = wq + h2v[kk] * bv[kk] * own[kk];
+        a.w[e * L3 + col + L2 * k] = wq;
+        if constexpr (CG) pap += own[kk] * wq;
       }
     }
     __syncthreads();  // work planes free for the next element
@@ -500,40 +379,29 @@ __global__ void __launch_bounds__(AxCgCfg<LX, S, KS, AL>::THREADS)
   }
   if (failed) {
     if (tid == 0) {
-      atomicExch(err ? err : &nb_dropin_error, 1);
+      atomicExch(a.err ? a.err : &nb_dropin_error, 1);
       // bounded wait for this CTA's copies still in flight
       for (int q = t; q < nt && q < t + S; q++) mbar_wait(&full[q % S], (uint32_t)((q / S) & 1));
     }
     __syncthreads();
   }
-  double tot;  // every block takes part, a failed one with its partial sum
-  if (grid_sum<THREADS>(pap, partials, counter, &tot)) {
-    if (st) {
-      st->pap = tot;
-      st->alpha = st->rtz1 / tot;
-    } else if (pap_out) {
-      *pap_out = tot;
+  if constexpr (CG) {
+    double tot;  // every block takes part, a failed one with its partial sum
+    if (grid_sum<THREADS>(pap, a.partials, a.counter, &tot)) {
+      if (a.st) {
+        a.st->pap = tot;
+        a.st->alpha = a.st->rtz1 / tot;
+      } else if (a.pap_out) {
+        *a.pap_out = tot;
+      }
     }
   }
 }
 
-// Operands of one fused step (see ax_cg_fused).
-template <typename TZ>
-struct AxCgArgs {
-  double *w, *p;
-  const TZ *z;
-  const double *D, *Dt, *h1, *g[6], *h2, *B;
-  int nelv;
-  CgState *st;
-  double beta, *pap_out, *partials;
-  unsigned *counter;
-  int max_grid, *err;
-};
-
-template <int LX, int S, int KS, typename TZ, bool AL, bool H2>
-static cudaError_t launch_ax_cg(const AxCgArgs<TZ> &a, cudaStream_t s) {
-  using C = AxCgCfg<LX, S, KS, AL>;
-  auto kern = ax_cg_fused_kernel<LX, S, KS, TZ, AL, H2>;
+template <int LX, int S, int KS, int NE, bool CG, bool AL, bool H2, typename TZ>
+static cudaError_t launch_ax_stream_as(const AxArgs<TZ> &a, cudaStream_t st) {
+  using C = AxCfgS<LX, S, KS, NE, CG, AL>;
+  auto kern = ax_stream_kernel<LX, S, KS, NE, CG, AL, H2, TZ>;
   static int grid_per_dev[64] = {0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -549,19 +417,67 @@ static cudaError_t launch_ax_cg(const AxCgArgs<TZ> &a, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     g = (per_sm > 0 ? per_sm : 1) * sms;
   }
-  int grid = a.nelv < g ? a.nelv : g;
-  if (grid > a.max_grid) grid = a.max_grid;
-  launch_chained((long)a.nelv * C::L3, kern, grid, C::THREADS, C::SMEM, s, a.w, a.p, a.z, a.D,
-                 a.Dt, a.h1, a.g[0], a.g[1], a.g[2],
-                                         a.g[3], a.g[4], a.g[5], a.h2, a.B, a.nelv, a.st, a.beta,
-                                         a.pap_out, a.partials, a.counter, a.err);
-  return cudaGetLastError();
+  if (a.nelv <= 0) return cudaSuccess;
+  const int ngroup = (a.nelv + NE - 1) / NE;
+  int grid = ngroup < g ? ngroup : g;
+  if (CG && grid > a.max_grid) grid = a.max_grid;
+  return launch_chained((long)a.nelv * C::L3, kern, grid, C::THREADS, C::SMEM, st, a);
+}
+
+// Stages, k split and overlay of an order, without and with h2.  A larger split
+// (more threads an element) hides the loads of h2 and B, which come past the
+// ring: lx 8 with h2 takes 102 us at 7.1 M points split by 4, 126 by 2.  A
+// smaller one leaves registers for another block: the step at lx 10 takes 128
+// us at 6.9 M points split by 2, 156 by 5 with a third, overlaid stage, and at
+// lx 8 105 us at 7.1 M points unsplit, 113 split by 2.
+template <int LX, int NE, bool CG, int S, int KS, bool AL, int S2, int KS2, bool AL2, typename TZ>
+static cudaError_t launch_ax_stream(const AxArgs<TZ> &a, cudaStream_t st) {
+  return a.h2 ? launch_ax_stream_as<LX, S2, KS2, NE, CG, AL2, true>(a, st)
+              : launch_ax_stream_as<LX, S, KS, NE, CG, AL, false>(a, st);
+}
+
+// Whether the streaming form takes the operands: every copied array on a
+// 16-byte boundary.
+static bool bulk_aligned(std::initializer_list<const void *> ptrs) {
+  for (const void *p : ptrs)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+  return true;
+}
+
+// Dispatch of the streaming operator; returns cudaErrorNotSupported when no
+// instantiation covers lx or a pointer is not 16-byte aligned.
+cudaError_t ax_helm_stream(double *w, const double *u, const double *D, const double *Dt,
+                           const double *h1, const double *g11, const double *g22,
+                           const double *g33, const double *g12, const double *g13,
+                           const double *g23, const double *h2, const double *B, int nelv, int lx,
+                           cudaStream_t s, const int *skip, int *err) {
+  if (!bulk_aligned({u, h1, g11, g22, g33, g12, g13, g23, h2, B})) return cudaErrorNotSupported;
+  AxArgs<double> a{};
+  a.w = w, a.u = u, a.D = D, a.Dt = Dt, a.h1 = h1;
+  a.g[0] = g11, a.g[1] = g22, a.g[2] = g33, a.g[3] = g12, a.g[4] = g13, a.g[5] = g23;
+  a.h2 = h2, a.B = B, a.nelv = nelv, a.skip = skip, a.err = err;
+  switch (lx) {
+    case 4: return launch_ax_stream<4, 1, false, 4, 4, false, 4, 4, false>(a, s);
+    case 5: return launch_ax_stream<5, 2, false, 3, 1, false, 3, 1, false>(a, s);
+    case 6: return launch_ax_stream<6, 1, false, 3, 3, false, 3, 3, false>(a, s);
+    case 7:
+      // While a block takes two pairs of elements at most, a single stage, which
+      // lets a third block run: 23 against 28 us for the operator with h2,
+      // gather-scatter and mask on 453 thousand points out of cache.  With more
+      // of them a second stage: 127 against 157 us at 6.8 M points.
+      return nelv <= 12 * device_sms()
+                 ? launch_ax_stream<7, 2, false, 1, 2, false, 1, 2, false>(a, s)
+                 : launch_ax_stream<7, 2, false, 2, 1, false, 2, 2, false>(a, s);
+    case 8: return launch_ax_stream<8, 1, false, 2, 2, true, 2, 4, false>(a, s);
+    case 9: return launch_ax_stream<9, 2, false, 1, 3, false, 2, 2, true>(a, s);
+    case 10: return launch_ax_stream<10, 1, false, 2, 5, false, 2, 2, false>(a, s);
+    default: return cudaErrorNotSupported;
+  }
 }
 
 // The fused step for the other orders and for operands that are not 16-byte
-// aligned (a bulk copy moves whole 16-byte units, and lx^3 values are not one
-// for odd lx): NE elements a block with plain coalesced loads, the element
-// loop of ax_helm_kernel.
+// aligned: NE elements a block with plain coalesced loads, the element loop of
+// ax_helm_kernel.
 template <int LX, int NE>
 struct AxCgGen {
   static constexpr int L2 = LX * LX, L3 = L2 * LX;
@@ -571,7 +487,7 @@ struct AxCgGen {
 
 template <int LX, int NE, typename TZ>
 __global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS)
-    ax_cg_gen_kernel(const AxCgArgs<TZ> a) {
+    ax_cg_gen_kernel(const AxArgs<TZ> a) {
   using C = AxCgGen<LX, NE>;
   constexpr int L2 = C::L2, L3 = C::L3;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -656,7 +572,7 @@ __global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS)
 }
 
 template <int LX, typename TZ>
-static cudaError_t launch_ax_cg_gen(const AxCgArgs<TZ> &a, cudaStream_t s) {
+static cudaError_t launch_ax_cg_gen(const AxArgs<TZ> &a, cudaStream_t s) {
   using C = AxCgGen<LX, AxCfg<LX>::NE>;
   auto kern = ax_cg_gen_kernel<LX, AxCfg<LX>::NE, TZ>;
   if (C::SMEM > 48 * 1024) {
@@ -679,26 +595,28 @@ cudaError_t ax_cg_fused(double *w, double *p, const TZ *z, const double *D, cons
                         double beta, double *pap_out, double *partials, unsigned *counter,
                         int max_grid, cudaStream_t s, int *err) {
   if (nelv <= 0) return cudaErrorNotSupported;
-  const AxCgArgs<TZ> a{w,    p,  z,    D,       Dt,       h1,      {g11, g22, g33, g12, g13, g23},
-                       h2,   B,  nelv, st,      beta,     pap_out, partials,
-                       counter, max_grid, err};
-  bool aligned = ((size_t)lx * lx * lx * sizeof(TZ)) % 16 == 0;
-  const void *ptrs[] = {z, p, h1, g11, g22, g33, g12, g13, g23};
-  for (const void *q : ptrs)
-    if (reinterpret_cast<uintptr_t>(q) & 15) aligned = false;
-  if (aligned) {
-#define NB_CG_CASE(LX, S, KS, AL)                                              \
-  case LX:                                                                     \
-    return h2 ? launch_ax_cg<LX, S, KS, TZ, AL, true>(a, s)                    \
-              : launch_ax_cg<LX, S, KS, TZ, AL, false>(a, s);
+  AxArgs<TZ> a{};
+  a.w = w, a.p = p, a.z = z, a.D = D, a.Dt = Dt, a.h1 = h1;
+  a.g[0] = g11, a.g[1] = g22, a.g[2] = g33, a.g[3] = g12, a.g[4] = g13, a.g[5] = g23;
+  a.h2 = h2, a.B = B, a.nelv = nelv, a.err = err;
+  a.st = st, a.beta = beta, a.pap_out = pap_out, a.partials = partials, a.counter = counter;
+  a.max_grid = max_grid;
+  if (bulk_aligned({z, p, h1, g11, g22, g33, g12, g13, g23, h2, B})) {
     switch (lx) {
-      NB_CG_CASE(4, 4, 4, false)
-      NB_CG_CASE(6, 3, 2, false)
-      NB_CG_CASE(8, 2, 2, false)
-      NB_CG_CASE(10, 3, 5, true)
+      case 4: return launch_ax_stream<4, 1, true, 4, 4, false, 4, 4, false>(a, s);
+      case 6: return launch_ax_stream<6, 1, true, 3, 3, false, 3, 3, false>(a, s);
+      case 8: return launch_ax_stream<8, 1, true, 2, 1, false, 2, 2, false>(a, s);
+      case 10: return launch_ax_stream<10, 1, true, 2, 2, false, 2, 2, false>(a, s);
       default: break;
     }
-#undef NB_CG_CASE
+    if constexpr (sizeof(TZ) == 8) {  // pairs of FP32 z are not whole 16-byte units
+      switch (lx) {
+        case 5: return launch_ax_stream<5, 2, true, 2, 2, false, 2, 2, false>(a, s);
+        case 7: return launch_ax_stream<7, 2, true, 1, 2, false, 1, 2, false>(a, s);
+        case 9: return launch_ax_stream<9, 2, true, 1, 3, false, 2, 2, true>(a, s);
+        default: break;
+      }
+    }
   }
   switch (lx) {
 #define NB_CG_GEN(N) \
@@ -742,18 +660,12 @@ int take_dropin_error() {
   return v;
 }
 
-template cudaError_t ax_helm_stream<double>(double *, const double *, const double *,
-                                            const double *, const double *, const double *,
-                                            const double *, const double *, const double *,
-                                            const double *, const double *, int, int,
-                                            cudaStream_t, const int *, int *);
-
 template <typename T, int LX>
 static cudaError_t launch_ax(T *w, const T *u, const T *dx, const T *dy, const T *dz,
                              const T *dxt, const T *dyt, const T *dzt, const T *h1,
                              const T *g11, const T *g22, const T *g33, const T *g12,
-                             const T *g13, const T *g23, int nelv, cudaStream_t s,
-                             const int *skip) {
+                             const T *g13, const T *g23, const T *h2, const T *B, int nelv,
+                             cudaStream_t s, const int *skip) {
   constexpr int NE = AxCfg<LX>::NE;
   const size_t smem = sizeof(T) * (6 * LX * LX + NE * 3 * LX * LX * LX);
   auto kern = ax_helm_kernel<T, LX, NE>;
@@ -766,7 +678,7 @@ static cudaError_t launch_ax(T *w, const T *u, const T *dx, const T *dy, const T
   if (nelv <= 0) return cudaSuccess;
   launch_chained((long)nelv * LX * LX * LX, kern, grid, block, smem, s, w, u, dx, dy, dz, dxt,
                  dyt, dzt, h1, g11, g22, g33, g12,
-                                 g13, g23, nelv, skip);
+                 g13, g23, h2, B, nelv, skip);
   return cudaGetLastError();
 }
 
@@ -774,11 +686,11 @@ template <typename T>
 cudaError_t ax_helm(T *w, const T *u, const T *dx, const T *dy, const T *dz, const T *dxt,
                     const T *dyt, const T *dzt, const T *h1, const T *g11, const T *g22,
                     const T *g33, const T *g12, const T *g13, const T *g23, int nelv, int lx,
-                    cudaStream_t s, const int *skip) {
+                    cudaStream_t s, const int *skip, const T *h2, const T *B) {
 #define NB_AX_CASE(N)                                                                  \
   case N:                                                                              \
     return launch_ax<T, N>(w, u, dx, dy, dz, dxt, dyt, dzt, h1, g11, g22, g33, g12, g13, \
-                           g23, nelv, s, skip);
+                           g23, h2, B, nelv, s, skip);
   switch (lx) {
     NB_AX_CASE(2)
     NB_AX_CASE(3)
@@ -806,12 +718,7 @@ template cudaError_t ax_helm<double>(double *, const double *, const double *, c
                                      const double *, const double *, const double *,
                                      const double *, const double *, const double *,
                                      const double *, const double *, int, int, cudaStream_t,
-                                     const int *);
-template cudaError_t ax_helm<float>(float *, const float *, const float *, const float *,
-                                    const float *, const float *, const float *, const float *,
-                                    const float *, const float *, const float *, const float *,
-                                    const float *, const float *, const float *, int, int,
-                                    cudaStream_t, const int *);
+                                     const int *, const double *, const double *);
 
 }  // namespace nb
 
@@ -856,11 +763,11 @@ extern "C" void cuda_ax_helm(void *w, void *u, void *dx, void *dy, void *dz, voi
   }
   cudaError_t e = cudaErrorNotSupported;
   if (nb::same_derivatives(dx, dy, dz, dxt, dyt, dzt, *lx))
-    e = nb::ax_helm_stream<double>((double *)w, (const double *)u, (const double *)dx,
+    e = nb::ax_helm_stream((double *)w, (const double *)u, (const double *)dx,
                                    (const double *)dxt, (const double *)h1, (const double *)g11,
                                    (const double *)g22, (const double *)g33, (const double *)g12,
-                                   (const double *)g13, (const double *)g23, *nelv, *lx,
-                                   nb::default_stream(), nullptr, nullptr);
+                                   (const double *)g13, (const double *)g23, nullptr, nullptr,
+                                   *nelv, *lx, nb::default_stream(), nullptr, nullptr);
   if (e == cudaErrorNotSupported)
     e = nb::ax_helm<double>(
       (double *)w, (const double *)u, (const double *)dx, (const double *)dy,

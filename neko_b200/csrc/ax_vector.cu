@@ -15,6 +15,7 @@
 
 #include <cstdint>
 
+#include "nb_chain.cuh"
 #include "nb_kernels.h"
 #include "nb_problem.h"
 #include "nb_tma.cuh"
@@ -40,12 +41,12 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
                       const double *__restrict__ h1, const double *__restrict__ g11,
                       const double *__restrict__ g22, const double *__restrict__ g33,
                       const double *__restrict__ g12, const double *__restrict__ g13,
-                      const double *__restrict__ g23, const int nelv, int *__restrict__ err,
+                      const double *__restrict__ g23, const double *__restrict__ h2,
+                      const double *__restrict__ Bm, const int nelv, int *__restrict__ err,
                       const int *__restrict__ skip) {
   using C = AxVecCfg<LX, S, KS>;
   constexpr int L2 = C::L2, L3 = C::L3, NA = C::NA, KP = LX / KS;
   static_assert(LX % KS == 0, "k split must divide lx");
-  if (skip && *skip) return;
   extern __shared__ __align__(128) unsigned char smem_vec[];
   double *stage = reinterpret_cast<double *>(smem_vec);
   double *sur = stage + S * NA * L3, *sus = sur + L3, *sut = sus + L3;
@@ -59,6 +60,8 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
     for (int s = 0; s < S; s++) mbar_init(&full[s], 1);
     fence_barrier_init();
   }
+  chain();
+  if (skip && *skip) return;
   for (int q = tid; q < L2; q += C::THREADS) {
     sD[q] = D[q];
     sDt[q] = Dt[q];
@@ -72,6 +75,10 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
 #pragma unroll
     for (int a = 0; a < NA; a++)
       bulk_g2s(stage + (size_t)(s * NA + a) * L3, src[a] + e * L3, (uint32_t)C::ABYTES, &full[s]);
+    if (h2) {  // read by each thread for its own points: to L2 meanwhile
+      bulk_prefetch_l2(h2 + e * L3, (uint32_t)C::ABYTES);
+      bulk_prefetch_l2(Bm + e * L3, (uint32_t)C::ABYTES);
+    }
   };
   if (tid == 0)
     for (int t = 0; t < S && t < nt; t++) issue(t, t);
@@ -92,12 +99,20 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
   bool failed = false;
   for (; t < nt; t++) {
     const int s = t % S;
+    const long e = b + (long)t * G;
+    double hb[KP];  // h2 B at this thread's points
+    if (act) {
+#pragma unroll
+      for (int kk = 0; kk < KP; kk++) {
+        const long g = e * L3 + col + L2 * (k0 + kk);
+        hb[kk] = h2 ? __ldg(h2 + g) * __ldg(Bm + g) : 0.0;
+      }
+    }
     const bool ok = mbar_wait(&full[s], (uint32_t)((t / S) & 1));
     if (__syncthreads_or(!ok)) {
       failed = true;
       break;
     }
-    const long e = b + (long)t * G;
     const double *slot = stage + (size_t)s * NA * L3;
     const double *sh = slot + 3 * L3, *s11 = slot + 4 * L3, *s22 = slot + 5 * L3,
                  *s33 = slot + 6 * L3, *s12 = slot + 7 * L3, *s13 = slot + 8 * L3,
@@ -105,10 +120,13 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const double *su = slot + c * L3;
+      double own[KP];  // the component at this thread's points
       if (act) {
         double ru[LX];
 #pragma unroll
         for (int l = 0; l < LX; l++) ru[l] = su[col + L2 * l];
+#pragma unroll
+        for (int kk = 0; kk < KP; kk++) own[kk] = su[col + L2 * (k0 + kk)];
 #pragma unroll
         for (int kk = 0; kk < KP; kk++) {
           const int k = k0 + kk;
@@ -145,7 +163,9 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
             cc += Dtj[l] * sus[i + LX * l + L2 * k];
             d += sDt[k + LX * l] * rt[l];
           }
-          wo[e * L3 + col + L2 * k] = a + cc + d;
+          double v = a + cc + d;
+          if (h2) v = v + hb[kk] * own[kk];  // the part2 term, in its order
+          wo[e * L3 + col + L2 * k] = v;
         }
       }
       __syncthreads();  // work planes free for the next component / element
@@ -165,8 +185,8 @@ template <int LX, int S, int KS>
 static cudaError_t launch_vec(const VecIo &io, const double *D, const double *Dt,
                               const double *h1, const double *g11, const double *g22,
                               const double *g33, const double *g12, const double *g13,
-                              const double *g23, int nelv, cudaStream_t st, int *err,
-                              const int *skip) {
+                              const double *g23, const double *h2, const double *B, int nelv,
+                              cudaStream_t st, int *err, const int *skip) {
   using C = AxVecCfg<LX, S, KS>;
   auto kern = ax_vec_tma_kernel<LX, S, KS>;
   static int grid_per_dev[64] = {0};
@@ -186,37 +206,45 @@ static cudaError_t launch_vec(const VecIo &io, const double *D, const double *Dt
   if (!err) err = dropin_error_word();
   if (!err) return cudaErrorInvalidSymbol;
   const int grid = nelv < g ? nelv : g;
-  kern<<<grid, C::THREADS, C::SMEM, st>>>(io, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv,
-                                          err, skip);
-  return cudaGetLastError();
+  return launch_chained(3L * nelv * C::L3, kern, grid, C::THREADS, C::SMEM, st, io, D, Dt, h1,
+                        g11, g22, g33, g12,
+                        g13, g23, h2, B, nelv, err, skip);
 }
 
-// (au, av, aw) = A (u, v, w) (h1 part).  The streaming kernel for even lx in
-// 4..10 with 16-byte aligned operands, otherwise the general kernel once per
-// component.
+// (au, av, aw) = A (u, v, w), plus h2 B (u, v, w) when h2 is given.  One pass
+// for even lx in 4..10 with 16-byte aligned operands, otherwise the scalar
+// operator (streaming for lx 5, 7, 9) once per component.
 cudaError_t ax_helm_vector(double *au, double *av, double *aw, const double *u,
                            const double *v, const double *w, const double *D,
                            const double *Dt, const double *h1, const double *g11,
                            const double *g22, const double *g33, const double *g12,
-                           const double *g13, const double *g23, int nelv, int lx,
-                           cudaStream_t s, int *err, const int *skip) {
+                           const double *g13, const double *g23, const double *h2,
+                           const double *B, int nelv, int lx, cudaStream_t s, int *err,
+                           const int *skip) {
   VecIo io{{au, av, aw}, {u, v, w}};
   bool aligned = true;
-  const void *ptrs[] = {u, v, w, h1, g11, g22, g33, g12, g13, g23};
+  const void *ptrs[] = {u, v, w, h1, g11, g22, g33, g12, g13, g23, h2, B};
   for (const void *q : ptrs)
     if (reinterpret_cast<uintptr_t>(q) & 15) aligned = false;
   if (aligned) {
+#define NB_VEC(LX, S, KS) \
+  case LX:                \
+    return launch_vec<LX, S, KS>(io, D, Dt, h1, g11, g22, g33, g12, g13, g23, h2, B, nelv, s, err, skip);
     switch (lx) {
-      case 4: return launch_vec<4, 4, 1>(io, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, s, err, skip);
-      case 6: return launch_vec<6, 3, 2>(io, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, s, err, skip);
-      case 8: return launch_vec<8, 2, 2>(io, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, s, err, skip);
-      case 10: return launch_vec<10, 2, 5>(io, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, s, err, skip);
+      NB_VEC(4, 4, 1)
+      NB_VEC(6, 3, 2)
+      NB_VEC(8, 2, 2)
+      NB_VEC(10, 2, 5)
       default: break;
     }
+#undef NB_VEC
   }
   for (int c = 0; c < 3; c++) {
-    cudaError_t e = ax_helm<double>(io.out[c], io.in[c], D, D, D, Dt, Dt, Dt, h1, g11, g22, g33,
-                                    g12, g13, g23, nelv, lx, s, skip);
+    cudaError_t e = ax_helm_stream(io.out[c], io.in[c], D, Dt, h1, g11, g22, g33, g12, g13, g23,
+                                   h2, B, nelv, lx, s, skip, err);
+    if (e == cudaErrorNotSupported)
+      e = ax_helm<double>(io.out[c], io.in[c], D, D, D, Dt, Dt, Dt, h1, g11, g22, g33, g12, g13,
+                          g23, nelv, lx, s, skip, h2, B);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -254,7 +282,7 @@ extern "C" void cuda_ax_helm_vector(void *au, void *av, void *aw, void *u, void 
   auto d = [](void *p) { return (double *)p; };
   if (same_derivatives(dx, dy, dz, dxt, dyt, dzt, *lx)) {
     e = ax_helm_vector(d(au), d(av), d(aw), d(u), d(v), d(w), d(dx), d(dxt), d(h1), d(g11),
-                       d(g22), d(g33), d(g12), d(g13), d(g23), *nelv, *lx, s, nullptr);
+                       d(g22), d(g33), d(g12), d(g13), d(g23), nullptr, nullptr, *nelv, *lx, s, nullptr);
   } else {
     double *outs[3] = {d(au), d(av), d(aw)}, *ins[3] = {d(u), d(v), d(w)};
     e = cudaSuccess;
@@ -284,11 +312,7 @@ extern "C" nb_status nb_ax_vector(nb_problem *p, double *au, double *av, double 
   }
   const cudaStream_t s = (cudaStream_t)stream;
   NB_CUDA_TRY(ax_helm_vector(au, av, aw, u, v, w, p->D, p->Dt, p->h1, p->g11, p->g22, p->g33,
-                             p->g12, p->g13, p->g23, p->nelv, p->lx, s, p->err));
-  if (p->ifh2) {
-    ax_vec_part2_kernel<<<stream_grid(p->n, 256), 256, 0, s>>>(au, av, aw, u, v, w, p->h2, p->B,
-                                                              p->n);
-    NB_CUDA_TRY(cudaGetLastError());
-  }
+                             p->g12, p->g13, p->g23, p->ifh2 ? p->h2 : nullptr,
+                             p->ifh2 ? p->B : nullptr, p->nelv, p->lx, s, p->err));
   return NB_OK;
 }

@@ -48,15 +48,6 @@ __global__ void jacobi_scale_kernel(double *d, const double *h1, const double *h
   }
 }
 
-__global__ void addcol4_kernel(double *w, const double *h2, const double *B, const double *u,
-                               long n, const int *skip) {
-  chain();
-  if (skip && *skip) return;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
-       i += (long)gridDim.x * blockDim.x)
-    w[i] = w[i] + h2[i] * B[i] * u[i];
-}
-
 // ---------------------------------------------------------------------------
 // CG kernels.  Every kernel returns immediately once st->done is set.
 // ---------------------------------------------------------------------------
@@ -490,13 +481,13 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, cuda
   // continuous and zero wherever w is masked: f is assembled and masked, so r
   // and every preconditioner's output are)
   cudaError_t e = cudaErrorNotSupported;
-  const double *h2 = P->ifh2 ? P->h2 : nullptr;
+  const double *h2 = P->ifh2 ? P->h2 : nullptr, *h2B = P->ifh2 ? P->B : nullptr;
   if (P->use_stream_ax)
     e = zf ? ax_cg_fused(W.w, W.p, zf, P->D, P->Dt, P->h1, P->g11, P->g22, P->g33, P->g12,
-                         P->g13, P->g23, h2, P->B, (int)P->nelv, P->lx, W.st, 0.0, nullptr,
+                         P->g13, P->g23, h2, h2B, (int)P->nelv, P->lx, W.st, 0.0, nullptr,
                          W.partials, W.counter, kCgMaxPartials, s, P->err)
            : ax_cg_fused(W.w, W.p, (const double *)W.z, P->D, P->Dt, P->h1, P->g11, P->g22,
-                         P->g33, P->g12, P->g13, P->g23, h2, P->B, (int)P->nelv, P->lx, W.st,
+                         P->g33, P->g12, P->g13, P->g23, h2, h2B, (int)P->nelv, P->lx, W.st,
                          0.0, nullptr, W.partials, W.counter, kCgMaxPartials, s, P->err);
   W.fused = e == cudaSuccess;
   if (e != cudaSuccess && e != cudaErrorNotSupported) return e;
@@ -505,10 +496,8 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, cuda
       launch_chained(n, cg_update_p_kernel<float>, eg, 256, 0, s, W.p, zf, n, W.st);
     else
       launch_chained(n, cg_update_p_kernel<double>, eg, 256, 0, s, W.p, W.z, n, W.st);
-    e = P->ax_raw(W.w, W.p, s, &W.st->done);
+    e = P->ax(W.w, W.p, s, &W.st->done);
     if (e != cudaSuccess) return e;
-    if (P->ifh2) launch_chained(n, addcol4_kernel, eg, 256, 0, s, W.w, P->h2, P->B, W.p, n,
-                                &W.st->done);
   }
   e = gs_add_fused<double>(P->gsd, W.w, true, s, &W.st->done);
   if (e != cudaSuccess) return e;
@@ -527,10 +516,8 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, cuda
   if (W.recompute_every > 0) {  // w = A x, gs, mask; r = f - w (scheduled iterations only)
     // x through z (free until the next preconditioner apply overwrites it)
     launch_chained(n, cg_copy_x_kernel, eg, 256, 0, s, W.z, n, W.st);
-    e = P->ax_raw(W.w, W.z, s, &W.st->skip_rc);
+    e = P->ax(W.w, W.z, s, &W.st->skip_rc);
     if (e != cudaSuccess) return e;
-    if (P->ifh2) launch_chained(n, addcol4_kernel, eg, 256, 0, s, W.w, P->h2, P->B, W.z, n,
-                                &W.st->skip_rc);
     e = gs_add_fused<double>(P->gsd, W.w, true, s, &W.st->skip_rc);
     if (e != cudaSuccess) return e;
     launch_chained(n, cg_true_residual_kernel, rb, kRedThreads, 0, s, W.r, W.w, P->mult,
@@ -633,8 +620,8 @@ nb_status cg_start(CgRun &R) {
     // inner products formed by the preconditioner a one-block finishing
     // launch replaces the dot pass
     const int pc_launches = pc ? pc->launches() - (pc->output_f32() ? 1 : 0) : 0;
-    W.launches_per_iter = (W.fused ? 4 : 6 + (P->ifh2 ? 1 : 0)) - (W.fold ? 1 : 0) + pc_launches +
-                          (W.recompute_every > 0 ? 4 + (P->ifh2 ? 1 : 0) : 0);
+    W.launches_per_iter = (W.fused ? 4 : 6) - (W.fold ? 1 : 0) + pc_launches +
+                          (W.recompute_every > 0 ? 4 : 0);
     cudaError_t ee = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
     if (ce != cudaSuccess) {

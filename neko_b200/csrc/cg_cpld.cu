@@ -229,11 +229,9 @@ static cudaError_t cpld_op(nb_problem *P, int op, const V3 &w, const V3 &p, cons
     e = problem_ax_stress(P, w.c[0], w.c[1], w.c[2], p.c[0], p.c[1], p.c[2], s, skip);
   } else {
     e = ax_helm_vector(w.c[0], w.c[1], w.c[2], p.c[0], p.c[1], p.c[2], P->D, P->Dt, P->h1,
-                       P->g11, P->g22, P->g33, P->g12, P->g13, P->g23, P->nelv, P->lx, s, P->err,
-                       skip);
-    if (e == cudaSuccess && P->ifh2)
-      e = ax_stress_part2(w.c[0], w.c[1], w.c[2], p.c[0], p.c[1], p.c[2], P->h2, P->B, P->n, s,
-                          skip);
+                       P->g11, P->g22, P->g33, P->g12, P->g13, P->g23,
+                       P->ifh2 ? P->h2 : nullptr, P->ifh2 ? P->B : nullptr, P->nelv, P->lx, s,
+                       P->err, skip);
   }
   if (e == cudaSuccess) e = gs_add_fused3(P->gsd, w.c[0], w.c[1], w.c[2], true, s, skip);
   return e;
@@ -320,11 +318,11 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
         ce = cudaGetLastError();
       }
     }
-    // the operator: one launch, plus a separate h2 launch except on the
-    // full-stress streaming kernel, which folds the h2 term in
-    const bool h2_folded =
-        op == NB_AX_STRESS && (P->lx == 4 || P->lx == 6 || P->lx == 8 || P->lx == 10);
-    const int op_launches = 1 + (P->ifh2 && !h2_folded ? 1 : 0);
+    // the operator is one launch on its streaming form, three (one a
+    // component) for ax_helm_vector at other lx; the general full-stress
+    // kernel adds the h2 term in a launch of its own
+    const bool one = P->lx == 4 || P->lx == 6 || P->lx == 8 || P->lx == 10;
+    const int op_launches = one ? 1 : op == NB_AX_STRESS ? 1 + (P->ifh2 ? 1 : 0) : 3;
     W.launches_per_iter = fused ? 1 + 1 + 1 : 1 + op_launches + 1 + 2;
     cudaError_t ee = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);

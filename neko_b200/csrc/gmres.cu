@@ -364,10 +364,8 @@ __global__ void gm_copy_x_kernel(double *__restrict__ y, long n, const GmresStat
 // nothing when *skip != 0.
 static cudaError_t apply_op(nb_problem *P, double *w, const double *u, const int *skip,
                             cudaStream_t s) {
-  cudaError_t e = P->ax_raw(w, u, s, skip);
+  cudaError_t e = P->ax(w, u, s, skip);
   if (e != cudaSuccess) return e;
-  if (P->ifh2)
-    addcol4_kernel<<<stream_grid(P->n, 256), 256, 0, s>>>(w, P->h2, P->B, u, P->n, skip);
   return gs_add_fused<double>(P->gsd, w, true, s, skip);
 }
 
@@ -381,7 +379,7 @@ static cudaError_t gmres_cycle(nb_problem *P, GmresWorkspace &W, Precond *pc, bo
   launch_chained(n, gm_copy_x_kernel, eg, 256, 0, s, W.Z[0], n, W.st);
   cudaError_t e = apply_op(P, W.w, W.Z[0], &W.st->done, s);
   if (e != cudaSuccess) return e;
-  L += 3 + (P->ifh2 ? 1 : 0);
+  L += 3;
   launch_chained(n, gm_cycle_start_kernel, rb, kRedThreads, 0, s, W.r, W.w, P->mult, P->multf, n,
                  W.st,
                                                    W.partials, W.counter);
@@ -399,7 +397,7 @@ static cudaError_t gmres_cycle(nb_problem *P, GmresWorkspace &W, Precond *pc, bo
     }
     e = apply_op(P, W.w, W.Z[j], &W.st->stop, s);
     if (e != cudaSuccess) return e;
-    L += 2 + (P->ifh2 ? 1 : 0);
+    L += 2;
     launch_chained(n, gm_many_dot_kernel, rb, kRedThreads, 0, s, W.w, W.Vp, P->mult, P->multf, n,
                    j, W.st,
                                                   W.partials, W.counter);

@@ -13,20 +13,22 @@ namespace nb {
 cudaStream_t default_stream();
 void set_default_stream(cudaStream_t s);
 
+// w = A u (+ h2 B u when h2 is given), any lx in 2..16.
 template <typename T>
 cudaError_t ax_helm(T *w, const T *u, const T *dx, const T *dy, const T *dz, const T *dxt,
                     const T *dyt, const T *dzt, const T *h1, const T *g11, const T *g22,
                     const T *g33, const T *g12, const T *g13, const T *g23, int nelv, int lx,
-                    cudaStream_t s, const int *skip = nullptr);
+                    cudaStream_t s, const int *skip = nullptr, const T *h2 = nullptr,
+                    const T *B = nullptr);
 
-// Persistent bulk-copy variant of ax_helm (dx = dy = dz); returns
-// cudaErrorNotSupported when it has no instantiation for (T, lx) or the
-// pointers are not 16-byte aligned.
-template <typename T>
-cudaError_t ax_helm_stream(T *w, const T *u, const T *D, const T *Dt, const T *h1,
-                           const T *g11, const T *g22, const T *g33, const T *g12,
-                           const T *g13, const T *g23, int nelv, int lx, cudaStream_t s,
-                           const int *skip = nullptr, int *err = nullptr);
+// Persistent bulk-copy variant of ax_helm (dx = dy = dz) for lx 4..10; returns
+// cudaErrorNotSupported for other lx and when the pointers are not 16-byte
+// aligned.
+cudaError_t ax_helm_stream(double *w, const double *u, const double *D, const double *Dt,
+                           const double *h1, const double *g11, const double *g22,
+                           const double *g33, const double *g12, const double *g13,
+                           const double *g23, const double *h2, const double *B, int nelv, int lx,
+                           cudaStream_t s, const int *skip = nullptr, int *err = nullptr);
 
 // True when dx, dy, dz (and dxt, dyt, dzt) hold the same lx x lx matrix
 // (pointer-equal, or equal contents, compared once per pointer set).
@@ -39,14 +41,15 @@ int take_dropin_error();
 // Device address of that word on the current device (looked up once).
 int *dropin_error_word();
 
-// (au, av, aw) = A (u, v, w), h1 part, one set of coefficients
-// (ax_vector.cu).
+// (au, av, aw) = A (u, v, w), one set of coefficients, plus h2 B (u, v, w)
+// when h2 is given (ax_vector.cu).
 cudaError_t ax_helm_vector(double *au, double *av, double *aw, const double *u,
                            const double *v, const double *w, const double *D,
                            const double *Dt, const double *h1, const double *g11,
                            const double *g22, const double *g33, const double *g12,
-                           const double *g13, const double *g23, int nelv, int lx,
-                           cudaStream_t s, int *err, const int *skip = nullptr);
+                           const double *g13, const double *g23, const double *h2,
+                           const double *B, int nelv, int lx, cudaStream_t s, int *err,
+                           const int *skip = nullptr);
 
 // (au, av, aw) = A_stress (u, v, w): the full-stress operator with
 // cofactors cof[0..8] = drdx, drdy, drdz, dsdx, dsdy, dsdz, dtdx, dtdy, dtdz
@@ -67,8 +70,9 @@ struct CgState;
 // pap = sum p * w in one launch (ax_helm.cu).  With a CG state, beta is read
 // from it, the launch returns at once when st->done is set, and pap and
 // alpha = rtz / pap are written to it; without one, beta is the argument and
-// pap goes to *pap_out (device, may be null).  The streaming kernel for lx 4,
-// 6, 8, 10 with 16-byte aligned operands, a general one otherwise;
+// pap goes to *pap_out (device, may be null).  The streaming kernel for lx 4
+// to 10 with 16-byte aligned operands (even lx with an FP32 z), a general one
+// otherwise;
 // cudaErrorNotSupported for lx outside 2..16.
 // z may be FP32 (a mixed-precision preconditioner's output), widened as read.
 template <typename TZ>

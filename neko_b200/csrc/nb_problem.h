@@ -23,10 +23,6 @@ cudaError_t jacobi_diag(double *d, const double *dxt, const double *dyt, const d
 // d = d * h1 (+ h2 * B)
 __global__ void jacobi_scale_kernel(double *d, const double *h1, const double *h2,
                                     const double *B, long n);
-// w += h2 * B * u
-__global__ void addcol4_kernel(double *w, const double *h2, const double *B, const double *u,
-                               long n, const int *skip = nullptr);
-
 }  // namespace nb
 
 struct nb_problem {
@@ -77,8 +73,8 @@ struct nb_problem {
   ~nb_problem();
   cudaError_t update_jacobi(cudaStream_t s);
   bool use_stream_ax = true;  // NB_AX_KERNEL=classic selects the general kernel
-  cudaError_t ax(double *w, const double *u, cudaStream_t s) const;
-  cudaError_t ax_raw(double *w, const double *u, cudaStream_t s, const int *skip) const;
+  // w = A u (with the h2 term when it is on), element-local
+  cudaError_t ax(double *w, const double *u, cudaStream_t s, const int *skip = nullptr) const;
   void invalidate_solver_cache();
 };
 

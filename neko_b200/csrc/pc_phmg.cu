@@ -320,10 +320,7 @@ struct PhmgImpl : public Precond {
 
   // w = A u on a level: ax (+ h2 B u), gather-scatter add with the mask.
   cudaError_t op(nb_problem *P, double *w, const double *u, const int *skip, cudaStream_t s) {
-    PH_CALL(P->ax_raw(w, u, s, skip));
-    if (P->ifh2)
-      PH_LAUNCH(launch_chained(P->n, addcol4_kernel, grid(P->n), kPhThreads, 0, s, w, P->h2,
-                               P->B, u, P->n, skip));
+    PH_CALL(P->ax(w, u, s, skip));
     PH_CALL(gs_add_fused<double>(P->gsd, w, P->nmask > 0, s, skip));
     return cudaSuccess;
   }
@@ -369,11 +366,7 @@ struct PhmgImpl : public Precond {
                              A.fnode[l], C->n,
                                                                    skip));
     PH_CALL(gs_add_fused<double>(C->gsd, A.wi, m, s, skip, (const double *)C->mult));
-    PH_CALL(C->ax_raw(A.wo, A.wi, s, skip));
-    if (C->ifh2)
-      PH_LAUNCH(launch_chained(C->n, addcol4_kernel, grid(C->n), kPhThreads, 0, s, A.wo, C->h2,
-                               C->B, A.wi, C->n,
-                                                                  skip));
+    PH_CALL(C->ax(A.wo, A.wi, s, skip));
     PH_CALL(gs_add_fused<double>(C->gsd, A.wo, m, s, skip, (const double *)C->mult));
     const int nn = (int)A.n[l];
     PH_LAUNCH(launch_chained(nn, amg_sum_kernel, (nn + 127) / 128, 128, 0, s, out, A.wo,

@@ -239,10 +239,8 @@ struct PipeWorkspace {
 // w = A u, gs add, mask; nothing when *skip
 static cudaError_t pipe_op(nb_problem *P, double *w, const double *u, const int *skip,
                            cudaStream_t s) {
-  cudaError_t e = P->ax_raw(w, u, s, skip);
+  cudaError_t e = P->ax(w, u, s, skip);
   if (e != cudaSuccess) return e;
-  if (P->ifh2)
-    addcol4_kernel<<<stream_grid(P->n, 256), 256, 0, s>>>(w, P->h2, P->B, u, P->n, skip);
   return gs_add_fused<double>(P->gsd, w, true, s, skip);
 }
 
@@ -309,7 +307,7 @@ nb_status pipecg_solve(nb_problem *P, double *x, const double *f, const nb_solve
         ce = cudaGetLastError();
       }
     }
-    W.launches_per_iter = (pc ? pc->launches() : 1) + 2 + (P->ifh2 ? 1 : 0) + 2;
+    W.launches_per_iter = (pc ? pc->launches() : 1) + 2 + 2;
     cudaError_t ee = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
     if (ce != cudaSuccess) {

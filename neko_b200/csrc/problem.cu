@@ -548,25 +548,18 @@ extern "C" nb_status nb_problem_set_coefficients(nb_problem *p, const double *h1
   return NB_OK;
 }
 
-// h1 part of ax_helm: the streaming kernel where it has an instantiation,
-// the general one otherwise.
-cudaError_t nb_problem::ax_raw(double *w, const double *u, cudaStream_t s,
-                               const int *skip) const {
+// ax_helm with the h2 term when it is on: the streaming kernel where it has an
+// instantiation, the general one otherwise.
+cudaError_t nb_problem::ax(double *w, const double *u, cudaStream_t s, const int *skip) const {
   cudaError_t e = cudaErrorNotSupported;
+  const double *h = ifh2 ? h2 : nullptr, *b = ifh2 ? B : nullptr;
   if (use_stream_ax)
-    e = nb::ax_helm_stream<double>(w, u, D, Dt, h1, g11, g22, g33, g12, g13, g23, nelv, lx, s,
-                                   skip, err);
+    e = nb::ax_helm_stream(w, u, D, Dt, h1, g11, g22, g33, g12, g13, g23, h, b, nelv, lx, s,
+                           skip, err);
   if (e == cudaErrorNotSupported)
     e = nb::ax_helm<double>(w, u, D, D, D, Dt, Dt, Dt, h1, g11, g22, g33, g12, g13, g23, nelv,
-                            lx, s, skip);
+                            lx, s, skip, h, b);
   return e;
-}
-
-cudaError_t nb_problem::ax(double *w, const double *u, cudaStream_t s) const {
-  cudaError_t e = ax_raw(w, u, s, nullptr);
-  if (e != cudaSuccess || !ifh2) return e;
-  addcol4_kernel<<<stream_grid(n, 256), 256, 0, s>>>(w, h2, B, u, n, nullptr);
-  return cudaGetLastError();
 }
 
 int nb_problem::take_error() {
@@ -632,7 +625,7 @@ extern "C" nb_status nb_ax_update_p(nb_problem *p, double *w, double *pdir, cons
   cudaError_t e = cudaErrorNotSupported;
   if (p->use_stream_ax)
     e = ax_cg_fused(w, pdir, z, p->D, p->Dt, p->h1, p->g11, p->g22, p->g33, p->g12, p->g13,
-                    p->g23, p->ifh2 ? p->h2 : nullptr, p->B, p->nelv, p->lx, nullptr, beta, pap,
+                    p->g23, p->ifh2 ? p->h2 : nullptr, p->ifh2 ? p->B : nullptr, p->nelv, p->lx, nullptr, beta, pap,
                     p->red_partials, p->red_counter, kMaxRedBlocks, s, p->err);
   if (e != cudaErrorNotSupported) {
     NB_TRY(e);
