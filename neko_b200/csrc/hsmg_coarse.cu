@@ -114,19 +114,6 @@ __global__ void __launch_bounds__(256)
   f[q] = (double)acc_z;
 }
 
-// one slice of the matrix to shared memory
-__device__ __forceinline__ void stage_slice(const NodeOp &A, int s, double *val, int *col,
-                                            int lane) {
-  const int o = __ldg(A.soff + s), w = __ldg(A.soff + s + 1) - o;
-  const double *gv = A.val + 32 * (size_t)o + lane;
-  const int *gc = A.col + 32 * (size_t)o + lane;
-#pragma unroll 9
-  for (int k = 0; k < w; k++) {
-    val[32 * k + lane] = __ldg(gv + 32 * k);
-    col[32 * k + lane] = __ldg(gc + 32 * k);
-  }
-}
-
 // sum of the element-local right-hand side over a node's copies, in order
 __device__ __forceinline__ double node_rhs(const NodeOp &A, const double *__restrict__ f,
                                            int row) {

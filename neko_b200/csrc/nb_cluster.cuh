@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include "nb_chain.cuh"
+#include "nb_nodes.h"
 #include "nb_tma.cuh"
 
 namespace nb {
@@ -63,6 +64,19 @@ __device__ __forceinline__ void cluster_allsum2(double v0, double v1, ClusterSum
   t1 = __shfl_sync(0xffffffffu, a, 16);
 }
 static_assert(kCoarseWarps == 16, "a half-warp reads one slot of every warp");
+
+// one slice of the matrix to shared memory
+__device__ __forceinline__ void stage_slice(const NodeOp &A, int s, double *val, int *col,
+                                            int lane) {
+  const int o = __ldg(A.soff + s), w = __ldg(A.soff + s + 1) - o;
+  const double *gv = A.val + 32 * (size_t)o + lane;
+  const int *gc = A.col + 32 * (size_t)o + lane;
+#pragma unroll 9
+  for (int k = 0; k < w; k++) {
+    val[32 * k + lane] = __ldg(gv + 32 * k);
+    col[32 * k + lane] = __ldg(gc + 32 * k);
+  }
+}
 
 // sum over the w entries of a row (stride 32) of val times load(col), nine
 // entries (a third of a box row) at a time

@@ -156,6 +156,13 @@ cudaError_t hsmg_coarse_restrict(const CoarseArgs<T> &a, int lm, const int *skip
                                  cudaStream_t s);
 // The coarse Jacobi-CG, one cluster launch.
 cudaError_t hsmg_coarse_cg(const CoarseCg &a, const int *skip, cudaStream_t s);
+
+// out = (J x J x J) in from ni to no points an element (down: the transposed
+// J), with the transfer kernel of hsmg; cudaErrorNotSupported for pairs it has
+// no instantiation of.  J has the larger number of rows.
+cudaError_t hsmg_transfer(bool down, int ni, int no, const double *in, const double *J,
+                          double *out, long nelv, const int *skip, cudaStream_t s);
+
 // hsmg preconditioner of problem P, built on first use (pc_hsmg.cu).
 nb_status hsmg_get(nb_problem *P, const nb_solve_opts &o, Precond **out);
 

@@ -24,6 +24,8 @@ struct TamgCluster {
   const double *rhs = nullptr;           // element-local, assembled and masked
   double *z = nullptr;                   // element-local result
   long npts = 0;
+  int nelv = 0, copies = 0;  // elements; most copies of a vertex
+  int stage_slices = 0;      // set by the launch
   const int *skip = nullptr;
 };
 // z = `cycles` V-cycles from zero for the right-hand side rhs.

@@ -749,6 +749,22 @@ static cudaError_t prolong_add(int ni, int no, const TIN *in, const T *J, TOUT *
   return cudaErrorNotSupported;
 }
 
+cudaError_t hsmg_transfer(bool down, int ni, int no, const double *in, const double *J,
+                          double *out, long nelv, const int *skip, cudaStream_t s) {
+  if (down)
+    return restrict_level<double, double, double>(ni, no, in, nullptr, J, out, nelv, skip, s);
+#define NB_T(A, B)                                                                          \
+  if (ni == A && no == B)                                                                   \
+    return launch_chained(nelv * B * B * B,                                                 \
+                          tensor3_kernel<double, double, double, A, B, false, false>,       \
+                          (unsigned)nelv, kT3Threads, 0, s, in, nullptr, nullptr, J, out,   \
+                          nelv, skip, PrologDots{}, CoarseAdd<double>{});
+  NB_T(2, 4) NB_T(2, 3) NB_T(4, 5) NB_T(4, 6) NB_T(4, 7) NB_T(4, 8) NB_T(4, 9) NB_T(4, 10)
+  NB_T(4, 11) NB_T(4, 12) NB_T(4, 13) NB_T(4, 14) NB_T(3, 4)
+#undef NB_T
+  return cudaErrorNotSupported;
+}
+
 // ---------------------------------------------------------------------------
 // The preconditioner.  T is the precision of the smoothing levels (double
 // for the FP64 path, float for the mixed path); the coarse CG is FP64.
