@@ -833,9 +833,12 @@ struct HsmgImpl : public HsmgState {
   CoarseArgs<T> ca;
   CoarseCg cg;
 
-  // The fine level has no masked point: its Schwarz gather-scatter merges
-  // into the final one.
-  bool merged_assembly() const { return fine->nmask == 0; }
+  // The fine Schwarz output's gather-scatter merges into the final one, with
+  // the mask when there is one: the prolonged correction is zero on masked
+  // points, and so are the r and w of the inner products that the prolongation
+  // forms on the unassembled output.  A masked FP32 level keeps its own
+  // gather-scatter, whose rounding its results carry.
+  bool merged_assembly() const { return fine->nmask == 0 || sizeof(T) == 8; }
 
   int launches() const override {
     // 2 Schwarz x (fdm, post, gs) + restrict + gs + coarse restrict + coarse
@@ -864,9 +867,9 @@ struct HsmgImpl : public HsmgState {
     return apply_to(zf, r, skip, s);
   }
 
-  // Without a mask the output is assembled by one final gather-scatter of
-  // the prolongation's result, so the inner products with the continuous r
-  // and w_prev can be formed by the prolongation itself.
+  // A merged output is assembled by one final gather-scatter of the
+  // prolongation's result, so the inner products with the continuous r and
+  // w_prev can be formed by the prolongation itself.
   bool dots_in_apply() const override { return merged_assembly(); }
   cudaError_t apply_dots(double *z, const double *r, const double *w_prev, double *part,
                          const int *skip, cudaStream_t s) override {
@@ -928,8 +931,7 @@ struct HsmgImpl : public HsmgState {
         (e = cudaStreamWaitEvent(s, ev_join_hi, 0)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(s, ev_join_crs, 0)) != cudaSuccess)
       return e;
-    // prolong: zs += J (e_mid + J_c e_crs); z = mult * gs(zs).  Without a mask the fine
-    // Schwarz output's own gather-scatter is folded into this one: wt and
+    // prolong: zs += J (e_mid + J_c e_crs); z = mult * gs(zs).  Merged: wt and
     // mult are the same at every copy of a point, so
     // mult gs(gs(wt e) + J e_mid) = gs(wt e + mult J e_mid).
     CoarseAdd<T> crs_add;
@@ -940,7 +942,7 @@ struct HsmgImpl : public HsmgState {
                                   merged ? dots : nullptr)) !=
         cudaSuccess)
       return e;
-    if ((e = gs_add_fused<T>(fine->gsd, zs, false, s, skip, merged ? nullptr : mult_f)) !=
+    if ((e = gs_add_fused<T>(fine->gsd, zs, merged, s, skip, merged ? nullptr : mult_f)) !=
         cudaSuccess)
       return e;
     return cudaGetLastError();
