@@ -434,8 +434,11 @@ cudaError_t CgWorkspace::ensure(long n_) {
   return cudaSuccess;
 }
 
-// One CG iteration (all launches on s), precond chosen by pc.
-static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, cudaStream_t s) {
+// One CG iteration (all launches on s), precond chosen by pc.  `last`: the
+// last of its chunk, the only one that can be due a true residual (the
+// interval is a multiple of the chunk).
+static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, bool last,
+                                cudaStream_t s) {
   const long n = P->n;
   const int rb = red_blocks(n), eg = stream_grid(n, 256);
   // A preconditioner that computes in FP32 leaves z in FP32 and the kernels
@@ -513,7 +516,7 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, cuda
   launch_chained(n, cg_update_xr_kernel, wave_blocks(n), kRedThreads, 0, s, W.r, W.p, W.w,
                  P->mult, P->multf, n, W.st,
                                                  W.partials, W.counter);
-  if (W.recompute_every > 0) {  // w = A x, gs, mask; r = f - w (scheduled iterations only)
+  if (W.recompute_every > 0 && last) {  // w = A x, gs, mask; r = f - w (scheduled iterations only)
     // x through z (free until the next preconditioner apply overwrites it)
     launch_chained(n, cg_copy_x_kernel, eg, 256, 0, s, W.z, n, W.st);
     e = P->ax(W.w, W.z, s, &W.st->skip_rc);
@@ -603,7 +606,13 @@ nb_status cg_start(CgRun &R) {
                                                  (W.use_dots << 3) | (W.fold << 4)),
                         (const void *)(intptr_t)P->ifh2};
   bool same = W.graph_exec && !memcmp(key, W.graph_key, sizeof(key));
-  R.chunk = n > (1 << 22) ? 4 : 16;
+  // Iterations a graph launch: the host looks at the state after each, about
+  // 15 us, against launches of the chunk that find the solve finished.  Jacobi
+  // iterations on small problems are short and many.
+  R.chunk = n > (1 << 22) ? 4 : W.fold && n <= (1 << 20) ? 32 : 16;
+  // with true residuals every 50 iterations: a divisor of that, so that the
+  // four launches of one are in a chunk's last iteration only
+  if (W.recompute_every > 0) R.chunk = n > (1 << 22) ? 5 : 10;
   if (!same) {
     if (W.graph_exec) {
       cudaGraphExecDestroy(W.graph_exec);
@@ -615,13 +624,13 @@ nb_status cg_start(CgRun &R) {
     NB_CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     cudaError_t ce = cudaSuccess;
     for (int k = 0; k < R.chunk && ce == cudaSuccess; k++)
-      ce = cg_iteration(P, W, pc, cs);
+      ce = cg_iteration(P, W, pc, k == R.chunk - 1, cs);
     // an FP32-output preconditioner skips its conversion launch; with the
     // inner products formed by the preconditioner a one-block finishing
     // launch replaces the dot pass
     const int pc_launches = pc ? pc->launches() - (pc->output_f32() ? 1 : 0) : 0;
-    W.launches_per_iter = (W.fused ? 4 : 6) - (W.fold ? 1 : 0) + pc_launches +
-                          (W.recompute_every > 0 ? 4 : 0);
+    W.launches_per_iter = (W.fused ? 4 : 6) - (W.fold ? 1 : 0) + pc_launches;
+    W.launches_per_chunk = R.chunk * W.launches_per_iter + (W.recompute_every > 0 ? 4 : 0);
     cudaError_t ee = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
     if (ce != cudaSuccess) {
@@ -643,7 +652,7 @@ nb_status cg_start(CgRun &R) {
 nb_status cg_next_chunk(CgRun &R) {
   CgWorkspace &W = *(CgWorkspace *)R.P->solver_ws;
   NB_CUDA_TRY(cudaGraphLaunch(W.graph_exec, R.s));
-  R.launches += R.chunk * W.launches_per_iter;
+  R.launches += W.launches_per_chunk;
   NB_CUDA_TRY(cudaMemcpyAsync(W.host_state, W.st, sizeof(CgState), cudaMemcpyDeviceToHost, R.s));
   NB_CUDA_TRY(cudaEventRecord(W.ev, R.s));
   return NB_OK;

@@ -74,7 +74,7 @@ struct CgWorkspace {
   bool fused = false;  // the last captured iteration used ax_cg_fused
   bool fold = false;   // z = d r is formed by the x and r update
   int recompute_every = 0;
-  int launches_per_iter = 6;
+  int launches_per_iter = 6, launches_per_chunk = 0;
   cudaGraphExec_t graph_exec = nullptr;
   cudaEvent_t ev = nullptr;  // behind the state copy of the last chunk
   const void *graph_key[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
