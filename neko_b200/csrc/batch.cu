@@ -16,7 +16,7 @@
 //       forms rnorm, the convergence flag and the next beta.
 //
 // Per-slot sums are formed by the last block of the slot from per-item
-// partials in item order, so they do not depend on scheduling.  (p, mult
+// partials in a fixed order, so they do not depend on scheduling.  (p, mult
 // gs(w)) is formed as the sum of p * w over local points before the
 // gather-scatter: p is continuous and zero on masked points, so the two
 // agree (each global point's weights 1/k over its k copies add to one).
@@ -47,9 +47,16 @@
 namespace nb {
 
 constexpr int kBT = 256;         // threads of the batched kernels
+// Largest work items.  A small slot is cut into about eight (share): a box of
+// 27 elements was two Ax items, 118 us an iteration on two multiprocessors
+// while its hsmg neighbours ran.  The cut depends on the slot alone, so that a
+// solve's sums do not change with the solves beside it.
 constexpr int kItemElems = 24;   // elements per Ax work item
 constexpr long kChunk = 8192;    // points per vector chunk
 constexpr int kGsChunk = 4096;   // gs items per chunk
+static long share(long total, long least, long most) {
+  return std::max(least, std::min(most, (total + 7) / 8));
+}
 
 struct BSlot {
   int lx, nelv;
@@ -264,14 +271,17 @@ __global__ void __launch_bounds__(kBT)
       last_s = atomicAdd(&S.ax_counter, 1u) == (unsigned)S.ax_count - 1;
     }
     __syncthreads();
-    if (last_s && threadIdx.x == 0) {
+    if (last_s) {  // uniform over the block
       __threadfence();
       double pap = 0.0;
-      for (int q = S.ax_first; q < S.ax_first + S.ax_count; q++)
+      for (int q = S.ax_first + threadIdx.x; q < S.ax_first + S.ax_count; q += kBT)
         pap += *((volatile double *)part + q);
-      S.ax_counter = 0;
-      S.pap = pap;
-      S.alpha = S.rtz / pap;
+      pap = block_sum<kBT>(pap, red);
+      if (threadIdx.x == 0) {
+        S.ax_counter = 0;
+        S.pap = pap;
+        S.alpha = S.rtz / pap;
+      }
     }
     __syncthreads();
   }
@@ -299,13 +309,16 @@ __device__ __forceinline__ bool slot_sum2(BSlot &S, int c, double v0, double v1,
     last_s = atomicAdd(&S.vc_counter, 1u) == (unsigned)S.vc_count - 1;
   }
   __syncthreads();
-  if (!last_s || threadIdx.x != 0) return false;
+  if (!last_s) return false;
   __threadfence();
   t0 = t1 = 0.0;
-  for (int q = S.vc_first; q < S.vc_first + S.vc_count; q++) {
+  for (int q = S.vc_first + threadIdx.x; q < S.vc_first + S.vc_count; q += kBT) {
     t0 += *((volatile double *)part + 2 * q);
     t1 += *((volatile double *)part + 2 * q + 1);
   }
+  t0 = block_sum<kBT>(t0, sh);
+  t1 = block_sum<kBT>(t1, sh);
+  if (threadIdx.x != 0) return false;
   S.vc_counter = 0;
   return true;
 }
@@ -588,18 +601,23 @@ static nb_status rebuild(nb_batch *b, std::vector<BSlot> &host_slots) {
   for (int s : order) {
     BSlot &S = host_slots[s];
     S.ax_first = (int)items.size();
-    for (int e = 0; e < S.nelv; e += kItemElems)
-      items.push_back(AxItem{s, e, std::min(kItemElems, S.nelv - e), S.lx});
+    const int per_item = (int)share(S.nelv, 4, kItemElems);
+    for (int e = 0; e < S.nelv; e += per_item)
+      items.push_back(AxItem{s, e, std::min(per_item, S.nelv - e), S.lx});
     S.ax_count = (int)items.size() - S.ax_first;
   }
   for (int s = 0; s < ns; s++) {
     if (!b->slots[s].used) continue;
     BSlot &S = host_slots[s];
     S.vc_first = (int)vch.size();
-    for (long i = 0; i < S.n; i += kChunk) vch.push_back(VChunk{s, 0, i, std::min(S.n, i + kChunk)});
+    const long per_chunk = share(S.n, 1024, kChunk);
+    for (long i = 0; i < S.n; i += per_chunk)
+      vch.push_back(VChunk{s, 0, i, std::min(S.n, i + per_chunk)});
     S.vc_count = (int)vch.size() - S.vc_first;
     const int ng = (int)gs_items(S.gs, true);
-    for (int t = 0; t < ng; t += kGsChunk) gch.push_back(GChunk{s, t, std::min(ng, t + kGsChunk), 0});
+    const int per_gs = (int)share(ng, 512, kGsChunk);
+    for (int t = 0; t < ng; t += per_gs)
+      gch.push_back(GChunk{s, t, std::min(ng, t + per_gs), 0});
   }
   NB_BTRY(grow(b->d_slots, b->cap_slots, (size_t)std::max(ns, 1)));
   NB_BTRY(grow(b->d_items, b->cap_items, std::max<size_t>(items.size(), 1)));
