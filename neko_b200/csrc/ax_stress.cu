@@ -85,23 +85,21 @@ __device__ __forceinline__ void stress_point(const double g[3][3], const double 
 }
 
 // ---------------------------------------------------------------------------
-// Streaming kernel (lx 4, 6, 8, 10).  Bound by HBM (136 B a point, 152 with
+// Streaming kernel (lx 4, 6, 10; lx 8 below).  Bound by HBM (136 B a point, 152 with
 // h2; 184 / 200 in the CG form) with shared-memory wavefronts close behind.
 //
 // The nine flux planes lie over the nine cofactor arrays of the element's own
 // stage: a thread reads the nine cofactors of a point and writes that point's
 // nine fluxes over them, and no thread reads another point's cofactors.  So
-// a stage is all the memory an element needs (14 arrays), two blocks of two
-// stages share a multiprocessor at lx 8, and two stages of lx 10 (224 KB) fit
-// one.  With separate planes only one block of 256 threads was resident at
-// lx 8 (104 us a coupled-CG step on 2.1 M points, 62% of the copy rate) and
-// lx 10 had no streaming form (272 us on 2.2 M points, plus 29 us for the h2
-// term).  h2, B and (CG form) z go straight to registers instead of
+// a stage is all the memory an element needs (14 arrays) and two stages of
+// lx 10 (224 KB) fit a multiprocessor.  With separate planes lx 10 had no
+// streaming form (272 us on 2.2 M points, plus 29 us for the h2 term; 141 us
+// in this one).  h2, B and (CG form) z go straight to registers instead of
 // staging up to five more arrays; they are brought to L2 when the stage is
 // filled.
-// Registers (two blocks of 256 threads, or one of 512: 128 a thread) hold two
-// rows of D at a time, reloaded for the second pass, and the components are
-// differentiated one after the other.
+// Registers (512 threads a multiprocessor: 128 each) hold two rows of D at a
+// time, reloaded for the second pass, and the components are differentiated
+// one after the other.
 // ---------------------------------------------------------------------------
 template <int LX, int S, int KS>
 struct StressCfg {
@@ -321,6 +319,298 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS>::THREADS, StressCfg<LX, S
   }
 }
 
+// ---------------------------------------------------------------------------
+// lx = 8: the contractions within a k-plane on the FP64 matrix instruction.
+// An 8 x 8 plane is one m8n8k4 tile (two k-steps), with no padding.  The
+// kernel above is bound by shared-memory wavefronts (about 330 a warp of
+// points: an r or s derivative reads eight values a point, each load two
+// wavefronts); here a lane owns the points (j, i) = (lane / 4, 2 (lane % 4) +
+// {0, 1}) of a plane, the tile's result layout, and
+//   r derivative: A = the plane itself, its fragment the lane's own values
+//                 (the contraction index taken as 2 t + s in k-step s);
+//   s derivative: B = the plane, two loads a lane;
+//   r flux:       A = the flux, straight from the lane's registers;
+//   s flux:       through the warp's own plane of the stage, warp-synchronous;
+//   t:            plain FMAs down the lane's column, 16-byte loads.
+// About 95 wavefronts a warp of points.  Four warps an element, two planes
+// each.  The matrix instruction runs at the FP64 FMA rate (37 against 33
+// TFLOP/s measured), so it saves the operand traffic, not arithmetic.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+  asm volatile(
+      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+struct StressMma {
+  static constexpr int LX = 8, L2 = 64, L3 = 512, NA = 14, S = 2, THREADS = 128;
+  static constexpr size_t ABYTES = L3 * sizeof(double);
+  static constexpr size_t SMEM = S * NA * ABYTES + L2 * sizeof(double) + 16 * S;
+};
+
+template <bool CG>
+__global__ void __launch_bounds__(StressMma::THREADS, 2)
+    ax_stress_mma_kernel(StressIo io, StressGeo geo, const double *__restrict__ dx,
+                         const double *__restrict__ dy, const double *__restrict__ dz,
+                         const double *__restrict__ w3, const double *__restrict__ h2,
+                         const double *__restrict__ Bm, const int nelv, int *__restrict__ err,
+                         const int *__restrict__ skip, StressCg cg) {
+  using C = StressMma;
+  constexpr int LX = C::LX, L2 = C::L2, L3 = C::L3, NA = C::NA, S = C::S;
+  extern __shared__ __align__(128) unsigned char smem_stress[];
+  double *stage = reinterpret_cast<double *>(smem_stress);
+  double *sDz = stage + S * NA * L3;
+  uint64_t *full = reinterpret_cast<uint64_t *>(sDz + L2);
+
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int G = gridDim.x, b = blockIdx.x;
+  const int nt = b < nelv ? (nelv - b + G - 1) / G : 0;
+  if (tid == 0) {
+    for (int s = 0; s < S; s++) mbar_init(&full[s], 1);
+    fence_barrier_init();
+  }
+  chain();
+  if (skip && *skip) return;
+  if (CG && cg.st->done) return;
+  const double beta = CG ? cg.st->beta : 0.0;
+  for (int q = tid; q < L2; q += C::THREADS) sDz[q] = dz[q];
+  __syncthreads();
+  auto issue = [&](int t, int s) {
+    const long e = b + (long)t * G;
+    mbar_arrive_expect_tx(&full[s], (uint32_t)(NA * C::ABYTES));
+#pragma unroll
+    for (int a = 0; a < NA; a++) {
+      const double *src =
+          a < 3 ? io.in[a] : (a == 3 ? geo.h1 : (a == 4 ? geo.jacinv : geo.c[a - 5]));
+      bulk_g2s(stage + (size_t)(s * NA + a) * L3, src + e * L3, (uint32_t)C::ABYTES, &full[s]);
+    }
+    if (h2) {
+      bulk_prefetch_l2(h2 + e * L3, (uint32_t)C::ABYTES);
+      bulk_prefetch_l2(Bm + e * L3, (uint32_t)C::ABYTES);
+    }
+    if constexpr (CG) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) bulk_prefetch_l2(cg.z[c] + e * L3, (uint32_t)C::ABYTES);
+    }
+  };
+  if (tid == 0)
+    for (int t = 0; t < S && t < nt; t++) issue(t, t);
+
+  // tile coordinates: row m, column pair n
+  const int m = lane >> 2, n = lane & 3, k0 = 2 * wid;
+  const int own = LX * m + 2 * n;  // the lane's two points in a plane
+  // fragments of D: r derivative (B), s derivative (A), r flux (B), s flux (A)
+  double dr[2], ds[2], fr[2], fs[2];
+#pragma unroll
+  for (int s = 0; s < 2; s++) {
+    dr[s] = __ldg(dx + m + LX * (2 * n + s));
+    ds[s] = __ldg(dy + m + LX * (n + 4 * s));
+    fr[s] = __ldg(dx + (2 * n + s) + LX * m);
+    fs[s] = __ldg(dy + (n + 4 * s) + LX * m);
+  }
+  auto get2 = [](const double *p, double (&v)[2]) {
+    const double2 t = *reinterpret_cast<const double2 *>(p);
+    v[0] = t.x;
+    v[1] = t.y;
+  };
+  auto put2 = [](double *p, const double (&v)[2]) {
+    *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+  };
+
+  int t = 0;
+  bool failed = false;
+  double pap = 0.0;
+  for (; t < nt; t++) {
+    const int s = t % S;
+    const long e = b + (long)t * G;
+    double *slot = stage + (size_t)s * NA * L3;
+    const bool ok = mbar_wait(&full[s], (uint32_t)((t / S) & 1));
+    if (__syncthreads_or(!ok)) {
+      failed = true;
+      break;
+    }
+    if constexpr (CG) {  // p = z + beta p for the lane's points, in the stage and stored
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int kk = 0; kk < 2; kk++) {
+          const int q = L2 * (k0 + kk) + own;
+          const double2 z = __ldg(reinterpret_cast<const double2 *>(cg.z[c] + e * L3 + q));
+          double p[2];
+          get2(slot + c * L3 + q, p);
+          p[0] = z.x + beta * p[0];
+          p[1] = z.y + beta * p[1];
+          put2(slot + c * L3 + q, p);
+          put2(cg.pout[c] + e * L3 + q, p);
+        }
+      __syncthreads();  // the element's new directions complete in the stage
+    }
+    // t derivatives of both planes, down the lane's column
+    double ut[2][3][2];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+#pragma unroll
+      for (int kk = 0; kk < 2; kk++) ut[kk][c][0] = ut[kk][c][1] = 0.0;
+#pragma unroll
+      for (int l = 0; l < LX; l++) {
+        double v[2];
+        get2(slot + c * L3 + L2 * l + own, v);
+#pragma unroll
+        for (int kk = 0; kk < 2; kk++) {
+          const double d = sDz[k0 + kk + LX * l];
+          ut[kk][c][0] += d * v[0];
+          ut[kk][c][1] += d * v[1];
+        }
+      }
+    }
+    double acc[2][3][2];  // r and s flux divergence at the lane's points
+#pragma unroll
+    for (int kk = 0; kk < 2; kk++) {
+      const int base = L2 * (k0 + kk);
+      double g[2][3][3];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double *u = slot + c * L3 + base;
+        double v[2], ur[2] = {0.0, 0.0}, us[2] = {0.0, 0.0};
+        get2(u + own, v);
+#pragma unroll
+        for (int h = 0; h < 2; h++) mma_f64(ur, v[h], dr[h]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) mma_f64(us, ds[h], u[LX * (n + 4 * h) + m]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          g[h][c][0] = ur[h];
+          g[h][c][1] = us[h];
+          g[h][c][2] = ut[kk][c][h];
+        }
+      }
+      double cf[2][9], hv[2], jv[2], f[2][3][3];
+#pragma unroll
+      for (int a = 0; a < 9; a++) {
+        double v[2];
+        get2(slot + (5 + a) * L3 + base + own, v);
+        cf[0][a] = v[0];
+        cf[1][a] = v[1];
+      }
+      get2(slot + 3 * L3 + base + own, hv);
+      get2(slot + 4 * L3 + base + own, jv);
+      const double2 wv = __ldg(reinterpret_cast<const double2 *>(w3 + base + own));
+      stress_point(g[0], cf[0], hv[0] * wv.x * jv[0], f[0]);
+      stress_point(g[1], cf[1], hv[1] * wv.y * jv[1], f[1]);
+      // s and t fluxes over the cofactors just read, the lane's own points
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double vs[2] = {f[0][c][1], f[1][c][1]}, vt[2] = {f[0][c][2], f[1][c][2]};
+        put2(slot + (5 + c) * L3 + base + own, vs);
+        put2(slot + (8 + c) * L3 + base + own, vt);
+      }
+      __syncwarp();  // the plane's s fluxes, all from this warp
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double *v = slot + (5 + c) * L3 + base;
+        acc[kk][c][0] = acc[kk][c][1] = 0.0;
+#pragma unroll
+        for (int h = 0; h < 2; h++) mma_f64(acc[kk][c], f[h][c][0], fr[h]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) mma_f64(acc[kk][c], fs[h], v[LX * (n + 4 * h) + m]);
+      }
+    }
+    __syncthreads();  // every plane's t fluxes complete
+    double hb[2][2];
+    if (h2) {
+#pragma unroll
+      for (int kk = 0; kk < 2; kk++) {
+        const long q = e * L3 + L2 * (k0 + kk) + own;
+        const double2 x = __ldg(reinterpret_cast<const double2 *>(h2 + q)),
+                      y = __ldg(reinterpret_cast<const double2 *>(Bm + q));
+        hb[kk][0] = x.x * y.x;
+        hb[kk][1] = x.y * y.y;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      double d[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+      for (int l = 0; l < LX; l++) {
+        double v[2];
+        get2(slot + (8 + c) * L3 + L2 * l + own, v);
+#pragma unroll
+        for (int kk = 0; kk < 2; kk++) {
+          const double z = sDz[l + LX * (k0 + kk)];
+          d[kk][0] += z * v[0];
+          d[kk][1] += z * v[1];
+        }
+      }
+#pragma unroll
+      for (int kk = 0; kk < 2; kk++) {
+        const int q = L2 * (k0 + kk) + own;
+        double u[2], v[2];
+        get2(slot + c * L3 + q, u);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          v[h] = acc[kk][c][h] + d[kk][h];
+          if (h2) v[h] = v[h] + hb[kk][h] * u[h];  // au + h2 B u, the part2 order
+          if (CG) pap += u[h] * v[h];
+        }
+        put2(io.out[c] + e * L3 + q, v);
+      }
+    }
+    // this thread's writes to the stage come before the next copy into it
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();  // stage s consumed
+    if (tid == 0 && t + S < nt) issue(t + S, s);
+  }
+  if (failed) {
+    if (tid == 0) {
+      atomicExch(err, 1);
+      // bounded wait for this CTA's copies still in flight
+      for (int q = t; q < nt && q < t + S; q++) mbar_wait(&full[q % S], (uint32_t)((q / S) & 1));
+    }
+    __syncthreads();
+  }
+  if constexpr (CG) {
+    double tot;  // every block takes part, a failed one with its partial sum
+    if (grid_sum<C::THREADS>(pap, cg.partials, cg.counter, &tot)) {
+      cg.st->pap = tot;
+      cg.st->alpha = cg.st->rtz1 / tot;
+    }
+  }
+}
+
+template <bool CG>
+static cudaError_t launch_stress_mma(const StressIo &io, const StressGeo &geo, const double *dx,
+                                     const double *dy, const double *dz, const double *w3,
+                                     const double *h2, const double *Bm, int nelv,
+                                     cudaStream_t st, int *err, const int *skip,
+                                     const StressCg &cg = StressCg{}) {
+  using C = StressMma;
+  // results and directions are stored in 16-byte pairs, w3 is read in them
+  const void *ptrs[] = {io.out[0], io.out[1], io.out[2], w3, h2, Bm};
+  for (const void *q : ptrs)
+    if (reinterpret_cast<uintptr_t>(q) & 15) return cudaErrorNotSupported;
+  auto kern = ax_stress_mma_kernel<CG>;
+  static int grid_per_dev[64] = {0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  int &g = grid_per_dev[dev & 63];
+  if (g == 0) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::THREADS, C::SMEM);
+    if (e != cudaSuccess) return e;
+    g = (per_sm > 0 ? per_sm : 1) * device_sms();
+  }
+  if (nelv <= 0) return cudaSuccess;
+  if (!err) err = dropin_error_word();
+  if (!err) return cudaErrorInvalidSymbol;
+  return launch_chained(3L * nelv * C::L3, kern,
+                        nelv < g ? nelv : g, C::THREADS, C::SMEM, st, io, geo, dx, dy, dz,
+                        w3, h2, Bm, nelv, err, skip, cg);
+}
+
 template <int LX, int S, int KS, bool CG = false>
 static cudaError_t launch_stress_tma(const StressIo &io, const StressGeo &geo, const double *dx,
                                      const double *dy, const double *dz, const double *w3,
@@ -513,7 +803,12 @@ cudaError_t ax_stress(double *au, double *av, double *aw, const double *u, const
     switch (lx) {
       case 4: return launch_stress_tma<4, 3, 4>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
       case 6: return launch_stress_tma<6, 2, 3>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
-      case 8: return launch_stress_tma<8, 2, 4>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
+      case 8: {
+        const cudaError_t e =
+            launch_stress_mma<false>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
+        if (e != cudaErrorNotSupported) return e;
+        break;
+      }
       case 10: return launch_stress_tma<10, 2, 5>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
       default: break;
     }
@@ -726,7 +1021,7 @@ cudaError_t problem_ax_stress_cg(nb_problem *P, double *const w[3], double *cons
   switch (P->lx) {
     case 4: return launch_stress_tma<4, 3, 4, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
     case 6: return launch_stress_tma<6, 2, 3, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
-    case 8: return launch_stress_tma<8, 2, 4, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
+    case 8: return launch_stress_mma<true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
     case 10: return launch_stress_tma<10, 2, 5, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
     default: return cudaErrorNotSupported;
   }
