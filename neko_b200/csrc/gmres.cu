@@ -135,7 +135,7 @@ __global__ void gm_precond_kernel(double *__restrict__ z, const double *__restri
 // h(i, j) = (w, mult v_i) for i = 0..j: vectors in chunks of kGmresChunk per
 // pass over the points; block partials per vector, the last block sums them
 // in block order.
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, 4)
     gm_many_dot_kernel(const double *__restrict__ w, const double *const *__restrict__ V,
                        const double *__restrict__ mult, const float *__restrict__ multf, long n,
                        int j, GmresState *st, double *partials, unsigned *counter) {
@@ -167,13 +167,16 @@ __global__ void __launch_bounds__(kRedThreads)
   __syncthreads();
   if (!last) return;
   __threadfence();
-  __shared__ double shs[kRedThreads / 32];
-  for (int k = 0; k < nv; k++) {
+  // a warp a vector: its lanes take the blocks in turn, one fixed tree (one
+  // vector after the other by the whole block, this tail was most of the 13 us
+  // of a column on 453 thousand points)
+  const int lane = threadIdx.x & 31;
+  for (int k = threadIdx.x >> 5; k < nv; k += kRedThreads / 32) {
     double t = 0.0;
-    for (int b = threadIdx.x; b < G; b += kRedThreads)
-      t += *((volatile double *)partials + (size_t)k * G + b);
-    t = block_sum<kRedThreads>(t, shs);
-    if (threadIdx.x == 0) st->h[k + st->m * j] = t;
+#pragma unroll 4
+    for (int b = lane; b < G; b += 32) t += __ldcg(partials + (size_t)k * G + b);
+    t = warp_sum(t);
+    if (lane == 0) st->h[k + st->m * j] = t;
   }
   if (threadIdx.x == 0) *counter = 0;
 }
@@ -398,8 +401,8 @@ static cudaError_t gmres_cycle(nb_problem *P, GmresWorkspace &W, Precond *pc, bo
     e = apply_op(P, W.w, W.Z[j], &W.st->stop, s);
     if (e != cudaSuccess) return e;
     L += 2;
-    launch_chained(n, gm_many_dot_kernel, rb, kRedThreads, 0, s, W.w, W.Vp, P->mult, P->multf, n,
-                   j, W.st,
+    launch_chained(n, gm_many_dot_kernel, wave_blocks(n), kRedThreads, 0, s, W.w, W.Vp, P->mult,
+                   P->multf, n, j, W.st,
                                                   W.partials, W.counter);
     launch_chained(n, gm_part2_kernel, rb, kRedThreads, 0, s, W.w, W.Vp, P->mult, P->multf, n, j,
                    W.st,
