@@ -242,7 +242,8 @@ __global__ void __launch_bounds__(AxCfgS<LX, S, KS, NE, CG, AL>::THREADS)
     double *base = stage + (size_t)s * NA * AS;
     auto source = [&](int q) {
       return q < U0 ? nullptr
-                    : q == U0 ? (CG ? (const double *)a.p : a.u) : q == U0 + 1 ? a.h1 : a.g[q - U0 - 2];
+                    : q == U0 ? (CG ? (const double *)a.p : a.u)
+                              : q == U0 + 1 ? a.h1 : a.g[q - U0 - 2];
     };
     if (odd) {  // its last value of each array, before the arrival below
       if (CG) reinterpret_cast<TZ *>(base)[L3 - 1] = a.z[e0 * L3 + L3 - 1];
@@ -427,9 +428,10 @@ static cudaError_t launch_ax_stream_as(const AxArgs<TZ> &a, cudaStream_t st) {
 // Stages, k split and overlay of an order, without and with h2.  A larger split
 // (more threads an element) hides the loads of h2 and B, which come past the
 // ring: lx 8 with h2 takes 102 us at 7.1 M points split by 4, 126 by 2.  A
-// smaller one leaves registers for another block: the step at lx 10 takes 128
-// us at 6.9 M points split by 2, 156 by 5 with a third, overlaid stage, and at
-// lx 8 105 us at 7.1 M points unsplit, 113 split by 2.
+// smaller one loads less from shared memory, as every part of the split reads
+// its columns whole for the t derivatives: the step at lx 8 takes 105 us at 7.1
+// M points unsplit, 113 split by 2; at lx 10 128 us at 6.9 M points split by 2,
+// 156 by 5 (with a third, overlaid stage).
 template <int LX, int NE, bool CG, int S, int KS, bool AL, int S2, int KS2, bool AL2, typename TZ>
 static cudaError_t launch_ax_stream(const AxArgs<TZ> &a, cudaStream_t st) {
   return a.h2 ? launch_ax_stream_as<LX, S2, KS2, NE, CG, AL2, true>(a, st)
@@ -461,10 +463,12 @@ cudaError_t ax_helm_stream(double *w, const double *u, const double *D, const do
     case 5: return launch_ax_stream<5, 2, false, 3, 1, false, 3, 1, false>(a, s);
     case 6: return launch_ax_stream<6, 1, false, 3, 3, false, 3, 3, false>(a, s);
     case 7:
-      // While a block takes two pairs of elements at most, a single stage, which
-      // lets a third block run: 23 against 28 us for the operator with h2,
-      // gather-scatter and mask on 453 thousand points out of cache.  With more
-      // of them a second stage: 127 against 157 us at 6.8 M points.
+      // While a block (two a multiprocessor) takes three pairs of elements at
+      // most, a single stage: the copies of a second would share the bandwidth
+      // with those of the first pair, which every block waits for.  Operator with
+      // h2, gather-scatter and mask on 453 thousand points out of cache: 23 us,
+      // 28 with two stages.  With more pairs the second stage pays: 127 against
+      // 157 us at 6.8 M points.
       return nelv <= 12 * device_sms()
                  ? launch_ax_stream<7, 2, false, 1, 2, false, 1, 2, false>(a, s)
                  : launch_ax_stream<7, 2, false, 2, 1, false, 2, 2, false>(a, s);

@@ -49,8 +49,9 @@ namespace nb {
 constexpr int kBT = 256;         // threads of the batched kernels
 // Largest work items.  A small slot is cut into about eight (share): a box of
 // 27 elements was two Ax items, 118 us an iteration on two multiprocessors
-// while its hsmg neighbours ran.  The cut depends on the slot alone, so that a
-// solve's sums do not change with the solves beside it.
+// while its hsmg neighbours ran (24 uneven solves: 74 ms, 59 cut so).  The cut
+// depends on the slot alone, so that a solve's sums do not change with the
+// solves beside it.
 constexpr int kItemElems = 24;   // elements per Ax work item
 constexpr long kChunk = 8192;    // points per vector chunk
 constexpr int kGsChunk = 4096;   // gs items per chunk

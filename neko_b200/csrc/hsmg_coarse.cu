@@ -24,15 +24,14 @@
 // block before the barrier of the sums, and each block forms p for itself,
 // which leaves two cluster barriers an iteration and gathers that never leave
 // the block.  That takes one row a thread, 8192 vertices; larger meshes, and
-// those without a mask beyond kCoarseFreeNodes, keep
-// element-local vectors on a grid of all multiprocessors
-// (coarse_cg_grid_kernel).
+// those without a mask beyond kCoarseFreeNodes, keep element-local vectors on a
+// grid of all multiprocessors (coarse_cg_grid_kernel).
 //
 // A solve on 343 vertices (8^3 elements) took 124 us as a cooperative grid
 // with barriers in global memory and element-local vectors (33 barriers of
-// about 3.7 us with their sums), 67 us with p in global memory, and 22 so.
-// A cluster leaves the other multiprocessors to the fine-level smoother,
-// which runs beside it; the grid form holds one block on every one.
+// about 3.7 us with their sums), 67 us as a cluster with p in global memory
+// and 33 us so.  A cluster leaves the other multiprocessors to the fine-level
+// smoother, which runs beside it; the grid form holds one block on every one.
 //
 // The arithmetic is that of cg_init / cg_precond_dot / cg_update_p /
 // ax_helm / gs / cg_update_xr with sums over distinct points: a mult-weighted
