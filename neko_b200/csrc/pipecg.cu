@@ -21,6 +21,7 @@
 #include <cstring>
 #include <string>
 
+#include "nb_chain.cuh"
 #include "nb_kernels.h"
 #include "nb_precond.h"
 #include "nb_problem.h"
@@ -38,90 +39,50 @@ struct PipeState {
   double *x;  // the solve's x, read by the captured iterations
 };
 
-// (r, mult u), (w, mult u), (r, mult r) into st->red
-__device__ __forceinline__ void pipe_reduce3(double t1, double t2, double t3, PipeState *st,
+// (r, mult u), (w, mult u), (r, mult r) into st->red; true on thread 0 of the
+// last block, which has them.  The three sums take their stages side by side.
+__device__ __forceinline__ bool pipe_reduce3(double t1, double t2, double t3, PipeState *st,
                                              double *partials, unsigned *counter) {
-  __shared__ double sh[kRedThreads / 32];
+  constexpr int W = kRedThreads / 32;
+  __shared__ double sh[3][W];
   __shared__ bool last;
-  const double b1 = block_sum<kRedThreads>(t1, sh);
-  const double b2 = block_sum<kRedThreads>(t2, sh);
-  const double b3 = block_sum<kRedThreads>(t3, sh);
-  const int G = gridDim.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, G = gridDim.x;
+  double v[3] = {t1, t2, t3};
+  auto block_sum3 = [&] {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      v[k] = warp_sum(v[k]);
+      if (lane == 0) sh[k][wid] = v[k];
+    }
+    __syncthreads();
+    if (wid == 0) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) v[k] = warp_sum(lane < W ? sh[k][lane] : 0.0);
+    }
+    __syncthreads();
+  };
+  block_sum3();
   if (threadIdx.x == 0) {
-    partials[blockIdx.x] = b1;
-    partials[G + blockIdx.x] = b2;
-    partials[2 * G + blockIdx.x] = b3;
+    for (int k = 0; k < 3; k++) partials[k * G + blockIdx.x] = v[k];
     __threadfence();
     last = atomicAdd(counter, 1u) == (unsigned)G - 1;
   }
   __syncthreads();
-  if (!last) return;
+  if (!last) return false;
   __threadfence();
   for (int k = 0; k < 3; k++) {
-    double t = 0.0;
-    for (int b = threadIdx.x; b < G; b += kRedThreads)
-      t += *((volatile double *)partials + k * G + b);
-    t = block_sum<kRedThreads>(t, sh);
-    if (threadIdx.x == 0) st->red[k] = t;
+    v[k] = 0.0;
+    for (int b = threadIdx.x; b < G; b += kRedThreads) v[k] += __ldcg(partials + k * G + b);
   }
-  if (threadIdx.x == 0) *counter = 0;
-}
-
-// x = p = z = q = s = 0, r = f
-__global__ void pipe_zero_kernel(double *__restrict__ x, double *__restrict__ p,
-                                 double *__restrict__ z, double *__restrict__ q,
-                                 double *__restrict__ s, double *__restrict__ r,
-                                 const double *__restrict__ f, long n) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
-       i += (long)gridDim.x * blockDim.x) {
-    x[i] = 0.0;
-    p[i] = 0.0;
-    z[i] = 0.0;
-    q[i] = 0.0;
-    s[i] = 0.0;
-    r[i] = f[i];
-  }
-}
-
-// out = d v (Jacobi) or v; nothing when *skip
-__global__ void pipe_diag_kernel(double *__restrict__ out, const double *__restrict__ v,
-                                 const double *__restrict__ d, long n, const int *skip) {
-  if (skip && *skip) return;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
-       i += (long)gridDim.x * blockDim.x)
-    out[i] = d ? d[i] * v[i] : v[i];
-}
-
-// The first inner products: gamma, delta, rtr of r, u, w.
-__global__ void __launch_bounds__(kRedThreads)
-    pipe_first_dots_kernel(const double *__restrict__ r, const double *__restrict__ u,
-                           const double *__restrict__ w, const double *__restrict__ mult,
-                           const float *__restrict__ multf, long n, PipeState *st,
-                           double *partials, unsigned *counter) {
-  double t1 = 0, t2 = 0, t3 = 0;
-  for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
-       i += (long)gridDim.x * kRedThreads) {
-    const double m = MW(i);
-    t1 += r[i] * m * u[i];
-    t2 += w[i] * m * u[i];
-    t3 += r[i] * m * r[i];
-  }
-  pipe_reduce3(t1, t2, t3, st, partials, counter);
-}
-
-// res_start and the zero-residual exit
-__global__ void pipe_start_kernel(PipeState *st) {
-  st->gamma1 = 0.0;
-  st->rtr = st->red[2];
-  st->rnorm = sqrt(st->rtr) * st->norm_fac;
-  st->res_start = st->rnorm;
-  st->iter = 0;
-  st->nan = 0;
-  st->done = st->rnorm == 0.0 ? 1 : 0;
+  block_sum3();
+  if (threadIdx.x != 0) return false;
+  for (int k = 0; k < 3; k++) st->red[k] = v[k];
+  *counter = 0;
+  return true;
 }
 
 // Scalars of one iteration from the last vector pass's inner products.
-__global__ void pipe_scalar_kernel(PipeState *st) {
+__device__ __forceinline__ void pipe_scalars(PipeState *st) {
   if (st->done) return;
   if (st->iter >= st->max_iter) {  // the loop of max_iter iterations has ended
     st->done = 1;
@@ -153,14 +114,79 @@ __global__ void pipe_scalar_kernel(PipeState *st) {
   }
 }
 
-// The vector pass of one iteration and the next inner products.
+// x = p = z = q = s = 0, r = f
+__global__ void pipe_zero_kernel(double *__restrict__ x, double *__restrict__ p,
+                                 double *__restrict__ z, double *__restrict__ q,
+                                 double *__restrict__ s, double *__restrict__ r,
+                                 const double *__restrict__ f, long n) {
+  chain();
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
+       i += (long)gridDim.x * blockDim.x) {
+    x[i] = 0.0;
+    p[i] = 0.0;
+    z[i] = 0.0;
+    q[i] = 0.0;
+    s[i] = 0.0;
+    r[i] = f[i];
+  }
+}
+
+// out = d v (Jacobi) or v; nothing when *skip
+__global__ void pipe_diag_kernel(double *__restrict__ out, const double *__restrict__ v,
+                                 const double *__restrict__ d, long n, const int *skip) {
+  chain();
+  if (skip && *skip) return;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
+       i += (long)gridDim.x * blockDim.x)
+    out[i] = d ? d[i] * v[i] : v[i];
+}
+
+// res_start and the zero-residual exit
+__device__ __forceinline__ void pipe_start(PipeState *st) {
+  st->gamma1 = 0.0;
+  st->rtr = st->red[2];
+  st->rnorm = sqrt(st->rtr) * st->norm_fac;
+  st->res_start = st->rnorm;
+  st->iter = 0;
+  st->nan = 0;
+  st->done = st->rnorm == 0.0 ? 1 : 0;
+}
+
+// The first inner products: gamma, delta, rtr of r, u, w; the first scalars.
+__global__ void __launch_bounds__(kRedThreads)
+    pipe_first_dots_kernel(const double *__restrict__ r, const double *__restrict__ u,
+                           const double *__restrict__ w, const double *__restrict__ mult,
+                           const float *__restrict__ multf, long n, PipeState *st,
+                           double *partials, unsigned *counter) {
+  chain();
+  double t1 = 0, t2 = 0, t3 = 0;
+  for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
+       i += (long)gridDim.x * kRedThreads) {
+    const double m = MW(i);
+    t1 += r[i] * m * u[i];
+    t2 += w[i] * m * u[i];
+    t3 += r[i] * m * r[i];
+  }
+  if (pipe_reduce3(t1, t2, t3, st, partials, counter)) {
+    pipe_start(st);
+    pipe_scalars(st);
+  }
+}
+
+// The vector pass of one iteration, the next inner products and, on the last
+// block, the next scalars.  Without a preconditioner of its own (pc) the
+// pass also forms mi = d w (mi = w without d) for the next operator.  As launches
+// of their own the scalars and the diagonal were two of an iteration's five,
+// each a launch gap and a few microseconds.
 __global__ void __launch_bounds__(kRedThreads)
     pipe_vecops_kernel(double *__restrict__ p, double *__restrict__ q,
                        double *__restrict__ r, double *__restrict__ s, double *__restrict__ u,
                        double *__restrict__ w, double *__restrict__ z,
-                       const double *__restrict__ ni, const double *__restrict__ mi,
-                       const double *__restrict__ mult, const float *__restrict__ multf, long n,
-                       PipeState *st, double *partials, unsigned *counter) {
+                       const double *__restrict__ ni, double *__restrict__ mi, bool pc,
+                       const double *__restrict__ d, const double *__restrict__ mult,
+                       const float *__restrict__ multf, long n, PipeState *st,
+                       double *partials, unsigned *counter) {
+  chain();
   if (st->done) return;
   double *__restrict__ x = st->x;
   const double alpha = st->alpha, beta = st->beta;
@@ -183,12 +209,13 @@ __global__ void __launch_bounds__(kRedThreads)
     r[i] = rn;
     u[i] = un;
     w[i] = wn;
+    if (!pc) mi[i] = d ? d[i] * wn : wn;
     const double m = MW(i);
     t1 = t1 + rn * m * un;
     t2 = t2 + wn * m * un;
     t3 = t3 + rn * m * rn;
   }
-  pipe_reduce3(t1, t2, t3, st, partials, counter);
+  if (pipe_reduce3(t1, t2, t3, st, partials, counter)) pipe_scalars(st);
 }
 
 struct PipeWorkspace {
@@ -247,9 +274,8 @@ static cudaError_t pipe_op(nb_problem *P, double *w, const double *u, const int 
 static cudaError_t pipe_precond(nb_problem *P, Precond *pc, bool jacobi, double *out,
                                 const double *in, const int *skip, cudaStream_t s) {
   if (pc) return pc->apply(out, in, skip, s);
-  pipe_diag_kernel<<<stream_grid(P->n, 256), 256, 0, s>>>(out, in, jacobi ? P->jdiag : nullptr,
-                                                         P->n, skip);
-  return cudaGetLastError();
+  return launch_chained(P->n, pipe_diag_kernel, stream_grid(P->n, 256), 256, 0, s, out, in,
+                        jacobi ? P->jdiag : nullptr, P->n, skip);
 }
 
 static nb_status pfail(nb_status st, const std::string &m) {
@@ -277,16 +303,15 @@ nb_status pipecg_solve(nb_problem *P, double *x, const double *f, const nb_solve
   init.x = x;
   NB_CUDA_TRY(cudaMemcpyAsync(W.st, &init, sizeof(init), cudaMemcpyHostToDevice, s));
   // r = f, u = M r, w = A u and the first inner products (outside the graph)
-  pipe_zero_kernel<<<eg, 256, 0, s>>>(x, p, z, q, sv, r, f, n);
-  NB_CUDA_TRY(cudaGetLastError());
+  NB_CUDA_TRY(launch_chained(n, pipe_zero_kernel, eg, 256, 0, s, x, p, z, q, sv, r, f, n));
   NB_CUDA_TRY(pipe_precond(P, pc, jacobi, u, r, nullptr, s));
   NB_CUDA_TRY(pipe_op(P, w, u, nullptr, s));
-  pipe_first_dots_kernel<<<rb, kRedThreads, 0, s>>>(r, u, w, P->mult, P->multf, n, W.st,
-                                                     W.partials, W.counter);
-  pipe_start_kernel<<<1, 1, 0, s>>>(W.st);
-  NB_CUDA_TRY(cudaGetLastError());
+  NB_CUDA_TRY(launch_chained(n, pipe_first_dots_kernel, rb, kRedThreads, 0, s, r, u, w, P->mult,
+                             P->multf, n, W.st, W.partials, W.counter));
+  if (!pc) NB_CUDA_TRY(pipe_precond(P, pc, jacobi, mi, w, nullptr, s));
   const void *key[4] = {nullptr, nullptr, pc, (const void *)(intptr_t)(jacobi | (P->ifh2 << 1))};
-  const int chunk = n > (1 << 22) ? 4 : 16;
+  // as in the plain CG: short iterations are many, a look at the state 15 us
+  const int chunk = n > (1 << 22) ? 4 : !pc && n <= (1 << 20) ? 32 : 16;
   if (!W.graph || memcmp(key, W.key, sizeof(key))) {
     if (W.graph) {
       cudaGraphExecDestroy(W.graph);
@@ -298,16 +323,14 @@ nb_status pipecg_solve(nb_problem *P, double *x, const double *f, const nb_solve
     NB_CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     cudaError_t ce = cudaSuccess;
     for (int k = 0; k < chunk && ce == cudaSuccess; k++) {
-      ce = pipe_precond(P, pc, jacobi, mi, w, &W.st->done, cs);
+      if (pc) ce = pc->apply(mi, w, &W.st->done, cs);
       if (ce == cudaSuccess) ce = pipe_op(P, ni, mi, &W.st->done, cs);
-      if (ce == cudaSuccess) {
-        pipe_scalar_kernel<<<1, 1, 0, cs>>>(W.st);
-        pipe_vecops_kernel<<<rb, kRedThreads, 0, cs>>>(p, q, r, sv, u, w, z, ni, mi, P->mult,
-                                                       P->multf, n, W.st, W.partials, W.counter);
-        ce = cudaGetLastError();
-      }
+      if (ce == cudaSuccess)
+        ce = launch_chained(n, pipe_vecops_kernel, rb, kRedThreads, 0, cs, p, q, r, sv, u, w, z, ni,
+                            mi, pc != nullptr, jacobi ? P->jdiag : nullptr, P->mult, P->multf, n,
+                            W.st, W.partials, W.counter);
     }
-    W.launches_per_iter = (pc ? pc->launches() : 1) + 2 + 2;
+    W.launches_per_iter = (pc ? pc->launches() : 0) + 2 + 1;
     cudaError_t ee = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
     if (ce != cudaSuccess) {
@@ -320,7 +343,7 @@ nb_status pipecg_solve(nb_problem *P, double *x, const double *f, const nb_solve
     NB_CUDA_TRY(ee);
     memcpy(W.key, key, sizeof(key));
   }
-  int launches = 5 + (pc ? pc->launches() : 1);
+  int launches = 4 + (pc ? pc->launches() : 2);
   PipeState *hs = W.host;
   for (;;) {
     NB_CUDA_TRY(cudaMemcpyAsync(hs, W.st, sizeof(PipeState), cudaMemcpyDeviceToHost, s));
