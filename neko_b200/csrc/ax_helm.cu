@@ -41,7 +41,9 @@ struct AxCfg {
   static constexpr int NE = LX <= 3 ? 16 : (LX <= 5 ? 8 : (LX <= 8 ? 2 : 1));
 };
 
-template <typename T, int LX, int NE>
+// H2 adds the h2 B u term, reading u again (from cache): a column kept in
+// registers to the end costs a block an SM at the large orders.
+template <typename T, int LX, int NE, bool H2>
 __global__ void __launch_bounds__(LX *LX *NE)
     ax_helm_kernel(T *__restrict__ w, const T *__restrict__ u,
                    const T *__restrict__ dx, const T *__restrict__ dy,
@@ -125,7 +127,7 @@ __global__ void __launch_bounds__(LX *LX *NE)
     if (active) {
       const long g = base + k * L2;
       T v = acc + acc2 + acc3;
-      if (h2) v = v + __ldg(h2 + g) * __ldg(Bm + g) * ru[k];
+      if (H2) v = v + __ldg(h2 + g) * __ldg(Bm + g) * __ldg(u + g);
       w[g] = v;
     }
   }
@@ -672,7 +674,7 @@ static cudaError_t launch_ax(T *w, const T *u, const T *dx, const T *dy, const T
                              cudaStream_t s, const int *skip) {
   constexpr int NE = AxCfg<LX>::NE;
   const size_t smem = sizeof(T) * (6 * LX * LX + NE * 3 * LX * LX * LX);
-  auto kern = ax_helm_kernel<T, LX, NE>;
+  auto kern = h2 ? ax_helm_kernel<T, LX, NE, true> : ax_helm_kernel<T, LX, NE, false>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
