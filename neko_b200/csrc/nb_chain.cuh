@@ -34,13 +34,22 @@ __device__ __forceinline__ void chain() {
 // that wait on a multiprocessor cost a long kernel more than the launch gap.
 // Chained at every size, a coupled solve on 3 x 2.1 M points went from 32.1 to
 // 36.8 ms and a mixed hsmg solve on 4.1 M from 9.0 to 10.0 ms; the operator on
-// 262 thousand points went from 16.5 to 12.5 us and a Jacobi-CG solve there
-// from 7.84 to 7.36 ms.
+// 262 thousand points went from 16.5 to 12.5 us.
 constexpr long kChainPoints = 1L << 20;
 
+// Nor are launches that a graph captures: between the nodes of a graph the gap
+// is short already, and waiting blocks cost more than it (Jacobi-CG on 729
+// thousand points at lx 10: 18.7 ms chained, 17.0 not).
+inline bool chained(long points, cudaStream_t s) {
+  if (points > kChainPoints) return false;
+  if (!s) return true;  // the legacy stream is never captured
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+}
+
 template <typename... P, typename... A>
-inline cudaError_t launch_chained(long points, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
-                                  cudaStream_t s, A &&...args) {
+inline cudaError_t launch_chained(long points, void (*kern)(P...), dim3 grid, dim3 block,
+                                  size_t smem, cudaStream_t s, A &&...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -50,7 +59,7 @@ inline cudaError_t launch_chained(long points, void (*kern)(P...), dim3 grid, di
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = points <= kChainPoints ? 1 : 0;
+  cfg.numAttrs = chained(points, s) ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 

@@ -110,7 +110,7 @@ inline void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[2]
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = points <= kChainPoints ? 2 : 1;
+  cfg.numAttrs = chained(points, s) ? 2 : 1;
 }
 
 // Blocks of the largest cluster the device takes for a kernel: 16 (one GPC,
