@@ -46,7 +46,7 @@ struct NodeOp {
   void *base = nullptr;
 };
 // Beyond most_nodes only A.nn is set (A.val stays null).
-nb_status node_create(nb_problem *C, NodeOp &A, int most_nodes = 0x7fffffff);
+nb_status node_create(nb_problem *C, NodeOp &A, int most_nodes);
 // Matrix values and dinv from the level's current coefficients, on stream s.
 cudaError_t node_update(const nb_problem *C, const NodeOp &A, cudaStream_t s);
 

@@ -607,16 +607,18 @@ nb_status amg_power(PhmgImpl &H, int l) {
 }
 
 // Operands of the one-launch cycle: level 0 on the distinct vertices of C.
-// Left out (the separate launches stay) when C is not a vertex level or has
-// no unmasked vertex.
+// Left out (the separate launches stay) when C is not a vertex level, has no
+// unmasked vertex or more of them than the cycle takes.
 nb_status tamg_cluster_build(PhmgImpl &H, const TamgHost &T) {
   TamgDev &A = H.A;
   nb_problem *C = A.C;
   if (C->lx != 2) return NB_OK;
-  nb_status st = node_create(C, A.nodes);
+  int most = 0;
+  PH_TRY(tamg_cycle_nodes(most));
+  nb_status st = node_create(C, A.nodes, most);
   if (st != NB_OK) return st;
   const int nn = A.nodes.nn;
-  if (nn == 0) return NB_OK;
+  if (nn == 0 || !A.nodes.val) return NB_OK;
   PH_TRY(node_update(C, A.nodes, nullptr));
   std::vector<int> node_of(C->n), eptr(nn + 1);
   PH_TRY(cudaMemcpy(node_of.data(), A.nodes.node_of, C->n * sizeof(int), cudaMemcpyDeviceToHost));

@@ -274,10 +274,21 @@ __global__ void __launch_bounds__(kCoarseThreads) tamg_cycle_kernel(const TamgCl
   }
 }
 
-cudaError_t tamg_cycle(const TamgCluster &a, const int *skip, cudaStream_t s) {
+static cudaError_t tamg_limit(int &limit) {
   static int known[64];
+  return cluster_limit(tamg_cycle_kernel, kTamgStageBytes, known, limit);
+}
+
+cudaError_t tamg_cycle_nodes(int &most) {
+  int limit = 0;
+  const cudaError_t e = tamg_limit(limit);
+  most = limit * kCoarseThreads;
+  return e;
+}
+
+cudaError_t tamg_cycle(const TamgCluster &a, const int *skip, cudaStream_t s) {
   int limit = 0, nblk = 1;
-  cudaError_t e = cluster_limit(tamg_cycle_kernel, kTamgStageBytes, known, limit);
+  cudaError_t e = tamg_limit(limit);
   if (e != cudaSuccess) return e;
   // a block for every 128 vertices, as the hsmg coarse solve
   while (nblk < limit && nblk * 128 < a.A.nn) nblk *= 2;
