@@ -95,12 +95,16 @@ struct FdmCfg {
   static constexpr int P = PAIR && (NL / 2) % 2 == 0 ? NL + 2 : NL;
   static constexpr int VW = 16 / (int)sizeof(T);            // values per vector
   static constexpr int BUF = (P * N2 + VW - 1) / VW * VW;
-  // The matrices are kept twice, each row l of the forward (S(l, .)) and
-  // backward (S(., l)) forms contiguous with a pitch of whole 16-byte
-  // vectors, so a lane reads a row with NL*sizeof(T)/16 vector loads.
-  static constexpr int NLR = (NL + VW - 1) / VW * VW;       // row pitch
+  // One element a block: the matrices are kept twice, each row l of the
+  // forward (S(l, .)) and backward (S(., l)) forms contiguous with a pitch of
+  // whole 16-byte vectors, so a lane reads a row with NL*sizeof(T)/16 vector
+  // loads.  Elements that share a warp keep one copy and read single values:
+  // each has few lanes to lay the second copy out with (12.5 against 14.5 us a
+  // launch for up to 1716 elements at nl 6 in FP64, 18.6 against 20.7 at nl 7).
+  static constexpr bool VEC = EPW == 1;
+  static constexpr int NLR = VEC ? (NL + VW - 1) / VW * VW : NL;  // row pitch
   static constexpr int MS = NL * NLR;                       // one matrix
-  static constexpr int MAT = 6 * MS;
+  static constexpr int MAT = (VEC ? 6 : 3) * MS;
   static constexpr int STR0 = BUF + MAT + 3 * NL + 1;
   // per-element stride in whole vectors; with several elements in a warp an
   // odd number of them, so that their broadcast rows fall in distinct banks
@@ -109,10 +113,13 @@ struct FdmCfg {
   static constexpr size_t SMEM = ((size_t)EPW * STR * sizeof(T) + 15) / 16 * 16;
   // resident blocks per SM the register allocation is sized for: what the
   // shared memory allows (228 KB, 1 KB reserved per block), fewer if the
-  // M x NL sums and the operands in flight would not fit in the registers
+  // M x NL sums and the operands in flight would not fit in the registers.
+  // One-warp blocks of several elements spread over the four partitions, 512
+  // registers a lane each: 14 blocks leave 128 a thread, not 146, and spill.
   static constexpr int OCC = (int)(233472 / (SMEM + 1024));
-  static constexpr int REGS = sizeof(T) == 8 ? 3 * M * NL + 48 : 2 * M * NL + 4;
-  static constexpr int RB = 65536 / (TPE * REGS);
+  static constexpr int REGS =
+      sizeof(T) == 8 ? 3 * M * NL + 48 : 2 * M * NL + (EPW > 1 ? 20 : 4);
+  static constexpr int RB = EPW > 1 ? 512 / ((REGS + 7) / 8 * 8) * 4 : 65536 / (TPE * REGS);
   static constexpr int MINB0 = OCC < RB ? OCC : RB;
   static constexpr int MINB = MINB0 < 1 ? 1 : MINB0 > 32 / W ? 32 / W : MINB0;
   __device__ static __forceinline__ int pos(int t, int l) { return P * t + l; }
@@ -141,11 +148,12 @@ __device__ __forceinline__ void gather_elem(T *dst, const TIN *src, bool valid) 
 }
 
 // One pass over the element, in place: out(m,n,i) = sum_l R(l, i) in(l,m,n)
-// with row l of the pass's matrix at rows[NLR l].  SCALE multiplies each
+// with row l of the pass's matrix at rows[NLR l], or (one copy, mat) R(l, i) =
+// S(l, i) at l + NL i when FWD, else S(i, l).  SCALE multiplies each
 // value read by D^-1 (the first backward pass reads the third forward pass's
 // output); `out` != nullptr writes the natural (i,j,k) order to global memory
 // (last pass) instead of the rotated order over the buffer.
-template <typename T, int NL, bool SCALE>
+template <typename T, int NL, bool FWD, bool SCALE>
 __device__ __forceinline__ void fdm_pass(T *__restrict__ buf, const T *__restrict__ rows,
                                          const T *__restrict__ sL, T *__restrict__ out, int u) {
   using C = FdmCfg<T, NL>;
@@ -191,11 +199,16 @@ __device__ __forceinline__ void fdm_pass(T *__restrict__ buf, const T *__restric
     }
 #pragma unroll
     for (int h = 0; h < LS; h++) {
-      // row l of the pass's matrix in 16-byte vector loads (broadcast)
+      // row l of the pass's matrix (broadcast), in 16-byte vector loads
       T mr[C::NLR];
-      const V *row = reinterpret_cast<const V *>(rows + C::NLR * (l + h));
+      if constexpr (C::VEC) {
+        const V *row = reinterpret_cast<const V *>(rows + C::NLR * (l + h));
 #pragma unroll
-      for (int q = 0; q < C::NLR / C::VW; q++) reinterpret_cast<V *>(mr)[q] = row[q];
+        for (int q = 0; q < C::NLR / C::VW; q++) reinterpret_cast<V *>(mr)[q] = row[q];
+      } else {
+#pragma unroll
+        for (int i = 0; i < NL; i++) mr[i] = rows[FWD ? l + h + NL * i : i + NL * (l + h)];
+      }
 #pragma unroll
       for (int i = 0; i < NL; i++) {
 #pragma unroll
@@ -220,6 +233,30 @@ __device__ __forceinline__ void fdm_pass(T *__restrict__ buf, const T *__restric
   }
 }
 
+// NM matrices that arrived one after the other at `raw`, handed entry by entry
+// (matrix m, S_m(a, b) = v) to `place`, which may write over them: every entry
+// passes through a register.  As scattered asynchronous copies the layout took
+// longer (nl 9 in FP64, up to 100 elements: 13.3 us a launch so, 14.4 scattered;
+// nl 11 19.1 and 20.6).
+template <typename T, int NL, int NM, typename F>
+__device__ __forceinline__ void fdm_spread(const T *raw, int u, F &&place) {
+  using C = FdmCfg<T, NL>;
+  constexpr int R = (NM * C::N2 + C::LPE - 1) / C::LPE;
+  T v[R];
+#pragma unroll
+  for (int g = 0; g < R; g++) {
+    const int q = u + C::LPE * g;
+    v[g] = q < NM * C::N2 ? raw[q] : T(0);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int g = 0; g < R; g++) {
+    const int q = u + C::LPE * g, m = q / C::N2, w = q - m * C::N2;
+    if (q < NM * C::N2) place(m, w % NL, w / NL, v[g]);
+  }
+  __syncthreads();
+}
+
 template <typename TIN, typename T, int NL>
 __global__ void __launch_bounds__(FdmCfg<T, NL>::TPE, FdmCfg<T, NL>::MINB)
     fdm_kernel(const TIN *__restrict__ r, const int *__restrict__ fn,
@@ -234,8 +271,8 @@ __global__ void __launch_bounds__(FdmCfg<T, NL>::TPE, FdmCfg<T, NL>::MINB)
   const int es = threadIdx.x / C::LPE, ul = threadIdx.x - es * C::LPE;
   T *b0 = reinterpret_cast<T *>(fdm_smem) + es * C::STR;
   // the forward rows (S(l, i) at i + NLR*l), then the backward rows (S(i, l)
-  // at i + NLR*l), direction by direction
-  T *fwd = b0 + C::BUF, *bwd = fwd + 3 * C::MS;
+  // at i + NLR*l), direction by direction; or one copy of S
+  T *fwd = b0 + C::BUF, *bwd = C::VEC ? fwd + 3 * C::MS : fwd;
   T *sL = fwd + C::MAT;  // spectra + eps
   const long e = (long)blockIdx.x * C::EPW + es;
   if ((long)blockIdx.x * C::EPW >= nelv) return;
@@ -284,28 +321,28 @@ __global__ void __launch_bounds__(FdmCfg<T, NL>::TPE, FdmCfg<T, NL>::MINB)
       }
       b0[C::pos(b + NL * c, a)] = T(0);
     }
-    for (int q = u; q < 3 * N2; q += LPE) {  // S_d(a, b), copied to its place in both forms
-      const int d = q / N2, w = q - d * N2, a = w % NL, b = w / NL;
-      const T *src = S + e * 3 * N2 + q;
-      cp_async_elem<T>(fwd + d * C::MS + b + C::NLR * a, src, true);
-      cp_async_elem<T>(bwd + d * C::MS + a + C::NLR * b, src, true);
-    }
+    for (int q = u; q < 3 * N2; q += LPE) cp_async_elem<T>(fwd + q, S + e * 3 * N2 + q, true);
     for (int q = u; q < 3 * NL; q += LPE) cp_async_elem<T>(sL + q, lam + e * 3 * NL + q, true);
     if (u == 0) cp_async_elem<T>(sL + 3 * NL, eps + e, true);
   }
   cp_async_wait_all();
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, fwd, sL, nullptr, u);
+  if constexpr (C::VEC)
+    fdm_spread<T, NL, 3>(fwd, u, [&](int m, int a, int b, T v) {  // S_m(a, b) in both forms
+      fwd[m * C::MS + b + C::NLR * a] = v;
+      bwd[m * C::MS + a + C::NLR * b] = v;
+    });
+  fdm_pass<T, NL, true, false>(b0, fwd, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, fwd + C::MS, sL, nullptr, u);
+  fdm_pass<T, NL, true, false>(b0, fwd + C::MS, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, fwd + 2 * C::MS, sL, nullptr, u);
+  fdm_pass<T, NL, true, false>(b0, fwd + 2 * C::MS, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, true>(b0, bwd, sL, nullptr, u);
+  fdm_pass<T, NL, false, true>(b0, bwd, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, bwd + C::MS, sL, nullptr, u);
+  fdm_pass<T, NL, false, false>(b0, bwd + C::MS, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, bwd + 2 * C::MS, sL, out + e * N3, u);
+  fdm_pass<T, NL, false, false>(b0, bwd + 2 * C::MS, sL, out + e * N3, u);
 }
 
 // e(i,j,k) = ext interior + neighbours' ghost results on the first interior
@@ -561,12 +598,6 @@ __global__ void convert_kernel(TB *__restrict__ b, const TA *__restrict__ a, lon
     b[i] = (TB)a[i];
 }
 
-__global__ void mask_kernel(double *x, const int *msk, int m, const int *skip) {
-  if (skip && *skip) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < m) x[msk[i] - 1] = 0.0;
-}
-
 // ---------------------------------------------------------------------------
 // Schwarz level (smoother precision T)
 // ---------------------------------------------------------------------------
@@ -646,21 +677,29 @@ __global__ void __launch_bounds__(FdmCfg<double, NL>::TPE, FdmCfg<double, NL>::M
   // i = 0..nl-1.  The reference's transforms are tnsr3d(s(2,x), s(1,y),
   // s(1,z)) forward and tnsr3d(s(1,x), s(2,y), s(2,z)) backward, whose
   // first matrix contracts as A(i, l) and the other two as Bt(l, j).
-  for (int q = u; q < 6 * N2; q += LPE) {
-    const int dm = q / N2, w = q - dm * N2, dd = dm >> 1, a = w % NL, b = w / NL;
+  auto at = [&](int dm, int a, int b) {
     // s(., ., 1, .) serves the forward pass (the backward one of x), s(., .,
     // 2, .) the backward pass (the forward one of x)
-    T *to = ((dm & 1) == 0) == (dd != 0) ? fwd : bwd;
-    cp_async_elem<T>(to + dd * MS + (dd == 0 ? a + C::NLR * b : b + C::NLR * a),
-                     s + e * 6 * N2 + q, true);
+    const int dd = dm >> 1;
+    return (((dm & 1) == 0) == (dd != 0) ? fwd : bwd) + dd * MS +
+           (dd == 0 ? a + C::NLR * b : b + C::NLR * a);
+  };
+  // copied to their places at nl 8 (500 elements: 9.4 us, 10.4 through registers),
+  // through registers above (nl 9, 82 elements: 8.3 us, 10.4; nl 13 12.4, 13.4)
+  constexpr bool PLACED = NL <= 8;
+  for (int q = u; q < 6 * N2; q += LPE) {
+    const int dm = q / N2, w = q - dm * N2;
+    cp_async_elem<T>(PLACED ? at(dm, w % NL, w / NL) : fwd + q, s + e * 6 * N2 + q, true);
   }
   cp_async_wait_all();
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, fwd, sL, nullptr, u);
+  if constexpr (!PLACED)
+    fdm_spread<T, NL, 6>(fwd, u, [&](int dm, int a, int b, T v) { *at(dm, a, b) = v; });
+  fdm_pass<T, NL, true, false>(b0, fwd, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, fwd + MS, sL, nullptr, u);
+  fdm_pass<T, NL, true, false>(b0, fwd + MS, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, fwd + 2 * MS, sL, nullptr, u);
+  fdm_pass<T, NL, true, false>(b0, fwd + 2 * MS, sL, nullptr, u);
   __syncthreads();
   for (int q = u; q < N3; q += LPE) {  // r = d * (forward transform), kept for the backward one
     const int p = C::pos(q / NL, q % NL);
@@ -669,11 +708,11 @@ __global__ void __launch_bounds__(FdmCfg<double, NL>::TPE, FdmCfg<double, NL>::M
     r[e * N3 + q] = v;
   }
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, bwd, sL, nullptr, u);
+  fdm_pass<T, NL, false, false>(b0, bwd, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, bwd + MS, sL, nullptr, u);
+  fdm_pass<T, NL, false, false>(b0, bwd + MS, sL, nullptr, u);
   __syncthreads();
-  fdm_pass<T, NL, false>(b0, bwd + 2 * MS, sL, eo + e * N3, u);
+  fdm_pass<T, NL, false, false>(b0, bwd + 2 * MS, sL, eo + e * N3, u);
 }
 
 template <int NL>
