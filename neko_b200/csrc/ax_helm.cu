@@ -41,10 +41,24 @@ struct AxCfg {
   static constexpr int NE = LX <= 3 ? 16 : (LX <= 5 ? 8 : (LX <= 8 ? 2 : 1));
 };
 
-// H2 adds the h2 B u term, reading u again (from cache): a column kept in
-// registers to the end costs a block an SM at the large orders.
+// Blocks a multiprocessor that leave each thread about `regs` registers (0 in
+// __launch_bounds__: the compiler's own choice).
+constexpr int blocks_for(int threads, int regs) {
+  const int b = 65536 / ((threads + 31) / 32 * 32 * regs);
+  return b < 1 ? 1 : b;
+}
+
+// H2 adds the h2 B u term.  Its product h2 B is loaded with u, so that the loads
+// are in flight during the element; u comes from shared memory again.  Left to
+// itself the compiler gives this form 254 registers, one block a multiprocessor
+// where the other has two; with 128 (lx <= 8) or 168 of them the operator takes
+// 82 us on 2.3 M points at lx 12 (154 with 254 registers and u read from global
+// memory, 74 without the term, 88 with the term as a pass of its own), 78 at lx
+// 13 (150, 77, 91), 58 at lx 8 (76, -, 75).  With 128 lx 11 takes 23 us on 209
+// thousand points, 16 with 168.
 template <typename T, int LX, int NE, bool H2>
-__global__ void __launch_bounds__(LX *LX *NE)
+__global__ void __launch_bounds__(LX *LX *NE,
+                                  H2 ? blocks_for(LX * LX * NE, LX <= 8 ? 128 : 168) : 0)
     ax_helm_kernel(T *__restrict__ w, const T *__restrict__ u,
                    const T *__restrict__ dx, const T *__restrict__ dy,
                    const T *__restrict__ dz, const T *__restrict__ dxt,
@@ -79,11 +93,16 @@ __global__ void __launch_bounds__(LX *LX *NE)
   const bool active = e < nelv;
   const long base = e * L3 + i + LX * j;
 
-  T ru[LX], rut[LX];
+  T ru[LX], rut[LX], hb[H2 ? LX : 1];
 #pragma unroll
   for (int k = 0; k < LX; k++) {
     ru[k] = active ? __ldg(u + base + k * L2) : T(0);
     su[i + LX * j + L2 * k] = ru[k];
+  }
+  if constexpr (H2) {
+#pragma unroll
+    for (int k = 0; k < LX; k++)
+      hb[k] = active ? __ldg(h2 + base + k * L2) * __ldg(Bm + base + k * L2) : T(0);
   }
   __syncthreads();
 
@@ -127,7 +146,7 @@ __global__ void __launch_bounds__(LX *LX *NE)
     if (active) {
       const long g = base + k * L2;
       T v = acc + acc2 + acc3;
-      if (H2) v = v + __ldg(h2 + g) * __ldg(Bm + g) * __ldg(u + g);
+      if constexpr (H2) v = v + hb[k] * su[i + LX * j + L2 * k];
       w[g] = v;
     }
   }
