@@ -502,16 +502,24 @@ cudaError_t ax_helm_stream(double *w, const double *u, const double *D, const do
 
 // The fused step for the other orders and for operands that are not 16-byte
 // aligned: NE elements a block with plain coalesced loads, the element loop of
-// ax_helm_kernel.
+// ax_helm_kernel.  The new p stays in shared memory after the first pass and the
+// output loop is unrolled by two: unrolled fully with p in registers the kernel
+// takes 254 of them, one block a multiprocessor (lx 12, 2.3 M points: 140 us, 159
+// with h2; as separate passes 93 and 106).  With 168 it holds the columns; where
+// fewer than three blocks fit so, 128 are better up to lx 12 (78 and 84 us there
+// against 91 and 103; lx 11, where three fit, 18 and 23 on 209 thousand points),
+// beyond they spill (lx 14, 2.0 M points: 191 us, 127 with 168).
 template <int LX, int NE>
 struct AxCgGen {
   static constexpr int L2 = LX * LX, L3 = L2 * LX;
   static constexpr int THREADS = ((L2 * NE + 31) / 32) * 32;
+  static constexpr int BLOCKS =
+      blocks_for(THREADS, LX > 12 || blocks_for(THREADS, 168) >= 3 ? 168 : 128);
   static constexpr size_t SMEM = sizeof(double) * (2 * L2 + (size_t)NE * 3 * L3);
 };
 
-template <int LX, int NE, typename TZ>
-__global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS)
+template <int LX, int NE, bool H2, typename TZ>
+__global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS, AxCgGen<LX, NE>::BLOCKS)
     ax_cg_gen_kernel(const AxArgs<TZ> a) {
   using C = AxCgGen<LX, NE>;
   constexpr int L2 = C::L2, L3 = C::L3;
@@ -568,7 +576,7 @@ __global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS)
     }
     __syncthreads();
     if (active) {
-#pragma unroll
+#pragma unroll 2
       for (int k = 0; k < LX; k++) {
         double c0 = 0, c1 = 0, c2 = 0;
 #pragma unroll
@@ -578,10 +586,11 @@ __global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS)
           c2 += sDt[k + LX * l] * rut[l];
         }
         const long g = base + k * L2;
+        const double pk = su[col + L2 * k];
         double wv = c0 + c1 + c2;
-        if (a.h2) wv = wv + __ldg(a.h2 + g) * __ldg(a.B + g) * rp[k];
+        if constexpr (H2) wv = wv + __ldg(a.h2 + g) * __ldg(a.B + g) * pk;
         a.w[g] = wv;
-        pap += rp[k] * wv;
+        pap += pk * wv;
       }
     }
   }
@@ -599,7 +608,8 @@ __global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS)
 template <int LX, typename TZ>
 static cudaError_t launch_ax_cg_gen(const AxArgs<TZ> &a, cudaStream_t s) {
   using C = AxCgGen<LX, AxCfg<LX>::NE>;
-  auto kern = ax_cg_gen_kernel<LX, AxCfg<LX>::NE, TZ>;
+  auto kern = a.h2 ? ax_cg_gen_kernel<LX, AxCfg<LX>::NE, true, TZ>
+                   : ax_cg_gen_kernel<LX, AxCfg<LX>::NE, false, TZ>;
   if (C::SMEM > 48 * 1024) {
     cudaError_t e =
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
@@ -626,7 +636,15 @@ cudaError_t ax_cg_fused(double *w, double *p, const TZ *z, const double *D, cons
   a.h2 = h2, a.B = B, a.nelv = nelv, a.err = err;
   a.st = st, a.beta = beta, a.pap_out = pap_out, a.partials = partials, a.counter = counter;
   a.max_grid = max_grid;
-  if (bulk_aligned({z, p, h1, g11, g22, g33, g12, g13, g23, h2, B})) {
+  const bool rest = bulk_aligned({p, h1, g11, g22, g33, g12, g13, g23, h2, B});
+  // z alone off a 16-byte boundary: beyond 2^20 points the separate passes, whose
+  // operator streams p, are faster than the general kernel at these orders (lx 10,
+  // 2.7 M points: 72 us, 90; lx 8 58 and 62), below it is the launches that count
+  // (lx 8, 369 thousand points: 23 us, 13)
+  if (rest && !bulk_aligned({z}) && (lx == 6 || lx == 8 || lx == 10) &&
+      (long)nelv * lx * lx * lx > (1L << 20))
+    return cudaErrorNotSupported;
+  if (rest && bulk_aligned({z})) {
     switch (lx) {
       case 4: return launch_ax_stream<4, 1, true, 4, 4, false, 4, 4, false>(a, s);
       case 6: return launch_ax_stream<6, 1, true, 3, 3, false, 3, 3, false>(a, s);
