@@ -35,7 +35,7 @@ struct VecIo {
   const double *in[3];
 };
 
-template <int LX, int S, int KS>
+template <int LX, int S, int KS, bool H2>
 __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
     ax_vec_tma_kernel(VecIo io, const double *__restrict__ D, const double *__restrict__ Dt,
                       const double *__restrict__ h1, const double *__restrict__ g11,
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
 #pragma unroll
     for (int a = 0; a < NA; a++)
       bulk_g2s(stage + (size_t)(s * NA + a) * L3, src[a] + e * L3, (uint32_t)C::ABYTES, &full[s]);
-    if (h2) {  // read by each thread for its own points: to L2 meanwhile
+    if constexpr (H2) {  // read by each thread for its own points: to L2 meanwhile
       bulk_prefetch_l2(h2 + e * L3, (uint32_t)C::ABYTES);
       bulk_prefetch_l2(Bm + e * L3, (uint32_t)C::ABYTES);
     }
@@ -100,12 +100,18 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
   for (; t < nt; t++) {
     const int s = t % S;
     const long e = b + (long)t * G;
-    double hb[KP];  // h2 B at this thread's points
-    if (act) {
+    // h2 B at this thread's points; at lx 10, where the operator alone takes all
+    // 128 registers of a thread, read again for each component (148 us on 2.7 M
+    // points, 192 with them kept and others spilled)
+    constexpr bool KEEP = H2 && LX < 10;
+    double hb[KEEP ? KP : 1];
+    if constexpr (KEEP) {
+      if (act) {
 #pragma unroll
-      for (int kk = 0; kk < KP; kk++) {
-        const long g = e * L3 + col + L2 * (k0 + kk);
-        hb[kk] = h2 ? __ldg(h2 + g) * __ldg(Bm + g) : 0.0;
+        for (int kk = 0; kk < KP; kk++) {
+          const long g = e * L3 + col + L2 * (k0 + kk);
+          hb[kk] = __ldg(h2 + g) * __ldg(Bm + g);
+        }
       }
     }
     const bool ok = mbar_wait(&full[s], (uint32_t)((t / S) & 1));
@@ -120,13 +126,15 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const double *su = slot + c * L3;
-      double own[KP];  // the component at this thread's points
+      double own[H2 ? KP : 1];  // the component at this thread's points
       if (act) {
         double ru[LX];
 #pragma unroll
         for (int l = 0; l < LX; l++) ru[l] = su[col + L2 * l];
+        if constexpr (H2) {
 #pragma unroll
-        for (int kk = 0; kk < KP; kk++) own[kk] = su[col + L2 * (k0 + kk)];
+          for (int kk = 0; kk < KP; kk++) own[kk] = su[col + L2 * (k0 + kk)];
+        }
 #pragma unroll
         for (int kk = 0; kk < KP; kk++) {
           const int k = k0 + kk;
@@ -164,7 +172,12 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
             d += sDt[k + LX * l] * rt[l];
           }
           double v = a + cc + d;
-          if (h2) v = v + hb[kk] * own[kk];  // the part2 term, in its order
+          if constexpr (KEEP) {
+            v = v + hb[kk] * own[kk];
+          } else if constexpr (H2) {
+            const long g = e * L3 + col + L2 * k;
+            v = v + __ldg(h2 + g) * __ldg(Bm + g) * own[kk];
+          }  // the part2 term, in its order
           wo[e * L3 + col + L2 * k] = v;
         }
       }
@@ -181,14 +194,14 @@ __global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
   }
 }
 
-template <int LX, int S, int KS>
+template <int LX, int S, int KS, bool H2>
 static cudaError_t launch_vec(const VecIo &io, const double *D, const double *Dt,
                               const double *h1, const double *g11, const double *g22,
                               const double *g33, const double *g12, const double *g13,
                               const double *g23, const double *h2, const double *B, int nelv,
                               cudaStream_t st, int *err, const int *skip) {
   using C = AxVecCfg<LX, S, KS>;
-  auto kern = ax_vec_tma_kernel<LX, S, KS>;
+  auto kern = ax_vec_tma_kernel<LX, S, KS, H2>;
   static int grid_per_dev[64] = {0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -227,9 +240,14 @@ cudaError_t ax_helm_vector(double *au, double *av, double *aw, const double *u,
   for (const void *q : ptrs)
     if (reinterpret_cast<uintptr_t>(q) & 15) aligned = false;
   if (aligned) {
-#define NB_VEC(LX, S, KS) \
-  case LX:                \
-    return launch_vec<LX, S, KS>(io, D, Dt, h1, g11, g22, g33, g12, g13, g23, h2, B, nelv, s, err, skip);
+    // the h2 term is a form of its own: carried along it costs the other one 125
+    // against 105 us at lx 8 on 3.0 M points
+#define NB_VEC(LX, S, KS)                                                                   \
+  case LX:                                                                                  \
+    return h2 ? launch_vec<LX, S, KS, true>(io, D, Dt, h1, g11, g22, g33, g12, g13, g23,    \
+                                            h2, B, nelv, s, err, skip)                      \
+              : launch_vec<LX, S, KS, false>(io, D, Dt, h1, g11, g22, g33, g12, g13, g23,   \
+                                             h2, B, nelv, s, err, skip);
     switch (lx) {
       NB_VEC(4, 4, 1)
       NB_VEC(6, 3, 2)
