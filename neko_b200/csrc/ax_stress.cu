@@ -99,8 +99,10 @@ __device__ __forceinline__ void stress_point(const double g[3][3], const double 
 // staging up to five more arrays; they are brought to L2 when the stage is
 // filled.
 // Registers (512 threads a multiprocessor: 128 each) hold two rows of D at a
-// time, reloaded for the second pass, and the components are differentiated
-// one after the other.
+// time at lx 10, reloaded for the second pass, and the components are
+// differentiated one after the other.  At lx 4 and 6 the four rows fit and are
+// loaded once (HOLD): 76 against 92 us on 3.0 M points at lx 4, 101 against 113 at
+// lx 6 (84 and 99, 107 and 121 with h2).
 // ---------------------------------------------------------------------------
 template <int LX, int S, int KS>
 struct StressCfg {
@@ -111,6 +113,7 @@ struct StressCfg {
   static constexpr int BLOCKS0 = (int)(233472 / (SMEM + 1024 + 128));
   static constexpr int BLOCKS1 = BLOCKS0 * THREADS > 512 ? 512 / THREADS : BLOCKS0;
   static constexpr int BLOCKS = BLOCKS1 < 1 ? 1 : BLOCKS1;
+  static constexpr bool HOLD = LX <= 6;
 };
 
 template <int LX, int S, int KS, bool CG>
@@ -169,6 +172,27 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS>::THREADS, StressCfg<LX, S
   const int col = tid % L2, kh = tid / L2;
   const int i = col % LX, j = col / LX, k0 = kh * KP;
 
+  // rows of the derivative matrices: dx(i, l), dy(j, l), then dx(l, i), dy(l, j)
+  double Dxi[LX], Dyj[LX], Dxti[LX], Dytj[LX];
+  auto rows = [&] {
+#pragma unroll
+    for (int l = 0; l < LX; l++) {
+      Dxi[l] = __ldg(dx + i + LX * l);
+      Dyj[l] = __ldg(dy + j + LX * l);
+    }
+  };
+  auto rows_t = [&] {
+#pragma unroll
+    for (int l = 0; l < LX; l++) {
+      Dxti[l] = __ldg(dx + l + LX * i);
+      Dytj[l] = __ldg(dy + l + LX * j);
+    }
+  };
+  if (C::HOLD) {
+    rows();
+    rows_t();
+  }
+
   int t = 0;
   bool failed = false;
   double pap = 0.0;
@@ -210,12 +234,7 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS>::THREADS, StressCfg<LX, S
       __syncthreads();  // the element's new directions complete in the stage
     }
     if (act) {
-      double Dxi[LX], Dyj[LX];  // dx(i, l), dy(j, l)
-#pragma unroll
-      for (int l = 0; l < LX; l++) {
-        Dxi[l] = __ldg(dx + i + LX * l);
-        Dyj[l] = __ldg(dy + j + LX * l);
-      }
+      if (!C::HOLD) rows();
       double g[KP][3][3];
 #pragma unroll
       for (int c = 0; c < 3; c++) {
@@ -260,12 +279,7 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS>::THREADS, StressCfg<LX, S
     }
     __syncthreads();  // flux planes complete
     if (act) {
-      double Dxti[LX], Dytj[LX];  // dx(l, i), dy(l, j)
-#pragma unroll
-      for (int l = 0; l < LX; l++) {
-        Dxti[l] = __ldg(dx + l + LX * i);
-        Dytj[l] = __ldg(dy + l + LX * j);
-      }
+      if (!C::HOLD) rows_t();
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const double *fr = planes + (3 * c) * L3, *fs = fr + L3, *ft = fs + L3;
@@ -803,7 +817,7 @@ cudaError_t ax_stress(double *au, double *av, double *aw, const double *u, const
     if (reinterpret_cast<uintptr_t>(q) & 15) aligned = false;
   if (aligned) {
     switch (lx) {
-      case 4: return launch_stress_tma<4, 3, 4>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
+      case 4: return launch_stress_tma<4, 3, 2>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
       case 6: return launch_stress_tma<6, 2, 3>(io, geo, dx, dy, dz, w3, h2, Bm, nelv, s, err, skip);
       case 8: {
         const cudaError_t e =
@@ -1021,7 +1035,7 @@ cudaError_t problem_ax_stress_cg(nb_problem *P, double *const w[3], double *cons
     if (reinterpret_cast<uintptr_t>(q) & 15) return cudaErrorNotSupported;
   const double *h2 = P->ifh2 ? P->h2 : nullptr, *Bm = P->ifh2 ? P->B : nullptr;
   switch (P->lx) {
-    case 4: return launch_stress_tma<4, 3, 4, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
+    case 4: return launch_stress_tma<4, 2, 4, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
     case 6: return launch_stress_tma<6, 2, 3, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
     case 8: return launch_stress_mma<true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
     case 10: return launch_stress_tma<10, 2, 5, true>(io, geo, P->D, P->D, P->D, P->w3, h2, Bm, P->nelv, s, P->err, nullptr, cg);
