@@ -365,7 +365,8 @@ struct StressMma {
   static constexpr size_t SMEM = S * NA * ABYTES + L2 * sizeof(double) + 16 * S;
 };
 
-template <bool CG>
+// OUT2: results start on 16-byte boundaries and are stored in pairs.
+template <bool CG, bool OUT2>
 __global__ void __launch_bounds__(StressMma::THREADS, 2)
     ax_stress_mma_kernel(StressIo io, StressGeo geo, const double *__restrict__ dx,
                          const double *__restrict__ dy, const double *__restrict__ dz,
@@ -511,7 +512,7 @@ __global__ void __launch_bounds__(StressMma::THREADS, 2)
       }
       get2(slot + 3 * L3 + base + own, hv);
       get2(slot + 4 * L3 + base + own, jv);
-      const double2 wv = __ldg(reinterpret_cast<const double2 *>(w3 + base + own));
+      const double2 wv = make_double2(__ldg(w3 + base + own), __ldg(w3 + base + own + 1));
       stress_point(g[0], cf[0], hv[0] * wv.x * jv[0], f[0]);
       stress_point(g[1], cf[1], hv[1] * wv.y * jv[1], f[1]);
       // s and t fluxes over the cofactors just read, the lane's own points
@@ -569,7 +570,12 @@ __global__ void __launch_bounds__(StressMma::THREADS, 2)
           if (h2) v[h] = v[h] + hb[kk][h] * u[h];  // au + h2 B u, the part2 order
           if (CG) pap += u[h] * v[h];
         }
-        put2(io.out[c] + e * L3 + q, v);
+        if constexpr (OUT2) {
+          put2(io.out[c] + e * L3 + q, v);
+        } else {
+          io.out[c][e * L3 + q] = v[0];
+          io.out[c][e * L3 + q + 1] = v[1];
+        }
       }
     }
     // this thread's writes to the stage come before the next copy into it
@@ -601,12 +607,12 @@ static cudaError_t launch_stress_mma(const StressIo &io, const StressGeo &geo, c
                                      cudaStream_t st, int *err, const int *skip,
                                      const StressCg &cg = StressCg{}) {
   using C = StressMma;
-  // results and directions are stored in 16-byte pairs, w3 is read in them
-  const void *ptrs[] = {io.out[0], io.out[1], io.out[2], w3, h2, Bm};
-  for (const void *q : ptrs)
-    if (reinterpret_cast<uintptr_t>(q) & 15) return cudaErrorNotSupported;
-  auto kern = ax_stress_mma_kernel<CG>;
-  static int grid_per_dev[64] = {0};
+  auto off = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15) != 0; };
+  if (off(h2) || off(Bm)) return cudaErrorNotSupported;  // read in 16-byte pairs
+  const bool out2 = !off(io.out[0]) && !off(io.out[1]) && !off(io.out[2]);
+  auto kern = out2 ? ax_stress_mma_kernel<CG, true> : ax_stress_mma_kernel<CG, false>;
+  static int grids[2][64] = {{0}};
+  int(&grid_per_dev)[64] = grids[out2];
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;

@@ -68,3 +68,16 @@ def test_fused_step(nb, lx, nel, h2):
     op, step = _best(lambda: A.compute(w, z, P),
                      lambda: A.update_p_compute(w, p, z, 0.5, P, pap=pap))
     assert step < 1.25 * (13 / 11 if h2 else 11 / 9) * op
+
+
+@pytest.mark.parametrize("h2", [False, True])
+def test_stress_outputs_off_a_boundary(nb, h2):
+    """lx 8: results that start 8 bytes off a 16-byte boundary move the same
+    bytes as others and take the same sums."""
+    A, P = nb.AxHelmFull(), _problem(nb, (17, 16, 15), 8, h2)
+    u = [_rand(P.n) for _ in range(3)]
+    w = [[_rand(P.n, k) for _ in range(3)] for k in (0, 1)]
+    on, off = _best(lambda: A.compute_vector(*w[0], *u, P), lambda: A.compute_vector(*w[1], *u, P))
+    assert off < 1.25 * on
+    for a, b in zip(*w):
+        assert float((a - b).abs().max() / a.abs().max()) < 1e-14
