@@ -414,7 +414,8 @@ typedef enum {
  * zero-Dirichlet mask on each component, opts.pc NB_PC_JACOBI (the
  * problem's Jacobi diagonal on each component) or NB_PC_NONE (anything
  * else: NB_ERR_UNSUPPORTED), opts.max_iter and opts.abs_tol as nb_solve;
- * the other options are ignored.  op is an nb_ax_op.  Device arrays of n
+ * the other options are ignored.  fx, fy, fz are assembled and masked, or the
+ * curvature is the reference's own as in nb_solve.  op is an nb_ax_op.  Device arrays of n
  * doubles; synchronous on `stream`.  The reference's three monitors carry
  * the same values; res is one of them. */
 nb_status nb_solve_coupled(nb_problem *p, int op, double *x, double *y, double *z,
@@ -481,7 +482,11 @@ nb_status nb_pc_apply(nb_problem *p, int pc, double *z, const double *r, void *s
  * src/krylov/bcknd/device/cg_device.f90:162-238), restarted flexible
  * GMRES (NB_KSP_GMRES; gmres_device_solve) or pipelined CG (NB_KSP_PIPECG;
  * pipecg_device_solve), entirely on the device with device-resident
- * scalars.  x and f are device arrays of n doubles. */
+ * scalars.  x and f are device arrays of n doubles.  CG forms its curvature
+ * (p, A p), and the flexible one its products with z, before the gather-scatter,
+ * which gives the reference's values for an assembled and masked f; for an f
+ * whose copies of a point differ, or that is not zero on the mask, by more than
+ * 1e-10 of its root mean square it forms the reference's own, in more passes. */
 nb_status nb_solve(nb_problem *p, double *x, const double *f,
                    const nb_solve_opts *opts, nb_solve_result *res,
                    void *stream);

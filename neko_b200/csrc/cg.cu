@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kRedThreads)
     st->nan = 0;
     st->skip_rc = 1;
     st->restart = 0;
-    st->done = fabs(rn) < 2.220446049250313e-16 ? 1 : 0;
+    st->done = fabs(rn) < 2.220446049250313e-16 ? 1 : first_done(st, n);
   }
 }
 
@@ -391,17 +391,14 @@ static nb_status ws_fail(nb_status s, const std::string &m) {
 CgWorkspace::~CgWorkspace() {
   if (dots) cudaFree(dots);
   if (ev) cudaEventDestroy(ev);
-  if (graph_exec) cudaGraphExecDestroy(graph_exec);
+  for (Graph &g : graph) g.drop();
   if (base) cudaFree(base);
   if (host_state) cudaFreeHost(host_state);
 }
 
 cudaError_t CgWorkspace::ensure(long n_) {
   if (base && n == n_) return cudaSuccess;
-  if (graph_exec) {
-    cudaGraphExecDestroy(graph_exec);
-    graph_exec = nullptr;
-  }
+  for (Graph &g : graph) g.drop();
   if (base) cudaFree(base);
   base = nullptr;
   n = n_;
@@ -434,10 +431,10 @@ cudaError_t CgWorkspace::ensure(long n_) {
   return cudaSuccess;
 }
 
-// One CG iteration (all launches on s), precond chosen by pc.  `last`: the
-// last of its chunk, the only one that can be due a true residual (the
-// interval is a multiple of the chunk).
-static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, bool last,
+// One CG iteration (all launches on s), precond chosen by pc.  `rough`: for an
+// f that is not assembled and masked.  `last`: the last of its chunk, the only
+// one that can be due a true residual (the interval is a multiple of the chunk).
+static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, bool rough, bool last,
                                 cudaStream_t s) {
   const long n = P->n;
   const int rb = red_blocks(n), eg = stream_grid(n, 256);
@@ -480,12 +477,10 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, bool
                    W.use_jacobi ? P->jdiag : nullptr,
                                                      P->mult, P->multf, n, W.st, W.partials, W.counter);
   }
-  // p = z + beta p; w = A p; pap: one launch (the local form of pap needs p
-  // continuous and zero wherever w is masked: f is assembled and masked, so r
-  // and every preconditioner's output are)
+  // p = z + beta p; w = A p; pap: one launch with the local pap
   cudaError_t e = cudaErrorNotSupported;
   const double *h2 = P->ifh2 ? P->h2 : nullptr, *h2B = P->ifh2 ? P->B : nullptr;
-  if (P->use_stream_ax)
+  if (P->use_stream_ax && !rough)
     e = zf ? ax_cg_fused(W.w, W.p, zf, P->D, P->Dt, P->h1, P->g11, P->g22, P->g33, P->g12,
                          P->g13, P->g23, h2, h2B, (int)P->nelv, P->lx, W.st, 0.0, nullptr,
                          W.partials, W.counter, kCgMaxPartials, s, P->err)
@@ -538,23 +533,60 @@ void nb_problem::invalidate_solver_cache() {
   gmres_invalidate(this);
   pipecg_invalidate(this);
   cpld_invalidate(this);
-  if (solver_ws) {
-    CgWorkspace *W = (CgWorkspace *)solver_ws;
-    if (W->graph_exec) {
-      cudaGraphExecDestroy(W->graph_exec);
-      W->graph_exec = nullptr;
-    }
-  }
+  if (solver_ws)
+    for (auto &g : ((CgWorkspace *)solver_ws)->graph) g.drop();
 }
 
 namespace nb {
 
 // Runs the whole solve on stream s.  Iterations are replayed from a graph
 // holding `chunk` iterations; the host reads the state once per chunk.
-// Starts a solve on stream s: state, init kernel, the iteration graph
-// (captured again when the operands changed), the first chunk of
-// iterations, an asynchronous copy of the state to the host and an event
-// behind it.  cg_poll then follows the solve without blocking.
+// The first chunk of iterations of a started solve, its graph captured (again)
+// when the operands changed, and a copy of the state behind it.
+static nb_status cg_iterate(CgRun &R) {
+  nb_problem *P = R.P;
+  Precond *pc = R.pc;
+  CgWorkspace &W = *(CgWorkspace *)P->solver_ws;
+  CgWorkspace::Graph &G = W.graph[R.rough];
+  W.use_dots = W.flexible && pc->dots_in_apply() && !R.rough;
+  // x and f are read from the state: the graph depends on neither
+  const void *key[5] = {nullptr, nullptr, pc,
+                        (const void *)(intptr_t)(W.use_jacobi | (W.flexible << 1) |
+                                                 ((W.recompute_every > 0) << 2) |
+                                                 (W.use_dots << 3) | (W.fold << 4)),
+                        (const void *)(intptr_t)P->ifh2};
+  if (!G.exec || memcmp(key, G.key, sizeof(key))) {
+    G.drop();
+    cudaStream_t cs;
+    NB_CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+    cudaGraph_t g;
+    NB_CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
+    cudaError_t ce = cudaSuccess;
+    for (int k = 0; k < R.chunk && ce == cudaSuccess; k++)
+      ce = cg_iteration(P, W, pc, R.rough, k == R.chunk - 1, cs);
+    // an FP32-output preconditioner skips its conversion launch; with the
+    // inner products formed by the preconditioner a one-block finishing
+    // launch replaces the dot pass
+    const int pc_launches = pc ? pc->launches() - (pc->output_f32() ? 1 : 0) : 0;
+    const int per_iter = (W.fused ? 4 : 6) - (W.fold ? 1 : 0) + pc_launches;
+    G.launches = R.chunk * per_iter + (W.recompute_every > 0 ? 4 : 0);
+    cudaError_t ee = cudaStreamEndCapture(cs, &g);
+    cudaStreamDestroy(cs);
+    if (ce != cudaSuccess) {
+      if (ee == cudaSuccess) cudaGraphDestroy(g);
+      return ws_fail(NB_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
+    }
+    NB_CUDA_TRY(ee);
+    ee = cudaGraphInstantiate(&G.exec, g, 0);
+    cudaGraphDestroy(g);
+    NB_CUDA_TRY(ee);
+    memcpy(G.key, key, sizeof(key));
+  }
+  return cg_next_chunk(R);
+}
+
+// Starts a solve on stream s: state, init kernel and the first chunk of
+// iterations.  cg_poll then follows the solve without blocking.
 nb_status cg_start(CgRun &R) {
   nb_problem *P = R.P;
   const nb_solve_opts &o = R.o;
@@ -570,10 +602,9 @@ nb_status cg_start(CgRun &R) {
   W.use_jacobi = o.pc == NB_PC_JACOBI;
   W.flexible = (o.flexible != 0 || o.mixed != 0) && pc != nullptr;
   W.recompute_every = o.mixed ? 50 : 0;
-  W.use_dots = W.flexible && pc->dots_in_apply();
   // z = d r moves into the update, except where r may change after it
   W.fold = !pc && W.recompute_every == 0;
-  if (W.use_dots && (!W.dots || W.dots_n != P->nelv)) {
+  if (W.flexible && pc->dots_in_apply() && (!W.dots || W.dots_n != P->nelv)) {
     if (W.dots) cudaFree(W.dots);
     W.dots = nullptr;
     cudaError_t ae = cudaMalloc(&W.dots, 2 * (size_t)P->nelv * sizeof(double));
@@ -594,18 +625,12 @@ nb_status cg_start(CgRun &R) {
   init.skip_rc = 1;
   NB_CUDA_TRY(cudaMemcpyAsync(W.st, &init, sizeof(CgState), cudaMemcpyHostToDevice, s));
   const long n = P->n;
+  R.rough = false;
+  NB_CUDA_TRY(gs_jump(P->gsd, R.f, &W.st->jump, s));
   launch_chained(n, cg_init_kernel, red_blocks(n), kRedThreads, 0, s, 
       R.x, W.p, W.r, W.fold ? W.z : nullptr, W.use_jacobi ? P->jdiag : nullptr, R.f, P->mult,
       P->multf, n, W.st, W.partials, W.counter);
   NB_CUDA_TRY(cudaGetLastError());
-  // (Re)capture the iteration graph when the operands changed.
-  // x and f are read from the state: the graph depends on neither
-  const void *key[5] = {nullptr, nullptr, pc,
-                        (const void *)(intptr_t)(W.use_jacobi | (W.flexible << 1) |
-                                                 ((W.recompute_every > 0) << 2) |
-                                                 (W.use_dots << 3) | (W.fold << 4)),
-                        (const void *)(intptr_t)P->ifh2};
-  bool same = W.graph_exec && !memcmp(key, W.graph_key, sizeof(key));
   // Iterations a graph launch: the host looks at the state after each, about
   // 15 us, against launches of the chunk that find the solve finished.  Jacobi
   // iterations on small problems are short and many.
@@ -613,46 +638,16 @@ nb_status cg_start(CgRun &R) {
   // with true residuals every 50 iterations: a divisor of that, so that the
   // four launches of one are in a chunk's last iteration only
   if (W.recompute_every > 0) R.chunk = n > (1 << 22) ? 5 : 10;
-  if (!same) {
-    if (W.graph_exec) {
-      cudaGraphExecDestroy(W.graph_exec);
-      W.graph_exec = nullptr;
-    }
-    cudaStream_t cs;
-    NB_CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    cudaGraph_t g;
-    NB_CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    cudaError_t ce = cudaSuccess;
-    for (int k = 0; k < R.chunk && ce == cudaSuccess; k++)
-      ce = cg_iteration(P, W, pc, k == R.chunk - 1, cs);
-    // an FP32-output preconditioner skips its conversion launch; with the
-    // inner products formed by the preconditioner a one-block finishing
-    // launch replaces the dot pass
-    const int pc_launches = pc ? pc->launches() - (pc->output_f32() ? 1 : 0) : 0;
-    W.launches_per_iter = (W.fused ? 4 : 6) - (W.fold ? 1 : 0) + pc_launches;
-    W.launches_per_chunk = R.chunk * W.launches_per_iter + (W.recompute_every > 0 ? 4 : 0);
-    cudaError_t ee = cudaStreamEndCapture(cs, &g);
-    cudaStreamDestroy(cs);
-    if (ce != cudaSuccess) {
-      if (ee == cudaSuccess) cudaGraphDestroy(g);
-      return ws_fail(NB_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
-    }
-    NB_CUDA_TRY(ee);
-    ee = cudaGraphInstantiate(&W.graph_exec, g, 0);
-    cudaGraphDestroy(g);
-    NB_CUDA_TRY(ee);
-    memcpy(W.graph_key, key, sizeof(key));
-  }
-  R.launches = 1;
+  R.launches = 2;
   R.active = true;
-  return cg_next_chunk(R);
+  return cg_iterate(R);
 }
 
 // One more chunk of iterations, the state copy and the event behind them.
 nb_status cg_next_chunk(CgRun &R) {
   CgWorkspace &W = *(CgWorkspace *)R.P->solver_ws;
-  NB_CUDA_TRY(cudaGraphLaunch(W.graph_exec, R.s));
-  R.launches += W.launches_per_chunk;
+  NB_CUDA_TRY(cudaGraphLaunch(W.graph[R.rough].exec, R.s));
+  R.launches += W.graph[R.rough].launches;
   NB_CUDA_TRY(cudaMemcpyAsync(W.host_state, W.st, sizeof(CgState), cudaMemcpyDeviceToHost, R.s));
   NB_CUDA_TRY(cudaEventRecord(W.ev, R.s));
   return NB_OK;
@@ -672,8 +667,14 @@ int cg_poll(CgRun &R, bool wait, nb_solve_result *res, nb_status *status) {
     return 1;
   }
   const CgState *hs = (const CgState *)W.host_state;
-  if (!hs->done) {
-    *status = cg_next_chunk(R);
+  if (!hs->done || hs->done == kRough) {
+    if (hs->done) {  // nothing has run yet: r, z and the scalars are the initial ones
+      R.rough = true;
+      e = cudaMemsetAsync(&W.st->done, 0, sizeof(int), R.s);
+      *status = e == cudaSuccess ? cg_iterate(R) : ws_fail(NB_ERR_CUDA, cudaGetErrorString(e));
+    } else {
+      *status = cg_next_chunk(R);
+    }
     if (*status == NB_OK) return 0;
     R.active = false;
     return 1;

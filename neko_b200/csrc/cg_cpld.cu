@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kRedThreads)
     st->beta = 0.0;
     st->iter = 0;
     st->nan = 0;
-    st->done = rn == 0.0 ? 1 : 0;
+    st->done = rn == 0.0 ? 1 : first_done(st, n);
   }
 }
 
@@ -183,20 +183,25 @@ struct CpldWorkspace {
   CgState *st = nullptr;
   CgState *host = nullptr;
   V3 *xdev = nullptr;  // the solve's x, y, z pointers
-  cudaGraphExec_t graph = nullptr;
-  const void *key[9] = {nullptr};
-  int launches_per_iter = 0;
+  // a chunk of iterations, captured: [0] with the local curvature where the
+  // operator forms it, [1] with the reference's (kRough)
+  struct Graph {
+    cudaGraphExec_t exec = nullptr;
+    const void *key[3] = {nullptr};
+    int launches_per_iter = 0;
+    void drop() {
+      if (exec) cudaGraphExecDestroy(exec);
+      exec = nullptr;
+    }
+  } graph[2];
   ~CpldWorkspace() {
-    if (graph) cudaGraphExecDestroy(graph);
+    for (Graph &g : graph) g.drop();
     if (base) cudaFree(base);
     if (host) cudaFreeHost(host);
   }
   cudaError_t ensure(long n_) {
     if (base && n == n_) return cudaSuccess;
-    if (graph) {
-      cudaGraphExecDestroy(graph);
-      graph = nullptr;
-    }
+    for (Graph &g : graph) g.drop();
     if (base) cudaFree(base);
     base = nullptr;
     n = n_;
@@ -269,20 +274,21 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
   init.max_iter = o.max_iter;
   NB_CUDA_TRY(cudaMemcpyAsync(W.st, &init, sizeof(init), cudaMemcpyHostToDevice, s));
   NB_CUDA_TRY(cudaMemcpyAsync(W.xdev, &x, sizeof(V3), cudaMemcpyHostToDevice, s));
+  int launches = 1;
+  if (op == NB_AX_STRESS)  // the only operator that forms the curvature itself
+    for (int c = 0; c < 3; c++, launches++)
+      NB_CUDA_TRY(gs_jump(P->gsd, f.c[c], &W.st->jump, s));
   launch_chained(3 * n, cpld_init_kernel, rb, kRedThreads, 0, s, x, p, r, z, f, d, P->mult,
                  P->multf, n, W.st,
                                               W.partials, W.counter);
   NB_CUDA_TRY(cudaGetLastError());
   // x, y, z are read from the device copy: the graph depends on neither
   // the solution nor the right-hand side pointers
-  const void *key[9] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, d,
-                        (const void *)(intptr_t)op, (const void *)(intptr_t)P->ifh2};
+  const void *key[3] = {d, (const void *)(intptr_t)op, (const void *)(intptr_t)P->ifh2};
   const int chunk = n > (1 << 22) ? 4 : 16;
-  if (!W.graph || memcmp(key, W.key, sizeof(key))) {
-    if (W.graph) {
-      cudaGraphExecDestroy(W.graph);
-      W.graph = nullptr;
-    }
+  auto capture = [&](CpldWorkspace::Graph &G, bool rough) -> nb_status {
+    if (G.exec && !memcmp(key, G.key, sizeof(key))) return NB_OK;
+    G.drop();
     cudaStream_t cs;
     NB_CUDA_TRY(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     cudaGraph_t g;
@@ -293,7 +299,7 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
       // the full-stress operator on the streaming kernel takes the direction
       // update and the curvature into its pass; otherwise separate passes
       const cudaError_t fe =
-          op == NB_AX_STRESS
+          op == NB_AX_STRESS && !rough
               ? problem_ax_stress_cg(P, w.c, p.c, zc.c, W.st, W.partials, W.counter, cs)
               : cudaErrorNotSupported;
       if (fe == cudaSuccess) {
@@ -308,13 +314,11 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
         if (ce == cudaSuccess) ce = cpld_op(P, op, w, p, &W.st->done, cs);
         if (ce == cudaSuccess)
           launch_chained(3 * n, cpld_pap_kernel, rb, kRedThreads, 0, cs, wc, pc, P->mult,
-                         P->multf, n, W.st,
-                                                      W.partials, W.counter);
+                         P->multf, n, W.st, W.partials, W.counter);
       }
       if (ce == cudaSuccess) {
         launch_chained(3 * n, cpld_update_kernel, wave_blocks(n), kRedThreads, 0, cs, W.xdev, r,
-                       z, pc, wc, d, P->mult,
-                                                       P->multf, n, W.st, W.partials, W.counter);
+                       z, pc, wc, d, P->mult, P->multf, n, W.st, W.partials, W.counter);
         ce = cudaGetLastError();
       }
     }
@@ -323,7 +327,7 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
     // kernel adds the h2 term in a launch of its own
     const bool one = P->lx == 4 || P->lx == 6 || P->lx == 8 || P->lx == 10;
     const int op_launches = one ? 1 : op == NB_AX_STRESS ? 1 + (P->ifh2 ? 1 : 0) : 3;
-    W.launches_per_iter = fused ? 1 + 1 + 1 : 1 + op_launches + 1 + 2;
+    G.launches_per_iter = fused ? 1 + 1 + 1 : 1 + op_launches + 1 + 2;
     cudaError_t ee = cudaStreamEndCapture(cs, &g);
     cudaStreamDestroy(cs);
     if (ce != cudaSuccess) {
@@ -331,19 +335,28 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
       return cfail(NB_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
     }
     NB_CUDA_TRY(ee);
-    ee = cudaGraphInstantiate(&W.graph, g, 0);
+    ee = cudaGraphInstantiate(&G.exec, g, 0);
     cudaGraphDestroy(g);
     NB_CUDA_TRY(ee);
-    memcpy(W.key, key, sizeof(key));
-  }
-  int launches = 1;
+    memcpy(G.key, key, sizeof(key));
+    return NB_OK;
+  };
+  bool rough = false;
+  nb_status cst = capture(W.graph[0], false);
+  if (cst != NB_OK) return cst;
   CgState *hs = W.host;
   for (;;) {
     NB_CUDA_TRY(cudaMemcpyAsync(hs, W.st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
     NB_CUDA_TRY(cudaStreamSynchronize(s));
-    if (hs->done) break;
-    NB_CUDA_TRY(cudaGraphLaunch(W.graph, s));
-    launches += chunk * W.launches_per_iter;
+    if (hs->done == kRough) {
+      rough = true;
+      if ((cst = capture(W.graph[1], true)) != NB_OK) return cst;
+      NB_CUDA_TRY(cudaMemsetAsync(&W.st->done, 0, sizeof(int), s));
+    } else if (hs->done) {
+      break;
+    }
+    NB_CUDA_TRY(cudaGraphLaunch(W.graph[rough].exec, s));
+    launches += chunk * W.graph[rough].launches_per_iter;
   }
   if (res) {
     res->iter = hs->iter;
@@ -366,10 +379,8 @@ void cpld_free(nb_problem *P) {
 
 void cpld_invalidate(nb_problem *P) {
   CpldWorkspace *W = (CpldWorkspace *)P->cpld_ws;
-  if (W && W->graph) {
-    cudaGraphExecDestroy(W->graph);
-    W->graph = nullptr;
-  }
+  if (W)
+    for (auto &g : W->graph) g.drop();
 }
 
 }  // namespace nb

@@ -200,6 +200,64 @@ cudaError_t gs_add_fused(const GsDevice &g, T *u, bool with_mask, cudaStream_t s
   return cudaGetLastError();
 }
 
+// As gs_add_warp_kernel, without the sums: each lane against its segment's first.
+__global__ void __launch_bounds__(256)
+    gs_jump_kernel(const double *__restrict__ u, const GsDevice g,
+                   unsigned long long *__restrict__ jump) {
+  constexpr int CPW = 4;
+  chain();
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const long nwarps = (g.nchunk + CPW - 1) / CPW;
+  double d = 0.0;
+  auto more = [&](double v) {
+    if (v > d) d = v;
+  };
+  if (t < 32 * nwarps) {  // whole warps
+    const int lane = threadIdx.x & 31;
+    const long c0 = (t >> 5) * CPW;
+    int idx[CPW];
+    unsigned head[CPW];
+    double v[CPW];
+#pragma unroll
+    for (int j = 0; j < CPW; j++) {
+      const bool ok = c0 + j < g.nchunk;
+      idx[j] = ok ? __ldg(g.lane_idx + 32 * (c0 + j) + lane) : -1;
+      head[j] = ok ? __ldg(g.lane_head + c0 + j) : 0xffffffffu;
+    }
+#pragma unroll
+    for (int j = 0; j < CPW; j++) v[j] = idx[j] >= 0 ? u[idx[j]] : 0.0;
+#pragma unroll
+    for (int j = 0; j < CPW; j++) {
+      const int start = 31 - __clz(head[j] & (0xffffffffu >> (31 - lane)));
+      const double first = __shfl_sync(0xffffffffu, v[j], start);
+      if (idx[j] < 0) continue;
+      more(fabs(v[j] - first));
+      if ((__ldg(g.lane_zero + c0 + j) >> lane) & 1u) more(fabs(v[j]));
+    }
+  } else {
+    long q = t - 32 * nwarps;
+    if (q < g.nlong) {
+      const int sg = __ldg(g.seg_long + q);
+      const int a = __ldg(g.seg_ptr + sg), b = __ldg(g.seg_ptr + sg + 1);
+      const double first = u[__ldg(g.seg_idx + a)];
+      for (int k = a + 1; k < b; k++) more(fabs(u[__ldg(g.seg_idx + k)] - first));
+      if (g.seg_masked && g.seg_masked[sg]) more(fabs(first));
+    } else if ((q -= g.nlong) < g.nextra) {
+      more(fabs(u[__ldg(g.extra_mask + q)]));
+    }
+  }
+  // an assembled, masked vector has none: no atomics then
+  if (d > 0.0) atomicMax(jump, (unsigned long long)__double_as_longlong(d));
+}
+
+cudaError_t gs_jump(const GsDevice &g, const double *u, unsigned long long *jump,
+                    cudaStream_t s) {
+  const long total = 32L * ((g.nchunk + 3) / 4) + g.nlong + g.nextra;
+  if (total == 0) return cudaSuccess;
+  return launch_chained(32L * g.nchunk, gs_jump_kernel, (unsigned)((total + 255) / 256), 256, 0, s,
+                        u, g, jump);
+}
+
 // Two chunks a warp: six scattered loads in flight a thread.
 cudaError_t gs_add_fused3(const GsDevice &g, double *u0, double *u1, double *u2, bool with_mask,
                           cudaStream_t s, const int *skip) {

@@ -53,5 +53,9 @@ cudaError_t gs_add_fused(const GsDevice &g, T *u, bool with_mask, cudaStream_t s
 // The same on three vectors in one launch (no scale): each sum as above.
 cudaError_t gs_add_fused3(const GsDevice &g, double *u0, double *u1, double *u2, bool with_mask,
                           cudaStream_t s, const int *skip = nullptr);
+// How far u is from an assembled, masked vector: *jump (the bits of a double
+// >= 0) becomes the largest difference between copies of a point and the
+// largest magnitude at a masked one, if it was less.  NaNs do not count.
+cudaError_t gs_jump(const GsDevice &g, const double *u, unsigned long long *jump, cudaStream_t s);
 
 }  // namespace nb

@@ -18,11 +18,28 @@ struct CgState {
   int recompute_every;  // > 0: r = f - A x every that many iterations
   int skip_rc;          // 0 when the current iteration ends with a recompute
   int restart;          // next beta is 0 (after a recompute)
+  unsigned long long jump;  // of f, from gs_jump
   // The solve's x and f: the kernels of a captured iteration read them
   // here, so one graph serves every solve of the workspace.
   double *x;
   const double *f;
 };
+
+// The iterations form (p, w) of the unassembled w = A p over all local points
+// (and the flexible CG its products of an unassembled z), which equals the
+// reference's mult-weighted product of the assembled, masked vectors when p is
+// continuous and zero on masked points: f then is, and r, z and p with it.  A
+// solve whose f is not (its copies differ, or its masked points are not zero, by
+// more than kJump of its root mean square: the products then differ by about as
+// much) stops before its first iteration with `done` = kRough, and the host goes
+// on with iterations that form the reference's products.
+constexpr double kJump = 1e-10;
+constexpr int kRough = 2;
+// st->done of a solve that has not converged at its start
+__device__ __forceinline__ int first_done(const CgState *st, long n) {
+  return __longlong_as_double((long long)st->jump) > kJump * sqrt(st->rtr / (double)n) ? kRough
+                                                                                       : 0;
+}
 
 // pc_t%solve(z, r): z = M^-1 r on stream s; returns early when *skip != 0.
 struct Precond {
@@ -74,15 +91,23 @@ struct CgWorkspace {
   bool fused = false;  // the last captured iteration used ax_cg_fused
   bool fold = false;   // z = d r is formed by the x and r update
   int recompute_every = 0;
-  int launches_per_iter = 6, launches_per_chunk = 0;
-  cudaGraphExec_t graph_exec = nullptr;
+  // a chunk of iterations, captured: [0] with the local products, [1] with the
+  // reference's
+  struct Graph {
+    cudaGraphExec_t exec = nullptr;
+    const void *key[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    int launches = 0;
+    void drop() {
+      if (exec) cudaGraphExecDestroy(exec);
+      exec = nullptr;
+    }
+  } graph[2];
   cudaEvent_t ev = nullptr;  // behind the state copy of the last chunk
-  const void *graph_key[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   // per-element partial inner products of a preconditioner that forms them
   // (Precond::apply_dots): 2 x nelv doubles, allocated on first use
   double *dots = nullptr;
   long dots_n = 0;
-  bool use_dots = false;  // this solve's iterations take them
+  bool use_dots = false;  // the iterations being captured take them
   ~CgWorkspace();
   cudaError_t ensure(long n);
 };
@@ -100,6 +125,7 @@ struct CgRun {
   cudaStream_t s = nullptr;
   int chunk = 0, launches = 0;
   bool active = false;
+  bool rough = false;  // f is not assembled and masked
 };
 nb_status cg_start(CgRun &R);
 nb_status cg_next_chunk(CgRun &R);
