@@ -635,13 +635,12 @@ cudaError_t hsmg_coarse_nodes(int &most) {
 cudaError_t hsmg_coarse_cg(const CoarseCg &a, const int *skip, cudaStream_t s) {
   const NodeOp &A = a.A;
   if (A.nn == 0) return cudaSuccess;  // every vertex masked: no correction
-  static int known[64];
   CoarseCg b = a;
   b.skip = skip;
   int limit = 0, nblk = 1;
   cudaError_t e;
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[2];
+  cudaLaunchAttribute at[3];
   if (A.val) {  // assembled: z, p and, where it fits, the matrix resident
     if ((e = resident_limit(limit)) != cudaSuccess) return e;
     while (nblk < limit && nblk * kCoarseRowsPerBlock < A.nn) nblk *= 2;
@@ -649,7 +648,8 @@ cudaError_t hsmg_coarse_cg(const CoarseCg &a, const int *skip, cudaStream_t s) {
     const size_t slice = (size_t)A.maxw * 32 * (sizeof(double) + sizeof(int)),
                  vectors = 2 * (size_t)A.nn * sizeof(double);
     b.stage_slices = vectors + slices * slice <= kCoarseStageBytes ? slices : 0;
-    cluster_config(cfg, at, nblk, vectors + b.stage_slices * slice, s, 8L * a.nelv);
+    cluster_config(cfg, at, nblk, vectors + b.stage_slices * slice, s, 8L * a.nelv,
+                   a.priority);
     return cudaLaunchKernelEx(&cfg, coarse_cg_resident_kernel, b);
   }
   // element-local: a block for every 512 points of the middle level, at most one

@@ -95,10 +95,10 @@ __device__ __forceinline__ double row_dot(const double *val, const int *col, int
   return (acc[0] + acc[1]) + acc[2];
 }
 
-// The cluster launch, chained to its predecessor in the stream when the level
-// has few points (nb_chain.cuh).
-inline void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[2], int nblk,
-                           size_t bytes, cudaStream_t s, long points) {
+// The cluster launch, at `priority` in the order of pending launches and chained
+// to its predecessor in the stream when the level has few points (nb_chain.cuh).
+inline void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[3], int nblk,
+                           size_t bytes, cudaStream_t s, long points, int priority = 0) {
   cfg = {};
   cfg.gridDim = dim3((unsigned)nblk);
   cfg.blockDim = dim3(kCoarseThreads);
@@ -107,10 +107,12 @@ inline void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&at)[2]
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)nblk;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributePriority;
+  at[1].val.priority = priority;
+  at[2].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[2].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = chained(points, s) ? 2 : 1;
+  cfg.numAttrs = chained(points, s) ? 3 : 2;
 }
 
 // Blocks of the largest cluster the device takes for a kernel: 16 (one GPC,
@@ -130,7 +132,7 @@ cudaError_t cluster_limit(K kern, size_t bytes, int *known, int &limit) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
         cudaSuccess) {
       cudaLaunchConfig_t cfg;
-      cudaLaunchAttribute at[2];
+      cudaLaunchAttribute at[3];
       cluster_config(cfg, at, kMaxCluster, bytes, nullptr, 0);
       int n = 0;
       if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1)

@@ -164,6 +164,7 @@ struct CoarseCg {
   double *x = nullptr;        // solution: a value a node, or 8 an element (val null)
   double norm_fac = 0.0, tol = 0.0;
   int niter = 0, lm = 0, stage_slices = 0;
+  int priority = 0;           // of the cluster launch
   const int *skip = nullptr;
   // element-local form
   long nelv = 0;

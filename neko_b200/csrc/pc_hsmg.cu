@@ -815,19 +815,23 @@ struct HsmgState : public Precond {
   double tol = 1e-9;
   bool mixed = false;
   // The branches of the additive scheme share only the input r.  The middle
-  // level's residual and its restriction come first, on `crs`; then the
-  // coarse solve (a cluster of at most 16 blocks, on `crs`), the middle
-  // level's Schwarz (on `hi`) and the fine level's (on `side`) run side by
-  // side.  `crs` and `hi` have the greatest priority: the cluster needs its
-  // multiprocessors at once, so it is placed before the fine-level FDM fills
-  // the device, and the FDM then takes the others.
+  // level's residual and its restriction come first, on the caller's stream;
+  // then the coarse solve (a cluster of at most 16 blocks, on the caller's
+  // stream), the middle level's Schwarz (on `hi`) and the fine level's (on
+  // `side`) run side by side.  The cluster and `hi` have the greatest priority:
+  // the cluster needs its multiprocessors at once, so it is placed before the
+  // fine-level FDM fills the device, and the FDM then takes the others.
   // As a grid on every multiprocessor (larger meshes) the coarse solve gains
-  // nothing from its place: there the fine level starts at once, and the coarse
-  // solve follows the middle level's Schwarz (27.0 against 27.4 ms a solve of
+  // nothing from its place: there the fine level starts at once, and all of the
+  // rest follows on `hi`, the coarse solve last (27.0 against 27.4 ms a solve of
   // 20 applications on 32^3 elements).
-  cudaStream_t side = nullptr, hi = nullptr, crs_s = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_mid = nullptr, ev_join = nullptr, ev_join_hi = nullptr,
-              ev_join_crs = nullptr;
+  // Two streams beside the caller's: with the head and the cluster on a third an
+  // application took 11 event calls instead of 7 and 3 % longer (the mean over 100
+  // meshes and orders; 66 against 60 us at lx 10 on 6 x 5 x 4 elements), and its
+  // set-up one stream and two events more.
+  cudaStream_t side = nullptr, hi = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join_hi = nullptr;
+  int priority = 0;  // the greatest
   NodeOp nodes;  // the coarse problem over its distinct vertices
   cudaError_t ensure_side() {
     if (side) return cudaSuccess;
@@ -836,23 +840,17 @@ struct HsmgState : public Precond {
     if ((e = cudaDeviceGetStreamPriorityRange(&lo_prio, &hi_prio)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithPriority(&hi, cudaStreamNonBlocking, hi_prio)) != cudaSuccess ||
-        (e = cudaStreamCreateWithPriority(&crs_s, cudaStreamNonBlocking, hi_prio)) !=
-            cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&ev_mid, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&ev_join_crs, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ev_join_hi, cudaEventDisableTiming)) != cudaSuccess)
       return e;
+    priority = hi_prio;
     return cudaSuccess;
   }
   ~HsmgState() override {
     if (side) cudaStreamDestroy(side);
     if (hi) cudaStreamDestroy(hi);
-    if (crs_s) cudaStreamDestroy(crs_s);
     if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_mid) cudaEventDestroy(ev_mid);
-    if (ev_join_crs) cudaEventDestroy(ev_join_crs);
     if (nodes.base) cudaFree(nodes.base);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_join_hi) cudaEventDestroy(ev_join_hi);
@@ -937,38 +935,35 @@ struct HsmgImpl : public HsmgState {
     cudaError_t e;
     const long nelv = fine->nelv;
     const bool grid = cg.err != nullptr;  // the coarse solve takes every multiprocessor
-    if ((e = cudaEventRecord(ev_fork, s)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(crs_s, ev_fork, 0)) != cudaSuccess)
-      return e;
+    const cudaStream_t head = grid ? hi : s;
+    auto fork = [&] {
+      cudaError_t f = cudaEventRecord(ev_fork, s);
+      if (f == cudaSuccess) f = cudaStreamWaitEvent(hi, ev_fork, 0);
+      return f == cudaSuccess ? cudaStreamWaitEvent(side, ev_fork, 0) : f;
+    };
+    if (grid && (e = fork()) != cudaSuccess) return e;
     // restrict (r * mult) to the middle level, assemble, mask: w; restrict
     // (w * mult_mid) to the vertices (FP64)
     if ((e = restrict_level<double, T, T>(fine->lx, mid->lx, r, fine->mult, Jfm, w_mid, nelv,
-                                          skip, crs_s, fine->multf)) != cudaSuccess ||
-        (e = gs_add_fused<T>(mid->gsd, w_mid, true, crs_s, skip)) != cudaSuccess ||
-        (e = hsmg_coarse_restrict<T>(ca, mid->lx, skip, crs_s)) != cudaSuccess ||
-        (e = cudaEventRecord(ev_mid, crs_s)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(hi, ev_mid, 0)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(side, grid ? ev_fork : ev_mid, 0)) != cudaSuccess)
+                                          skip, head, fine->multf)) != cudaSuccess ||
+        (e = gs_add_fused<T>(mid->gsd, w_mid, true, head, skip)) != cudaSuccess ||
+        (e = hsmg_coarse_restrict<T>(ca, mid->lx, skip, head)) != cudaSuccess)
       return e;
     // coarse: assemble, mask, niter Jacobi-CG iterations (or abs tol)
-    auto coarse = [&](cudaStream_t cs) {
-      const cudaError_t r = hsmg_coarse_cg(cg, skip, cs);
-      return r != cudaSuccess ? r : cudaEventRecord(ev_join_crs, cs);
-    };
-    if (!grid && (e = coarse(crs_s)) != cudaSuccess) return e;
+    if (!grid && ((e = fork()) != cudaSuccess || (e = hsmg_coarse_cg(cg, skip, s)) != cudaSuccess))
+      return e;
     // middle Schwarz: e_mid = S_m w
     if ((e = schwarz_apply<T, T>(sm, w_mid, e_mid, skip, hi)) != cudaSuccess ||
+        (grid && (e = hsmg_coarse_cg(cg, skip, hi)) != cudaSuccess) ||
         (e = cudaEventRecord(ev_join_hi, hi)) != cudaSuccess)
       return e;
-    if (grid && (e = coarse(hi)) != cudaSuccess) return e;
     // fine Schwarz: zs = S_f r (left unassembled when the final
     // gather-scatter takes it, see below)
     const bool merged = merged_assembly();
     if ((e = schwarz_apply<double, T>(sf, r, zs, skip, side, !merged)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(ev_join, side)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(s, ev_join, 0)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(s, ev_join_hi, 0)) != cudaSuccess ||
-        (e = cudaStreamWaitEvent(s, ev_join_crs, 0)) != cudaSuccess)
+        (e = cudaStreamWaitEvent(s, ev_join_hi, 0)) != cudaSuccess)
       return e;
     // prolong: zs += J (e_mid + J_c e_crs); z = mult * gs(zs).  Merged: wt and
     // mult are the same at every copy of a point, so
@@ -1200,6 +1195,7 @@ static nb_status upload_impl(HsmgImpl<T> *H, const SchwarzHost &hf, const Schwar
     cg.err = reinterpret_cast<int *>(cg.bar + 2);
   }
   cg.norm_fac = 1.0 / std::sqrt(C->volume), cg.tol = H->tol, cg.niter = H->niter;
+  cg.priority = H->priority;
   auto upv = [&](size_t o, const std::vector<double> &v) {
     std::vector<T> t = cast_vec<T>(v);
     return t.empty() ? cudaSuccess
@@ -1271,7 +1267,7 @@ nb_status hsmg_get(nb_problem *P, const nb_solve_opts &o, Precond **out) {
     return st;
   }
   int most_nodes = 0;
-  if (hsmg_coarse_nodes(most_nodes) != cudaSuccess)
+  if (H->ensure_side() != cudaSuccess || hsmg_coarse_nodes(most_nodes) != cudaSuccess)
     st = hfail(NB_ERR_CUDA, "hsmg: coarse solve not available");
   if (!dirichlet) most_nodes = std::min(most_nodes, kCoarseFreeNodes);
   if (st != NB_OK || (st = node_create(H->crs, H->nodes, most_nodes)) != NB_OK) {
@@ -1298,7 +1294,7 @@ nb_status hsmg_get(nb_problem *P, const nb_solve_opts &o, Precond **out) {
              : upload_impl((HsmgImpl<double> *)H, hf, hm, Jfm, Jmc, ornt);
   // The uploads ran on the legacy stream (a pageable cudaMemcpy may return
   // before its DMA lands); finish them before any caller stream reads them.
-  if (st == NB_OK && (cudaDeviceSynchronize() != cudaSuccess || H->ensure_side() != cudaSuccess))
+  if (st == NB_OK && cudaDeviceSynchronize() != cudaSuccess)
     st = hfail(NB_ERR_CUDA, "hsmg: upload failed");
   if (st != NB_OK) {
     delete H;

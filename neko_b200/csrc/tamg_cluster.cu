@@ -301,7 +301,7 @@ cudaError_t tamg_cycle(const TamgCluster &a, const int *skip, cudaStream_t s) {
                         bytes <= kTamgStageBytes;
   b.stage_slices = resident ? slices : 0;
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute at[2];
+  cudaLaunchAttribute at[3];
   cluster_config(cfg, at, nblk, resident ? bytes : 0, s, a.npts);
   return cudaLaunchKernelEx(&cfg, tamg_cycle_kernel, b);
 }
