@@ -1,10 +1,7 @@
 // ax_helm.cu -- matrix-free Helmholtz operator w = D^T (h1 G D u) on sm_100a.
 //
-// One element per group of lx*lx threads; thread (i,j) owns the column
-// u(i,j,:).  The column is held in registers (t-derivative), the element is
-// staged once in shared memory for the r- and s-derivatives, and the
-// geometric factors stream in with read-only, coalesced loads (consecutive
-// threads read consecutive points of one k-plane).  The FP64 path is
+// The streaming forms, their dispatch and the entry points; other orders and
+// unaligned operands take ax_helm_gen.cu and ax_cg_gen.cu.  The FP64 path is
 // HBM-bound (72 B and 12 lx + 15 flop per point), so no tensor cores.
 //
 // Follows the arithmetic of ax_helm_lx (src/math/bcknd/cpu/ax_helm_cpu.f90:
@@ -21,6 +18,7 @@
 
 #include <cstdint>
 
+#include "nb_ax.cuh"
 #include "nb_chain.cuh"
 #include "nb_kernels.h"
 #include "nb_precond.h"
@@ -34,123 +32,6 @@ namespace nb {
 // points pass their problem's own word instead.  Read and cleared by
 // take_dropin_error() (after the synchronising drop-in reductions).
 __device__ int nb_dropin_error = 0;
-
-// Elements per block for each lx (threads = lx*lx*NE).
-template <int LX>
-struct AxCfg {
-  static constexpr int NE = LX <= 3 ? 16 : (LX <= 5 ? 8 : (LX <= 8 ? 2 : 1));
-};
-
-// Blocks a multiprocessor that leave each thread about `regs` registers (0 in
-// __launch_bounds__: the compiler's own choice).
-constexpr int blocks_for(int threads, int regs) {
-  const int b = 65536 / ((threads + 31) / 32 * 32 * regs);
-  return b < 1 ? 1 : b;
-}
-
-// H2 adds the h2 B u term.  Its product h2 B is loaded with u, so that the loads
-// are in flight during the element; u comes from shared memory again.  Left to
-// itself the compiler gives this form 254 registers, one block a multiprocessor
-// where the other has two; with 128 (lx <= 8) or 168 of them the operator takes
-// 82 us on 2.3 M points at lx 12 (154 with 254 registers and u read from global
-// memory, 74 without the term, 88 with the term as a pass of its own), 78 at lx
-// 13 (150, 77, 91), 58 at lx 8 (76, -, 75).  With 128 lx 11 takes 23 us on 209
-// thousand points, 16 with 168.
-template <typename T, int LX, int NE, bool H2>
-__global__ void __launch_bounds__(LX *LX *NE,
-                                  H2 ? blocks_for(LX * LX * NE, LX <= 8 ? 128 : 168) : 0)
-    ax_helm_kernel(T *__restrict__ w, const T *__restrict__ u,
-                   const T *__restrict__ dx, const T *__restrict__ dy,
-                   const T *__restrict__ dz, const T *__restrict__ dxt,
-                   const T *__restrict__ dyt, const T *__restrict__ dzt,
-                   const T *__restrict__ h1, const T *__restrict__ g11,
-                   const T *__restrict__ g22, const T *__restrict__ g33,
-                   const T *__restrict__ g12, const T *__restrict__ g13,
-                   const T *__restrict__ g23, const T *__restrict__ h2,
-                   const T *__restrict__ Bm, const int nelv, const int *__restrict__ skip) {
-  chain();
-  if (skip && *skip) return;  // solver finished: uniform early exit
-  constexpr int L2 = LX * LX, L3 = L2 * LX;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *sD = reinterpret_cast<T *>(smem_raw);  // 6 matrices, L2 each
-  T *sDx = sD, *sDy = sD + L2, *sDz = sD + 2 * L2;
-  T *sDxt = sD + 3 * L2, *sDyt = sD + 4 * L2, *sDzt = sD + 5 * L2;
-  const int tz = threadIdx.z;
-  T *su = sD + 6 * L2 + tz * 3 * L3;
-  T *sur = su + L3, *sus = su + 2 * L3;
-
-  const int i = threadIdx.x, j = threadIdx.y;
-  const int tid = i + LX * (j + LX * tz);
-  for (int q = tid; q < L2; q += L2 * NE) {
-    sDx[q] = dx[q];
-    sDy[q] = dy[q];
-    sDz[q] = dz[q];
-    sDxt[q] = dxt[q];
-    sDyt[q] = dyt[q];
-    sDzt[q] = dzt[q];
-  }
-  const long e = (long)blockIdx.x * NE + tz;
-  const bool active = e < nelv;
-  const long base = e * L3 + i + LX * j;
-
-  T ru[LX], rut[LX], hb[H2 ? LX : 1];
-#pragma unroll
-  for (int k = 0; k < LX; k++) {
-    ru[k] = active ? __ldg(u + base + k * L2) : T(0);
-    su[i + LX * j + L2 * k] = ru[k];
-  }
-  if constexpr (H2) {
-#pragma unroll
-    for (int k = 0; k < LX; k++)
-      hb[k] = active ? __ldg(h2 + base + k * L2) * __ldg(Bm + base + k * L2) : T(0);
-  }
-  __syncthreads();
-
-#pragma unroll
-  for (int k = 0; k < LX; k++) {
-    T ur = 0, us = 0, ut = 0;
-#pragma unroll
-    for (int l = 0; l < LX; l++) {
-      ur += sDx[i + LX * l] * su[l + LX * j + L2 * k];
-      us += sDy[j + LX * l] * su[i + LX * l + L2 * k];
-      ut += sDz[k + LX * l] * ru[l];
-    }
-    const long g = base + k * L2;
-    T G11 = 0, G22 = 0, G33 = 0, G12 = 0, G13 = 0, G23 = 0, H = 0;
-    if (active) {
-      G11 = __ldg(g11 + g);
-      G22 = __ldg(g22 + g);
-      G33 = __ldg(g33 + g);
-      G12 = __ldg(g12 + g);
-      G13 = __ldg(g13 + g);
-      G23 = __ldg(g23 + g);
-      H = __ldg(h1 + g);
-    }
-    sur[i + LX * j + L2 * k] = H * (G11 * ur + G12 * us + G13 * ut);
-    sus[i + LX * j + L2 * k] = H * (G12 * ur + G22 * us + G23 * ut);
-    rut[k] = H * (G13 * ur + G23 * us + G33 * ut);
-  }
-  __syncthreads();
-
-#pragma unroll
-  for (int k = 0; k < LX; k++) {
-    T acc = 0;
-#pragma unroll
-    for (int l = 0; l < LX; l++) acc += sDxt[i + LX * l] * sur[l + LX * j + L2 * k];
-    T acc2 = 0;
-#pragma unroll
-    for (int l = 0; l < LX; l++) acc2 += sDyt[j + LX * l] * sus[i + LX * l + L2 * k];
-    T acc3 = 0;
-#pragma unroll
-    for (int l = 0; l < LX; l++) acc3 += sDzt[k + LX * l] * rut[l];
-    if (active) {
-      const long g = base + k * L2;
-      T v = acc + acc2 + acc3;
-      if constexpr (H2) v = v + hb[k] * su[i + LX * j + L2 * k];
-      w[g] = v;
-    }
-  }
-}
 
 // ---------------------------------------------------------------------------
 // Streaming form: a persistent kernel in which each CTA walks its share of the
@@ -205,24 +86,6 @@ struct AxCfgS {
   static constexpr size_t SMEM =
       (S * NA + (AL ? 0 : 3)) * NE * ABYTES + 2 * L2 * sizeof(double) + 16 * S;
   static_assert((NE * L3 * sizeof(double)) % 16 == 0, "stage arrays are whole 16-byte units");
-};
-
-// Operands; u of the plain operator, or z and p of the fused step.
-template <typename TZ>
-struct AxArgs {
-  double *w;
-  const double *u;
-  double *p;
-  const TZ *z;
-  const double *D, *Dt, *h1, *g[6], *h2, *B;
-  int nelv;
-  const int *skip;
-  int *err;
-  // fused step
-  CgState *st;
-  double beta, *pap_out, *partials;
-  unsigned *counter;
-  int max_grid;
 };
 
 template <int LX, int S, int KS, int NE, bool CG, bool AL, bool H2, typename TZ>
@@ -500,128 +363,6 @@ cudaError_t ax_helm_stream(double *w, const double *u, const double *D, const do
   }
 }
 
-// The fused step for the other orders and for operands that are not 16-byte
-// aligned: NE elements a block with plain coalesced loads, the element loop of
-// ax_helm_kernel.  The new p stays in shared memory after the first pass and the
-// output loop is unrolled by two: unrolled fully with p in registers the kernel
-// takes 254 of them, one block a multiprocessor (lx 12, 2.3 M points: 140 us, 159
-// with h2; as separate passes 93 and 106).  With 168 it holds the columns; where
-// fewer than three blocks fit so, 128 are better up to lx 12 (78 and 84 us there
-// against 91 and 103; lx 11, where three fit, 18 and 23 on 209 thousand points),
-// beyond they spill (lx 14, 2.0 M points: 191 us, 127 with 168).
-template <int LX, int NE>
-struct AxCgGen {
-  static constexpr int L2 = LX * LX, L3 = L2 * LX;
-  static constexpr int THREADS = ((L2 * NE + 31) / 32) * 32;
-  static constexpr int BLOCKS =
-      blocks_for(THREADS, LX > 12 || blocks_for(THREADS, 168) >= 3 ? 168 : 128);
-  static constexpr size_t SMEM = sizeof(double) * (2 * L2 + (size_t)NE * 3 * L3);
-};
-
-template <int LX, int NE, bool H2, typename TZ>
-__global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS, AxCgGen<LX, NE>::BLOCKS)
-    ax_cg_gen_kernel(const AxArgs<TZ> a) {
-  using C = AxCgGen<LX, NE>;
-  constexpr int L2 = C::L2, L3 = C::L3;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double *sD = reinterpret_cast<double *>(smem_raw), *sDt = sD + L2;
-  const int tid = threadIdx.x, tz = tid / L2, col = tid - tz * L2;
-  const int i = col % LX, j = col / LX;
-  double *su = sDt + L2 + (tz < NE ? tz : 0) * 3 * L3, *sur = su + L3, *sus = sur + L3;
-  for (int q = tid; q < L2; q += C::THREADS) {
-    sD[q] = a.D[q];
-    sDt[q] = a.Dt[q];
-  }
-  chain();
-  if (a.st && a.st->done) return;
-  const double beta = a.st ? a.st->beta : a.beta;
-  double pap = 0.0;
-  for (long eb = (long)blockIdx.x * NE; eb < a.nelv; eb += (long)gridDim.x * NE) {
-    const long e = eb + tz;
-    const bool active = tz < NE && e < a.nelv;
-    const long base = e * L3 + col;
-    double rp[LX], rut[LX];
-    __syncthreads();  // matrices loaded; planes of the previous elements read
-    if (active) {
-#pragma unroll
-      for (int k = 0; k < LX; k++) {
-        const long g = base + k * L2;
-        rp[k] = (double)a.z[g] + beta * a.p[g];
-      }
-#pragma unroll
-      for (int k = 0; k < LX; k++) {
-        a.p[base + k * L2] = rp[k];
-        su[col + L2 * k] = rp[k];
-      }
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll
-      for (int k = 0; k < LX; k++) {
-        double ur = 0, us = 0, ut = 0;
-#pragma unroll
-        for (int l = 0; l < LX; l++) {
-          ur += sD[i + LX * l] * su[l + LX * j + L2 * k];
-          us += sD[j + LX * l] * su[i + LX * l + L2 * k];
-          ut += sD[k + LX * l] * rp[l];
-        }
-        const long g = base + k * L2;
-        const double G11 = __ldg(a.g[0] + g), G22 = __ldg(a.g[1] + g), G33 = __ldg(a.g[2] + g),
-                     G12 = __ldg(a.g[3] + g), G13 = __ldg(a.g[4] + g), G23 = __ldg(a.g[5] + g),
-                     H = __ldg(a.h1 + g);
-        sur[col + L2 * k] = H * (G11 * ur + G12 * us + G13 * ut);
-        sus[col + L2 * k] = H * (G12 * ur + G22 * us + G23 * ut);
-        rut[k] = H * (G13 * ur + G23 * us + G33 * ut);
-      }
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll 2
-      for (int k = 0; k < LX; k++) {
-        double c0 = 0, c1 = 0, c2 = 0;
-#pragma unroll
-        for (int l = 0; l < LX; l++) {
-          c0 += sDt[i + LX * l] * sur[l + LX * j + L2 * k];
-          c1 += sDt[j + LX * l] * sus[i + LX * l + L2 * k];
-          c2 += sDt[k + LX * l] * rut[l];
-        }
-        const long g = base + k * L2;
-        const double pk = su[col + L2 * k];
-        double wv = c0 + c1 + c2;
-        if constexpr (H2) wv = wv + __ldg(a.h2 + g) * __ldg(a.B + g) * pk;
-        a.w[g] = wv;
-        pap += pk * wv;
-      }
-    }
-  }
-  double tot;
-  if (grid_sum<C::THREADS>(pap, a.partials, a.counter, &tot)) {
-    if (a.st) {
-      a.st->pap = tot;
-      a.st->alpha = a.st->rtz1 / tot;
-    } else if (a.pap_out) {
-      *a.pap_out = tot;
-    }
-  }
-}
-
-template <int LX, typename TZ>
-static cudaError_t launch_ax_cg_gen(const AxArgs<TZ> &a, cudaStream_t s) {
-  using C = AxCgGen<LX, AxCfg<LX>::NE>;
-  auto kern = a.h2 ? ax_cg_gen_kernel<LX, AxCfg<LX>::NE, true, TZ>
-                   : ax_cg_gen_kernel<LX, AxCfg<LX>::NE, false, TZ>;
-  if (C::SMEM > 48 * 1024) {
-    cudaError_t e =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-    if (e != cudaSuccess) return e;
-  }
-  // every partial sum has a slot: blocks loop over the elements beyond that
-  const int ne = AxCfg<LX>::NE, need = (a.nelv + ne - 1) / ne;
-  launch_chained((long)a.nelv * C::L3, kern,
-                 need < a.max_grid ? need : a.max_grid, C::THREADS, C::SMEM, s, a);
-  return cudaGetLastError();
-}
-
 template <typename TZ>
 cudaError_t ax_cg_fused(double *w, double *p, const TZ *z, const double *D, const double *Dt,
                         const double *h1, const double *g11, const double *g22, const double *g33,
@@ -661,15 +402,7 @@ cudaError_t ax_cg_fused(double *w, double *p, const TZ *z, const double *D, cons
       }
     }
   }
-  switch (lx) {
-#define NB_CG_GEN(N) \
-  case N: return launch_ax_cg_gen<N, TZ>(a, s);
-    NB_CG_GEN(2) NB_CG_GEN(3) NB_CG_GEN(4) NB_CG_GEN(5) NB_CG_GEN(6) NB_CG_GEN(7) NB_CG_GEN(8)
-    NB_CG_GEN(9) NB_CG_GEN(10) NB_CG_GEN(11) NB_CG_GEN(12) NB_CG_GEN(13) NB_CG_GEN(14)
-    NB_CG_GEN(15) NB_CG_GEN(16)
-#undef NB_CG_GEN
-    default: return cudaErrorNotSupported;
-  }
+  return ax_cg_general<TZ>(a, lx, s);
 }
 template cudaError_t ax_cg_fused<double>(double *, double *, const double *, const double *,
                                          const double *, const double *, const double *,
@@ -702,66 +435,6 @@ int take_dropin_error() {
   if (v) cudaMemcpyToSymbol(nb_dropin_error, &zero, sizeof(int));
   return v;
 }
-
-template <typename T, int LX>
-static cudaError_t launch_ax(T *w, const T *u, const T *dx, const T *dy, const T *dz,
-                             const T *dxt, const T *dyt, const T *dzt, const T *h1,
-                             const T *g11, const T *g22, const T *g33, const T *g12,
-                             const T *g13, const T *g23, const T *h2, const T *B, int nelv,
-                             cudaStream_t s, const int *skip) {
-  constexpr int NE = AxCfg<LX>::NE;
-  const size_t smem = sizeof(T) * (6 * LX * LX + NE * 3 * LX * LX * LX);
-  auto kern = h2 ? ax_helm_kernel<T, LX, NE, true> : ax_helm_kernel<T, LX, NE, false>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  dim3 block(LX, LX, NE), grid((nelv + NE - 1) / NE);
-  if (nelv <= 0) return cudaSuccess;
-  launch_chained((long)nelv * LX * LX * LX, kern, grid, block, smem, s, w, u, dx, dy, dz, dxt,
-                 dyt, dzt, h1, g11, g22, g33, g12,
-                 g13, g23, h2, B, nelv, skip);
-  return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t ax_helm(T *w, const T *u, const T *dx, const T *dy, const T *dz, const T *dxt,
-                    const T *dyt, const T *dzt, const T *h1, const T *g11, const T *g22,
-                    const T *g33, const T *g12, const T *g13, const T *g23, int nelv, int lx,
-                    cudaStream_t s, const int *skip, const T *h2, const T *B) {
-#define NB_AX_CASE(N)                                                                  \
-  case N:                                                                              \
-    return launch_ax<T, N>(w, u, dx, dy, dz, dxt, dyt, dzt, h1, g11, g22, g33, g12, g13, \
-                           g23, h2, B, nelv, s, skip);
-  switch (lx) {
-    NB_AX_CASE(2)
-    NB_AX_CASE(3)
-    NB_AX_CASE(4)
-    NB_AX_CASE(5)
-    NB_AX_CASE(6)
-    NB_AX_CASE(7)
-    NB_AX_CASE(8)
-    NB_AX_CASE(9)
-    NB_AX_CASE(10)
-    NB_AX_CASE(11)
-    NB_AX_CASE(12)
-    NB_AX_CASE(13)
-    NB_AX_CASE(14)
-    NB_AX_CASE(15)
-    NB_AX_CASE(16)
-    default:
-      return cudaErrorInvalidValue;
-  }
-#undef NB_AX_CASE
-}
-
-template cudaError_t ax_helm<double>(double *, const double *, const double *, const double *,
-                                     const double *, const double *, const double *,
-                                     const double *, const double *, const double *,
-                                     const double *, const double *, const double *,
-                                     const double *, const double *, int, int, cudaStream_t,
-                                     const int *, const double *, const double *);
 
 }  // namespace nb
 
