@@ -96,7 +96,6 @@ __global__ void __launch_bounds__(kRedThreads)
     cg_precond_dot_kernel(double *__restrict__ z, const double *__restrict__ r,
                           const double *__restrict__ d, const double *__restrict__ mult, const float *__restrict__ multf,
                           long n, CgState *st, double *partials, unsigned *counter) {
-  chain();
   if (st->done) return;
   double s = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
@@ -121,7 +120,6 @@ __global__ void __launch_bounds__(kRedThreads)
     cg_dot_rz_kernel(const TZ *__restrict__ z, const double *__restrict__ r,
                      const double *__restrict__ mult, const float *__restrict__ multf, long n, CgState *st, double *partials,
                      unsigned *counter) {
-  chain();
   if (st->done) return;
   double s = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
@@ -144,7 +142,6 @@ __global__ void __launch_bounds__(kRedThreads)
     cg_dot_rz_flex_kernel(const TZ *__restrict__ z, const double *__restrict__ r,
                           const double *__restrict__ w_prev, const double *__restrict__ mult, const float *__restrict__ multf,
                           long n, CgState *st, double *partials, unsigned *counter) {
-  chain();
   if (st->done) return;
   double s0 = 0.0, s1 = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
@@ -167,7 +164,6 @@ __global__ void __launch_bounds__(kRedThreads)
 // fixed order.
 __global__ void __launch_bounds__(1024)
     cg_finish_flex_kernel(const double *__restrict__ part, long nelv, CgState *st) {
-  chain();
   if (st->done) return;
   // four independent chains a thread (loads in flight together), summed in
   // a fixed order
@@ -199,7 +195,6 @@ __global__ void __launch_bounds__(1024)
 template <typename TZ>
 __global__ void cg_update_p_kernel(double *__restrict__ p, const TZ *__restrict__ z,
                                    long n, const CgState *st) {
-  chain();
   if (st->done) return;
   const double beta = st->beta;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
@@ -212,7 +207,6 @@ __global__ void __launch_bounds__(kRedThreads)
     cg_pap_kernel(const double *__restrict__ w, const double *__restrict__ p,
                   const double *__restrict__ mult, const float *__restrict__ multf, long n, CgState *st, double *partials,
                   unsigned *counter) {
-  chain();
   if (st->done) return;
   double s = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
@@ -231,7 +225,6 @@ __global__ void __launch_bounds__(kRedThreads, 4)
                         const double *__restrict__ p, const double *__restrict__ w,
                         const double *__restrict__ mult, const float *__restrict__ multf, long n, CgState *st,
                         double *partials, unsigned *counter) {
-  chain();
   if (st->done) return;
   double *__restrict__ x = st->x;
   const double alpha = st->alpha, malpha = -alpha;
@@ -287,7 +280,6 @@ __global__ void __launch_bounds__(kRedThreads, 4)
                          const double *__restrict__ d, const double *__restrict__ mult,
                          const float *__restrict__ multf, long n, CgState *st, double *partials,
                          unsigned *counter) {
-  chain();
   if (st->done) return;
   double *__restrict__ x = st->x;
   const double alpha = st->alpha, malpha = -alpha;
@@ -345,7 +337,6 @@ __global__ void __launch_bounds__(kRedThreads)
     cg_true_residual_kernel(double *__restrict__ r,
                             const double *__restrict__ w, const double *__restrict__ mult, const float *__restrict__ multf, long n,
                             CgState *st, double *partials, unsigned *counter) {
-  chain();
   if (st->skip_rc) return;
   const double *__restrict__ f = st->f;
   double s = 0.0;
@@ -372,7 +363,6 @@ __global__ void __launch_bounds__(kRedThreads)
 
 // y = st->x (the recompute's operator input), on scheduled iterations only
 __global__ void cg_copy_x_kernel(double *__restrict__ y, long n, const CgState *st) {
-  chain();
   if (st->skip_rc) return;
   const double *__restrict__ x = st->x;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
@@ -448,34 +438,28 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, bool
     // unassembled output equal the mult-weighted ones of the assembled z)
     cudaError_t e = pc->apply_dots(W.z, W.r, W.w, W.dots, &W.st->done, s);
     if (e != cudaSuccess) return e;
-    launch_chained(n, cg_finish_flex_kernel, 1, 1024, 0, s, W.dots, W.dots_n, W.st);
+    cg_finish_flex_kernel<<<1, 1024, 0, s>>>(W.dots, W.dots_n, W.st);
   } else if (pc) {
     cudaError_t e = zf ? pc->apply_f32(W.r, &W.st->done, s) : pc->apply(W.z, W.r, &W.st->done, s);
     if (e != cudaSuccess) return e;
     if (W.flexible) {
       if (zf)
-        launch_chained(n, cg_dot_rz_flex_kernel<float>, rb, kRedThreads, 0, s, zf, W.r, W.w,
-                       P->mult, P->multf,
-                                                                n, W.st, W.partials, W.counter);
+        cg_dot_rz_flex_kernel<float><<<rb, kRedThreads, 0, s>>>(zf, W.r, W.w, P->mult, P->multf, n,
+            W.st, W.partials, W.counter);
       else
-        launch_chained(n, cg_dot_rz_flex_kernel<double>, rb, kRedThreads, 0, s, W.z, W.r, W.w,
-                       P->mult,
-                                                                 P->multf, n, W.st, W.partials,
-                                                                 W.counter);
+        cg_dot_rz_flex_kernel<double><<<rb, kRedThreads, 0, s>>>(W.z, W.r, W.w, P->mult, P->multf,
+            n, W.st, W.partials, W.counter);
     } else {
       if (zf)
-        launch_chained(n, cg_dot_rz_kernel<float>, rb, kRedThreads, 0, s, zf, W.r, P->mult,
-                       P->multf, n, W.st,
-                                                           W.partials, W.counter);
+        cg_dot_rz_kernel<float><<<rb, kRedThreads, 0, s>>>(zf, W.r, P->mult, P->multf, n, W.st,
+            W.partials, W.counter);
       else
-        launch_chained(n, cg_dot_rz_kernel<double>, rb, kRedThreads, 0, s, W.z, W.r, P->mult,
-                       P->multf, n,
-                                                            W.st, W.partials, W.counter);
+        cg_dot_rz_kernel<double><<<rb, kRedThreads, 0, s>>>(W.z, W.r, P->mult, P->multf, n, W.st,
+            W.partials, W.counter);
     }
   } else if (!W.fold) {
-    launch_chained(n, cg_precond_dot_kernel, rb, kRedThreads, 0, s, W.z, W.r,
-                   W.use_jacobi ? P->jdiag : nullptr,
-                                                     P->mult, P->multf, n, W.st, W.partials, W.counter);
+    cg_precond_dot_kernel<<<rb, kRedThreads, 0, s>>>(W.z, W.r, W.use_jacobi ? P->jdiag : nullptr,
+        P->mult, P->multf, n, W.st, W.partials, W.counter);
   }
   // p = z + beta p; w = A p; pap: one launch with the local pap
   cudaError_t e = cudaErrorNotSupported;
@@ -491,36 +475,33 @@ static cudaError_t cg_iteration(nb_problem *P, CgWorkspace &W, Precond *pc, bool
   if (e != cudaSuccess && e != cudaErrorNotSupported) return e;
   if (!W.fused) {
     if (zf)
-      launch_chained(n, cg_update_p_kernel<float>, eg, 256, 0, s, W.p, zf, n, W.st);
+      cg_update_p_kernel<float><<<eg, 256, 0, s>>>(W.p, zf, n, W.st);
     else
-      launch_chained(n, cg_update_p_kernel<double>, eg, 256, 0, s, W.p, W.z, n, W.st);
+      cg_update_p_kernel<double><<<eg, 256, 0, s>>>(W.p, W.z, n, W.st);
     e = P->ax(W.w, W.p, s, &W.st->done);
     if (e != cudaSuccess) return e;
   }
   e = gs_add_fused<double>(P->gsd, W.w, true, s, &W.st->done);
   if (e != cudaSuccess) return e;
   if (!W.fused)
-    launch_chained(n, cg_pap_kernel, rb, kRedThreads, 0, s, W.w, W.p, P->mult, P->multf, n, W.st,
-                   W.partials, W.counter);
+    cg_pap_kernel<<<rb, kRedThreads, 0, s>>>(W.w, W.p, P->mult, P->multf, n, W.st, W.partials,
+        W.counter);
   if (W.fold) {
-    launch_chained(n, cg_update_xrz_kernel, wave_blocks(n), kRedThreads, 0, s, W.r, W.z, W.p, W.w,
-                                                    W.use_jacobi ? P->jdiag : nullptr, P->mult,
-                                                    P->multf, n, W.st, W.partials, W.counter);
+    cg_update_xrz_kernel<<<wave_blocks(n), kRedThreads, 0, s>>>(W.r, W.z, W.p, W.w,
+        W.use_jacobi ? P->jdiag : nullptr, P->mult, P->multf, n, W.st, W.partials, W.counter);
     return cudaGetLastError();
   }
-  launch_chained(n, cg_update_xr_kernel, wave_blocks(n), kRedThreads, 0, s, W.r, W.p, W.w,
-                 P->mult, P->multf, n, W.st,
-                                                 W.partials, W.counter);
+  cg_update_xr_kernel<<<wave_blocks(n), kRedThreads, 0, s>>>(W.r, W.p, W.w, P->mult, P->multf, n,
+      W.st, W.partials, W.counter);
   if (W.recompute_every > 0 && last) {  // w = A x, gs, mask; r = f - w (scheduled iterations only)
     // x through z (free until the next preconditioner apply overwrites it)
-    launch_chained(n, cg_copy_x_kernel, eg, 256, 0, s, W.z, n, W.st);
+    cg_copy_x_kernel<<<eg, 256, 0, s>>>(W.z, n, W.st);
     e = P->ax(W.w, W.z, s, &W.st->skip_rc);
     if (e != cudaSuccess) return e;
     e = gs_add_fused<double>(P->gsd, W.w, true, s, &W.st->skip_rc);
     if (e != cudaSuccess) return e;
-    launch_chained(n, cg_true_residual_kernel, rb, kRedThreads, 0, s, W.r, W.w, P->mult,
-                   P->multf, n, W.st,
-                                                       W.partials, W.counter);
+    cg_true_residual_kernel<<<rb, kRedThreads, 0, s>>>(W.r, W.w, P->mult, P->multf, n, W.st,
+        W.partials, W.counter);
   }
   return cudaGetLastError();
 }
@@ -627,7 +608,7 @@ nb_status cg_start(CgRun &R) {
   const long n = P->n;
   R.rough = false;
   NB_CUDA_TRY(gs_jump(P->gsd, R.f, &W.st->jump, s));
-  launch_chained(n, cg_init_kernel, red_blocks(n), kRedThreads, 0, s, 
+  launch_chained(n, cg_init_kernel, red_blocks(n), kRedThreads, 0, s,
       R.x, W.p, W.r, W.fold ? W.z : nullptr, W.use_jacobi ? P->jdiag : nullptr, R.f, P->mult,
       P->multf, n, W.st, W.partials, W.counter);
   NB_CUDA_TRY(cudaGetLastError());

@@ -89,7 +89,6 @@ __global__ void __launch_bounds__(kRedThreads)
 
 // p_c = z_c + beta p_c
 __global__ void cpld_update_p_kernel(V3 p, C3 z, long n, const CgState *st) {
-  chain();
   if (st->done) return;
   const double beta = st->beta;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
@@ -103,7 +102,6 @@ __global__ void __launch_bounds__(kRedThreads)
     cpld_pap_kernel(C3 w, C3 p, const double *__restrict__ mult,
                     const float *__restrict__ multf, long n, CgState *st, double *partials,
                     unsigned *counter) {
-  chain();
   if (st->done) return;
   double s = 0.0;
   for (long i = blockIdx.x * (long)kRedThreads + threadIdx.x; i < n;
@@ -123,7 +121,6 @@ __global__ void __launch_bounds__(kRedThreads, 4)
                        const double *__restrict__ d, const double *__restrict__ mult,
                        const float *__restrict__ multf, long n, CgState *st, double *partials,
                        unsigned *counter) {
-  chain();
   if (st->done) return;
   const V3 x = *xp;  // the solve's x, y, z (device copy: one graph for every solve)
   const double alpha = st->alpha, alphm = -alpha;
@@ -309,16 +306,16 @@ nb_status cpld_solve(nb_problem *P, int op, double *const xs[3], const double *c
         ce = fe;
         break;
       } else {
-        launch_chained(3 * n, cpld_update_p_kernel, eg, 256, 0, cs, p, zc, n, W.st);
+        cpld_update_p_kernel<<<eg, 256, 0, cs>>>(p, zc, n, W.st);
         ce = cudaGetLastError();
         if (ce == cudaSuccess) ce = cpld_op(P, op, w, p, &W.st->done, cs);
         if (ce == cudaSuccess)
-          launch_chained(3 * n, cpld_pap_kernel, rb, kRedThreads, 0, cs, wc, pc, P->mult,
-                         P->multf, n, W.st, W.partials, W.counter);
+          cpld_pap_kernel<<<rb, kRedThreads, 0, cs>>>(wc, pc, P->mult, P->multf, n, W.st,
+              W.partials, W.counter);
       }
       if (ce == cudaSuccess) {
-        launch_chained(3 * n, cpld_update_kernel, wave_blocks(n), kRedThreads, 0, cs, W.xdev, r,
-                       z, pc, wc, d, P->mult, P->multf, n, W.st, W.partials, W.counter);
+        cpld_update_kernel<<<wave_blocks(n), kRedThreads, 0, cs>>>(W.xdev, r, z, pc, wc, d,
+            P->mult, P->multf, n, W.st, W.partials, W.counter);
         ce = cudaGetLastError();
       }
     }

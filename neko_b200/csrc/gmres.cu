@@ -77,7 +77,6 @@ __global__ void __launch_bounds__(kRedThreads)
                           const double *__restrict__ w, const double *__restrict__ mult,
                           const float *__restrict__ multf, long n, GmresState *st,
                           double *partials, unsigned *counter) {
-  chain();
   const double *__restrict__ f = st->f;
   if (st->done) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -114,7 +113,6 @@ __global__ void __launch_bounds__(kRedThreads)
 // a = b * inv_scale (v_1 = r / gam(1), v_(j+1) = w / alpha)
 __global__ void gm_scale_kernel(double *__restrict__ a, const double *__restrict__ b, long n,
                                 const GmresState *st) {
-  chain();
   if (st->stop) return;
   const double c = st->inv_scale;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
@@ -125,7 +123,6 @@ __global__ void gm_scale_kernel(double *__restrict__ a, const double *__restrict
 // z = d v (Jacobi; d null: z = v, the identity preconditioner)
 __global__ void gm_precond_kernel(double *__restrict__ z, const double *__restrict__ v,
                                   const double *__restrict__ d, long n, const GmresState *st) {
-  chain();
   if (st->stop) return;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
        i += (long)gridDim.x * blockDim.x)
@@ -139,7 +136,6 @@ __global__ void __launch_bounds__(kRedThreads, 4)
     gm_many_dot_kernel(const double *__restrict__ w, const double *const *__restrict__ V,
                        const double *__restrict__ mult, const float *__restrict__ multf, long n,
                        int j, GmresState *st, double *partials, unsigned *counter) {
-  chain();
   if (st->stop) return;
   __shared__ double sh[(kRedThreads / 32) * kGmresChunk];
   __shared__ bool last;
@@ -187,7 +183,6 @@ __global__ void __launch_bounds__(kRedThreads)
     gm_part2_kernel(double *__restrict__ w, const double *const *__restrict__ V,
                     const double *__restrict__ mult, const float *__restrict__ multf, long n,
                     int j, GmresState *st, double *partials, unsigned *counter) {
-  chain();
   if (st->stop) return;
   __shared__ double hs[kGmresMaxM];
   const int m = st->m;
@@ -259,7 +254,6 @@ __global__ void __launch_bounds__(kRedThreads)
 // columns (every block computes it), then x += sum_k z_k y_k.
 __global__ void __launch_bounds__(kRedThreads)
     gm_update_x_kernel(const double *const *__restrict__ Z, long n, const GmresState *st) {
-  chain();
   double *__restrict__ x = st->x;
   const int j = st->j_used, m = st->m;
   if (j <= 0) return;
@@ -355,7 +349,6 @@ struct GmresWorkspace {
 
 // y = st->x, the operator input of the cycle's residual
 __global__ void gm_copy_x_kernel(double *__restrict__ y, long n, const GmresState *st) {
-  chain();
   if (st->done) return;
   const double *__restrict__ x = st->x;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
@@ -379,14 +372,13 @@ static cudaError_t gmres_cycle(nb_problem *P, GmresWorkspace &W, Precond *pc, bo
   const int rb = red_blocks(n), eg = stream_grid(n, 256);
   int L = 0;
   // x through Z[0], which this cycle's first preconditioner apply overwrites
-  launch_chained(n, gm_copy_x_kernel, eg, 256, 0, s, W.Z[0], n, W.st);
+  gm_copy_x_kernel<<<eg, 256, 0, s>>>(W.Z[0], n, W.st);
   cudaError_t e = apply_op(P, W.w, W.Z[0], &W.st->done, s);
   if (e != cudaSuccess) return e;
   L += 3;
-  launch_chained(n, gm_cycle_start_kernel, rb, kRedThreads, 0, s, W.r, W.w, P->mult, P->multf, n,
-                 W.st,
-                                                   W.partials, W.counter);
-  launch_chained(n, gm_scale_kernel, eg, 256, 0, s, W.V[0], W.r, n, W.st);
+  gm_cycle_start_kernel<<<rb, kRedThreads, 0, s>>>(W.r, W.w, P->mult, P->multf, n, W.st,
+      W.partials, W.counter);
+  gm_scale_kernel<<<eg, 256, 0, s>>>(W.V[0], W.r, n, W.st);
   L += 2;
   for (int j = 0; j < W.m; j++) {
     if (pc) {
@@ -394,26 +386,23 @@ static cudaError_t gmres_cycle(nb_problem *P, GmresWorkspace &W, Precond *pc, bo
       if (e != cudaSuccess) return e;
       L += pc->launches();
     } else {
-      launch_chained(n, gm_precond_kernel, eg, 256, 0, s, W.Z[j], W.V[j],
-                     jacobi ? P->jdiag : nullptr, n, W.st);
+      gm_precond_kernel<<<eg, 256, 0, s>>>(W.Z[j], W.V[j], jacobi ? P->jdiag : nullptr, n, W.st);
       L += 1;
     }
     e = apply_op(P, W.w, W.Z[j], &W.st->stop, s);
     if (e != cudaSuccess) return e;
     L += 2;
-    launch_chained(n, gm_many_dot_kernel, wave_blocks(n), kRedThreads, 0, s, W.w, W.Vp, P->mult,
-                   P->multf, n, j, W.st,
-                                                  W.partials, W.counter);
-    launch_chained(n, gm_part2_kernel, rb, kRedThreads, 0, s, W.w, W.Vp, P->mult, P->multf, n, j,
-                   W.st,
-                                               W.partials, W.counter);
+    gm_many_dot_kernel<<<wave_blocks(n), kRedThreads, 0, s>>>(W.w, W.Vp, P->mult, P->multf, n, j,
+        W.st, W.partials, W.counter);
+    gm_part2_kernel<<<rb, kRedThreads, 0, s>>>(W.w, W.Vp, P->mult, P->multf, n, j, W.st,
+        W.partials, W.counter);
     L += 2;
     if (j + 1 < W.m) {
-      launch_chained(n, gm_scale_kernel, eg, 256, 0, s, W.V[j + 1], W.w, n, W.st);
+      gm_scale_kernel<<<eg, 256, 0, s>>>(W.V[j + 1], W.w, n, W.st);
       L += 1;
     }
   }
-  launch_chained(n, gm_update_x_kernel, eg, kRedThreads, 0, s, W.Zp, n, W.st);
+  gm_update_x_kernel<<<eg, kRedThreads, 0, s>>>(W.Zp, n, W.st);
   L += 1;
   *launches = L;
   return cudaGetLastError();

@@ -1,16 +1,21 @@
 // nb_chain.cuh -- launches that chain through programmatic dependent launch.
 //
-// An iteration of a solver is a chain of kernels of a few microseconds each,
-// and between two of them an ordinary stream dependency costs the drain of
-// the first and the launch of the second.  A chained kernel lets its successor
-// be scheduled as soon as all of its own blocks run (chain_next) and waits for
-// its predecessor's completion and memory before it touches anything
-// (chain_wait), so the successor's launch and start-up run under the
-// predecessor.  Every kernel launched this way, and every kernel before one,
-// calls chain() first; whatever runs ahead of chain_wait() reads only data
-// that no kernel of the stream writes (index maps, derivative matrices).
-// Completion stays transitive: a kernel completes only after its wait, so its
-// successor's wait covers everything before it.
+// An operator application, a preconditioner application and the start of a solve
+// are chains of kernels of a few microseconds each, and between two of them an
+// ordinary stream dependency costs the drain of the first and the launch of the
+// second.  A chained kernel lets its successor be scheduled as soon as all of its
+// own blocks run (chain_next) and waits for its predecessor's completion and
+// memory before it touches anything (chain_wait), so the successor's launch and
+// start-up run under the predecessor.
+//
+// The rules: a kernel launched with the attribute (launch_chained,
+// cluster_config) waits before it touches anything that a kernel of the stream
+// writes; ahead of the wait it reads index maps and derivative matrices only.  A
+// kernel lets its successor go only after its own wait, so a kernel completes
+// only after everything before it has, and its successor's wait covers that too.
+// A predecessor that does neither (a caller's kernel, the iterations of a solver,
+// which run captured) lets its successor go when it completes; a successor
+// without the attribute waits for the whole of its predecessor.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -186,7 +186,6 @@ __global__ void __launch_bounds__(kRedThreads)
                        const double *__restrict__ d, const double *__restrict__ mult,
                        const float *__restrict__ multf, long n, PipeState *st,
                        double *partials, unsigned *counter) {
-  chain();
   if (st->done) return;
   double *__restrict__ x = st->x;
   const double alpha = st->alpha, beta = st->beta;
@@ -325,10 +324,12 @@ nb_status pipecg_solve(nb_problem *P, double *x, const double *f, const nb_solve
     for (int k = 0; k < chunk && ce == cudaSuccess; k++) {
       if (pc) ce = pc->apply(mi, w, &W.st->done, cs);
       if (ce == cudaSuccess) ce = pipe_op(P, ni, mi, &W.st->done, cs);
-      if (ce == cudaSuccess)
-        ce = launch_chained(n, pipe_vecops_kernel, rb, kRedThreads, 0, cs, p, q, r, sv, u, w, z, ni,
-                            mi, pc != nullptr, jacobi ? P->jdiag : nullptr, P->mult, P->multf, n,
-                            W.st, W.partials, W.counter);
+      if (ce == cudaSuccess) {
+        pipe_vecops_kernel<<<rb, kRedThreads, 0, cs>>>(p, q, r, sv, u, w, z, ni, mi,
+            pc != nullptr, jacobi ? P->jdiag : nullptr, P->mult, P->multf, n, W.st, W.partials,
+            W.counter);
+        ce = cudaGetLastError();
+      }
     }
     W.launches_per_iter = (pc ? pc->launches() : 0) + 2 + 1;
     cudaError_t ee = cudaStreamEndCapture(cs, &g);
