@@ -349,10 +349,11 @@ cudaError_t ax_helm_stream(double *w, const double *u, const double *D, const do
     case 7:
       // While a block (two a multiprocessor) takes three pairs of elements at
       // most, a single stage: the copies of a second would share the bandwidth
-      // with those of the first pair, which every block waits for.  Operator with
-      // h2, gather-scatter and mask on 453 thousand points out of cache: 23 us,
-      // 28 with two stages.  With more pairs the second stage pays: 127 against
-      // 157 us at 6.8 M points.
+      // with those of the first pair, which every block waits for.  Out of cache,
+      // operator with h2 and gather-scatter: 26 us against 30 with two stages on
+      // 1320 elements, 30 and 34 on 1760, 44 and 46 on 3000, 52 and 52 on 4000, 73
+      // and 62 on 6000; in cache the operator alone takes 12.3 and 11.6 us on 1320,
+      // 27.7 and 23.5 on 3000.
       return nelv <= 12 * device_sms()
                  ? launch_ax_stream<7, 2, false, 1, 2, false, 1, 2, false>(a, s)
                  : launch_ax_stream<7, 2, false, 2, 1, false, 2, 2, false>(a, s);

@@ -182,21 +182,21 @@ __global__ void __launch_bounds__(256) gs_add_warp_kernel(const GsVec<T, NC> vec
 
 template <typename T, int CPW, int NC>
 static void launch_warp_form(const GsDevice &g, const GsVec<T, NC> &u, bool with_mask, cudaStream_t s,
-                             const int *skip, const T *scale) {
+                             const int *skip, const T *scale, bool chain) {
   const long total = 32L * ((g.nchunk + CPW - 1) / CPW) + g.nlong + (with_mask ? g.nextra : 0);
   const int threads = 256;
   const int blocks = (int)((total + threads - 1) / threads);
-  launch_chained(32L * NC * g.nchunk, gs_add_warp_kernel<T, CPW, NC>, blocks, threads, 0, s, u,
-                 g, with_mask, skip, scale);
+  launch_chained(chain ? 32L * NC * g.nchunk : kNotChained, gs_add_warp_kernel<T, CPW, NC>,
+                 blocks, threads, 0, s, u, g, with_mask, skip, scale);
 }
 
 template <typename T>
 cudaError_t gs_add_fused(const GsDevice &g, T *u, bool with_mask, cudaStream_t s,
-                         const int *skip, const T *scale) {
+                         const int *skip, const T *scale, bool chain) {
   if (g.nchunk == 0 && g.nlong == 0 && (!with_mask || g.nextra == 0)) return cudaSuccess;
   // four chunks a warp: 70 us against 80 (two) and 77 (eight) for the
   // 9.7 M entries of a 32^3-element box at lx = 8
-  launch_warp_form<T, 4, 1>(g, GsVec<T, 1>{{u}}, with_mask, s, skip, scale);
+  launch_warp_form<T, 4, 1>(g, GsVec<T, 1>{{u}}, with_mask, s, skip, scale, chain);
   return cudaGetLastError();
 }
 
@@ -262,13 +262,13 @@ cudaError_t gs_jump(const GsDevice &g, const double *u, unsigned long long *jump
 cudaError_t gs_add_fused3(const GsDevice &g, double *u0, double *u1, double *u2, bool with_mask,
                           cudaStream_t s, const int *skip) {
   if (g.nchunk == 0 && g.nlong == 0 && (!with_mask || g.nextra == 0)) return cudaSuccess;
-  launch_warp_form<double, 2, 3>(g, GsVec<double, 3>{{u0, u1, u2}}, with_mask, s, skip, nullptr);
+  launch_warp_form<double, 2, 3>(g, GsVec<double, 3>{{u0, u1, u2}}, with_mask, s, skip, nullptr, true);
   return cudaGetLastError();
 }
 template cudaError_t gs_add_fused<double>(const GsDevice &, double *, bool, cudaStream_t,
-                                          const int *, const double *);
+                                          const int *, const double *, bool);
 template cudaError_t gs_add_fused<float>(const GsDevice &, float *, bool, cudaStream_t,
-                                         const int *, const float *);
+                                         const int *, const float *, bool);
 
 // Host-side re-layout of reference maps into the fused form.  `masked`
 // (n flags, may be empty) marks zero-Dirichlet points.

@@ -39,8 +39,15 @@ __device__ __forceinline__ void chain() {
 // that wait on a multiprocessor cost a long kernel more than the launch gap.
 // Chained at every size, a coupled solve on 3 x 2.1 M points went from 32.1 to
 // 36.8 ms and a mixed hsmg solve on 4.1 M from 9.0 to 10.0 ms; the operator on
-// 262 thousand points went from 16.5 to 12.5 us.
+// 262 thousand points went from 16.5 to 12.5 us, an hsmg application from 70.5 to 65
+// us there and from 94 to 90 on 885 thousand (113 and 112 us on 1.4 M: nothing left
+// to gain).
 constexpr long kChainPoints = 1L << 20;
+// Points of a launch that is not chained whatever its size: in an hsmg application
+// whose coarse solve is a grid on every multiprocessor, waiting blocks keep that
+// grid and the fine level's smoother from their places (lx 4, 28^3 elements, FP32
+// smoothing: 383 us chained, 325 not; 346 before there were chained launches).
+constexpr long kNotChained = kChainPoints + 1;
 
 // Nor are launches that a graph captures: between the nodes of a graph the gap
 // is short already, and waiting blocks cost more than it (Jacobi-CG on 729

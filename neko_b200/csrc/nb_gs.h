@@ -46,10 +46,11 @@ bool gs_pairs_regular(const GsMaps &m);
 
 // u = gs_add(u) over g; masked entries become 0 when with_mask; when scale
 // is given every written entry is multiplied by scale[index] (points outside
-// the maps are not touched).  Returns at once when *skip != 0.
+// the maps are not touched).  Returns at once when *skip != 0.  chain: the launch
+// may be chained (nb_chain.cuh).
 template <typename T>
 cudaError_t gs_add_fused(const GsDevice &g, T *u, bool with_mask, cudaStream_t s,
-                         const int *skip = nullptr, const T *scale = nullptr);
+                         const int *skip = nullptr, const T *scale = nullptr, bool chain = true);
 // The same on three vectors in one launch (no scale): each sum as above.
 cudaError_t gs_add_fused3(const GsDevice &g, double *u0, double *u1, double *u2, bool with_mask,
                           cudaStream_t s, const int *skip = nullptr);

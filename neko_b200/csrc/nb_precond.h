@@ -180,7 +180,7 @@ struct CoarseCg {
 // f = restriction of (w_mid mult_m), element by element (lm = 3 or 4).
 template <typename T>
 cudaError_t hsmg_coarse_restrict(const CoarseArgs<T> &a, int lm, const int *skip,
-                                 cudaStream_t s);
+                                 cudaStream_t s, bool chain);
 // The coarse Jacobi-CG, one cluster launch.
 cudaError_t hsmg_coarse_cg(const CoarseCg &a, const int *skip, cudaStream_t s);
 

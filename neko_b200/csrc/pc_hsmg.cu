@@ -613,7 +613,7 @@ struct SchwarzLevel {
 
 template <typename TIN, typename T, int LX>
 static cudaError_t launch_fdm_post(const SchwarzLevel<T> &L, const TIN *r, T *e, const int *skip,
-                                   cudaStream_t s) {
+                                   cudaStream_t s, bool chain) {
   constexpr int NL = LX + 2;
   using C = FdmCfg<T, NL>;
   auto kern = fdm_kernel<TIN, T, NL>;
@@ -626,29 +626,29 @@ static cudaError_t launch_fdm_post(const SchwarzLevel<T> &L, const TIN *r, T *e,
     if (err != cudaSuccess) return err;
     attr_set = true;
   }
-  launch_chained(4 * L.nelv * C::N3, kern, (unsigned)((L.nelv + C::EPW - 1) / C::EPW), C::TPE,
-                 C::SMEM, s, r, L.fn, L.ornt, L.S, L.lam, L.eps, L.ext, (int)L.nelv, skip);
-  const long n = L.nelv * LX * LX * LX;
-  launch_chained(4 * n, schwarz_post_kernel<T, LX>, (unsigned)((n + 255) / 256), 256, 0, s, 
-      L.ext, L.fn, L.ornt, L.wt, e, L.nelv, skip);
+  const long n = L.nelv * LX * LX * LX, points = chain ? n : kNotChained;
+  launch_chained(points, kern, (unsigned)((L.nelv + C::EPW - 1) / C::EPW), C::TPE, C::SMEM, s, r,
+                 L.fn, L.ornt, L.S, L.lam, L.eps, L.ext, (int)L.nelv, skip);
+  launch_chained(points, schwarz_post_kernel<T, LX>, (unsigned)((n + 255) / 256), 256, 0, s, L.ext,
+                 L.fn, L.ornt, L.wt, e, L.nelv, skip);
   return cudaGetLastError();
 }
 
 // e = Schwarz(r) on level L (r already masked): FDM + overlap + gs + mask.
 template <typename TIN, typename T>
 static cudaError_t schwarz_apply(const SchwarzLevel<T> &L, const TIN *r, T *e, const int *skip,
-                                 cudaStream_t s, bool assemble = true) {
+                                 cudaStream_t s, bool chain, bool assemble = true) {
   cudaError_t err;
   switch (L.lx) {
 #define NB_S(N) \
-  case N: err = launch_fdm_post<TIN, T, N>(L, r, e, skip, s); break;
+  case N: err = launch_fdm_post<TIN, T, N>(L, r, e, skip, s, chain); break;
     NB_S(3) NB_S(4) NB_S(5) NB_S(6) NB_S(7) NB_S(8) NB_S(9) NB_S(10) NB_S(11) NB_S(12)
     NB_S(13) NB_S(14)
 #undef NB_S
     default: return cudaErrorNotSupported;
   }
   if (err != cudaSuccess || !assemble) return err;
-  return gs_add_fused<T>(L.P->gsd, e, true, s, skip);
+  return gs_add_fused<T>(L.P->gsd, e, true, s, skip, nullptr, chain);
 }
 
 // Drop-in form of the FDM (cuda_fdm_do_fast, src/math/bcknd/device/cuda/
@@ -749,12 +749,13 @@ cudaError_t fdm_dropin(double *eo, double *r, const double *s, const double *d, 
 template <typename TIN, typename TOUT, typename T>
 static cudaError_t restrict_level(int ni, int no, const TIN *in, const TIN *scale, const T *J,
                                   TOUT *out, long nelv, const int *skip, cudaStream_t s,
-                                  const float *scale_f = nullptr) {
+                                  const float *scale_f = nullptr, bool chain = true) {
 #define NB_R(A, B)                                                                          \
   if (ni == A && no == B) {                                                                 \
-    launch_chained(4 * nelv * A * A * A, tensor3_kernel<TIN, TOUT, T, A, B, true, false>,   \
-                   (unsigned)nelv, kT3Threads, 0, s,          \
-        in, scale, scale_f, J, out, nelv, skip, PrologDots{}, CoarseAdd<T>{});              \
+    launch_chained(chain ? nelv * A * A * A : kNotChained,                                  \
+                   tensor3_kernel<TIN, TOUT, T, A, B, true, false>, (unsigned)nelv,         \
+                   kT3Threads, 0, s, in, scale, scale_f, J, out, nelv, skip, PrologDots{},  \
+                   CoarseAdd<T>{});                                                         \
     return cudaGetLastError();                                                              \
   }
   NB_R(4, 2) NB_R(3, 2) NB_R(5, 4) NB_R(6, 4) NB_R(7, 4) NB_R(8, 4) NB_R(9, 4) NB_R(10, 4)
@@ -766,20 +767,21 @@ static cudaError_t restrict_level(int ni, int no, const TIN *in, const TIN *scal
 // prolongation out += (J x J x J) in from ni to no points (J: no x ni)
 template <typename TIN, typename TOUT, typename T>
 static cudaError_t prolong_add(int ni, int no, const TIN *in, const T *J, TOUT *out, long nelv,
-                               const int *skip, cudaStream_t s, const CoarseAdd<T> &crs,
+                               const int *skip, cudaStream_t s, bool chain,
+                               const CoarseAdd<T> &crs,
                                const TIN *oscale = nullptr, const float *oscale_f = nullptr,
                                const PrologDots *dots = nullptr) {
   const PrologDots d0 = dots ? *dots : PrologDots{};
 #define NB_P(A, B)                                                                          \
   if (ni == A && no == B) {                                                                 \
     const unsigned g = (unsigned)nelv;                                                      \
+    const long points = chain ? nelv * B * B * B : kNotChained;                             \
     if (dots)                                                                               \
-      launch_chained(4 * nelv * B * B * B, tensor3_kernel<TIN, TOUT, T, A, B, false, true, true>,\
-                     g, kT3Threads, 0, s, in, oscale, oscale_f, J, out, nelv, skip, d0,     \
-                     crs);          \
+      launch_chained(points, tensor3_kernel<TIN, TOUT, T, A, B, false, true, true>, g,      \
+                     kT3Threads, 0, s, in, oscale, oscale_f, J, out, nelv, skip, d0, crs);  \
     else                                                                                    \
-      launch_chained(4 * nelv * B * B * B, tensor3_kernel<TIN, TOUT, T, A, B, false, true>, g,\
-                     kT3Threads, 0, s, in, oscale, oscale_f, J, out, nelv, skip, d0, crs);     \
+      launch_chained(points, tensor3_kernel<TIN, TOUT, T, A, B, false, true>, g, kT3Threads, \
+                     0, s, in, oscale, oscale_f, J, out, nelv, skip, d0, crs);              \
     return cudaGetLastError();                                                              \
   }
   NB_P(2, 4) NB_P(2, 3) NB_P(4, 5) NB_P(4, 6) NB_P(4, 7) NB_P(4, 8) NB_P(4, 9) NB_P(4, 10)
@@ -945,22 +947,24 @@ struct HsmgImpl : public HsmgState {
     // restrict (r * mult) to the middle level, assemble, mask: w; restrict
     // (w * mult_mid) to the vertices (FP64)
     if ((e = restrict_level<double, T, T>(fine->lx, mid->lx, r, fine->mult, Jfm, w_mid, nelv,
-                                          skip, head, fine->multf)) != cudaSuccess ||
-        (e = gs_add_fused<T>(mid->gsd, w_mid, true, head, skip)) != cudaSuccess ||
-        (e = hsmg_coarse_restrict<T>(ca, mid->lx, skip, head)) != cudaSuccess)
+                                          skip, head, fine->multf, !grid)) != cudaSuccess ||
+        (e = gs_add_fused<T>(mid->gsd, w_mid, true, head, skip, nullptr, !grid)) !=
+            cudaSuccess ||
+        (e = hsmg_coarse_restrict<T>(ca, mid->lx, skip, head, !grid)) != cudaSuccess)
       return e;
     // coarse: assemble, mask, niter Jacobi-CG iterations (or abs tol)
     if (!grid && ((e = fork()) != cudaSuccess || (e = hsmg_coarse_cg(cg, skip, s)) != cudaSuccess))
       return e;
     // middle Schwarz: e_mid = S_m w
-    if ((e = schwarz_apply<T, T>(sm, w_mid, e_mid, skip, hi)) != cudaSuccess ||
+    if ((e = schwarz_apply<T, T>(sm, w_mid, e_mid, skip, hi, !grid)) != cudaSuccess ||
         (grid && (e = hsmg_coarse_cg(cg, skip, hi)) != cudaSuccess) ||
         (e = cudaEventRecord(ev_join_hi, hi)) != cudaSuccess)
       return e;
     // fine Schwarz: zs = S_f r (left unassembled when the final
     // gather-scatter takes it, see below)
     const bool merged = merged_assembly();
-    if ((e = schwarz_apply<double, T>(sf, r, zs, skip, side, !merged)) != cudaSuccess) return e;
+    if ((e = schwarz_apply<double, T>(sf, r, zs, skip, side, !grid, !merged)) != cudaSuccess)
+      return e;
     if ((e = cudaEventRecord(ev_join, side)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(s, ev_join, 0)) != cudaSuccess ||
         (e = cudaStreamWaitEvent(s, ev_join_hi, 0)) != cudaSuccess)
@@ -970,13 +974,13 @@ struct HsmgImpl : public HsmgState {
     // mult gs(gs(wt e) + J e_mid) = gs(wt e + mult J e_mid).
     CoarseAdd<T> crs_add;
     if (nodes.nn > 0) crs_add = CoarseAdd<T>{cg.x, nodes.node_of, Jmc};
-    if ((e = prolong_add<T, T, T>(mid->lx, fine->lx, e_mid, Jfm, zs, nelv, skip, s, crs_add,
+    if ((e = prolong_add<T, T, T>(mid->lx, fine->lx, e_mid, Jfm, zs, nelv, skip, s, !grid, crs_add,
                                   merged ? mult_f : nullptr,
                                   merged && sizeof(T) == 8 ? fine->multf : nullptr,
                                   merged ? dots : nullptr)) !=
         cudaSuccess)
       return e;
-    if ((e = gs_add_fused<T>(fine->gsd, zs, merged, s, skip, merged ? nullptr : mult_f)) !=
+    if ((e = gs_add_fused<T>(fine->gsd, zs, merged, s, skip, merged ? nullptr : mult_f, !grid)) !=
         cudaSuccess)
       return e;
     return cudaGetLastError();

@@ -290,7 +290,9 @@ cudaError_t tamg_cycle(const TamgCluster &a, const int *skip, cudaStream_t s) {
   int limit = 0, nblk = 1;
   cudaError_t e = tamg_limit(limit);
   if (e != cudaSuccess) return e;
-  // a block for every 128 vertices, as the hsmg coarse solve
+  // a block for every 128 vertices: with 64, 128, 256 and 512 an application at lx 6
+  // takes 261, 259, 265 and 283 us on 8^3 elements, 275, 273, 284 and 303 on 10^3, 475,
+  // 469, 469 and 489 on 16^3
   while (nblk < limit && nblk * 128 < a.A.nn) nblk *= 2;
   TamgCluster b = a;
   b.skip = skip;
