@@ -567,7 +567,9 @@ def run_velocity(args):
                                              "h1 = 1 + 0.5 sin x sin y sin z, h2 = 10")
                    + ", three components", "iterations": mons[0].iter,
                    "converged": mons[0].converged, "r0": r0},
-        "roofline": {"bound": "hbm", "kernel": f"ax_stress_tma_kernel<{cfg['lx']}> "
+        "roofline": {"bound": "hbm",
+                     "kernel": ("ax_stress_mma_kernel " if cfg["lx"] == 8
+                                else f"ax_stress_tma_kernel<{cfg['lx']}> ")
                      "(nb_ax_stress, three components)", "achieved": gbs,
                      "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": gbs / peaks["hbm_gbs"],
                      "peak_source": src, "bytes_per_launch": nbytes, "launch_ms": t_op * 1e3,

@@ -347,8 +347,8 @@ __global__ void __launch_bounds__(StressCfg<LX, S, KS>::THREADS, StressCfg<LX, S
 //   r flux:       A = the flux, straight from the lane's registers;
 //   s flux:       through the warp's own plane of the stage, warp-synchronous;
 //   t:            plain FMAs down the lane's column, 16-byte loads.
-// About 95 wavefronts a warp of points.  Four warps an element, two planes
-// each.  The matrix instruction runs at the FP64 FMA rate (37 against 33
+// About 95 wavefronts a warp of points (132 measured, with the copies into the
+// stage and 18 of conflicts).  Four warps an element, two planes each.  The matrix instruction runs at the FP64 FMA rate (37 against 33
 // TFLOP/s measured), so it saves the operand traffic, not arithmetic.
 // A fused step on 3 x 2.1 M points: 78 us, 104 with the kernel above.
 // ---------------------------------------------------------------------------

@@ -62,13 +62,14 @@ __device__ __forceinline__ void face_map(unsigned code, int lx, int s1, int s2, 
 // entries M(., l), which are the same for the whole element (broadcast
 // reads), and updates M*NL independent sums, so a matrix read serves M lines.
 //
-// The passes are bound by shared-memory wavefronts.  Line t starts at P t,
-// and for even NL a lane reads its lines two values at a time: with P / 2
+// What bounds the passes is latency, with shared memory the busiest pipe (64 % at
+// nl = 10 in FP64, the FP64 pipe 48 %, 11 warps a multiprocessor).  Line t starts
+// at P t, and for even NL a lane reads its lines two values at a time: with P / 2
 // odd, the eight lanes of a quarter-warp (sixteen of a half-warp in FP32)
 // then hit distinct banks, and where P = NL the rotated writes of
-// consecutive lines are consecutive addresses.  For nl = 10 in FP64 that is
-// 80 + 80 + 50 wavefronts a pass (line reads, writes, matrix rows) against
-// 140 + 84 + 50 with single-value reads of a padded layout.  Odd NL read
+// consecutive lines are consecutive addresses.  An element of nl = 10 in FP64
+// takes 1143 load and 482 store wavefronts so, 19 and 37 of them conflicts, where
+// single-value reads of a padded layout took 1487 and 451 with 382.  Odd NL read
 // single values, conflict-free at their odd pitch.
 //
 // Every pass works in place: the lanes read their lines, the block meets at
