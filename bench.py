@@ -570,7 +570,7 @@ def run_velocity(args):
         "roofline": {"bound": "hbm",
                      "kernel": ("ax_stress_mma_kernel " if cfg["lx"] == 8
                                 else f"ax_stress_tma_kernel<{cfg['lx']}> ")
-                     "(nb_ax_stress, three components)", "achieved": gbs,
+                     + "(nb_ax_stress, three components)", "achieved": gbs,
                      "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": gbs / peaks["hbm_gbs"],
                      "peak_source": src, "bytes_per_launch": nbytes, "launch_ms": t_op * 1e3,
                      "traffic": None},
