@@ -28,6 +28,11 @@ struct AxVecCfg {
   static constexpr int THREADS = ((L2 * KS + 31) / 32) * 32;
   static constexpr size_t ABYTES = (size_t)L3 * sizeof(double);
   static constexpr size_t SMEM = S * NA * ABYTES + 3 * ABYTES + 2 * L2 * sizeof(double) + 16 * S;
+  // As many blocks a multiprocessor as the shared memory has room for; the compiler
+  // may use the registers that this leaves each.  Left to itself it takes 96 at lx 6:
+  // 119 us on 3.0 M points with the bound, 133 without; lx 8 with h2 115 and 132; the
+  // other forms are the same either way.
+  static constexpr int BLOCKS = (int)(233472 / (SMEM + 1024));
 };
 
 struct VecIo {
@@ -36,7 +41,7 @@ struct VecIo {
 };
 
 template <int LX, int S, int KS, bool H2>
-__global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS)
+__global__ void __launch_bounds__(AxVecCfg<LX, S, KS>::THREADS, AxVecCfg<LX, S, KS>::BLOCKS)
     ax_vec_tma_kernel(VecIo io, const double *__restrict__ D, const double *__restrict__ Dt,
                       const double *__restrict__ h1, const double *__restrict__ g11,
                       const double *__restrict__ g22, const double *__restrict__ g33,
