@@ -15,14 +15,14 @@ namespace nb {
 // H2 adds the h2 B u term.  Its product h2 B is loaded with u, so that the loads
 // are in flight during the element; u comes from shared memory again.  Left to
 // itself the compiler gives this form 254 registers, one block a multiprocessor
-// where the other has two; with 128 (lx <= 8) or 168 of them the operator takes
+// where the other has two; with 128 (lx <= 7) or 168 of them the operator takes
 // 82 us on 2.3 M points at lx 12 (154 with 254 registers and u read from global
 // memory, 74 without the term, 88 with the term as a pass of its own), 78 at lx
-// 13 (150, 77, 91), 58 at lx 8 (76, -, 75).  With 128 lx 11 takes 23 us on 209
-// thousand points, 16 with 168.
+// 13 (150, 77, 91), 60 at lx 8 (76, -, 75).  With 128 lx 11 takes 23 us on 209
+// thousand points, 16 with 168; lx 8 10.2 and 8.3 on 369 thousand.
 template <typename T, int LX, int NE, bool H2>
 __global__ void __launch_bounds__(LX *LX *NE,
-                                  H2 ? blocks_for(LX * LX * NE, LX <= 8 ? 128 : 168) : 0)
+                                  H2 ? blocks_for(LX * LX * NE, LX <= 7 ? 128 : 168) : 0)
     ax_helm_kernel(T *__restrict__ w, const T *__restrict__ u,
                    const T *__restrict__ dx, const T *__restrict__ dy,
                    const T *__restrict__ dz, const T *__restrict__ dxt,
