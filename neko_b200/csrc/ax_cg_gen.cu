@@ -9,19 +9,27 @@ namespace nb {
 
 // The fused step for the other orders and for operands that are not 16-byte
 // aligned: NE elements a block with plain coalesced loads, the element loop of
-// ax_helm_kernel.  The new p stays in shared memory after the first pass and the
-// output loop is unrolled by two: unrolled fully with p in registers the kernel
-// takes 254 of them, one block a multiprocessor (lx 12, 2.3 M points: 140 us, 159
-// with h2; as separate passes 93 and 106).  With 168 it holds the columns; where
-// fewer than three blocks fit so, 128 are better up to lx 12 (78 and 84 us there
-// against 91 and 103; lx 11, where three fit, 18 and 23 on 209 thousand points),
-// beyond they spill (lx 14, 2.0 M points: 191 us, 127 with 168).
+// ax_helm_kernel.  In the middle orders the new p stays in shared memory after the
+// first pass and the output loop is unrolled by two: unrolled fully with p in
+// registers the kernel takes 254 of them, one block a multiprocessor (lx 12, 2.3 M
+// points: 119 us, 167 with h2; as separate passes 93 and 106).  With 168 it holds the
+// columns; where fewer than three blocks fit so, 128 are better up to lx 12 (77 and
+// 84 us there against 94 and 107; lx 11, where three fit, 18 and 23 on 209 thousand
+// points), beyond they spill (lx 14, 2.0 M points: 191 us, 127 with 168).  The short
+// columns (lx 3, 4) and the long ones that leave one block a multiprocessor either
+// way (lx 15, 16) keep p in registers: 421 thousand points at lx 3 16.6 -> 13.5 us,
+// 2.5 M at lx 4 49.1 -> 43.3, 2.1 M at lx 16 95.6 -> 97.0, with h2 114.5 -> 98.5.
 template <int LX, int NE>
 struct AxCgGen {
   static constexpr int L2 = LX * LX, L3 = L2 * LX;
   static constexpr int THREADS = ((L2 * NE + 31) / 32) * 32;
+  // p in registers to the end, the output loop unrolled fully
+  static constexpr bool HELD = LX == 3 || LX == 4 || LX >= 15;
+  static constexpr int UNROLL = HELD ? LX : 2;
   static constexpr int BLOCKS =
-      blocks_for(THREADS, LX > 12 || blocks_for(THREADS, 168) >= 3 ? 168 : 128);
+      LX == 3 || LX == 4
+          ? 0
+          : blocks_for(THREADS, LX > 12 || blocks_for(THREADS, 168) >= 3 ? 168 : 128);
   static constexpr size_t SMEM = sizeof(double) * (2 * L2 + (size_t)NE * 3 * L3);
 };
 
@@ -83,7 +91,7 @@ __global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS, AxCgGen<LX, NE>::BLO
     }
     __syncthreads();
     if (active) {
-#pragma unroll 2
+#pragma unroll(C::UNROLL)
       for (int k = 0; k < LX; k++) {
         double c0 = 0, c1 = 0, c2 = 0;
 #pragma unroll
@@ -93,7 +101,11 @@ __global__ void __launch_bounds__(AxCgGen<LX, NE>::THREADS, AxCgGen<LX, NE>::BLO
           c2 += sDt[k + LX * l] * rut[l];
         }
         const long g = base + k * L2;
-        const double pk = su[col + L2 * k];
+        double pk;
+        if constexpr (C::HELD)
+          pk = rp[k];
+        else
+          pk = su[col + L2 * k];
         double wv = c0 + c1 + c2;
         if constexpr (H2) wv = wv + __ldg(a.h2 + g) * __ldg(a.B + g) * pk;
         a.w[g] = wv;
